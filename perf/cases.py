@@ -14,7 +14,7 @@ from forkmatch_gb300 import synth as S
 
 MB, GB = 1 << 20, 1 << 30
 WALK_PARTIALS = 1 << 23       # partial matches and embeddings that a walk query of these cases may have
-WALK_ROWS = 1 << 19
+WALK_ROWS = 1 << 17
 CYCLE_ROWS = 1 << 22
 HOST_ROWS = 1 << 14
 
@@ -306,6 +306,7 @@ def prepare(case, seed):
         st["stream"] = torch.cuda.Stream()
         cap = WALK_ROWS if case["shape"] == "walk" else CYCLE_ROWS
         st["tables"] = [torch.zeros(cap, q.q, dtype=torch.int32, device="cuda") for q in queries]
+        st["mix"] = torch.tensor([pow(0x5851F42D4C957F2D, i + 1, 1 << 63) for i in range(16)], device="cuda")
     elif task == "batch":
         st["batch"] = fm.Batch(ctx, graph, queries, mode=fm.MODE_COUNT)
     elif task == "serve":
@@ -318,12 +319,10 @@ class _DeviceRows:
         self.__cuda_array_interface__ = {"shape": (n, q), "typestr": "<i4", "data": (ptr, False), "version": 3}
 
 
-def _row_set(rows):
-    """The rows in an order that depends on their values alone."""
-    key = rows[:, 0].long()
-    for c in range(1, rows.shape[1]):
-        key = key * 0x5851F42D4C957F2D + rows[:, c]
-    return rows[torch.argsort(key)]
+def _row_set(r, mix, out):
+    """The rows of a device table, put into `out` in an order that depends on their values alone."""
+    rows = torch.as_tensor(_DeviceRows(r.rows_device, r.rows, r.q), device="cuda")
+    torch.index_select(rows, 0, torch.argsort((rows * mix).sum(1)), out=out[:r.rows])
 
 
 def run(state):
@@ -344,7 +343,7 @@ def run(state):
             for q, table in zip(state["queries"], state["tables"]):
                 r = fm.match(ctx, state["graph"], q, stream=state["stream"].cuda_stream)
                 if r.rows:
-                    table[:r.rows] = _row_set(torch.as_tensor(_DeviceRows(r.rows_device, r.rows, r.q), device="cuda"))
+                    _row_set(r, state["mix"][:r.q], table)
                 out += [r.count, table]
         return out
     if task == "batch":
