@@ -233,10 +233,8 @@ void* fm_context_stream(fm_context* ctx) { return ctx ? (void*)ctx->stream : nul
 // ------------------------------------------------------------------ graphs
 
 static void free_device_graph(DeviceGraph& g) {
-    if (g.seg) cudaFree(g.seg);
-    if (g.nbr) cudaFree(g.nbr);
-    if (g.heads) cudaFree(g.heads);
-    if (g.bitmaps) cudaFree(g.bitmaps);
+    if (g.block) cudaFree(g.block);
+    g.block = nullptr;
     g.bitmaps = nullptr;
     g.seg = nullptr;
     g.nbr = nullptr;
@@ -253,28 +251,13 @@ void fm_graph_free(fm_graph* g) {
 static fm_status graph_from_host_arrays(fm_context* ctx, uint32_t V, uint32_t L, uint64_t E, const uint32_t* src,
                                         const uint32_t* dst, const uint32_t* lab, fm_graph** out) {
     FM_CUDA(cudaSetDevice(ctx->device));
-    uint32_t* d = nullptr;
-    if (E) {
-        cudaError_t e = cudaMalloc(&d, E * 12);
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            set_error("cannot allocate edge staging buffers");
-            return FM_ERR_NOMEM;
-        }
-        FM_CUDA(cudaMemcpyAsync(d, src, E * 4, cudaMemcpyHostToDevice, ctx->stream));
-        FM_CUDA(cudaMemcpyAsync(d + E, dst, E * 4, cudaMemcpyHostToDevice, ctx->stream));
-        FM_CUDA(cudaMemcpyAsync(d + 2 * E, lab, E * 4, cudaMemcpyHostToDevice, ctx->stream));
-    }
     std::unique_ptr<fm_graph> g(new fm_graph());
-    fm_status st = build_device_graph(g->g, V, L, E, d, d + E, d + 2 * E, ctx->stream);
-    cudaStreamSynchronize(ctx->stream);
-    if (d) cudaFree(d);
+    const fm_status st = build_from_edges(g->g, V, L, E, src, dst, lab, ctx->stream);
     if (st != FM_OK) {
+        cudaStreamSynchronize(ctx->stream);
         free_device_graph(g->g);
         return st;
     }
-    g->g.label_count.assign(L, 0);   // label frequencies for the matching-order cost model
-    for (uint64_t i = 0; i < E; i++) g->g.label_count[lab[i]]++;
     *out = g.release();
     return FM_OK;
 }
@@ -297,6 +280,7 @@ fm_status fm_graph_load_text(fm_context* ctx, const char* text, uint64_t len, fm
     std::unique_ptr<fm_graph> g(new fm_graph());
     fm_status st = parse_data_text_device(text, len, ctx->stream, g->g);
     if (st != FM_OK) {
+        cudaStreamSynchronize(ctx->stream);
         free_device_graph(g->g);
         return st;
     }

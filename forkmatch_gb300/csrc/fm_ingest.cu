@@ -12,15 +12,16 @@
 //      numbers the newlines, and every line start is written in file order;
 //   4. k_parse_lines: one thread per line parses "v id label" or
 //      "e src dst label" with the same grammar and range checks as the host
-//      parser (fm_parse.cpp) and records the first bad line;
-//   5. the kept e-lines (label < label slots) are compacted with CUB and go
-//      straight to the device graph build, without a round trip to the host.
+//      parser (fm_parse.cpp), records the first bad line, counts labels and
+//      appends the kept e-lines (label < label slots) as sort keys;
+//   5. the keys go straight to the device graph build, without a round trip
+//      to the host.  The build sorts them, so the order in which blocks
+//      append does not matter and no stable compaction is needed.
 #include <cub/cub.cuh>
 
 #include <algorithm>
 #include <cstring>
 #include <string>
-#include <vector>
 
 #include "fm_internal.h"
 
@@ -60,8 +61,10 @@ __global__ void k_count_lines(const unsigned char* __restrict__ body, uint64_t n
 }
 
 // Start offset of every line: line 0 starts at 0, line i+1 after newline i.
+// Starts past `cap` are not kept (see parse_data_text_device).
 __global__ void k_line_starts(const unsigned char* __restrict__ body, uint64_t n,
-                              const unsigned long long* __restrict__ block_base, uint64_t* __restrict__ starts) {
+                              const unsigned long long* __restrict__ block_base, uint64_t cap,
+                              uint64_t* __restrict__ starts) {
     typedef cub::BlockScan<uint32_t, kIngestBlock> Scan;
     __shared__ typename Scan::TempStorage tmp;
     const uint64_t pos = blockIdx.x * kBytesPerBlock + 16ull * threadIdx.x;
@@ -73,7 +76,7 @@ __global__ void k_line_starts(const unsigned char* __restrict__ body, uint64_t n
     while (mask) {
         const int b = __ffs(mask) - 1;
         mask &= mask - 1;
-        starts[line + 1] = pos + b + 1;
+        if (line < cap) starts[line + 1] = pos + b + 1;
         line++;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) starts[0] = 0;
@@ -92,51 +95,63 @@ __device__ __forceinline__ bool dparse_u32(const unsigned char* b, uint64_t& p, 
     return true;
 }
 
-// One thread per line (lines [0, nlines), each ending with '\n').  An e-line
-// that is kept writes its three values at its line index; flags[i] = 1 then.
+// One thread per line (lines [0, min(lines, cap)), each ending with '\n').  A
+// block appends its kept e-lines as sort keys with one atomic per 256 lines.
 __global__ void k_parse_lines(const unsigned char* __restrict__ body, const uint64_t* __restrict__ starts,
-                              uint64_t nlines, uint32_t V, uint32_t EL, uint32_t L, uint32_t* __restrict__ src,
-                              uint32_t* __restrict__ dst, uint32_t* __restrict__ lab, uint8_t* __restrict__ keep,
-                              unsigned long long* __restrict__ first_bad) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < nlines;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        uint64_t p = starts[i];
-        const uint64_t end = starts[i + 1];   // one past this line's '\n'
-        bool ok = end >= p + 2;
-        uint8_t k = 0;
-        uint32_t v[3] = {0, 0, 0};
-        if (ok) {
-            const unsigned char kind = body[p];
-            ok = (kind == 'v' || kind == 'e') && body[p + 1] == ' ';
-            const int nv = kind == 'e' ? 3 : 2;
-            p += 2;
-            for (int f = 0; f < nv && ok; f++) {
-                ok = dparse_u32(body, p, end, v[f]) && p < end && body[p] == ((f == nv - 1) ? '\n' : ' ');
-                ++p;
-            }
-            if (ok) {
-                if (kind == 'v') ok = v[0] < V;
-                else ok = v[0] < V && v[1] < V && v[2] <= EL;
-            }
-            if (ok && kind == 'e' && v[2] < L) k = 1;
-        }
-        if (!ok) atomicMin(first_bad, (unsigned long long)i);
-        keep[i] = k;
-        src[i] = v[0];
-        dst[i] = v[1];
-        lab[i] = v[2];
-    }
-}
-
-__global__ void k_label_hist(const uint32_t* __restrict__ lab, uint64_t n, unsigned long long* __restrict__ hist) {
+                              uint64_t cap, uint32_t V, uint32_t EL, uint32_t L, uint32_t vbits,
+                              uint64_t* __restrict__ keys, BuildStats* __restrict__ st) {
     __shared__ unsigned int h[FM_MAX_LABEL + 1];
+    __shared__ uint32_t n_s[kIngestBlock / 32];
+    __shared__ unsigned long long base_s;
     for (uint32_t i = threadIdx.x; i <= FM_MAX_LABEL; i += blockDim.x) h[i] = 0;
-    __syncthreads();
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        atomicAdd(&h[lab[i] & FM_MAX_LABEL], 1u);
+    const uint64_t nlines = st->lines < cap ? st->lines : cap;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x; i0 < nlines; i0 += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t i = i0 + threadIdx.x;
+        bool keep = false;
+        uint32_t v[3] = {0, 0, 0};
+        if (i < nlines) {
+            uint64_t p = starts[i];
+            const uint64_t end = starts[i + 1];   // one past this line's '\n'
+            bool ok = end >= p + 2;
+            if (ok) {
+                const unsigned char kind = body[p];
+                ok = (kind == 'v' || kind == 'e') && body[p + 1] == ' ';
+                const int nv = kind == 'e' ? 3 : 2;
+                p += 2;
+                for (int f = 0; f < nv && ok; f++) {
+                    ok = dparse_u32(body, p, end, v[f]) && p < end && body[p] == ((f == nv - 1) ? '\n' : ' ');
+                    ++p;
+                }
+                if (ok) {
+                    if (kind == 'v') ok = v[0] < V;
+                    else ok = v[0] < V && v[1] < V && v[2] <= EL;
+                }
+                keep = ok && kind == 'e' && v[2] < L;
+            }
+            if (!ok) atomicMin(&st->first_bad, (unsigned long long)i);
+        }
+        const unsigned b = __ballot_sync(0xffffffffu, keep);
+        if (lane == 0) n_s[warp] = __popc(b);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            uint32_t n = 0;
+            for (int w = 0; w < kIngestBlock / 32; w++) n += n_s[w];
+            base_s = n ? atomicAdd(&st->kept, (unsigned long long)n) : 0ull;
+        }
+        __syncthreads();
+        if (keep) {
+            uint64_t at = base_s + __popc(b & ((1u << lane) - 1u));
+            for (uint32_t w = 0; w < warp; w++) at += n_s[w];
+            keys[at] = ((uint64_t)v[2] << (2 * vbits)) | ((uint64_t)v[0] << vbits) | (uint64_t)v[1];
+            atomicAdd(&h[v[2]], 1u);
+            if (v[0] == v[1]) atomicOr(&st->loops, 1u);
+        }
+        __syncthreads();                          // n_s and base_s are written again
+    }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i <= FM_MAX_LABEL; i += blockDim.x)
-        if (h[i]) atomicAdd(hist + i, (unsigned long long)h[i]);
+        if (h[i]) atomicAdd(&st->label_count[i], (unsigned long long)h[i]);
 }
 
 struct DBuf {
@@ -219,117 +234,78 @@ fm_status parse_data_text_device(const char* text, uint64_t len, cudaStream_t s,
     int dev = 0, sms = 1;
     FM_CUDA(cudaGetDevice(&dev));
     FM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    // body on the device (16-byte aligned, padded to whole 16-byte words)
-    DBuf d_body;
-    FM_TRY(dev_alloc(d_body, (blen + 31) & ~15ull));
-    if (blen) FM_CUDA(cudaMemcpyAsync(d_body.p, body, blen, cudaMemcpyHostToDevice, s));
     const uint64_t nblocks = std::max<uint64_t>(1, (blen + kBytesPerBlock - 1) / kBytesPerBlock);
     if (nblocks > 0x7fffffffull) {
         set_error("data graph text too large");
         return FM_ERR_UNSUPPORTED;
     }
-    DBuf d_cnt, d_base;
-    FM_TRY(dev_alloc(d_cnt, nblocks * 8));
-    FM_TRY(dev_alloc(d_base, nblocks * 8));
-    const unsigned char* b = d_body.as<unsigned char>();
-    k_count_lines<<<(unsigned)nblocks, kIngestBlock, 0, s>>>(b, blen, d_cnt.as<unsigned long long>());
-    FM_CUDA(cudaGetLastError());
-    size_t tb = 0;
-    FM_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, d_cnt.as<unsigned long long>(), d_base.as<unsigned long long>(),
-                                          (int64_t)nblocks, s));
-    DBuf d_tmp;
-    FM_TRY(dev_alloc(d_tmp, tb));
-    FM_CUDA(cub::DeviceScan::ExclusiveSum(d_tmp.p, tb, d_cnt.as<unsigned long long>(), d_base.as<unsigned long long>(),
-                                          (int64_t)nblocks, s));
-    unsigned long long last_base = 0, last_cnt = 0;
-    FM_CUDA(cudaMemcpyAsync(&last_base, d_base.as<unsigned long long>() + (nblocks - 1), 8, cudaMemcpyDeviceToHost, s));
-    FM_CUDA(cudaMemcpyAsync(&last_cnt, d_cnt.as<unsigned long long>() + (nblocks - 1), 8, cudaMemcpyDeviceToHost, s));
-    FM_CUDA(cudaStreamSynchronize(s));
-    const uint64_t nlines = last_base + last_cnt;   // every line ends with '\n'
-    DBuf d_starts;
-    FM_TRY(dev_alloc(d_starts, (nlines + 1) * 8));
-    k_line_starts<<<(unsigned)nblocks, kIngestBlock, 0, s>>>(b, blen, d_base.as<unsigned long long>(),
-                                                             d_starts.as<uint64_t>());
-    FM_CUDA(cudaGetLastError());
-
-    DBuf d_vals, d_keep, d_bad;
-    FM_TRY(dev_alloc(d_vals, std::max<uint64_t>(1, nlines) * 12));
-    FM_TRY(dev_alloc(d_keep, std::max<uint64_t>(1, nlines)));
-    FM_TRY(dev_alloc(d_bad, 8));
-    FM_CUDA(cudaMemsetAsync(d_bad.p, 0xff, 8, s));
-    uint32_t* vsrc = d_vals.as<uint32_t>();
-    uint32_t* vdst = vsrc + nlines;
-    uint32_t* vlab = vdst + nlines;
-    if (nlines) {
-        const unsigned grid = (unsigned)std::min<uint64_t>((nlines + 255) / 256, (uint64_t)sms * 32);
-        k_parse_lines<<<grid, 256, 0, s>>>(b, d_starts.as<uint64_t>(), nlines, V, EL, L, vsrc, vdst, vlab,
-                                            d_keep.as<uint8_t>(), d_bad.as<unsigned long long>());
-        FM_CUDA(cudaGetLastError());
+    // a header that no graph can have is reported after the lines are checked
+    uint32_t vbits = 0, lbits = 0;
+    if (graph_key_layout(V, L, 0, vbits, lbits) != FM_OK) vbits = lbits = 16;
+    const uint32_t key_bits = 2 * vbits + lbits;
+    // body (16-byte aligned, padded to whole 16-byte words) and newline counts
+    const uint64_t body_bytes = (blen + 31 + 255) & ~255ull, text_bytes = body_bytes + nblocks * 8;
+    // A valid line takes at least 6 bytes, so the text bounds the number of
+    // lines (a text with more lines has its first bad line among those).
+    // Texts up to 64 MiB use that bound for the build's arrays (33 bytes per
+    // possible line) and put body and arrays in one allocation; larger ones,
+    // where the bound would cost gigabytes, count the lines first.
+    const bool bound = blen <= (64ull << 20);
+    BuildArena arena;
+    DBuf d_text;
+    uint64_t cap = blen / 6 + 1;
+    char* text_mem = nullptr;
+    if (bound) {
+        FM_TRY(arena.alloc(cap + 1, key_bits, text_bytes));
+        text_mem = arena.extra;
+    } else {
+        FM_TRY(dev_alloc(d_text, text_bytes + 8));
+        text_mem = d_text.as<char>();
     }
-    unsigned long long bad = ~0ull;
-    FM_CUDA(cudaMemcpyAsync(&bad, d_bad.p, 8, cudaMemcpyDeviceToHost, s));
+    unsigned char* b = (unsigned char*)text_mem;
+    unsigned long long* counts = (unsigned long long*)(text_mem + body_bytes);
+    if (blen) FM_CUDA(cudaMemcpyAsync(b, body, blen, cudaMemcpyHostToDevice, s));
+    k_count_lines<<<(unsigned)nblocks, kIngestBlock, 0, s>>>(b, blen, counts);
+    FM_CUDA(cudaGetLastError());
+    unsigned long long* lines = nullptr;
+    if (!bound) {
+        // counts[nblocks] takes the number of lines (every line ends with '\n')
+        lines = counts + nblocks;
+        FM_CUDA(scan_tiles_u64(counts, nblocks, lines, s));
+        unsigned long long n = 0;
+        FM_CUDA(cudaMemcpyAsync(&n, lines, 8, cudaMemcpyDeviceToHost, s));
+        FM_CUDA(cudaStreamSynchronize(s));
+        cap = n;
+        FM_TRY(arena.alloc(cap + 1, key_bits, 0));
+    }
+    FM_CUDA(cudaMemsetAsync(arena.stats, 0, sizeof(BuildStats), s));
+    FM_CUDA(cudaMemsetAsync(&arena.stats->first_bad, 0xff, 8, s));
+    if (bound) FM_CUDA(scan_tiles_u64(counts, nblocks, &arena.stats->lines, s));
+    else FM_CUDA(cudaMemcpyAsync(&arena.stats->lines, lines, 8, cudaMemcpyDeviceToDevice, s));
+    uint64_t* starts = arena.alt;
+    k_line_starts<<<(unsigned)nblocks, kIngestBlock, 0, s>>>(b, blen, counts, cap, starts);
+    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((cap + 255) / 256, (uint64_t)sms * 8));
+    k_parse_lines<<<grid, kIngestBlock, 0, s>>>(b, starts, cap, V, EL, L, vbits, arena.keys, arena.stats);
+    FM_CUDA(cudaGetLastError());
+    BuildStats st;
+    FM_CUDA(cudaMemcpyAsync(&st, arena.stats, sizeof(st), cudaMemcpyDeviceToHost, s));
     FM_CUDA(cudaStreamSynchronize(s));
-    if (bad != ~0ull) {
+    if (st.first_bad != ~0ull) {
         uint64_t at = 0;
-        FM_CUDA(cudaMemcpy(&at, d_starts.as<uint64_t>() + bad, 8, cudaMemcpyDeviceToHost));
+        FM_CUDA(cudaMemcpy(&at, starts + st.first_bad, 8, cudaMemcpyDeviceToHost));
         const char* line = body + at;
         const char* nl = (const char*)std::memchr(line, '\n', (size_t)(end - line));
         std::string txt(line, nl ? (size_t)(nl - line) : std::min<size_t>(40, (size_t)(end - line)));
         set_error("malformed or out-of-range data line: \"" + txt.substr(0, 80) + "\"");
         return FM_ERR_DATA_LINE;
     }
-    d_starts.reset();
-    d_body.reset();
-
-    // compact the kept e-lines (three flagged selections share the flags)
-    DBuf d_edges, d_nsel;
-    FM_TRY(dev_alloc(d_edges, std::max<uint64_t>(1, nlines) * 12));
-    FM_TRY(dev_alloc(d_nsel, 8));
-    uint32_t* esrc = d_edges.as<uint32_t>();
-    uint32_t* edst = esrc + nlines;
-    uint32_t* elab = edst + nlines;
-    uint64_t E = 0;
-    if (nlines) {
-        size_t tb2 = 0;
-        FM_CUDA(cub::DeviceSelect::Flagged(nullptr, tb2, vsrc, d_keep.as<uint8_t>(), esrc,
-                                           d_nsel.as<unsigned long long>(), (int64_t)nlines, s));
-        DBuf d_tmp2;
-        FM_TRY(dev_alloc(d_tmp2, tb2));
-        FM_CUDA(cub::DeviceSelect::Flagged(d_tmp2.p, tb2, vsrc, d_keep.as<uint8_t>(), esrc,
-                                           d_nsel.as<unsigned long long>(), (int64_t)nlines, s));
-        FM_CUDA(cub::DeviceSelect::Flagged(d_tmp2.p, tb2, vdst, d_keep.as<uint8_t>(), edst,
-                                           d_nsel.as<unsigned long long>(), (int64_t)nlines, s));
-        FM_CUDA(cub::DeviceSelect::Flagged(d_tmp2.p, tb2, vlab, d_keep.as<uint8_t>(), elab,
-                                           d_nsel.as<unsigned long long>(), (int64_t)nlines, s));
-        unsigned long long ne = 0;
-        FM_CUDA(cudaMemcpyAsync(&ne, d_nsel.p, 8, cudaMemcpyDeviceToHost, s));
-        FM_CUDA(cudaStreamSynchronize(s));
-        E = ne;
-    }
+    const uint64_t E = st.kept;
     if (E > Ehdr) {
         set_error("more e-lines than the header's edge count");
         return FM_ERR_DATA_LINE;
     }
-    d_vals.reset();
-    d_keep.reset();
-    // label frequencies for the matching-order cost model
-    DBuf d_hist;
-    FM_TRY(dev_alloc(d_hist, (FM_MAX_LABEL + 1) * 8));
-    FM_CUDA(cudaMemsetAsync(d_hist.p, 0, (FM_MAX_LABEL + 1) * 8, s));
-    if (E) {
-        k_label_hist<<<(unsigned)std::min<uint64_t>((E + 255) / 256, (uint64_t)sms * 8), 256, 0, s>>>(
-            elab, E, d_hist.as<unsigned long long>());
-        FM_CUDA(cudaGetLastError());
-    }
-    std::vector<unsigned long long> hist(FM_MAX_LABEL + 1);
-    FM_CUDA(cudaMemcpyAsync(hist.data(), d_hist.p, hist.size() * 8, cudaMemcpyDeviceToHost, s));
-    FM_CUDA(cudaStreamSynchronize(s));
-    fm_status st = build_device_graph(g, V, L, E, esrc, edst, elab, s);
-    cudaStreamSynchronize(s);
-    if (st != FM_OK) return st;
-    g.label_count.assign(L, 0);
-    for (uint32_t l = 0; l < L; l++) g.label_count[l] = hist[l];
-    return FM_OK;
+    if (!bound) d_text.reset();
+    return build_from_keys(g, V, L, E, arena, s);
 }
 
 }  // namespace fm

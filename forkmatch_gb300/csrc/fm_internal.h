@@ -41,6 +41,7 @@ struct DeviceGraph {
     uint32_t L = 0;            // label slots
     uint32_t vbits = 0;        // bits per vertex id in the sort key
     uint64_t E = 0;
+    void* block = nullptr;     // the device allocation that holds every array below
     uint4* seg = nullptr;      // L*V records, index label*V + v
     uint32_t* nbr = nullptr;   // out-of-line lists
     // Source vertex of every non-empty segment, label-major: the vertices with
@@ -325,9 +326,53 @@ fm_status batch_create_scratch(fm_context* ctx, const fm_graph* graph, const fm_
 // (independent e-lines, label frequencies): the server's footprint model.
 void estimate_level_rows(const Plan& P, const DeviceGraph& g, double est[kMaxQ]);
 
-// Device graph build from device edge arrays (fm_graph.cu).
-fm_status build_device_graph(DeviceGraph& g, uint32_t V, uint32_t L, uint64_t E, const uint32_t* d_src,
-                             const uint32_t* d_dst, const uint32_t* d_lab, cudaStream_t s);
+// Device graph build (fm_graph.cu).
+// What the build finds out on the device, read back once.
+struct BuildStats {
+    unsigned int error;               // an e-line was out of range
+    unsigned int dup, loops;          // a repeated e-line, an e-line v -> v
+    unsigned int nseg, total16;       // segments; 16-byte units of out-of-line lists
+    unsigned int max_len;             // longest list
+    unsigned int bm_count;            // bitmap indices given out
+    unsigned int hist[32];            // lists by floor(log2(length))
+    unsigned long long kept;          // text: e-lines kept
+    unsigned long long first_bad;     // text: first malformed line
+    unsigned long long lines;         // text: lines
+    unsigned long long label_count[FM_MAX_LABEL + 1];
+    unsigned long long first[FM_MAX_LABEL + 1];   // first segment of a label; all ones: none
+};
+
+// Every temporary of one build, in one device allocation sized for `cap` keys
+// of `key_bits` bits (plus `extra` bytes for the caller).
+struct BuildArena {
+    void* mem = nullptr;
+    BuildStats* stats = nullptr;
+    uint64_t* keys = nullptr;         // cap e-line keys, to be sorted
+    uint64_t* alt = nullptr;          // cap: the sort's other buffer; free before it
+    uint32_t* seg_start = nullptr;    // cap + 1; free before the sort is done
+    uint32_t* off16 = nullptr;        // cap
+    uint32_t* tile_keys = nullptr;
+    uint32_t* tile_segs = nullptr;
+    void* temp = nullptr;
+    size_t temp_bytes = 0;
+    char* extra = nullptr;
+    BuildArena() = default;
+    BuildArena(const BuildArena&) = delete;
+    BuildArena& operator=(const BuildArena&) = delete;
+    ~BuildArena();
+    fm_status alloc(uint64_t cap, uint32_t key_bits, uint64_t extra);
+};
+// Bits of a vertex id and of a label in a key, and the limits of a graph.
+fm_status graph_key_layout(uint32_t V, uint32_t L, uint64_t E, uint32_t& vbits, uint32_t& lbits);
+// Host edge arrays -> device graph.
+fm_status build_from_edges(DeviceGraph& g, uint32_t V, uint32_t L, uint64_t E, const uint32_t* src,
+                           const uint32_t* dst, const uint32_t* lab, cudaStream_t s);
+// E unsorted keys (label << 2 vbits | src << vbits | dst) in a.keys, label
+// frequencies and flags in a.stats -> device graph.  The stream is idle when
+// it returns FM_OK.
+fm_status build_from_keys(DeviceGraph& g, uint32_t V, uint32_t L, uint64_t E, BuildArena& a, cudaStream_t s);
+// Exclusive prefix sum in place, total to *total (device pointers).
+cudaError_t scan_tiles_u64(unsigned long long* v, uint64_t n, unsigned long long* total, cudaStream_t s);
 
 // Host parsers (fm_parse.cpp).
 struct EdgeArrays {
