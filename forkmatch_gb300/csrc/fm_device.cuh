@@ -110,6 +110,56 @@ __device__ __forceinline__ uint32_t count_members(const uint4& s, const uint32_t
     return found;
 }
 
+// Which of the row's vertices (column-major rows_s[c*32 + j], c < n_row, c !=
+// skip) are in the list of record s: bit c.  Graphs without duplicate e-lines
+// only.  Same three kinds of lists as count_members.
+__device__ __forceinline__ uint32_t member_mask(const uint4& s, const uint32_t* rows_s, uint32_t j, uint32_t n_row,
+                                                uint32_t skip, const uint32_t* __restrict__ nbr,
+                                                const uint32_t* __restrict__ bm, uint32_t bm_words) {
+    uint32_t mask = 0;
+    if (s.x == 0) return 0;
+    if (s.x <= 3) {
+        for (uint32_t i = 0; i < n_row; i++) {
+            const uint32_t v = rows_s[i * 32 + j];
+            if (i != skip && (s.y == v || s.z == v || s.w == v)) mask |= 1u << i;
+        }
+        return mask;
+    }
+    if (s.z & kBitmapMark) {
+        const uint32_t* b = bm + (uint64_t)(s.z & ~kBitmapMark) * bm_words;
+        for (uint32_t i = 0; i < n_row; i++) {
+            const uint32_t v = rows_s[i * 32 + j];
+            if (i != skip && v <= s.w && ((__ldg(b + (v >> 5)) >> (v & 31)) & 1u)) mask |= 1u << i;
+        }
+        return mask;
+    }
+    const uint32_t* a = nbr + (uint64_t)s.y * 4;
+    for (uint32_t g = 0; g < n_row; g += 4) {
+        uint32_t key[4], base[4];
+        bool act[4];
+#pragma unroll
+        for (uint32_t u = 0; u < 4; u++) {
+            const uint32_t i = g + u;
+            key[u] = i < n_row ? rows_s[i * 32 + j] : 0u;
+            act[u] = i < n_row && i != skip && key[u] >= s.z && key[u] <= s.w;
+            base[u] = 0;
+        }
+        if (!(act[0] || act[1] || act[2] || act[3])) continue;
+        uint32_t len = s.x;
+        while (len > 1) {
+            const uint32_t half = len >> 1;
+#pragma unroll
+            for (uint32_t u = 0; u < 4; u++)
+                if (act[u] && __ldg(a + base[u] + half) <= key[u]) base[u] += half;
+            len -= half;
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < 4; u++)
+            if (act[u] && __ldg(a + base[u]) == key[u]) mask |= 1u << (g + u);
+    }
+    return mask;
+}
+
 // ------------------------------------------------- staged membership lists
 //
 // A list tested for membership by many candidates of a chunk is copied once

@@ -18,11 +18,12 @@
 // (BuildArena) and every resident array from another: on this machine a pair
 // of cudaMalloc and cudaFree costs 0.2-0.5 ms, more than most of the kernels.
 #include <algorithm>
+#include <cstddef>
 #include <cstdlib>
 
 #include <cub/cub.cuh>
 
-#include "fm_internal.h"
+#include "fm_device.cuh"
 
 namespace fm {
 namespace {
@@ -321,6 +322,32 @@ __global__ void k_place(const uint64_t* __restrict__ keys, uint64_t E, uint32_t 
     }
 }
 
+// Does every e-line have its reverse?  Without duplicates it is enough that
+// every e-line with src < dst has one and that there are as many with
+// src > dst: half of the lookups.  Bound by the scattered record loads.
+__global__ void k_symmetry(const uint64_t* __restrict__ keys, uint64_t E, uint32_t V, uint32_t vbits,
+                           const uint4* __restrict__ seg, const uint32_t* __restrict__ nbr,
+                           const uint32_t* __restrict__ bm, uint32_t bm_words, BuildStats* __restrict__ st) {
+    const uint64_t vmask = (1ull << vbits) - 1;
+    uint32_t up = 0, down = 0;
+    bool bad = false;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < E; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t k = keys[i];
+        const uint32_t d = (uint32_t)(k & vmask), s = (uint32_t)((k >> vbits) & vmask);
+        down += s > d;
+        if (s >= d) continue;
+        up += 1;
+        bad |= !dev::seg_has(dev::ldg4(seg + (k >> (2 * vbits)) * V + d), s, 1, nbr, bm, bm_words);
+    }
+    up = __reduce_add_sync(0xffffffffu, up);
+    down = __reduce_add_sync(0xffffffffu, down);
+    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) st->asym = 1u;
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&st->up, up);
+        atomicAdd(&st->down, down);
+    }
+}
+
 // One block per bitmap: set the bit of every entry.
 __global__ void k_bm_fill(const uint32_t* __restrict__ nbr, const uint2* __restrict__ bm_list, uint32_t n_bm,
                           uint32_t bm_words, uint32_t* __restrict__ bitmaps) {
@@ -567,10 +594,15 @@ fm_status build_from_keys(DeviceGraph& g, uint32_t V, uint32_t L, uint64_t E, Bu
             g.bm_words = words;
             g.bm_min_len = thresh;
         }
+        if (!h.dup)
+            k_symmetry<<<grid_for(E, sms), 256, 0, s>>>(sorted, E, V, vbits, g.seg, g.nbr, g.bitmaps, g.bm_words,
+                                                        a.stats);
         FM_CUDA(cudaGetLastError());
+        FM_CUDA(cudaMemcpyAsync(&h, a.stats, offsetof(BuildStats, hist), cudaMemcpyDeviceToHost, s));
     }
     FM_CUDA(cudaEventRecord(ev.b, s));
     FM_CUDA(cudaStreamSynchronize(s));
+    g.symmetric = !h.dup && !h.asym && h.up == h.down;
     float ms = 0;
     cudaEventElapsedTime(&ms, ev.a, ev.b);
     g.build_ms = ms;

@@ -472,6 +472,22 @@ struct MatchRun {
     // survivors' extensions (ExpandParams::pre_count) and depth q-1 is never
     // launched
     bool pre = false;
+    // pre-count by sums: the counting level's plan, and whether the vertex
+    // sums have been computed in this match
+    bool sums = false, sums_ready = false;
+    uint32_t sum_label = 0, sum_last = 0;
+    uint2* vsum = nullptr;                  // null: the rule needs none
+
+    size_t level_smem(uint32_t d) const {
+        const uint32_t k = sums && d == last_depth() ? 2u : nreq_depth[d];
+        return expand_smem_bytes(d, k, block / 32, nreq_depth[d] >= 2 ? base.stage_words : 0);
+    }
+    cudaError_t vertex_sums(const ExpandParams& p, const unsigned long long* parents) {
+        if (!vsum) return cudaSuccess;
+        const uint64_t h = g->head_off[sum_label];
+        return launch_vertex_sums(p, g->heads + h, (uint32_t)(g->head_off[sum_label + 1] - h), sum_label, sum_last, vsum,
+                                  parents, s);
+    }
 
     uint32_t last_depth() const { return plan->q - 1 - (pre ? 1u : 0u); }
 
@@ -540,8 +556,7 @@ struct MatchRun {
         for (uint32_t d = 1; d <= last; d++) {
             const int mode = mode_of(d);
             const bool roots = d == 1;
-            const size_t smem = expand_smem_bytes(d, nreq_depth[d], block / 32,
-                                                  nreq_depth[d] >= 2 ? base.stage_words : 0);
+            const size_t smem = level_smem(d);
             const int per_sm = expand_blocks_per_sm(mode, roots, dups, smem, block);
             const int full = ctx->sms * per_sm;
             ExpandParams p = base;
@@ -566,6 +581,10 @@ struct MatchRun {
             }
             FM_CUDA(cudaMemsetAsync(ctx->ctl + d, 0, sizeof(LaunchCtl), s));
             if (profile) FM_TRY(begin_timing(ev[d][0], ev[d][1]));
+            if (sums && d == last) {
+                p.sum_rule = 1;
+                FM_CUDA(vertex_sums(p, p.n_parents_dev));
+            }
             FM_CUDA(launch_expand(p, mode, roots, dups, grid, full, block, smem, s));
             if (profile) FM_CUDA(cudaEventRecord(ev[d][1], s));
         }
@@ -586,6 +605,7 @@ struct MatchRun {
                 return FM_ERR_DEVICE;
             }
         }
+        if (sums) sums_ready = 4 * n_parents[last] >= base.sum_heads;
         if (over_limit()) return FM_ERR_LIMIT;
         LaunchCtl snap[kMaxQ];
         std::memcpy(snap, ctx->h_ctl, q * sizeof(LaunchCtl));
@@ -674,8 +694,7 @@ struct MatchRun {
         const uint32_t q = plan->q;
         const int mode = mode_of(d);
         const uint64_t n_chunks = (n_parents + 31) / 32;
-        const size_t smem =
-            expand_smem_bytes(d, nreq_depth[d], block / 32, nreq_depth[d] >= 2 ? base.stage_words : 0);
+        const size_t smem = level_smem(d);
         const int per_sm = expand_blocks_per_sm(mode, roots, dups, smem, block);
         (void)q;
         while (true) {
@@ -701,6 +720,14 @@ struct MatchRun {
             FM_CUDA(cudaMemsetAsync(ctx->ctl + d, 0, sizeof(LaunchCtl), s));
             cudaEvent_t e0 = nullptr, e1 = nullptr;
             if (profile) FM_TRY(begin_timing(e0, e1));
+            if (sums && d == last_depth()) {
+                if (!sums_ready && 4 * n_parents >= base.sum_heads) {
+                    p.sum_rule = 2;
+                    FM_CUDA(vertex_sums(p, nullptr));
+                    sums_ready = true;
+                }
+                p.sum_rule = sums_ready ? 2 : 0;
+            }
             FM_CUDA(launch_expand(p, mode, roots, dups, grid, ctx->sms * per_sm, block, smem, s));
             if (profile) FM_CUDA(cudaEventRecord(e1, s));
             FM_CUDA(cudaMemcpyAsync(ctx->h_ctl + d, ctx->ctl + d, sizeof(LaunchCtl), cudaMemcpyDeviceToHost, s));
@@ -863,14 +890,42 @@ fm_status match_impl(fm_context* ctx, const fm_graph* graph, const fm_query* que
         const uint32_t stored = q - (run.pre ? 1u : 0u);   // depths with a level buffer: 2 .. stored-1
         uint64_t sum_cols = 0;
         for (uint32_t d = 2; d < stored; d++) sum_cols += d;
-        uint64_t cap = sum_cols ? ctx->soln_bytes / (4ull * sum_cols) : 0;
         const uint64_t bank = ctx->knobs.bank_rows;
-        if (sum_cols) {
+        auto rows_in = [&](uint64_t bytes) {
+            uint64_t cap = sum_cols ? bytes / (4ull * sum_cols) : 0;
             cap = std::min<uint64_t>(cap, 0xffffffffull - 64);   // parent indices are 32-bit
-            cap = cap / bank * bank;
-            if (cap < (uint64_t)g.max_len * 32 + 32 || cap == 0) {
-                set_error("SOLN_PREALLOC cannot hold one 32-parent chunk per level for this graph");
-                return FM_ERR_POOL;
+            return cap / bank * bank;
+        };
+        auto enough = [&](uint64_t cap) { return !sum_cols || (cap >= (uint64_t)g.max_len * 32 + 32 && cap > 0); };
+        uint64_t cap = rows_in(ctx->soln_bytes);
+        if (!enough(cap)) {
+            set_error("SOLN_PREALLOC cannot hold one 32-parent chunk per level for this graph");
+            return FM_ERR_POOL;
+        }
+        // Pre-count by sums: the counting level has one back edge too, no
+        // vertex is in its own list, and a chain's lists can be read from
+        // either end.  A work limit counts candidate by candidate.  Depth 1
+        // is left to enumeration: its parents are the label's lists, each of
+        // which the vertex sums would walk once as well.  The sums take 8
+        // bytes a vertex of the level memory, at most an eighth of it.
+        if (run.pre && q >= 4 && nreq[q - 2] == 1 && !g.has_self_loops && !opts.work_limit &&
+            (opts.engine != FM_ENGINE_PERSISTENT || opts.profile)) {
+            const uint32_t a = dp.req_anc[dp.req_begin[q - 2]], l = dp.req_label[dp.req_begin[q - 2]];
+            const uint32_t b = dp.req_anc[dp.req_begin[q - 1]], ll = dp.req_label[dp.req_begin[q - 1]];
+            const bool chain = b == q - 2;
+            const bool vertex = chain || (a == b && l != ll);
+            const uint64_t vbytes = vertex ? (uint64_t)g.V * sizeof(uint2) : 0;
+            const uint64_t voff = 8 * vbytes <= ctx->soln_bytes ? (ctx->soln_bytes - vbytes) & ~255ull : 0;
+            if ((!chain || g.symmetric) && enough(rows_in(voff))) {
+                run.sums = true;
+                run.sum_label = l;
+                run.sum_last = ll;
+                cap = rows_in(voff);
+                if (vertex) {
+                    run.vsum = (uint2*)(ctx->soln + voff);
+                    run.base.vsum = run.vsum;
+                    run.base.sum_heads = (uint32_t)(g.head_off[l + 1] - g.head_off[l]);
+                }
             }
         }
         run.ctx = ctx;

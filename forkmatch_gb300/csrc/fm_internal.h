@@ -61,6 +61,7 @@ struct DeviceGraph {
     uint32_t max_len = 0;
     int has_dups = 0;
     int has_self_loops = 0;    // some e-line has src == dst
+    int symmetric = 0;         // every e-line's reverse (same label) is there too
     int device = 0;
     double build_ms = 0;
     std::vector<uint64_t> label_count;   // e-lines per label slot
@@ -203,6 +204,14 @@ struct ExpandParams {
     // The graph has an e-line v -> v: only then can a vertex be in its own
     // list, so only then does pre-count test the new vertex against its list.
     uint32_t self_loops;
+    // Pre-count by sums (see expand_sum_main): 0 off; 1 on when the level has
+    // at least a quarter as many parents as the vertex sums took lists
+    // (sum_heads), decided on the device; 2 on.
+    uint32_t sum_rule;
+    uint32_t sum_heads;
+    const uint2* vsum;              // per vertex v with a list of the level's label: the sum of its
+                                    // neighbours' last-label list lengths, and the neighbours that are
+                                    // also in v's own last-label list
 };
 constexpr unsigned int kLimitFlag = 2u;
 
@@ -273,6 +282,11 @@ cudaError_t launch_sched_init(SchedState* S, unsigned q, unsigned long long n_ro
 cudaError_t launch_expand(const ExpandParams& p, int mode, bool roots, bool dups, int grid, int heavy_grid,
                           int block, size_t smem, cudaStream_t s);
 size_t expand_smem_bytes(uint32_t depth, uint32_t nreq, int warps, uint32_t stage_words);
+// Vertex sums of pre-count by sums for the lists of `label` (n root-list
+// entries at `heads`); with `parents` set, skipped on the device when the level
+// has too few parents for the rule.
+cudaError_t launch_vertex_sums(const ExpandParams& p, const uint32_t* heads, uint32_t n, uint32_t label,
+                               uint32_t last_label, uint2* vsum, const unsigned long long* parents, cudaStream_t s);
 // Let kernel f launch with up to the device's opt-in shared memory (once per
 // device; safe from several host threads).
 void allow_dynamic_smem(const void* f);
@@ -334,6 +348,8 @@ struct BuildStats {
     unsigned int nseg, total16;       // segments; 16-byte units of out-of-line lists
     unsigned int max_len;             // longest list
     unsigned int bm_count;            // bitmap indices given out
+    unsigned int asym;                // an e-line without its reverse
+    unsigned int up, down;            // e-lines with src < dst, src > dst
     unsigned int hist[32];            // lists by floor(log2(length))
     unsigned long long kept;          // text: e-lines kept
     unsigned long long first_bad;     // text: first malformed line

@@ -1,0 +1,94 @@
+"""Pre-count by sums (count mode, one back edge at each of the last two depths):
+counts and the per-level work counters equal the oracle's enumeration on
+graphs where the two lists meet in every way -- pairs joined by two labels (a
+vertex's lists of two labels share neighbours), hubs longer than a piece and
+than the block limit of the vertex sums, lists of every kind, graphs whose
+e-lines lack their reverse or loop (where the rule must not be used), and level
+buffers small enough to drain.  Integer work: no tolerance."""
+import numpy as np
+import pytest
+
+import forkmatch_gb300 as fm
+from forkmatch_gb300 import synth as S
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from forkmatch_gb300 import build
+    build.build()
+    c = fm.Context(prealloc_bytes=2 << 30, soln_prealloc_bytes=512 << 20, output_prealloc_bytes=64 << 20,
+                   bank_rows=256)
+    yield c
+    c.close()
+
+
+def _edges(kind):
+    """Directed e-lines (src, dst, label), no duplicates."""
+    rng = np.random.default_rng(17)
+    n, m = 400, 1800
+    a, b = rng.integers(0, n, m), rng.integers(0, n, m)
+    lab = rng.integers(1, 4, m)
+    if kind == "hub":                                # label 1: two hubs of 1500 common neighbours
+        n = 1600
+        x = np.arange(2, 1502)
+        a = np.concatenate([a, np.zeros(1500, int), np.ones(1500, int)])
+        b = np.concatenate([b, x, x])
+        lab = np.concatenate([lab, np.ones(1500, int), np.where(x % 3 == 0, 1, 2)])
+    if kind == "two_labels":                         # every third edge carries a second label
+        a, b, lab = np.concatenate([a, a[::3]]), np.concatenate([b, b[::3]]), np.concatenate([lab, lab[::3] % 3 + 1])
+    keep = a != b
+    a, b, lab = a[keep], b[keep], lab[keep]
+    e = np.stack([np.concatenate([a, b]), np.concatenate([b, a]), np.concatenate([lab, lab])], 1)
+    if kind == "one_way":
+        e = e[rng.random(len(e)) < 0.8]
+    if kind == "loops":
+        v = np.arange(0, n, 5)
+        e = np.concatenate([e, np.stack([v, v, np.ones(len(v), int)], 1)])
+    e = np.unique(e, axis=0).astype(np.uint32)
+    return n, [np.ascontiguousarray(e[:, i]) for i in range(3)]
+
+
+def _queries():
+    """Paths, stars, and trees whose last two vertices hang on different ancestors, labels equal and mixed."""
+    qs = [S.query_path(4, [1, 2, 3]), S.query_path(4, [1, 1, 1]), S.query_path(4, [2, 1, 2]),
+          S.query_path(5, [1, 2, 1, 2]), S.query_path(5, [3, 1, 2, 3]), S.query_star(4, [1, 2, 3]),
+          S.query_star(4, [1, 1, 2]), S.query_star(4, [2, 2, 2]),
+          S.Query(5, [(0, 1, 1), (0, 2, 2), (1, 3, 3), (2, 4, 1)]), S.Query(5, [(0, 1, 2), (1, 2, 1), (1, 3, 2), (0, 4, 1)]),
+          S.Query(5, [(0, 1, 1), (1, 2, 2), (0, 2, 3), (2, 3, 1), (3, 4, 2)])]
+    return [q.to_g_text() for q in qs]
+
+
+@pytest.mark.parametrize("bitmaps", ["default", "none", "short"])
+@pytest.mark.parametrize("kind", ["plain", "two_labels", "hub", "one_way", "loops"])
+def test_sums_equal_enumeration(ctx, monkeypatch, kind, bitmaps):
+    if bitmaps == "none":
+        monkeypatch.setenv("FM_BITMAP_BYTES", "0")
+    if bitmaps == "short":
+        monkeypatch.setenv("FM_BITMAP_MIN_LEN", "4")
+    V, (src, dst, lab) = _edges(kind)
+    g = fm.Graph.from_edges(ctx, V, 4, src, dst, lab)
+    og = O.Graph.from_edges(V, 4, src, dst, lab)
+    small = fm.Context(prealloc_bytes=256 << 20, soln_prealloc_bytes=8 * 4 * 5 * (32 * g.info().max_list + 64) + 8 * V,
+                       output_prealloc_bytes=1 << 20, bank_rows=1)
+    for text in _queries():
+        p = O.plan(text, enumerate_aut=0)
+        want, _, st = O.match(og, p, count_rule=True, limit=1 << 40)
+        q = fm.Query.from_text(text)
+        # an e-line is read from the vertex matched first, so without its
+        # reverse the count belongs to one order: the oracle's is the reference's
+        for order in (fm.ORDER_REFERENCE,) if kind == "one_way" else (fm.ORDER_REFERENCE, fm.ORDER_AUTO):
+            assert fm.match(ctx, g, q, mode=fm.MODE_COUNT, order=order).count == want
+            assert fm.match(small, g, q, mode=fm.MODE_COUNT, order=order).count == want
+        r = fm.match(ctx, g, q, mode=fm.MODE_COUNT, order=fm.ORDER_REFERENCE)
+        assert r.count == want
+        for d in range(2, p.q):
+            assert r.level[d].lookups == st.lookups[d], ("lookups", d)
+            assert r.level[d].list_words == st.list_words[d], ("list_words", d)
+            assert r.level[d].parents == st.partials[d - 1], ("parents", d)
+        for d in range(1, p.q - 1):
+            assert r.level[d].produced == st.partials[d], ("produced", d)
+    small.close()
+    g.close()
