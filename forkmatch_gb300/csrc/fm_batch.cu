@@ -87,7 +87,7 @@ using dev::kFull;
 using dev::ldg4;
 using dev::seg_at;
 using dev::seg_has;
-using dev::slot_locate;
+using dev::SlotWalk;
 
 constexpr int kBWarps = 8;
 constexpr uint32_t kBStage = 128;
@@ -127,7 +127,7 @@ __device__ __forceinline__ BTune make_btune(const BatchParams& P) {
 struct BMem {
     uint32_t* rows_s;   // [d][32]
     uint4* segs_s;      // [kmax][32]
-    uint32_t* excl_s;   // [32]
+    uint2* start_s;     // [32] parents with candidates: first slot, lane (dev::SlotWalk)
     uint32_t* drv_s;    // [32]
     uint32_t* k_s;      // [32] requirements of the parent's query at this depth
     uint32_t* qid_s;    // [32]
@@ -141,7 +141,7 @@ struct BMem {
 };
 
 __host__ __device__ constexpr uint32_t bper_warp_bytes(uint32_t d, uint32_t kmax, uint32_t stage_words = 0) {
-    return 128 * d + 512 * kmax + 6 * 128 + 12 * kBStage + 4 * stage_words;
+    return 128 * d + 512 * kmax + 7 * 128 + 12 * kBStage + 4 * stage_words;
 }
 
 __device__ __forceinline__ BMem bmem(unsigned char* smem, uint32_t warp, uint32_t d, uint32_t kmax,
@@ -151,17 +151,17 @@ __device__ __forceinline__ BMem bmem(unsigned char* smem, uint32_t warp, uint32_
     m.rows_s = (uint32_t*)w;
     m.segs_s = (uint4*)(w + 128 * d);
     uint32_t* s = (uint32_t*)(w + 128 * d + 512 * kmax);
-    m.excl_s = s;
-    m.drv_s = s + 32;
-    m.k_s = s + 64;
-    m.qid_s = s + 96;
-    m.pidx_s = s + 128;
-    m.fin_s = s + 160;
-    m.stp = s + 192;
+    m.start_s = (uint2*)s;
+    m.drv_s = s + 64;
+    m.k_s = s + 96;
+    m.qid_s = s + 128;
+    m.pidx_s = s + 160;
+    m.fin_s = s + 192;
+    m.stp = s + 224;
     m.stx = m.stp + kBStage;
     m.stq = m.stx + kBStage;
     m.mbar = mbar_s + warp;
-    m.stage = (uint32_t*)(w + 128 * d + 512 * kmax + 6 * 128 + 12 * kBStage);
+    m.stage = (uint32_t*)(w + 128 * d + 512 * kmax + 7 * 128 + 12 * kBStage);
     return m;
 }
 
@@ -228,7 +228,7 @@ __device__ __forceinline__ uint32_t bload_chunk(const BatchParams& P, const BMem
                                                 uint32_t d, unsigned long long n_parents, bool& valid,
                                                 uint32_t& k_out, unsigned long long& words, uint32_t sw,
                                                 uint32_t& phase, bool& stage_ok, unsigned long long& rule_cnt,
-                                                uint32_t& cont_total) {
+                                                uint32_t& cont_total, uint32_t& excl, uint32_t& n) {
     uint32_t qid, pidx;
     if (ROOTS) {
         qid = chunk / P.chunks_per_query;
@@ -243,7 +243,8 @@ __device__ __forceinline__ uint32_t bload_chunk(const BatchParams& P, const BMem
         qid = valid ? __ldg(P.pin + (uint64_t)d * P.pstride + p) : 0u;
         for (uint32_t c = 0; c < d; c++) m.rows_s[c * 32 + lane] = valid ? __ldg(P.pin + c * P.pstride + p) : 0u;
     }
-    uint32_t n = 0, drv = 0, k = 0, fin = 0;
+    uint32_t drv = 0, k = 0, fin = 0;
+    n = 0;
     words = 0;
     rule_cnt = 0;
     if (valid) {
@@ -288,7 +289,7 @@ __device__ __forceinline__ uint32_t bload_chunk(const BatchParams& P, const BMem
         const uint32_t t = __shfl_up_sync(kFull, incl, o);
         if ((int)lane >= o) incl += t;
     }
-    m.excl_s[lane] = incl - n;
+    excl = incl - n;
     m.drv_s[lane] = drv;
     m.k_s[lane] = k;
     m.qid_s[lane] = qid;
@@ -374,18 +375,18 @@ __device__ __forceinline__ void bprecount(const BatchParams& P, const BMem& m, b
 // single-query kernel); each slot's survivor is then counted or written
 // (its query ends here), pre-counted, or staged for the next level.
 template <bool ROOTS>
-__device__ __forceinline__ void bprocess(const BatchParams& P, const BMem& m, uint32_t chunk, uint32_t begin,
-                                         uint32_t end, uint32_t lane, uint32_t d, uint32_t& nst) {
+__device__ __forceinline__ void bprocess(const BatchParams& P, const BMem& m, uint32_t chunk, uint32_t excl, uint32_t n,
+                                         uint32_t begin, uint32_t end, uint32_t lane, uint32_t d, uint32_t& nst) {
+    SlotWalk walk(m.start_s, excl, n, begin, lane);
     for (uint32_t base = begin; base < end; base += 32 * kBSlots) {
         uint32_t j[kBSlots], t[kBSlots], x[kBSlots];
         bool ok[kBSlots];
 #pragma unroll
         for (uint32_t u = 0; u < kBSlots; u++) {
-            const uint32_t s = base + 32 * u + lane;
-            j[u] = t[u] = x[u] = 0;
-            ok[u] = s < end;
+            walk.window(m.start_s, base + 32 * u, lane, j[u], t[u]);
+            x[u] = 0;
+            ok[u] = base + 32 * u + lane < end;
             if (ok[u]) {
-                slot_locate(s, m.excl_s, j[u], t[u]);
                 x[u] = seg_at(m.segs_s[m.drv_s[j[u]] * 32 + j[u]], t[u], P.nbr);
             }
         }
@@ -467,9 +468,9 @@ __device__ __forceinline__ void bexpand_main(const BatchParams& P, unsigned char
             bool valid, stage_ok;
             uint32_t k;
             unsigned long long w, rule_cnt;
-            uint32_t cont;
+            uint32_t cont, excl, n;
             const uint32_t total = bload_chunk<ROOTS>(P, m, chunk, lane, d, T.n_parents, valid, k, w, sw, phase,
-                                                      stage_ok, rule_cnt, cont);
+                                                      stage_ok, rule_cnt, cont, excl, n);
             last_chunk = chunk;
             if (!stage_ok) {
                 done = true;
@@ -532,7 +533,7 @@ __device__ __forceinline__ void bexpand_main(const BatchParams& P, unsigned char
                 pub = __shfl_sync(kFull, pub, 0);
                 if (pub) continue;
             }
-            bprocess<ROOTS>(P, m, chunk, 0, total, lane, d, nst);
+            bprocess<ROOTS>(P, m, chunk, excl, n, 0, total, lane, d, nst);
             // the stage refers to this chunk's query ids only through stq, and to
             // its parents through pidx: it can outlive the chunk
         }
@@ -582,11 +583,12 @@ __device__ __forceinline__ void bexpand_heavy(const BatchParams& P, unsigned cha
         bool valid, stage_ok;
         uint32_t k;
         unsigned long long w, rule_cnt;   // counted by the main pass
-        uint32_t cont;
-        bload_chunk<ROOTS>(P, m, e.chunk, lane, d, T.n_parents, valid, k, w, sw, phase, stage_ok, rule_cnt, cont);
+        uint32_t cont, excl, n;
+        bload_chunk<ROOTS>(P, m, e.chunk, lane, d, T.n_parents, valid, k, w, sw, phase, stage_ok, rule_cnt, cont, excl,
+                           n);
         last_chunk = e.chunk;
         if (!stage_ok) break;
-        bprocess<ROOTS>(P, m, e.chunk, begin, end, lane, d, nst);
+        bprocess<ROOTS>(P, m, e.chunk, excl, n, begin, end, lane, d, nst);
     }
     if (nst) bflush<ROOTS>(P, m, nst, lane, d, last_chunk);
 }

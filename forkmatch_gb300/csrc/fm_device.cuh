@@ -16,6 +16,45 @@ __device__ __forceinline__ uint32_t seg_at(const uint4& s, uint32_t t, const uin
     return __ldg(nbr + (uint64_t)s.y * 4 + t);
 }
 
+// ------------------------------------------------------------ e-line filter
+//
+// "Is x in the list of (label, v)?" answered "no" by one 4-byte load for all
+// but about 1 % of the candidates that are not: three bits of one word of the
+// label's slice, chosen by v and x.  A level's candidates mostly fail, and an
+// exact test (inline compare, bitmap word or binary search, by list) makes
+// the lanes of a warp take all three ways one after another, the search with
+// up to a dozen dependent loads; the filter costs every lane the same 20
+// instructions and one load from a slice of 2 bytes an e-line, which stays in
+// L2.  Only what passes is tested exactly.  With 16 bits an e-line a word has
+// two e-lines on average; 8 bits would pass 5 %, 32 bits 0.4 % from twice the
+// memory.
+struct FilterSlice {
+    const uint32_t* words;
+    uint32_t n;
+};
+
+__device__ __forceinline__ uint32_t filter_seed(uint32_t v) { return v * 0x9E3779B1u; }
+
+// Word of the slice and the three bits.
+__device__ __forceinline__ uint32_t filter_place(uint32_t seed, uint32_t x, uint32_t n, uint32_t& bits) {
+    uint32_t h = x * 0x2C1B3C6Du + seed;
+    h = (h ^ (h >> 16)) * 0x297A2D39u;
+    const uint32_t g = h * 0x7FEB352Du;
+    bits = (1u << (g >> 27)) | (1u << ((g >> 22) & 31u)) | (1u << ((g >> 17) & 31u));
+    return __umulhi(h, n);
+}
+
+__device__ __forceinline__ FilterSlice filter_slice(const uint32_t* efilter, const uint32_t* off, uint32_t label) {
+    const uint32_t a = __ldg(off + label);
+    return {efilter + a, __ldg(off + label + 1) - a};
+}
+
+__device__ __forceinline__ bool filter_has(const FilterSlice& f, uint32_t seed, uint32_t x) {
+    uint32_t bits;
+    const uint32_t at = filter_place(seed, x, f.n, bits);
+    return (__ldg(f.words + at) & bits) == bits;
+}
+
 // lower_bound of x in a[0, n)
 __device__ __forceinline__ uint32_t lower_bound_g(const uint32_t* __restrict__ a, uint32_t n, uint32_t x) {
     uint32_t lo = 0;
@@ -111,51 +150,20 @@ __device__ __forceinline__ uint32_t count_members(const uint4& s, const uint32_t
 }
 
 // Which of the row's vertices (column-major rows_s[c*32 + j], c < n_row, c !=
-// skip) are in the list of record s: bit c.  Graphs without duplicate e-lines
-// only.  Same three kinds of lists as count_members.
+// skip) are in the list s of vertex v: bit c.  The filter answers almost all of
+// them.  Graphs without duplicate e-lines only.
 __device__ __forceinline__ uint32_t member_mask(const uint4& s, const uint32_t* rows_s, uint32_t j, uint32_t n_row,
-                                                uint32_t skip, const uint32_t* __restrict__ nbr,
-                                                const uint32_t* __restrict__ bm, uint32_t bm_words) {
+                                                uint32_t skip, const FilterSlice& f, uint32_t v,
+                                                const uint32_t* __restrict__ nbr, const uint32_t* __restrict__ bm,
+                                                uint32_t bm_words) {
     uint32_t mask = 0;
     if (s.x == 0) return 0;
-    if (s.x <= 3) {
-        for (uint32_t i = 0; i < n_row; i++) {
-            const uint32_t v = rows_s[i * 32 + j];
-            if (i != skip && (s.y == v || s.z == v || s.w == v)) mask |= 1u << i;
-        }
-        return mask;
-    }
-    if (s.z & kBitmapMark) {
-        const uint32_t* b = bm + (uint64_t)(s.z & ~kBitmapMark) * bm_words;
-        for (uint32_t i = 0; i < n_row; i++) {
-            const uint32_t v = rows_s[i * 32 + j];
-            if (i != skip && v <= s.w && ((__ldg(b + (v >> 5)) >> (v & 31)) & 1u)) mask |= 1u << i;
-        }
-        return mask;
-    }
-    const uint32_t* a = nbr + (uint64_t)s.y * 4;
-    for (uint32_t g = 0; g < n_row; g += 4) {
-        uint32_t key[4], base[4];
-        bool act[4];
-#pragma unroll
-        for (uint32_t u = 0; u < 4; u++) {
-            const uint32_t i = g + u;
-            key[u] = i < n_row ? rows_s[i * 32 + j] : 0u;
-            act[u] = i < n_row && i != skip && key[u] >= s.z && key[u] <= s.w;
-            base[u] = 0;
-        }
-        if (!(act[0] || act[1] || act[2] || act[3])) continue;
-        uint32_t len = s.x;
-        while (len > 1) {
-            const uint32_t half = len >> 1;
-#pragma unroll
-            for (uint32_t u = 0; u < 4; u++)
-                if (act[u] && __ldg(a + base[u] + half) <= key[u]) base[u] += half;
-            len -= half;
-        }
-#pragma unroll
-        for (uint32_t u = 0; u < 4; u++)
-            if (act[u] && __ldg(a + base[u]) == key[u]) mask |= 1u << (g + u);
+    const uint32_t seed = filter_seed(v);
+    for (uint32_t i = 0; i < n_row; i++)
+        if (i != skip && filter_has(f, seed, rows_s[i * 32 + j])) mask |= 1u << i;
+    for (uint32_t t = mask; t; t &= t - 1) {
+        const uint32_t i = __ffs(t) - 1;
+        if (!seg_has(s, rows_s[i * 32 + j], 1, nbr, bm, bm_words)) mask &= ~(1u << i);
     }
     return mask;
 }
@@ -287,15 +295,37 @@ __device__ __forceinline__ uint32_t order_lists(uint4* recs, uint32_t lane, uint
     return 0;
 }
 
-// Slot s of a chunk belongs to parent j (the last j with excl[j] <= s), at
-// position t of that parent's driver list.
-__device__ __forceinline__ void slot_locate(uint32_t s, const uint32_t* excl_s, uint32_t& j, uint32_t& t) {
-    j = 0;
-#pragma unroll
-    for (uint32_t step = 16; step; step >>= 1)
-        if (excl_s[j + step] <= s) j += step;
-    t = s - excl_s[j];
-}
+// Which parent a candidate slot of a chunk belongs to.  The parents with
+// candidates are listed in order (`start`: first slot and lane of each); a
+// window of 32 consecutive slots starts in the middle of some parent's range,
+// and the parents that start inside the window are marked in one word
+// (`__reduce_or_sync` over the lanes' first slots).  A slot's parent is then a
+// popcount away: about 11 instructions and one shared load, where a binary
+// search over the 32 first slots takes 25 and five dependent shared loads.
+// Windows are visited in order, 32 slots at a time.
+struct SlotWalk {
+    uint32_t first;      // this lane's first slot, 0xffffffff if it has none
+    uint32_t before;     // parents that start before the next window
+
+    // `excl`, `n`: this lane's first slot and slot count; `begin`: first slot of the walk.
+    __device__ __forceinline__ SlotWalk(uint2* start, uint32_t excl, uint32_t n, uint32_t begin, uint32_t lane) {
+        const unsigned has = __ballot_sync(kFull, n > 0);
+        if (n > 0) start[__popc(has & ((1u << lane) - 1u))] = make_uint2(excl, lane);
+        first = n > 0 ? excl : 0xffffffffu;
+        before = __popc(__ballot_sync(kFull, first < begin));
+        __syncwarp();
+    }
+    // Slot base + lane: parent j (a lane) and position t in its candidates.
+    // Only meaningful for slots below the chunk's total.
+    __device__ __forceinline__ void window(const uint2* start, uint32_t base, uint32_t lane, uint32_t& j, uint32_t& t) {
+        const uint32_t at = first - base;
+        const unsigned mask = __reduce_or_sync(kFull, at < 32u ? 1u << at : 0u);
+        const uint2 s = start[before + __popc(mask & (0xffffffffu >> (31u - lane))) - 1u];
+        before += __popc(mask);
+        j = s.y;
+        t = base + lane - s.x;
+    }
+};
 
 // ------------------------------------------------------- persistent engine
 

@@ -348,6 +348,20 @@ __global__ void k_symmetry(const uint64_t* __restrict__ keys, uint64_t E, uint32
     }
 }
 
+// E-line filter (dev::filter_place).  Bound by the atomics, one per e-line.
+__global__ void k_filter(const uint64_t* __restrict__ keys, uint64_t E, uint32_t vbits,
+                         const uint32_t* __restrict__ off, uint32_t* __restrict__ efilter) {
+    const uint64_t vmask = (1ull << vbits) - 1;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < E; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t k = keys[i];
+        const uint32_t l = (uint32_t)(k >> (2 * vbits)), a = __ldg(off + l);
+        uint32_t bits;
+        const uint32_t at = dev::filter_place(dev::filter_seed((uint32_t)((k >> vbits) & vmask)), (uint32_t)(k & vmask),
+                                              __ldg(off + l + 1) - a, bits);
+        atomicOr(efilter + a + at, bits);
+    }
+}
+
 // One block per bitmap: set the bit of every entry.
 __global__ void k_bm_fill(const uint32_t* __restrict__ nbr, const uint2* __restrict__ bm_list, uint32_t n_bm,
                           uint32_t bm_words, uint32_t* __restrict__ bitmaps) {
@@ -573,12 +587,25 @@ fm_status build_from_keys(DeviceGraph& g, uint32_t V, uint32_t L, uint64_t E, Bu
     const uint64_t seg_bytes = up256((uint64_t)L * V * sizeof(uint4));
     const uint64_t nbr_bytes = up256((g.nbr_words ? g.nbr_words : 4) * 4);
     const uint64_t head_bytes = up256((nseg ? nseg : 4) * 4);
-    const uint64_t bm_bytes = n_bm * words * 4ull;
-    FM_CUDA(cudaMalloc(&g.block, seg_bytes + nbr_bytes + head_bytes + bm_bytes));
+    const uint64_t bm_bytes = up256(n_bm * words * 4ull);
+    // half a word of filter per e-line, at least one word per label
+    std::vector<uint32_t> foff(L + 1, 0);
+    for (uint32_t l = 0; l < L; l++) foff[l + 1] = foff[l] + (uint32_t)(h.label_count[l] / 2 + 1);
+    const uint64_t filter_bytes = h.dup ? 0 : up256((uint64_t)foff[L] * 4), foff_bytes = h.dup ? 0 : up256((L + 1) * 4ull);
+    FM_CUDA(cudaMalloc(&g.block, seg_bytes + nbr_bytes + head_bytes + bm_bytes + filter_bytes + foff_bytes));
     g.seg = (uint4*)g.block;
     g.nbr = (uint32_t*)((char*)g.block + seg_bytes);
     g.heads = (uint32_t*)((char*)g.block + seg_bytes + nbr_bytes);
     FM_CUDA(cudaMemsetAsync(g.seg, 0, (size_t)L * V * sizeof(uint4), s));
+    if (!h.dup) {
+        char* f = (char*)g.heads + head_bytes + bm_bytes;
+        g.efilter = (uint32_t*)f;
+        g.efilter_off = (uint32_t*)(f + filter_bytes);
+        FM_CUDA(cudaMemsetAsync(g.efilter, 0, filter_bytes, s));
+        FM_CUDA(cudaMemcpyAsync(g.efilter_off, foff.data(), (L + 1) * 4, cudaMemcpyHostToDevice, s));
+        k_filter<<<grid_for(E, sms), 256, 0, s>>>(sorted, E, vbits, g.efilter_off, g.efilter);
+        FM_CUDA(cudaGetLastError());
+    }
     if (E) {
         uint2* bm_list = (uint2*)spare;
         if (n_bm) {

@@ -236,6 +236,7 @@ static void free_device_graph(DeviceGraph& g) {
     if (g.block) cudaFree(g.block);
     g.block = nullptr;
     g.bitmaps = nullptr;
+    g.efilter = g.efilter_off = nullptr;
     g.seg = nullptr;
     g.nbr = nullptr;
     g.heads = nullptr;
@@ -480,7 +481,8 @@ struct MatchRun {
 
     size_t level_smem(uint32_t d) const {
         const uint32_t k = sums && d == last_depth() ? 2u : nreq_depth[d];
-        return expand_smem_bytes(d, k, block / 32, nreq_depth[d] >= 2 ? base.stage_words : 0);
+        return expand_smem_bytes(d, k, block / 32, nreq_depth[d] >= 2 ? base.stage_words : 0,
+                                 mode_of(d) != kModeLastCount);
     }
     cudaError_t vertex_sums(const ExpandParams& p, const unsigned long long* parents) {
         if (!vsum) return cudaSuccess;
@@ -907,7 +909,9 @@ fm_status match_impl(fm_context* ctx, const fm_graph* graph, const fm_query* que
         // either end.  A work limit counts candidate by candidate.  Depth 1
         // is left to enumeration: its parents are the label's lists, each of
         // which the vertex sums would walk once as well.  The sums take 8
-        // bytes a vertex of the level memory, at most an eighth of it.
+        // bytes a vertex of the level memory, at most an eighth of it, and a
+        // launch of their own: below 4096 lists that launch (3 us) is more
+        // than the level saves (300 vertices: 86 us a match with, 83 without).
         if (run.pre && q >= 4 && nreq[q - 2] == 1 && !g.has_self_loops && !opts.work_limit &&
             (opts.engine != FM_ENGINE_PERSISTENT || opts.profile)) {
             const uint32_t a = dp.req_anc[dp.req_begin[q - 2]], l = dp.req_label[dp.req_begin[q - 2]];
@@ -916,7 +920,8 @@ fm_status match_impl(fm_context* ctx, const fm_graph* graph, const fm_query* que
             const bool vertex = chain || (a == b && l != ll);
             const uint64_t vbytes = vertex ? (uint64_t)g.V * sizeof(uint2) : 0;
             const uint64_t voff = 8 * vbytes <= ctx->soln_bytes ? (ctx->soln_bytes - vbytes) & ~255ull : 0;
-            if ((!chain || g.symmetric) && enough(rows_in(voff))) {
+            const uint64_t lists = l < g.L ? g.head_off[l + 1] - g.head_off[l] : 0;
+            if ((!chain || g.symmetric) && lists >= 4096 && enough(rows_in(voff))) {
                 run.sums = true;
                 run.sum_label = l;
                 run.sum_last = ll;
@@ -924,7 +929,7 @@ fm_status match_impl(fm_context* ctx, const fm_graph* graph, const fm_query* que
                 if (vertex) {
                     run.vsum = (uint2*)(ctx->soln + voff);
                     run.base.vsum = run.vsum;
-                    run.base.sum_heads = (uint32_t)(g.head_off[l + 1] - g.head_off[l]);
+                    run.base.sum_heads = (uint32_t)lists;
                 }
             }
         }
@@ -948,6 +953,8 @@ fm_status match_impl(fm_context* ctx, const fm_graph* graph, const fm_query* que
         b.nbr = g.nbr;
         b.bm = g.bitmaps;
         b.bm_words = g.bm_words;
+        b.efilter = g.efilter;
+        b.efilter_off = g.efilter_off;
         b.V = g.V;
         b.root_begin = rb;
         // Over the full vertex range the roots are the vertices that have an

@@ -54,6 +54,11 @@ struct DeviceGraph {
     // bitmaps + (z & ~kBitmapMark) * bm_words instead of its minimum.
     uint32_t* bitmaps = nullptr;
     uint32_t bm_words = 0;
+    // E-line filter: 16 bits per e-line, three of them set in one word chosen
+    // by (src, dst), in a slice per label (words efilter[efilter_off[l] ..
+    // efilter_off[l + 1])).  Null for graphs with duplicate e-lines.
+    uint32_t* efilter = nullptr;
+    uint32_t* efilter_off = nullptr;
     uint32_t n_bitmaps = 0;
     uint32_t bm_min_len = 0;
     uint64_t nbr_words = 0;
@@ -149,6 +154,8 @@ struct ExpandParams {
     const uint32_t* nbr;
     const uint32_t* bm;             // list bitmaps (see DeviceGraph)
     uint32_t bm_words;
+    const uint32_t* efilter;        // e-line filter and its slices by label (see DeviceGraph)
+    const uint32_t* efilter_off;
     uint32_t V;
     // parents
     const uint32_t* pin;            // SoA: column c at pin + c*pstride (null for roots)
@@ -281,7 +288,8 @@ cudaError_t launch_sched_init(SchedState* S, unsigned q, unsigned long long n_ro
 // (fm_match.cu).
 cudaError_t launch_expand(const ExpandParams& p, int mode, bool roots, bool dups, int grid, int heavy_grid,
                           int block, size_t smem, cudaStream_t s);
-size_t expand_smem_bytes(uint32_t depth, uint32_t nreq, int warps, uint32_t stage_words);
+// `staged`: the level writes survivors (a middle or a table level).
+size_t expand_smem_bytes(uint32_t depth, uint32_t nreq, int warps, uint32_t stage_words, bool staged);
 // Vertex sums of pre-count by sums for the lists of `label` (n root-list
 // entries at `heads`); with `parents` set, skipped on the device when the level
 // has too few parents for the rule.

@@ -51,11 +51,16 @@ using dev::ldg4;
 using dev::lower_bound_g;
 using dev::seg_at;
 using dev::seg_has;
-using dev::slot_locate;
+using dev::SlotWalk;
 
 constexpr int kWarps = 8;
-constexpr uint32_t kStage = 256;           // staged survivors per warp
+// Staged survivors per warp: levels with one back edge flush most (every
+// candidate survives) and have no filter queue; 128 entries there cost 10-14 %
+// against 256, which elsewhere cost more in L1 than they save in flushes.
+constexpr uint32_t kStage = 128, kStageOne = 256;
+__host__ __device__ constexpr uint32_t stage_rows(uint32_t k) { return k == 1 ? kStageOne : kStage; }
 constexpr uint32_t kSlots = 2;             // candidate slots per lane per round
+constexpr uint32_t kPend = 32 * kSlots + 32;  // candidates that wait for their exact test, per warp
 constexpr uint32_t kHeavyMaxPieces = 65536;
 
 // Rank of position t within its run of equal values.
@@ -115,52 +120,44 @@ __device__ __forceinline__ void defer_chunk(const ExpandParams& P, uint32_t chun
     else atomicOr(&P.ctl->error, 1u);
 }
 
-// Does driver value x (position t of parent j's driver list dj) survive?
-// Membership in the other lists first (most candidates fail there), then
-// injectivity against the parent's row in shared memory (rarely fails).
-template <bool DUPS>
-__device__ __forceinline__ bool slot_check(const ExpandParams& P, uint32_t x, uint32_t t, uint32_t j, uint32_t dj,
-                                           const uint4& ds, const uint4* segs_s, const uint32_t* rows_s,
-                                           uint32_t k, uint32_t d, const uint32_t* stage) {
-    bool ok = true;
-    uint32_t need = 1;
-    if (DUPS) need = seg_rank(ds, t, x, P.nbr) + 1;
-    for (uint32_t i = 0; i < k && ok; i++) {
-        if (i == dj) continue;
-        ok = dev::seg_has_st(segs_s[i * 32 + j], x, need, P.nbr, P.bm, P.bm_words, stage);
-    }
-    for (uint32_t c = 0; c < d && ok; c++) ok = rows_s[c * 32 + j] != x;
-    return ok;
-}
-
 // Per-warp shared memory.
 struct WarpMem {
     uint32_t* rows_s;   // [d][32] parent rows of the current chunk, column-major
     uint4* segs_s;      // [k][32] segment records
-    uint32_t* excl_s;   // [32] exclusive prefix of driver lengths
-    uint32_t* drv_s;    // [32] driver list of each parent
-    uint32_t* stp;      // [kStage] staged survivors: parent index in the level
-    uint32_t* stx;      // [kStage] staged survivors: new vertex
+    uint2* start_s;     // [32] parents with candidates: first slot, lane (dev::SlotWalk)
+    uint8_t* drv_s;     // [32] driver list of each parent
+    uint32_t* stp;      // [stage_rows] staged survivors: parent index in the level
+    uint32_t* stx;      // [stage_rows] staged survivors: new vertex
+    uint32_t* px;       // [kPend] candidates the filter let pass: vertex
+    uint8_t* pj;        // [kPend] and parent (lane) in the chunk
     uint64_t* mbar;     // completion barrier of the list stage's bulk copies
     uint32_t* stage;    // [stage_words] membership lists copied in by TMA (optional)
 };
 
-__host__ __device__ constexpr uint32_t per_warp_bytes(uint32_t d, uint32_t k, uint32_t stage_words = 0) {
-    return 128 * d + 512 * k + 256 + 8 * kStage + 4 * stage_words;
+// Counting levels store no survivors and have no stage.  The bytes matter: what
+// the blocks of an SM do not take of its 256 KB is its L1, which serves the
+// records, lists and filter words (with 6 blocks, 33 KB a block instead of 31
+// leaves 28 KB of L1 instead of 60 and made the counting level of a 5-vertex
+// path 1.5 times slower).
+__host__ __device__ constexpr uint32_t per_warp_bytes(uint32_t d, uint32_t k, uint32_t stage_words, bool staged) {
+    return 128 * d + 512 * k + 256 + 32 + (staged ? 8 * stage_rows(k) : 0u) + (k == 1 ? 0u : 5 * kPend) + 4 * stage_words;
 }
+static_assert(5 * kPend % 16 == 0 && 8 * kStage % 16 == 0, "the list stage is 16-byte aligned");
 
 __device__ __forceinline__ WarpMem warp_mem(unsigned char* smem_raw, uint32_t warp, uint32_t d, uint32_t k,
-                                            uint32_t stage_words, uint64_t* mbar_s) {
-    unsigned char* ws = smem_raw + warp * per_warp_bytes(d, k, stage_words);
+                                            uint32_t stage_words, bool staged, uint64_t* mbar_s) {
+    unsigned char* ws = smem_raw + warp * per_warp_bytes(d, k, stage_words, staged);
     WarpMem m;
     m.rows_s = (uint32_t*)ws;
     m.segs_s = (uint4*)(ws + 128 * d);
-    m.excl_s = (uint32_t*)(ws + 128 * d + 512 * k);
-    m.drv_s = m.excl_s + 32;
-    m.stp = (uint32_t*)(ws + 128 * d + 512 * k + 256);
-    m.stx = m.stp + kStage;
+    m.start_s = (uint2*)(ws + 128 * d + 512 * k);
+    m.drv_s = (uint8_t*)(m.start_s + 32);
+    m.stp = (uint32_t*)(m.drv_s + 32);
+    m.stx = m.stp + stage_rows(k);
+    m.px = m.stp + (staged ? 2 * stage_rows(k) : 0u);
+    m.pj = (uint8_t*)(m.px + kPend);
     m.mbar = mbar_s + warp;
-    m.stage = (uint32_t*)(ws + 128 * d + 512 * k + 256 + 8 * kStage);
+    m.stage = (uint32_t*)(m.pj + kPend);
     return m;
 }
 
@@ -297,11 +294,11 @@ __device__ __forceinline__ void flush_stage(const ExpandParams& P, const WarpMem
 // Load the 32 parents of `chunk`, look up their k lists (independent 16-byte
 // loads), pick each parent's shortest list as its driver and prefix-sum the
 // driver lengths.  Returns the chunk's candidate slots (warp-uniform).
-template <bool ROOTS>
+template <bool ROOTS, bool DUPS>
 __device__ __forceinline__ uint32_t load_chunk(const ExpandParams& P, const WarpMem& m, uint32_t chunk, uint32_t lane,
                                                uint32_t d, uint32_t k, uint32_t rb, unsigned long long n_parents,
                                                bool& valid, unsigned long long& words, uint32_t& phase,
-                                               bool& stage_ok) {
+                                               bool& stage_ok, uint32_t& excl, uint32_t& n) {
     const uint64_t p = (uint64_t)chunk * 32 + lane;
     valid = p < n_parents;
     if (ROOTS) {
@@ -309,7 +306,8 @@ __device__ __forceinline__ uint32_t load_chunk(const ExpandParams& P, const Warp
     } else {
         for (uint32_t c = 0; c < d; c++) m.rows_s[c * 32 + lane] = valid ? P.pin[c * P.pstride + p] : 0u;
     }
-    uint32_t n = 0, drv = 0;
+    uint32_t drv = 0;
+    n = 0;
     words = 0;
     if (valid) {
         uint32_t best = 0xffffffffu;
@@ -326,7 +324,8 @@ __device__ __forceinline__ uint32_t load_chunk(const ExpandParams& P, const Warp
             }
         }
         n = best;
-        if (k > 2) drv = dev::order_lists(m.segs_s, lane, k, drv);
+        // shortest list first where every candidate is tested exactly
+        if (DUPS && k > 2) drv = dev::order_lists(m.segs_s, lane, k, drv);
     }
     stage_ok = true;
     if (P.stage_words && k >= 2) stage_ok = stage_lists(P, m, lane, k, drv, n, valid, phase);
@@ -336,8 +335,8 @@ __device__ __forceinline__ uint32_t load_chunk(const ExpandParams& P, const Warp
         const uint32_t t = __shfl_up_sync(kFull, incl, o);
         if ((int)lane >= o) incl += t;
     }
-    m.excl_s[lane] = incl - n;
-    m.drv_s[lane] = drv;
+    excl = incl - n;
+    m.drv_s[lane] = (uint8_t)drv;
     __syncwarp();
     return __shfl_sync(kFull, incl, 31);
 }
@@ -365,86 +364,172 @@ __device__ __forceinline__ void flush_pre(const ExpandParams& P, PreAcc& pre, ui
     }
 }
 
+// The back edges' filter slices and columns of a level, the same for every
+// parent (in shared memory, one copy per block).
+struct LevelLists {
+    uint2 slice[kMaxQ];              // first word, words
+    uint8_t anc[kMaxQ];
+    __device__ __forceinline__ dev::FilterSlice at(const ExpandParams& P, uint32_t i) const {
+        return {P.efilter + slice[i].x, slice[i].y};
+    }
+};
+
+__device__ __forceinline__ void level_lists_init(const ExpandParams& P, LevelLists& L, uint32_t d) {
+    const uint32_t k = P.plan.nreq[d], rb = P.plan.req_begin[d];
+    if (threadIdx.x < k) {
+        const uint32_t l = P.plan.req_label[rb + threadIdx.x];
+        L.anc[threadIdx.x] = P.plan.req_anc[rb + threadIdx.x];
+        if (P.efilter) {
+            const uint32_t a = __ldg(P.efilter_off + l);
+            L.slice[threadIdx.x] = make_uint2(a, __ldg(P.efilter_off + l + 1) - a);
+        }
+    }
+    __syncthreads();
+}
+
+// What survives a warp round at its level: lane's candidate x of parent j,
+// `ok` if it survived.  Counted, pre-counted, or staged for the next level or
+// the table; the stage is flushed when it cannot take another round.
+struct Emit {
+    uint32_t& nst;                        // staged survivors (warp-uniform), of cap
+    uint32_t cap;
+    unsigned long long& n_count;          // counted (warp-uniform)
+    unsigned long long lane_count = 0;    // pre-counted by this lane
+};
+
+template <int MODE, bool ROOTS, bool DUPS>
+__device__ __forceinline__ void emit(const ExpandParams& P, const WarpMem& m, uint32_t chunk, bool ok, uint32_t j,
+                                     uint32_t x, uint32_t lane, uint32_t d, const uint8_t* col_depth_s, Emit& e,
+                                     PreAcc& pre) {
+    if (MODE == kModeLastCount && !DUPS && P.pre_count) {
+        // Pre-count: each survivor's extensions at the last depth (one back
+        // edge: ancestor anc, label lab) are the entries of that list minus
+        // the row's vertices found in it; the survivor is never stored.
+        if (!ok) return;
+        const uint32_t rb = P.plan.req_begin[d + 1];
+        const uint32_t anc = P.plan.req_anc[rb];
+        const uint4* segl = P.seg + (uint64_t)P.plan.req_label[rb] * P.V;
+        const uint4 sg = ldg4(segl + (anc == d ? x : m.rows_s[anc * 32 + j]));
+        e.lane_count += sg.x - dev::count_members(sg, m.rows_s, j, d, x, P.self_loops || anc != d, P.nbr, P.bm, P.bm_words);
+        pre.parents += 1;
+        pre.words += sg.x;
+        return;
+    }
+    const unsigned b = __ballot_sync(kFull, ok);
+    if (MODE == kModeLastCount) {
+        e.n_count += __popc(b);
+        return;
+    }
+    if (ok) {
+        const uint32_t q = e.nst + __popc(b & ((1u << lane) - 1u));
+        m.stp[q] = chunk * 32 + j;
+        m.stx[q] = x;
+    }
+    e.nst += __popc(b);
+    __syncwarp();
+    if (e.nst > e.cap - 32) {
+        flush_stage<MODE, ROOTS>(P, m, e.nst, lane, d, col_depth_s, chunk);
+        e.nst = 0;
+        __syncwarp();
+    }
+}
+
 // Evaluate slots [begin, end) of the loaded chunk: kSlots slots per lane per
-// round with all their driver loads in flight; survivors go to the stage,
-// which is flushed whenever it cannot take another round.
+// round with all their driver loads in flight.  With several back edges the
+// filter rejects most candidates where they stand; the few it lets pass are
+// collected and tested exactly 32 at a time, so that the exact tests (which
+// differ from list to list and diverge) run with full warps.  Bound by issue
+// slots and by the L1's rate for scattered words.  Closing level of a 4-cycle on
+// a 2^20-vertex R-MAT graph with 64 labels (1.7e7 parents): 740 us, 1100 us with
+// an exact test per candidate and a binary search per slot for its parent.
 template <int MODE, bool ROOTS, bool DUPS>
 __device__ __forceinline__ void process_slots(const ExpandParams& P, const WarpMem& m, uint32_t chunk,
-                                              uint32_t begin, uint32_t end, uint32_t lane, uint32_t d, uint32_t k,
+                                              uint32_t excl, uint32_t n, uint32_t begin, uint32_t end, uint32_t lane,
+                                              uint32_t d, uint32_t k, const LevelLists& L,
                                               const uint8_t* col_depth_s, uint32_t& nst,
                                               unsigned long long& n_count, PreAcc& pre) {
-    const uint32_t pbase = chunk * 32;
-    unsigned long long lane_count = 0;   // pre-count: this lane's counts, summed over the warp at the end
+    Emit e{nst, stage_rows(k), n_count};
+    SlotWalk walk(m.start_s, excl, n, begin, lane);
+    uint32_t pend = 0;
     for (uint32_t base = begin; base < end; base += 32 * kSlots) {
-        uint32_t j[kSlots], t[kSlots], x[kSlots];
+        uint32_t j[kSlots], t[kSlots], x[kSlots], dj[kSlots];
         bool ok[kSlots];
         // every driver load of the round is issued before any check
 #pragma unroll
         for (uint32_t u = 0; u < kSlots; u++) {
-            const uint32_t s = base + 32 * u + lane;
-            j[u] = t[u] = x[u] = 0;
-            ok[u] = s < end;
+            walk.window(m.start_s, base + 32 * u, lane, j[u], t[u]);
+            x[u] = dj[u] = 0;
+            ok[u] = base + 32 * u + lane < end;
             if (ok[u]) {
-                slot_locate(s, m.excl_s, j[u], t[u]);
-                x[u] = seg_at(m.segs_s[m.drv_s[j[u]] * 32 + j[u]], t[u], P.nbr);
+                dj[u] = m.drv_s[j[u]];
+                x[u] = seg_at(m.segs_s[dj[u] * 32 + j[u]], t[u], P.nbr);
             }
         }
-#pragma unroll
-        for (uint32_t u = 0; u < kSlots; u++) {
-            if (ok[u]) {
-                const uint32_t dj = m.drv_s[j[u]];
-                ok[u] = slot_check<DUPS>(P, x[u], t[u], j[u], dj, m.segs_s[dj * 32 + j[u]], m.segs_s, m.rows_s, k, d,
-                                         m.stage);
-            }
-        }
-        if (MODE == kModeLastCount && !DUPS && P.pre_count) {
-            // Pre-count: each survivor's extensions at the last depth (one back
-            // edge: ancestor anc, label lab) are the entries of that list minus
-            // the row's vertices found in it; the survivor is never stored.
-            const uint32_t rb = P.plan.req_begin[d + 1];
-            const uint32_t anc = P.plan.req_anc[rb];
-            const uint4* segl = P.seg + (uint64_t)P.plan.req_label[rb] * P.V;
+        if (DUPS || k == 1) {
+            // membership first (with duplicates: enough copies), then
+            // injectivity against the parent's row in shared memory
 #pragma unroll
             for (uint32_t u = 0; u < kSlots; u++) {
-                uint32_t c = 0;
                 if (ok[u]) {
-                    const uint4 sg = ldg4(segl + (anc == d ? x[u] : m.rows_s[anc * 32 + j[u]]));
-                    c = sg.x - dev::count_members(sg, m.rows_s, j[u], d, x[u], P.self_loops || anc != d, P.nbr,
-                                                  P.bm, P.bm_words);
-                    pre.parents += 1;
-                    pre.words += sg.x;
+                    if (DUPS) {
+                        const uint32_t need = seg_rank(m.segs_s[dj[u] * 32 + j[u]], t[u], x[u], P.nbr) + 1;
+                        for (uint32_t i = 0; i < k && ok[u]; i++)
+                            if (i != dj[u])
+                                ok[u] = dev::seg_has_st(m.segs_s[i * 32 + j[u]], x[u], need, P.nbr, P.bm, P.bm_words,
+                                                        m.stage);
+                    }
+                    for (uint32_t c = 0; c < d && ok[u]; c++) ok[u] = m.rows_s[c * 32 + j[u]] != x[u];
                 }
-                lane_count += c;
             }
+#pragma unroll
+            for (uint32_t u = 0; u < kSlots; u++)
+                emit<MODE, ROOTS, DUPS>(P, m, chunk, ok[u], j[u], x[u], lane, d, col_depth_s, e, pre);
             continue;
         }
-        const unsigned lt = (1u << lane) - 1u;
+        if constexpr (!DUPS) {
+            for (uint32_t i = 0; i < k; i++) {
+                const dev::FilterSlice f = L.at(P, i);
+                const uint32_t* col = m.rows_s + L.anc[i] * 32;
 #pragma unroll
-        for (uint32_t u = 0; u < kSlots; u++) {
-            const unsigned b = __ballot_sync(kFull, ok[u]);
-            if (MODE == kModeLastCount) {
-                n_count += __popc(b);
-                continue;
+                for (uint32_t u = 0; u < kSlots; u++)
+                    if (ok[u] && dj[u] != i) ok[u] = dev::filter_has(f, dev::filter_seed(col[j[u]]), x[u]);
             }
-            if (ok[u]) {
-                const uint32_t q = nst + __popc(b & lt);
-                m.stp[q] = pbase + j[u];
-                m.stx[q] = x[u];
+#pragma unroll
+            for (uint32_t u = 0; u < kSlots; u++) {
+                const unsigned b = __ballot_sync(kFull, ok[u]);
+                if (ok[u]) {
+                    const uint32_t q = pend + __popc(b & ((1u << lane) - 1u));
+                    m.px[q] = x[u];
+                    m.pj[q] = (uint8_t)j[u];
+                }
+                pend += __popc(b);
             }
-            nst += __popc(b);
-        }
-        if (MODE == kModeLastCount) continue;
-        if (nst > kStage - 32 * kSlots) {
+            const bool last = base + 32 * kSlots >= end;
+            while (pend >= 32 || (last && pend)) {
+                const uint32_t take = min(pend, 32u);
+                pend -= take;
+                __syncwarp();
+                bool in = lane < take;
+                uint32_t jj = 0, xx = 0;
+                if (in) {
+                    jj = m.pj[pend + lane];
+                    xx = m.px[pend + lane];
+                    const uint32_t dd = m.drv_s[jj];
+                    for (uint32_t i = 0; i < k && in; i++)
+                        if (i != dd)
+                            in = dev::seg_has_st(m.segs_s[i * 32 + jj], xx, 1, P.nbr, P.bm, P.bm_words, m.stage);
+                    for (uint32_t c = 0; c < d && in; c++) in = m.rows_s[c * 32 + jj] != xx;
+                }
+                emit<MODE, ROOTS, DUPS>(P, m, chunk, in, jj, xx, lane, d, col_depth_s, e, pre);
+            }
             __syncwarp();
-            flush_stage<MODE, ROOTS>(P, m, nst, lane, d, col_depth_s, chunk);
-            nst = 0;
         }
-        __syncwarp();
     }
+    __syncwarp();
     if (MODE == kModeLastCount && !DUPS && P.pre_count) {
 #pragma unroll
-        for (int o = 16; o; o >>= 1) lane_count += __shfl_xor_sync(kFull, lane_count, o);
-        n_count += lane_count;
+        for (int o = 16; o; o >>= 1) e.lane_count += __shfl_xor_sync(kFull, e.lane_count, o);
+        n_count += e.lane_count;
     }
 }
 
@@ -478,14 +563,14 @@ __device__ __forceinline__ bool over_limit(const ExpandParams& P, uint32_t lane,
 // Main pass: warps claim batches of chunks; long candidate ranges are
 // published to the heavy list instead of being walked by one warp.
 template <int MODE, bool ROOTS, bool DUPS>
-__device__ __forceinline__ void expand_main(const ExpandParams& P, unsigned char* smem_raw,
+__device__ __forceinline__ void expand_main(const ExpandParams& P, unsigned char* smem_raw, const LevelLists& L,
                                             const uint8_t* col_depth_s, uint64_t* mbar_s, uint32_t& phase) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t d = P.depth;
     const uint32_t k = P.plan.nreq[d];
     const uint32_t rb = P.plan.req_begin[d];
     const uint32_t sw = k >= 2 ? P.stage_words : 0;   // only levels with membership tests stage lists
-    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, k, sw, mbar_s);
+    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, k, sw, MODE != kModeLastCount, mbar_s);
     const Tune T = make_tune(P, true);
 
     unsigned long long n_count = 0, n_lookups = 0, n_words = 0, n_parents = 0;
@@ -522,8 +607,9 @@ __device__ __forceinline__ void expand_main(const ExpandParams& P, unsigned char
             }
             bool valid, stage_ok;
             unsigned long long w;
-            const uint32_t total = load_chunk<ROOTS>(P, m, chunk, lane, d, k, rb, T.n_parents, valid, w, phase,
-                                                     stage_ok);
+            uint32_t excl, n;
+            const uint32_t total = load_chunk<ROOTS, DUPS>(P, m, chunk, lane, d, k, rb, T.n_parents, valid, w, phase,
+                                                     stage_ok, excl, n);
             last_chunk = chunk;
             if (!stage_ok) {
                 done = true;
@@ -596,7 +682,8 @@ __device__ __forceinline__ void expand_main(const ExpandParams& P, unsigned char
                 pub = __shfl_sync(kFull, pub, 0);
                 if (pub) continue;
             }
-            process_slots<MODE, ROOTS, DUPS>(P, m, chunk, 0, total, lane, d, k, col_depth_s, nst, n_count, pre);
+            process_slots<MODE, ROOTS, DUPS>(P, m, chunk, excl, n, 0, total, lane, d, k, L, col_depth_s, nst, n_count,
+                                             pre);
         }
     }
     if (MODE != kModeLastCount && nst) flush_stage<MODE, ROOTS>(P, m, nst, lane, d, col_depth_s, last_chunk);
@@ -622,7 +709,7 @@ __device__ __forceinline__ void expand_main(const ExpandParams& P, unsigned char
 // that finished their own chunks take over the work of the hub chunks.  The
 // main pass already holds the chunk's output budget and counted its work.
 template <int MODE, bool ROOTS, bool DUPS>
-__device__ __forceinline__ void expand_heavy(const ExpandParams& P, unsigned char* smem_raw,
+__device__ __forceinline__ void expand_heavy(const ExpandParams& P, unsigned char* smem_raw, const LevelLists& L,
                                              const uint8_t* col_depth_s, uint64_t* mbar_s, uint32_t& phase) {
     const unsigned long long h = *(volatile unsigned long long*)&P.ctl->heavy;
     const uint32_t nent = (uint32_t)(h >> 32);
@@ -633,7 +720,7 @@ __device__ __forceinline__ void expand_heavy(const ExpandParams& P, unsigned cha
     const uint32_t k = P.plan.nreq[d];
     const uint32_t rb = P.plan.req_begin[d];
     const uint32_t sw = k >= 2 ? P.stage_words : 0;
-    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, k, sw, mbar_s);
+    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, k, sw, MODE != kModeLastCount, mbar_s);
     const Tune T = make_tune(P, false);
     unsigned long long n_count = 0, n_flushed = 0;
     PreAcc pre;
@@ -656,10 +743,12 @@ __device__ __forceinline__ void expand_heavy(const ExpandParams& P, unsigned cha
         const uint32_t end = min(begin + T.heavy_piece, e.total);
         bool valid, stage_ok;
         unsigned long long w;
-        load_chunk<ROOTS>(P, m, e.chunk, lane, d, k, rb, T.n_parents, valid, w, phase, stage_ok);
+        uint32_t excl, n;
+        load_chunk<ROOTS, DUPS>(P, m, e.chunk, lane, d, k, rb, T.n_parents, valid, w, phase, stage_ok, excl, n);
         last_chunk = e.chunk;
         if (!stage_ok) break;
-        process_slots<MODE, ROOTS, DUPS>(P, m, e.chunk, begin, end, lane, d, k, col_depth_s, nst, n_count, pre);
+        process_slots<MODE, ROOTS, DUPS>(P, m, e.chunk, excl, n, begin, end, lane, d, k, L, col_depth_s, nst, n_count,
+                                             pre);
     }
     if (MODE != kModeLastCount && nst) flush_stage<MODE, ROOTS>(P, m, nst, lane, d, col_depth_s, last_chunk);
     if (MODE == kModeLastCount && lane == 0 && n_count > n_flushed) atomicAdd(&P.tot->count, n_count - n_flushed);
@@ -684,15 +773,16 @@ __device__ __forceinline__ void expand_heavy(const ExpandParams& P, unsigned cha
 // depth come from the same sums.
 //
 // Bound by the intersections' dependent loads.  A 5-vertex path on a 2^22-vertex
-// R-MAT graph with 64 labels (1.2e8 parents with 3.4e9 candidates): 25.6 ms, against 85.0 ms candidate by
+// R-MAT graph with 64 labels (1.2e8 parents with 3.4e9 candidates): 14.4 ms, against 85.0 ms candidate by
 // candidate.
 
 // Intersection of A with the last label's list of row vertex u: the shorter
 // list drives.  Returns the chunk's candidate slots (warp-uniform).
 __device__ __forceinline__ uint32_t sum_lists(const ExpandParams& P, const WarpMem& m, uint32_t lane, uint32_t u,
-                                              const uint4* last, bool live) {
+                                              const uint4* last, bool live, uint32_t& excl, uint32_t& n) {
     uint4 b = make_uint4(0, 0, 0, 0);
-    uint32_t n = 0, drv = 0;
+    uint32_t drv = 0;
+    n = 0;
     if (live) {
         b = ldg4(last + m.rows_s[u * 32 + lane]);
         const uint32_t na = m.segs_s[lane].x;
@@ -706,39 +796,10 @@ __device__ __forceinline__ uint32_t sum_lists(const ExpandParams& P, const WarpM
         const uint32_t t = __shfl_up_sync(kFull, incl, o);
         if ((int)lane >= o) incl += t;
     }
-    m.excl_s[lane] = incl - n;
-    m.drv_s[lane] = drv;
+    excl = incl - n;
+    m.drv_s[lane] = (uint8_t)drv;
     __syncwarp();
     return __shfl_sync(kFull, incl, 31);
-}
-
-// Members of both lists outside the row, over slots [begin, end) (lane-private).
-__device__ __forceinline__ uint32_t sum_slots(const ExpandParams& P, const WarpMem& m, uint32_t begin, uint32_t end,
-                                              uint32_t lane, uint32_t d) {
-    uint32_t hits = 0;
-    for (uint32_t base = begin; base < end; base += 32 * kSlots) {
-        uint32_t j[kSlots], t[kSlots], x[kSlots];
-        bool ok[kSlots];
-#pragma unroll
-        for (uint32_t u = 0; u < kSlots; u++) {
-            const uint32_t s = base + 32 * u + lane;
-            j[u] = t[u] = x[u] = 0;
-            ok[u] = s < end;
-            if (ok[u]) {
-                slot_locate(s, m.excl_s, j[u], t[u]);
-                x[u] = seg_at(m.segs_s[m.drv_s[j[u]] * 32 + j[u]], t[u], P.nbr);
-            }
-        }
-#pragma unroll
-        for (uint32_t u = 0; u < kSlots; u++) {
-            if (!ok[u]) continue;
-            bool in = seg_has(m.segs_s[(m.drv_s[j[u]] ^ 1u) * 32 + j[u]], x[u], 1, P.nbr, P.bm, P.bm_words);
-            for (uint32_t c = 0; c < d && in; c++) in = m.rows_s[c * 32 + j[u]] != x[u];
-            hits += in ? 1u : 0u;
-        }
-    }
-    __syncwarp();
-    return hits;
 }
 
 struct SumPlan {
@@ -746,6 +807,7 @@ struct SumPlan {
     bool same;                       // fork of one vertex by one label: both lists are A
     const uint4* seg;                // records of l
     const uint4* last;               // records of l'
+    dev::FilterSlice seg_f, last_f;
 };
 
 __device__ __forceinline__ SumPlan sum_plan(const ExpandParams& P) {
@@ -756,7 +818,61 @@ __device__ __forceinline__ SumPlan sum_plan(const ExpandParams& P) {
     s.same = s.last_anc == s.anc && P.plan.req_label[rb] == P.plan.req_label[rl];
     s.seg = P.seg + (uint64_t)P.plan.req_label[rb] * P.V;
     s.last = P.seg + (uint64_t)P.plan.req_label[rl] * P.V;
+    s.seg_f = dev::filter_slice(P.efilter, P.efilter_off, P.plan.req_label[rb]);
+    s.last_f = dev::filter_slice(P.efilter, P.efilter_off, P.plan.req_label[rl]);
     return s;
+}
+
+// Members of A and the last label's list of row vertex w, outside the row, over
+// slots [begin, end) (lane-private).
+__device__ __forceinline__ uint32_t sum_slots(const ExpandParams& P, const WarpMem& m, const SumPlan& sp, uint32_t w,
+                                              uint32_t excl, uint32_t n, uint32_t begin, uint32_t end, uint32_t lane,
+                                              uint32_t d) {
+    uint32_t hits = 0, pend = 0;
+    SlotWalk walk(m.start_s, excl, n, begin, lane);
+    for (uint32_t base = begin; base < end; base += 32 * kSlots) {
+        uint32_t j[kSlots], t[kSlots], x[kSlots];
+        bool ok[kSlots], b[kSlots];      // b: the last label's list drives
+#pragma unroll
+        for (uint32_t u = 0; u < kSlots; u++) {
+            walk.window(m.start_s, base + 32 * u, lane, j[u], t[u]);
+            x[u] = 0;
+            b[u] = false;
+            ok[u] = base + 32 * u + lane < end;
+            if (ok[u]) {
+                b[u] = m.drv_s[j[u]] != 0;
+                x[u] = seg_at(m.segs_s[(b[u] ? 32 : 0) + j[u]], t[u], P.nbr);
+            }
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < kSlots; u++) {
+            if (ok[u])
+                ok[u] = dev::filter_has(b[u] ? sp.seg_f : sp.last_f,
+                                        dev::filter_seed(m.rows_s[(b[u] ? sp.anc : w) * 32 + j[u]]), x[u]);
+            const unsigned bl = __ballot_sync(kFull, ok[u]);
+            if (ok[u]) {
+                const uint32_t q = pend + __popc(bl & ((1u << lane) - 1u));
+                m.px[q] = x[u];
+                m.pj[q] = (uint8_t)j[u];
+            }
+            pend += __popc(bl);
+        }
+        const bool last = base + 32 * kSlots >= end;
+        while (pend >= 32 || (last && pend)) {
+            const uint32_t take = min(pend, 32u);
+            pend -= take;
+            __syncwarp();
+            if (lane < take) {
+                const uint32_t jj = m.pj[pend + lane], xx = m.px[pend + lane];
+                bool in = seg_has(m.segs_s[(m.drv_s[jj] ? 0 : 32) + jj], xx, 1, P.nbr, P.bm, P.bm_words);
+                for (uint32_t c = 0; c < d && in; c++) in = m.rows_s[c * 32 + jj] != xx;
+                hits += in ? 1u : 0u;
+            }
+        }
+        __syncwarp();
+    }
+    __syncwarp();
+    return hits;
 }
 
 __device__ __forceinline__ bool sum_rule_on(const ExpandParams& P, unsigned long long n_parents) {
@@ -782,7 +898,7 @@ __device__ __forceinline__ bool sum_needs(const SumPlan& sp, uint32_t d, uint32_
 __device__ __forceinline__ void expand_sum_main(const ExpandParams& P, unsigned char* smem_raw, uint64_t* mbar_s) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t d = P.depth;
-    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, 2, 0, mbar_s);
+    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, 2, 0, false, mbar_s);
     const Tune T = make_tune(P, true);
     const SumPlan sp = sum_plan(P);
     const bool chain = sp.last_anc == d;
@@ -803,7 +919,7 @@ __device__ __forceinline__ void expand_sum_main(const ExpandParams& P, unsigned 
             const bool live = a.x > 0;
             if (live) {
                 const uint32_t va = m.rows_s[sp.anc * 32 + lane];
-                uint32_t in_a = dev::member_mask(a, m.rows_s, lane, d, sp.anc, P.nbr, P.bm, P.bm_words);
+                uint32_t in_a = dev::member_mask(a, m.rows_s, lane, d, sp.anc, sp.seg_f, va, P.nbr, P.bm, P.bm_words);
                 const unsigned long long free_a = a.x - __popc(in_a);
                 pre.parents += free_a;
                 if (chain) {
@@ -822,8 +938,10 @@ __device__ __forceinline__ void expand_sum_main(const ExpandParams& P, unsigned 
                     pre.words += words;
                     n_count += c;
                 } else {
-                    const uint4 b = ldg4(sp.last + m.rows_s[sp.last_anc * 32 + lane]);
-                    const uint32_t in_b = dev::member_mask(b, m.rows_s, lane, d, sp.last_anc, P.nbr, P.bm, P.bm_words);
+                    const uint32_t vb = m.rows_s[sp.last_anc * 32 + lane];
+                    const uint4 b = ldg4(sp.last + vb);
+                    const uint32_t in_b =
+                        dev::member_mask(b, m.rows_s, lane, d, sp.last_anc, sp.last_f, vb, P.nbr, P.bm, P.bm_words);
                     n_count += free_a * (b.x - __popc(in_b));
                     pre.words += free_a * b.x;
                     if (sp.same) n_count -= free_a;
@@ -832,7 +950,8 @@ __device__ __forceinline__ void expand_sum_main(const ExpandParams& P, unsigned 
             }
             for (uint32_t u = 0; u < d; u++) {
                 if (!sum_needs(sp, d, u)) continue;
-                const uint32_t total = sum_lists(P, m, lane, u, sp.last, live);
+                uint32_t excl, n;
+                const uint32_t total = sum_lists(P, m, lane, u, sp.last, live, excl, n);
                 if (total > T.heavy_thresh) {
                     int pub = 0;
                     const uint32_t np = (total + T.heavy_piece - 1) / T.heavy_piece;
@@ -855,7 +974,7 @@ __device__ __forceinline__ void expand_sum_main(const ExpandParams& P, unsigned 
                         continue;
                     }
                 }
-                n_count -= sum_slots(P, m, 0, total, lane, d);
+                n_count -= sum_slots(P, m, sp, u, excl, n, 0, total, lane, d);
             }
             __syncwarp();
         }
@@ -882,7 +1001,7 @@ __device__ __forceinline__ void expand_sum_heavy(const ExpandParams& P, unsigned
     if (nent == 0) return;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t d = P.depth;
-    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, 2, 0, mbar_s);
+    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, 2, 0, false, mbar_s);
     const Tune T = make_tune(P, false);
     const SumPlan sp = sum_plan(P);
     unsigned long long hits = 0;
@@ -901,8 +1020,9 @@ __device__ __forceinline__ void expand_sum_heavy(const ExpandParams& P, unsigned
         const uint32_t begin = ((uint32_t)gp - e.piece0) * T.heavy_piece;
         const uint32_t end = min(begin + T.heavy_piece, e.total);
         sum_load(P, m, sp, e.chunk, lane, d, T.n_parents);
-        sum_lists(P, m, lane, e.pieces >> 24, sp.last, m.segs_s[lane].x > 0);
-        hits += sum_slots(P, m, begin, end, lane, d);
+        uint32_t excl, n;
+        sum_lists(P, m, lane, e.pieces >> 24, sp.last, m.segs_s[lane].x > 0, excl, n);
+        hits += sum_slots(P, m, sp, e.pieces >> 24, excl, n, begin, end, lane, d);
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1) hits += __shfl_xor_sync(kFull, hits, o);
@@ -919,12 +1039,14 @@ __global__ void __launch_bounds__(kWarps * 32) k_vertex_sums(const __grid_consta
                                                              uint32_t label, uint32_t last_label,
                                                              uint2* __restrict__ vsum,
                                                              const unsigned long long* parents) {
-    __shared__ uint32_t excl_s[kWarps][32], sum_s[kWarps][32], both_s[kWarps][32], v_s[kWarps][32];
+    __shared__ uint2 start_s[kWarps][32];
+    __shared__ uint32_t sum_s[kWarps][32], both_s[kWarps][32], v_s[kWarps][32];
     __shared__ uint32_t long_s[kWarps * 32], n_long, lsum, lboth;
     if (parents && !sum_rule_on(P, *(const volatile unsigned long long*)parents)) return;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint4* seg = P.seg + (uint64_t)label * P.V;
     const uint4* last = P.seg + (uint64_t)last_label * P.V;
+    const dev::FilterSlice lf = dev::filter_slice(P.efilter, P.efilter_off, last_label);
     if (threadIdx.x == 0) n_long = 0;
     __syncthreads();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -943,19 +1065,21 @@ __global__ void __launch_bounds__(kWarps * 32) k_vertex_sums(const __grid_consta
         const uint32_t t = __shfl_up_sync(kFull, incl, o);
         if ((int)lane >= o) incl += t;
     }
-    excl_s[warp][lane] = incl - len;
     sum_s[warp][lane] = both_s[warp][lane] = 0;
     v_s[warp][lane] = v;
     const uint32_t total = __shfl_sync(kFull, incl, 31);
-    __syncwarp();
-    for (uint32_t s = lane; s < total; s += 32) {
+    SlotWalk walk(start_s[warp], incl - len, len, 0, lane);
+    for (uint32_t base = 0; base < total; base += 32) {
         uint32_t j, t;
-        slot_locate(s, excl_s[warp], j, t);
+        walk.window(start_s[warp], base, lane, j, t);
+        if (base + lane >= total) continue;
         const uint32_t vj = v_s[warp][j];
         const uint32_t x = seg_at(ldg4(seg + vj), t, P.nbr);
         const uint32_t w = __ldg(&last[x].x);
         if (w) atomicAdd(&sum_s[warp][j], w);
-        if (label == last_label || seg_has(ldg4(last + vj), x, 1, P.nbr, P.bm, P.bm_words)) atomicAdd(&both_s[warp][j], 1u);
+        if (label == last_label || (dev::filter_has(lf, dev::filter_seed(vj), x) &&
+                                    seg_has(ldg4(last + vj), x, 1, P.nbr, P.bm, P.bm_words)))
+            atomicAdd(&both_s[warp][j], 1u);
     }
     __syncwarp();
     if (len) vsum[v] = make_uint2(sum_s[warp][lane], both_s[warp][lane]);
@@ -988,6 +1112,8 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_expand(const __grid_constant
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint8_t col_depth_s[kMaxQ];
     __shared__ uint64_t mbar_s[kWarps];
+    __shared__ LevelLists L;
+    level_lists_init(P, L, P.depth);
     if (threadIdx.x < (unsigned)kMaxQ) col_depth_s[threadIdx.x] = P.plan.col_depth[threadIdx.x];
     dev::stage_barriers_init(mbar_s);
     if (MODE == kModeLastCount && !ROOTS && !DUPS && P.sum_rule && sum_rule_on(P, make_tune(P, true).n_parents)) {
@@ -995,7 +1121,7 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_expand(const __grid_constant
         return;
     }
     uint32_t phase = 0;
-    expand_main<MODE, ROOTS, DUPS>(P, smem_raw, col_depth_s, mbar_s, phase);
+    expand_main<MODE, ROOTS, DUPS>(P, smem_raw, L, col_depth_s, mbar_s, phase);
 }
 
 template <int MODE, bool ROOTS, bool DUPS>
@@ -1003,6 +1129,8 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_expand_heavy(const __grid_co
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint8_t col_depth_s[kMaxQ];
     __shared__ uint64_t mbar_s[kWarps];
+    __shared__ LevelLists L;
+    level_lists_init(P, L, P.depth);
     if (threadIdx.x < (unsigned)kMaxQ) col_depth_s[threadIdx.x] = P.plan.col_depth[threadIdx.x];
     dev::stage_barriers_init(mbar_s);
     if (MODE == kModeLastCount && !ROOTS && !DUPS && P.sum_rule && sum_rule_on(P, make_tune(P, false).n_parents)) {
@@ -1010,7 +1138,7 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_expand_heavy(const __grid_co
         return;
     }
     uint32_t phase = 0;
-    expand_heavy<MODE, ROOTS, DUPS>(P, smem_raw, col_depth_s, mbar_s, phase);
+    expand_heavy<MODE, ROOTS, DUPS>(P, smem_raw, L, col_depth_s, mbar_s, phase);
 }
 
 // ------------------------------------------------------- persistent engine
@@ -1026,25 +1154,25 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_expand_heavy(const __grid_co
 
 template <int LAST, bool DUPS>
 __device__ __forceinline__ void persist_main(const ExpandParams& P, unsigned char* smem, const uint8_t* cd,
-                                             bool roots, bool last, uint64_t* mb, uint32_t& ph) {
+                                             bool roots, bool last, const LevelLists& L, uint64_t* mb, uint32_t& ph) {
     if (last) {
-        if (roots) expand_main<LAST, true, DUPS>(P, smem, cd, mb, ph);
-        else expand_main<LAST, false, DUPS>(P, smem, cd, mb, ph);
+        if (roots) expand_main<LAST, true, DUPS>(P, smem, L, cd, mb, ph);
+        else expand_main<LAST, false, DUPS>(P, smem, L, cd, mb, ph);
     } else {
-        if (roots) expand_main<kModeMid, true, DUPS>(P, smem, cd, mb, ph);
-        else expand_main<kModeMid, false, DUPS>(P, smem, cd, mb, ph);
+        if (roots) expand_main<kModeMid, true, DUPS>(P, smem, L, cd, mb, ph);
+        else expand_main<kModeMid, false, DUPS>(P, smem, L, cd, mb, ph);
     }
 }
 
 template <int LAST, bool DUPS>
 __device__ __forceinline__ void persist_heavy(const ExpandParams& P, unsigned char* smem, const uint8_t* cd,
-                                              bool roots, bool last, uint64_t* mb, uint32_t& ph) {
+                                              bool roots, bool last, const LevelLists& L, uint64_t* mb, uint32_t& ph) {
     if (last) {
-        if (roots) expand_heavy<LAST, true, DUPS>(P, smem, cd, mb, ph);
-        else expand_heavy<LAST, false, DUPS>(P, smem, cd, mb, ph);
+        if (roots) expand_heavy<LAST, true, DUPS>(P, smem, L, cd, mb, ph);
+        else expand_heavy<LAST, false, DUPS>(P, smem, L, cd, mb, ph);
     } else {
-        if (roots) expand_heavy<kModeMid, true, DUPS>(P, smem, cd, mb, ph);
-        else expand_heavy<kModeMid, false, DUPS>(P, smem, cd, mb, ph);
+        if (roots) expand_heavy<kModeMid, true, DUPS>(P, smem, L, cd, mb, ph);
+        else expand_heavy<kModeMid, false, DUPS>(P, smem, L, cd, mb, ph);
     }
 }
 
@@ -1056,6 +1184,7 @@ __global__ void __launch_bounds__(kWarps * 32, 5) k_persist(const __grid_constan
     __shared__ uint8_t col_depth_s[kMaxQ];
     __shared__ unsigned flag_s, cur_s;
     __shared__ uint64_t mbar_s[kWarps];
+    __shared__ LevelLists L;
     SchedState* S = A.sched;
     {
         const uint32_t* src = (const uint32_t*)&P0;
@@ -1097,10 +1226,11 @@ __global__ void __launch_bounds__(kWarps * 32, 5) k_persist(const __grid_constan
         const unsigned d = cur_s;
         if (d == 0) break;
         const bool roots = d == 1, last = d + 1 + P0.pre_count == q;
-        persist_main<LAST, DUPS>(P, smem_raw, col_depth_s, roots, last, mbar_s, phase);
+        level_lists_init(P, L, d);
+        persist_main<LAST, DUPS>(P, smem_raw, col_depth_s, roots, last, L, mbar_s, phase);
         if (!dev::grid_barrier(S, first && A.hold_first_barrier && blockIdx.x == 0, &flag_s)) break;
         first = false;
-        persist_heavy<LAST, DUPS>(P, smem_raw, col_depth_s, roots, last, mbar_s, phase);
+        persist_heavy<LAST, DUPS>(P, smem_raw, col_depth_s, roots, last, L, mbar_s, phase);
         if (!dev::grid_barrier(S, false, &flag_s)) break;
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             const bool limit_hit = P.work_limit && (*(volatile unsigned*)&P.tot->error & kLimitFlag);
@@ -1162,7 +1292,7 @@ cudaError_t launch_sched_init(SchedState* S, unsigned q, unsigned long long n_ro
 size_t persist_smem_bytes(const DevPlan& plan, const uint32_t* nreq_depth, uint32_t stage_words) {
     size_t best = 0;
     for (uint32_t d = 1; d < plan.q; d++)
-        best = std::max<size_t>(best, per_warp_bytes(d, nreq_depth[d], nreq_depth[d] >= 2 ? stage_words : 0));
+        best = std::max<size_t>(best, per_warp_bytes(d, nreq_depth[d], nreq_depth[d] >= 2 ? stage_words : 0, true));
     return best * kWarps;
 }
 
@@ -1204,8 +1334,8 @@ cudaError_t launch_vertex_sums(const ExpandParams& p, const uint32_t* heads, uin
     return cudaGetLastError();
 }
 
-size_t expand_smem_bytes(uint32_t depth, uint32_t nreq, int warps, uint32_t stage_words) {
-    return (size_t)warps * per_warp_bytes(depth, nreq, stage_words);
+size_t expand_smem_bytes(uint32_t depth, uint32_t nreq, int warps, uint32_t stage_words, bool staged) {
+    return (size_t)warps * per_warp_bytes(depth, nreq, stage_words, staged);
 }
 
 void allow_dynamic_smem(const void* f) {

@@ -91,7 +91,7 @@ struct StaticRun {
         uint32_t* def_b = def_a + kStaticDefCap;
         uint32_t ndef_in = 0;
         uint64_t fresh = 0;
-        const size_t smem = expand_smem_bytes(d, nreq[d], block / 32, 0);
+        const size_t smem = expand_smem_bytes(d, nreq[d], block / 32, 0, mode != kModeLastCount);
         const int per_sm = expand_blocks_per_sm(mode, roots, dups, smem, block);
         // A launch defers at most 8 chunks per warp (the largest claim batch),
         // so a grid of at most kStaticDefCap / (8 * warps per block) blocks
@@ -265,6 +265,8 @@ extern "C" fm_status fm_match_static(const fm_graph* graph, const fm_query* quer
     b.nbr = g.nbr;
     b.bm = g.bitmaps;
     b.bm_words = g.bm_words;
+    b.efilter = g.efilter;
+    b.efilter_off = g.efilter_off;
     b.V = g.V;
     b.root_begin = 0;
     b.table = rows_out;

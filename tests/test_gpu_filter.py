@@ -1,0 +1,50 @@
+"""The e-line filter and the queue of candidates it lets pass: graphs where every
+candidate passes (complete graphs: full queues, remainders at every chunk's
+end), and labels whose slice is one word.  Closed forms; no tolerance."""
+import math
+
+import numpy as np
+import pytest
+
+import forkmatch_gb300 as fm
+from forkmatch_gb300 import synth as S
+from tests.helpers import complete_graph
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from forkmatch_gb300 import build
+    build.build()
+    c = fm.Context(prealloc_bytes=1 << 30, soln_prealloc_bytes=512 << 20, output_prealloc_bytes=256 << 20,
+                   bank_rows=256)
+    yield c
+    c.close()
+
+
+@pytest.mark.parametrize("n", [3, 4, 31, 32, 33, 34, 65])
+def test_every_candidate_passes(ctx, n):
+    V, s, d, l = complete_graph(n)
+    g = fm.Graph.from_edges(ctx, V, 2, s, d, l)
+    for q in (S.query_cycle(3, [1] * 3), S.query_cycle(4, [1] * 4), S.query_clique(4, [1])):
+        query = fm.Query.from_text(q.to_g_text())
+        want = math.perm(n, q.k)
+        assert fm.match(ctx, g, query, mode=fm.MODE_COUNT).count == want
+        cnt, rows, _ = fm.match_table(ctx, g, query, max_rows=max(1, want))
+        assert cnt == want == len(rows) == len(np.unique(rows, axis=0))
+        assert all(len(set(r)) == q.k for r in rows[:100].tolist())
+    g.close()
+
+
+@pytest.mark.parametrize("labels", [1, 3, 255])
+def test_one_edge_per_label(ctx, labels):
+    """A triangle whose edges carry labels of their own, among other single edges."""
+    e = [(0, 1, 1), (1, 2, min(2, labels)), (2, 0, min(3, labels))] + [(0, 10 + i, 1 + i) for i in range(3, labels)]
+    src = np.array([a for a, _, _ in e] + [b for _, b, _ in e], dtype=np.uint32)
+    dst = np.array([b for _, b, _ in e] + [a for a, _, _ in e], dtype=np.uint32)
+    lab = np.array([x for _, _, x in e] * 2, dtype=np.uint32)
+    g = fm.Graph.from_edges(ctx, 300, labels + 1, src, dst, lab)
+    q = fm.Query.from_text(S.query_cycle(3, [1, min(2, labels), min(3, labels)]).to_g_text())
+    assert fm.match(ctx, g, q, mode=fm.MODE_COUNT).count == (6 if labels == 1 else 1)
+    g.close()

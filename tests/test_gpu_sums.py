@@ -28,11 +28,10 @@ def ctx():
 def _edges(kind):
     """Directed e-lines (src, dst, label), no duplicates."""
     rng = np.random.default_rng(17)
-    n, m = 400, 1800
+    n, m = 6000, 27000                               # over 4096 lists of each label: the rule's least
     a, b = rng.integers(0, n, m), rng.integers(0, n, m)
     lab = rng.integers(1, 4, m)
     if kind == "hub":                                # label 1: two hubs of 1500 common neighbours
-        n = 1600
         x = np.arange(2, 1502)
         a = np.concatenate([a, np.zeros(1500, int), np.ones(1500, int)])
         b = np.concatenate([b, x, x])
