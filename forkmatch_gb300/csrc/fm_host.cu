@@ -53,7 +53,7 @@ struct fm_context {
     HeavyEntry* heavy = nullptr;  // heavy-chunk entries of the current launch
     uint32_t heavy_cap = 0;
     SchedState* sched = nullptr;  // persistent engine schedule (device)
-    LaunchCtl* h_ctl = nullptr; // pinned mirrors
+    LaunchCtl* h_ctl = nullptr; // pinned mirrors (one MatchCtl)
     MatchTotals* h_tot = nullptr;
     SchedState* h_sched = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -86,15 +86,15 @@ bool fm::pre_count_knob() {
 
 namespace {
 
-// [0, 4 KiB) control blocks, [4 KiB, 8 KiB) match totals and the persistent
-// schedule, [8 KiB, 48 MiB) deferred-chunk lists (two per depth, which the
+// [0, 4 KiB) control blocks and match totals (one MatchCtl), [4 KiB, 8 KiB) the
+// persistent schedule, [8 KiB, 48 MiB) deferred-chunk lists (two per depth, which the
 // persistent engine uses as one ring per depth), [48 MiB, 64 MiB) heavy-chunk
 // entries
 void set_misc(fm_context* c, char* misc) {
-    static_assert(kMaxQ * sizeof(LaunchCtl) <= 4096, "per-level control blocks must fit in 4 KiB");
-    static_assert(256 + sizeof(SchedState) <= 4096, "totals and schedule must fit in 4 KiB");
-    c->ctl = (LaunchCtl*)misc;                 // one control block per depth
-    c->tot = (MatchTotals*)(misc + 4096);
+    static_assert(sizeof(MatchCtl) <= 4096, "control blocks and totals must fit in 4 KiB");
+    static_assert(256 + sizeof(SchedState) <= 4096, "the schedule must fit in 4 KiB");
+    c->ctl = ((MatchCtl*)misc)->level;         // one control block per depth
+    c->tot = &((MatchCtl*)misc)->tot;
     c->sched = (SchedState*)(misc + 4096 + 256);
     c->defs = (uint32_t*)(misc + 8192);
     c->def_cap = (uint32_t)(((48ull << 20) - 8192) / 4 / (2 * kMaxQ));
@@ -180,7 +180,6 @@ void fm_context_destroy(fm_context* c) {
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
     if (c->h_ctl) cudaFreeHost(c->h_ctl);
-    if (c->h_tot) cudaFreeHost(c->h_tot);
     if (c->h_sched) cudaFreeHost(c->h_sched);
     if (c->slab) cudaFree(c->slab);
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -219,8 +218,8 @@ fm_status fm_context_create(const fm_knobs* knobs, fm_context** out) {
     c->output = (uint32_t*)(c->slab + ((k.soln_prealloc_bytes + 255) & ~255ull));
     // control blocks hold 64-bit atomics: keep them 256-byte aligned whatever PREALLOC is
     set_misc(c.get(), c->slab + ((k.prealloc_bytes - kMiscBytes) & ~255ull));
-    FM_CUDA(cudaHostAlloc(&c->h_ctl, kMaxQ * sizeof(LaunchCtl), cudaHostAllocDefault));
-    FM_CUDA(cudaHostAlloc(&c->h_tot, sizeof(MatchTotals), cudaHostAllocDefault));
+    FM_CUDA(cudaHostAlloc(&c->h_ctl, sizeof(MatchCtl), cudaHostAllocDefault));
+    c->h_tot = &((MatchCtl*)c->h_ctl)->tot;
     FM_CUDA(cudaHostAlloc(&c->h_sched, sizeof(SchedState), cudaHostAllocDefault));
     FM_CUDA(cudaEventCreate(&c->ev0));
     FM_CUDA(cudaEventCreate(&c->ev1));
@@ -504,21 +503,27 @@ struct MatchRun {
         return (d == last_depth()) ? (table ? kModeLastTable : kModeLastCount) : kModeMid;
     }
 
+    // Control blocks and totals to the host, with one copy; ev1 ends the
+    // device window.
+    fm_status read_back() {
+        FM_CUDA(cudaEventRecord(ctx->ev1, s));
+        FM_CUDA(cudaMemcpyAsync(ctx->h_ctl, ctx->ctl, sizeof(MatchCtl), cudaMemcpyDeviceToHost, s));
+        FM_CUDA(cudaStreamSynchronize(s));
+        return FM_OK;
+    }
+
     // Pre-count: the last depth's work counters, which the counting level
     // added to the last depth's control block, and the counting level's
-    // survivors (its "produced" rows, never stored).
-    fm_status finish_pre() {
-        if (!pre) return FM_OK;
+    // survivors (its "produced" rows, never stored).  After read_back.
+    void finish_pre() {
+        if (!pre) return;
         const uint32_t q = plan->q;
-        FM_CUDA(cudaMemcpyAsync(ctx->h_ctl + q - 1, ctx->ctl + q - 1, sizeof(LaunchCtl), cudaMemcpyDeviceToHost, s));
-        FM_CUDA(cudaStreamSynchronize(s));
         const LaunchCtl& c = ctx->h_ctl[q - 1];
         fm_level_stats& ls = res->level[q - 1];
         ls.parents = c.parents;
         ls.lookups = c.lookups;
         ls.list_words = c.list_words;
         res->level[q - 2].produced = c.parents;
-        return FM_OK;
     }
     uint32_t* def_list(uint32_t d, int which) const {
         return ctx->defs + (size_t)(2 * d + which) * ctx->def_cap;
@@ -554,7 +559,6 @@ struct MatchRun {
         const uint32_t q = plan->q;
         const uint32_t last = last_depth();
         cudaEvent_t ev[kMaxQ][2] = {};
-        if (pre) FM_CUDA(cudaMemsetAsync(ctx->ctl + q - 1, 0, sizeof(LaunchCtl), s));
         for (uint32_t d = 1; d <= last; d++) {
             const int mode = mode_of(d);
             const bool roots = d == 1;
@@ -581,17 +585,15 @@ struct MatchRun {
             } else {
                 p.n_parents_dev = &ctx->ctl[d - 1].produced;
             }
-            FM_CUDA(cudaMemsetAsync(ctx->ctl + d, 0, sizeof(LaunchCtl), s));
             if (profile) FM_TRY(begin_timing(ev[d][0], ev[d][1]));
             if (sums && d == last) {
                 p.sum_rule = 1;
                 FM_CUDA(vertex_sums(p, p.n_parents_dev));
             }
-            FM_CUDA(launch_expand(p, mode, roots, dups, grid, full, block, smem, s));
+            FM_CUDA(launch_expand(p, mode, roots, dups, !roots, grid, full, block, smem, s));
             if (profile) FM_CUDA(cudaEventRecord(ev[d][1], s));
         }
-        FM_CUDA(cudaMemcpyAsync(ctx->h_ctl, ctx->ctl, q * sizeof(LaunchCtl), cudaMemcpyDeviceToHost, s));
-        FM_CUDA(cudaStreamSynchronize(s));
+        FM_TRY(read_back());
         uint64_t n_parents[kMaxQ] = {};
         for (uint32_t d = 1; d <= last; d++) {
             const LaunchCtl& c = ctx->h_ctl[d];
@@ -611,6 +613,7 @@ struct MatchRun {
         if (over_limit()) return FM_ERR_LIMIT;
         LaunchCtl snap[kMaxQ];
         std::memcpy(snap, ctx->h_ctl, q * sizeof(LaunchCtl));
+        bool drained = false;
         for (uint32_t d = last; d >= 1; d--) {
             if (mode_of(d) != kModeMid) continue;   // the last level never defers
             const LaunchCtl& c = snap[d];
@@ -619,10 +622,13 @@ struct MatchRun {
             if (c.ndef == 0 && claimed == items) continue;
             // every chunk claimed in the optimistic pass was fresh and was either
             // processed or deferred (its id is in the pass's def_out list)
+            drained = true;
             fm_status st = drain_level(d, n_parents[d], d == 1, c.ndef, claimed, def_list(d, 1), def_list(d, 0));
             if (st != FM_OK) return st;
         }
-        return finish_pre();
+        if (drained) FM_TRY(read_back());
+        finish_pre();
+        return FM_OK;
     }
 
     // Persistent engine: one cooperative launch runs every pass; the device
@@ -640,7 +646,6 @@ struct MatchRun {
         const unsigned long long wait_ns =
             (unsigned long long)(opts.wait_limit_ms ? opts.wait_limit_ms : 60000u) * 1000000ull;
         FM_CUDA(launch_sched_init(ctx->sched, q, n_roots, work_limit, wait_ns, s));
-        FM_CUDA(cudaMemsetAsync(ctx->ctl, 0, q * sizeof(LaunchCtl), s));
         PersistArgs a;
         std::memset(&a, 0, sizeof(a));
         a.sched = ctx->sched;
@@ -655,7 +660,7 @@ struct MatchRun {
         p.ctl = ctx->ctl;
         FM_CUDA(launch_persist(p, a, last_mode, dups, grid, smem, s));
         FM_CUDA(cudaMemcpyAsync(&h, ctx->sched, sizeof(h), cudaMemcpyDeviceToHost, s));
-        FM_CUDA(cudaStreamSynchronize(s));
+        FM_TRY(read_back());
         for (uint32_t d = 1; d < q; d++) {
             fm_level_stats& ls = res->level[d];
             ls.parents += h.lv[d].parents;
@@ -684,7 +689,8 @@ struct MatchRun {
             return FM_ERR_POOL;
         }
         if (h.error & kSchedErrLimit) return FM_ERR_LIMIT;
-        return finish_pre();
+        finish_pre();
+        return FM_OK;
     }
 
     // Host-driven depth-first loop for one level (used when a level's buffer
@@ -730,7 +736,7 @@ struct MatchRun {
                 }
                 p.sum_rule = sums_ready ? 2 : 0;
             }
-            FM_CUDA(launch_expand(p, mode, roots, dups, grid, ctx->sms * per_sm, block, smem, s));
+            FM_CUDA(launch_expand(p, mode, roots, dups, false, grid, ctx->sms * per_sm, block, smem, s));
             if (profile) FM_CUDA(cudaEventRecord(e1, s));
             FM_CUDA(cudaMemcpyAsync(ctx->h_ctl + d, ctx->ctl + d, sizeof(LaunchCtl), cudaMemcpyDeviceToHost, s));
             FM_CUDA(cudaStreamSynchronize(s));
@@ -875,9 +881,9 @@ fm_status match_impl(fm_context* ctx, const fm_graph* graph, const fm_query* que
         return FM_ERR_UNSUPPORTED;
     }
 
-    FM_CUDA(cudaMemsetAsync(ctx->tot, 0, sizeof(MatchTotals), s));
+    FM_CUDA(cudaMemsetAsync(ctx->ctl, 0, sizeof(MatchCtl), s));
     FM_CUDA(cudaEventRecord(ctx->ev0, s));
-    bool limited = false;
+    bool limited = false, launched = false;
     if (q == 1) {
         uint64_t n = re - rb;
         if (table && n) {
@@ -979,6 +985,7 @@ fm_status match_impl(fm_context* ctx, const fm_graph* graph, const fm_query* que
         b.tot = ctx->tot;
         b.heavy = ctx->heavy;
         b.heavy_cap = ctx->heavy_cap;
+        b.max_list = g.max_len;
         b.work_limit = opts.work_limit;
         b.stage_words = stage_words_knob();
         b.pre_count = run.pre ? 1u : 0u;
@@ -992,12 +999,19 @@ fm_status match_impl(fm_context* ctx, const fm_graph* graph, const fm_query* que
             if (st != FM_ERR_UNSUPPORTED) out->engine = FM_ENGINE_PERSISTENT;
         }
         if (st == FM_ERR_UNSUPPORTED) st = run.run(n_roots);
-        if (st == FM_ERR_LIMIT) limited = true;
-        else if (st != FM_OK) return st;
+        launched = true;                        // the totals are on the host
+        if (st == FM_ERR_LIMIT) {
+            limited = true;
+            FM_TRY(run.read_back());            // a drain may have counted since
+        } else if (st != FM_OK) {
+            return st;
+        }
     }
-    FM_CUDA(cudaEventRecord(ctx->ev1, s));
-    FM_CUDA(cudaMemcpyAsync(ctx->h_tot, ctx->tot, sizeof(MatchTotals), cudaMemcpyDeviceToHost, s));
-    FM_CUDA(cudaStreamSynchronize(s));
+    if (!launched) {
+        std::memset(ctx->h_tot, 0, sizeof(MatchTotals));
+        FM_CUDA(cudaEventRecord(ctx->ev1, s));
+        FM_CUDA(cudaStreamSynchronize(s));
+    }
     float ms = 0;
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
     out->device_ms = ms;
@@ -1055,8 +1069,8 @@ fm_status fm::context_create_view(fm_context* owner, char* misc, fm_context** ou
     FM_CUDA(cudaSetDevice(c->device));
     FM_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     set_misc(c.get(), misc);
-    FM_CUDA(cudaHostAlloc(&c->h_ctl, kMaxQ * sizeof(LaunchCtl), cudaHostAllocDefault));
-    FM_CUDA(cudaHostAlloc(&c->h_tot, sizeof(MatchTotals), cudaHostAllocDefault));
+    FM_CUDA(cudaHostAlloc(&c->h_ctl, sizeof(MatchCtl), cudaHostAllocDefault));
+    c->h_tot = &((MatchCtl*)c->h_ctl)->tot;
     FM_CUDA(cudaHostAlloc(&c->h_sched, sizeof(SchedState), cudaHostAllocDefault));
     FM_CUDA(cudaEventCreate(&c->ev0));
     FM_CUDA(cudaEventCreate(&c->ev1));

@@ -145,6 +145,13 @@ struct MatchTotals {
     unsigned int pad[3];
 };
 
+// What one match clears and reads back: one control block per depth and the
+// totals, together.
+struct MatchCtl {
+    LaunchCtl level[kMaxQ];
+    MatchTotals tot;
+};
+
 enum KernelMode { kModeMid = 0, kModeLastTable = 1, kModeLastCount = 2 };
 
 struct ExpandParams {
@@ -194,6 +201,7 @@ struct ExpandParams {
     HeavyEntry* heavy;
     uint32_t heavy_cap;             // entries; chunks are published only while room remains
     uint32_t max_warps;             // warps of the heavy pass (bounds concurrent publishers)
+    uint32_t max_list;              // the graph's longest list
     // last level: stop once the count (or reserved table rows) exceeds this,
     // setting bit kLimitFlag in tot->error; 0 = no limit
     unsigned long long work_limit;
@@ -286,8 +294,13 @@ cudaError_t launch_sched_init(SchedState* S, unsigned q, unsigned long long n_ro
 
 // Launch one level expansion: the main pass, then the heavy-chunk pass
 // (fm_match.cu).
-cudaError_t launch_expand(const ExpandParams& p, int mode, bool roots, bool dups, int grid, int heavy_grid,
-                          int block, size_t smem, cudaStream_t s);
+// `overlap`: the pass may start while the launch before it drains.
+cudaError_t launch_expand(const ExpandParams& p, int mode, bool roots, bool dups, bool overlap, int grid,
+                          int heavy_grid, int block, size_t smem, cudaStream_t s);
+cudaError_t launch_pass(const void* f, int grid, int block, size_t smem, void** args, bool overlap, cudaStream_t s);
+// Resident blocks per SM of kernel f (0: does not fit), asked of the driver
+// once per kernel and shared memory size.
+int blocks_per_sm(const void* f, int block, size_t smem);
 // `staged`: the level writes survivors (a middle or a table level).
 size_t expand_smem_bytes(uint32_t depth, uint32_t nreq, int warps, uint32_t stage_words, bool staged);
 // Vertex sums of pre-count by sums for the lists of `label` (n root-list

@@ -37,8 +37,10 @@
 // relaunches this level on the deferred chunks plus the unclaimed remainder.
 // Nothing spins and nothing traps.
 #include <algorithm>
+#include <map>
 #include <mutex>
 #include <set>
+#include <tuple>
 #include <utility>
 
 #include "fm_device.cuh"
@@ -62,6 +64,9 @@ __host__ __device__ constexpr uint32_t stage_rows(uint32_t k) { return k == 1 ? 
 constexpr uint32_t kSlots = 2;             // candidate slots per lane per round
 constexpr uint32_t kPend = 32 * kSlots + 32;  // candidates that wait for their exact test, per warp
 constexpr uint32_t kHeavyMaxPieces = 65536;
+// A level none of whose chunks can have more candidates than this (32 parents
+// with the graph's longest list) has no heavy pass.
+constexpr uint32_t kHeavyLeast = 512;
 
 // Rank of position t within its run of equal values.
 __device__ __forceinline__ uint32_t seg_rank(const uint4& s, uint32_t t, uint32_t x, const uint32_t* __restrict__ nbr) {
@@ -104,6 +109,7 @@ __device__ __forceinline__ Tune make_tune(const ExpandParams& P, bool main_pass)
     const unsigned long long cb = P.ocap / (4 * all_warps);
     t.credit_block = (uint32_t)(cb < 1024 ? cb : 1024);
     t.heavy_thresh = t.n_items >= 4 * all_warps ? 4096u : (t.n_items >= all_warps ? 1024u : 256u);
+    if (32ull * P.max_list <= kHeavyLeast) t.heavy_thresh = 0xffffffffu;   // there is no heavy pass
     t.heavy_piece = t.heavy_thresh / 2;
     return t;
 }
@@ -111,6 +117,11 @@ __device__ __forceinline__ Tune make_tune(const ExpandParams& P, bool main_pass)
 __device__ __forceinline__ uint32_t item_chunk(const ExpandParams& P, unsigned long long item) {
     return item < P.ndef_in ? P.def_in[(P.def_in_pos + item) % P.def_cap]
                             : (uint32_t)(P.fresh_base + (item - P.ndef_in));
+}
+
+__device__ __forceinline__ HeavyEntry heavy_entry(const HeavyEntry* p) {
+    const uint4 v = __ldcg((const uint4*)p);
+    return {v.x, v.y, v.z, v.w};
 }
 
 __device__ __forceinline__ void defer_chunk(const ExpandParams& P, uint32_t chunk) {
@@ -228,7 +239,7 @@ __device__ __forceinline__ bool stage_lists(const ExpandParams& P, const WarpMem
 template <bool ROOTS>
 __device__ __forceinline__ uint32_t parent_col(const ExpandParams& P, uint32_t c, uint32_t p) {
     if (ROOTS) return P.root_list ? __ldg(P.root_list + p) : P.root_begin + p;
-    return __ldg(P.pin + c * P.pstride + p);
+    return __ldcg(P.pin + c * P.pstride + p);
 }
 
 // Column c of staged parent p: from the warp's copy of chunk `cur` in shared
@@ -304,7 +315,7 @@ __device__ __forceinline__ uint32_t load_chunk(const ExpandParams& P, const Warp
     if (ROOTS) {
         m.rows_s[lane] = !P.root_list ? P.root_begin + (uint32_t)p : valid ? __ldg(P.root_list + p) : 0u;
     } else {
-        for (uint32_t c = 0; c < d; c++) m.rows_s[c * 32 + lane] = valid ? P.pin[c * P.pstride + p] : 0u;
+        for (uint32_t c = 0; c < d; c++) m.rows_s[c * 32 + lane] = valid ? __ldcg(P.pin + c * P.pstride + p) : 0u;
     }
     uint32_t drv = 0;
     n = 0;
@@ -735,10 +746,10 @@ __device__ __forceinline__ void expand_heavy(const ExpandParams& P, unsigned cha
         uint32_t lo = 0, hi = nent;      // last entry with piece0 <= gp
         while (hi - lo > 1) {
             const uint32_t mid = (lo + hi) >> 1;
-            if (P.heavy[mid].piece0 <= gp) lo = mid;
+            if (__ldcg(&P.heavy[mid].piece0) <= gp) lo = mid;
             else hi = mid;
         }
-        const HeavyEntry e = P.heavy[lo];
+        const HeavyEntry e = heavy_entry(P.heavy + lo);
         const uint32_t begin = ((uint32_t)gp - e.piece0) * T.heavy_piece;
         const uint32_t end = min(begin + T.heavy_piece, e.total);
         bool valid, stage_ok;
@@ -884,7 +895,7 @@ __device__ __forceinline__ bool sum_load(const ExpandParams& P, const WarpMem& m
                                          uint32_t lane, uint32_t d, unsigned long long n_parents) {
     const uint64_t p = (uint64_t)chunk * 32 + lane;
     const bool valid = p < n_parents;
-    for (uint32_t c = 0; c < d; c++) m.rows_s[c * 32 + lane] = valid ? P.pin[c * P.pstride + p] : 0u;
+    for (uint32_t c = 0; c < d; c++) m.rows_s[c * 32 + lane] = valid ? __ldcg(P.pin + c * P.pstride + p) : 0u;
     m.segs_s[lane] = valid ? ldg4(sp.seg + m.rows_s[sp.anc * 32 + lane]) : make_uint4(0, 0, 0, 0);
     return valid;
 }
@@ -923,7 +934,7 @@ __device__ __forceinline__ void expand_sum_main(const ExpandParams& P, unsigned 
                 const unsigned long long free_a = a.x - __popc(in_a);
                 pre.parents += free_a;
                 if (chain) {
-                    const uint2 w = __ldg(P.vsum + va);
+                    const uint2 w = __ldcg(P.vsum + va);
                     unsigned long long words = w.x, c = (unsigned long long)w.x - w.y;
                     if (in_a) {
                         const uint4 own = ldg4(sp.last + va);
@@ -945,7 +956,7 @@ __device__ __forceinline__ void expand_sum_main(const ExpandParams& P, unsigned 
                     n_count += free_a * (b.x - __popc(in_b));
                     pre.words += free_a * b.x;
                     if (sp.same) n_count -= free_a;
-                    else if (sp.last_anc == sp.anc) n_count -= __ldg(&P.vsum[va].y) - __popc(in_a & in_b);
+                    else if (sp.last_anc == sp.anc) n_count -= __ldcg(&P.vsum[va].y) - __popc(in_a & in_b);
                 }
             }
             for (uint32_t u = 0; u < d; u++) {
@@ -1013,10 +1024,10 @@ __device__ __forceinline__ void expand_sum_heavy(const ExpandParams& P, unsigned
         uint32_t lo = 0, hi = nent;      // last entry with piece0 <= gp
         while (hi - lo > 1) {
             const uint32_t mid = (lo + hi) >> 1;
-            if (P.heavy[mid].piece0 <= gp) lo = mid;
+            if (__ldcg(&P.heavy[mid].piece0) <= gp) lo = mid;
             else hi = mid;
         }
-        const HeavyEntry e = P.heavy[lo];
+        const HeavyEntry e = heavy_entry(P.heavy + lo);
         const uint32_t begin = ((uint32_t)gp - e.piece0) * T.heavy_piece;
         const uint32_t end = min(begin + T.heavy_piece, e.total);
         sum_load(P, m, sp, e.chunk, lane, d, T.n_parents);
@@ -1042,6 +1053,8 @@ __global__ void __launch_bounds__(kWarps * 32) k_vertex_sums(const __grid_consta
     __shared__ uint2 start_s[kWarps][32];
     __shared__ uint32_t sum_s[kWarps][32], both_s[kWarps][32], v_s[kWarps][32];
     __shared__ uint32_t long_s[kWarps * 32], n_long, lsum, lboth;
+    dev::pass_begin();
+    dev::pass_wait();
     if (parents && !sum_rule_on(P, *(const volatile unsigned long long*)parents)) return;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint4* seg = P.seg + (uint64_t)label * P.V;
@@ -1113,9 +1126,11 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_expand(const __grid_constant
     __shared__ uint8_t col_depth_s[kMaxQ];
     __shared__ uint64_t mbar_s[kWarps];
     __shared__ LevelLists L;
+    dev::pass_begin();
     level_lists_init(P, L, P.depth);
     if (threadIdx.x < (unsigned)kMaxQ) col_depth_s[threadIdx.x] = P.plan.col_depth[threadIdx.x];
     dev::stage_barriers_init(mbar_s);
+    dev::pass_wait();
     if (MODE == kModeLastCount && !ROOTS && !DUPS && P.sum_rule && sum_rule_on(P, make_tune(P, true).n_parents)) {
         expand_sum_main(P, smem_raw, mbar_s);
         return;
@@ -1130,9 +1145,11 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_expand_heavy(const __grid_co
     __shared__ uint8_t col_depth_s[kMaxQ];
     __shared__ uint64_t mbar_s[kWarps];
     __shared__ LevelLists L;
+    dev::pass_begin();
     level_lists_init(P, L, P.depth);
     if (threadIdx.x < (unsigned)kMaxQ) col_depth_s[threadIdx.x] = P.plan.col_depth[threadIdx.x];
     dev::stage_barriers_init(mbar_s);
+    dev::pass_wait();
     if (MODE == kModeLastCount && !ROOTS && !DUPS && P.sum_rule && sum_rule_on(P, make_tune(P, false).n_parents)) {
         expand_sum_heavy(P, smem_raw, mbar_s);
         return;
@@ -1299,12 +1316,7 @@ size_t persist_smem_bytes(const DevPlan& plan, const uint32_t* nreq_depth, uint3
 int persist_blocks_per_sm(int last_mode, bool dups, size_t smem) {
     void* f = persist_ptr(last_mode, dups);
     allow_dynamic_smem(f);
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, kWarps * 32, smem) != cudaSuccess) {
-        cudaGetLastError();
-        n = 0;
-    }
-    return n;
+    return blocks_per_sm(f, kWarps * 32, smem);
 }
 
 cudaError_t launch_persist(const ExpandParams& p, const PersistArgs& a, int last_mode, bool dups, int grid,
@@ -1326,12 +1338,28 @@ cudaError_t launch_persist(const ExpandParams& p, const PersistArgs& a, int last
     return cudaLaunchKernelExC(&cfg, persist_ptr(last_mode, dups), args);
 }
 
+// One launch; `overlap`: may start while the launch before it drains (see
+// dev::pass_wait).
+cudaError_t launch_pass(const void* f, int grid, int block, size_t smem, void** args, bool overlap, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelExC(&cfg, f, args);
+}
+
 cudaError_t launch_vertex_sums(const ExpandParams& p, const uint32_t* heads, uint32_t n, uint32_t label,
                                uint32_t last_label, uint2* vsum, const unsigned long long* parents, cudaStream_t s) {
     if (!n) return cudaSuccess;
-    k_vertex_sums<<<(n + kWarps * 32 - 1) / (kWarps * 32), kWarps * 32, 0, s>>>(p, heads, n, label, last_label, vsum,
-                                                                               parents);
-    return cudaGetLastError();
+    void* args[] = {(void*)&p, (void*)&heads, (void*)&n, (void*)&label, (void*)&last_label, (void*)&vsum, (void*)&parents};
+    return launch_pass((const void*)&k_vertex_sums, (int)((n + kWarps * 32 - 1) / (kWarps * 32)), kWarps * 32, 0, args,
+                       parents != nullptr, s);
 }
 
 size_t expand_smem_bytes(uint32_t depth, uint32_t nreq, int warps, uint32_t stage_words, bool staged) {
@@ -1360,17 +1388,32 @@ void allow_dynamic_smem(const void* f) {
         cudaGetLastError();   // the launch reports a size it cannot take
 }
 
+int blocks_per_sm(const void* f, int block, size_t smem) {
+    static std::mutex mu;
+    static std::map<std::tuple<int, const void*, int, size_t>, int> known;   // kernels x shared memory sizes
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = known.find({dev, f, block, smem});
+    if (it != known.end()) return it->second;
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, block, smem) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    known[{dev, f, block, smem}] = n;
+    return n;
+}
+
 int expand_blocks_per_sm(int mode, bool roots, bool dups, size_t smem, int block) {
     void* f = pick(mode, roots, dups, false);
     allow_dynamic_smem(f);
     allow_dynamic_smem(pick(mode, roots, dups, true));
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, block, smem) != cudaSuccess || n < 1) n = 1;
-    return n;
+    return std::max(1, blocks_per_sm(f, block, smem));
 }
 
-cudaError_t launch_expand(const ExpandParams& p, int mode, bool roots, bool dups, int grid, int heavy_grid,
-                          int block, size_t smem, cudaStream_t s) {
+cudaError_t launch_expand(const ExpandParams& p, int mode, bool roots, bool dups, bool overlap, int grid,
+                          int heavy_grid, int block, size_t smem, cudaStream_t s) {
     void* f = pick(mode, roots, dups, false);
     void* fh = pick(mode, roots, dups, true);
     if (!f || !fh) return cudaErrorInvalidValue;
@@ -1379,10 +1422,10 @@ cudaError_t launch_expand(const ExpandParams& p, int mode, bool roots, bool dups
     // and from max_warps, the warps of the heavy pass
     q.max_warps = (uint32_t)heavy_grid * (uint32_t)(block / 32);
     void* args[] = {(void*)&q};
-    cudaError_t e = cudaLaunchKernel(f, dim3(grid), dim3(block), args, smem, s);
-    if (e != cudaSuccess) return e;
+    cudaError_t e = launch_pass(f, grid, block, smem, args, overlap, s);
+    if (e != cudaSuccess || 32ull * p.max_list <= kHeavyLeast) return e;
     // the heavy pass always gets a full grid: a few heavy chunks can hold most of the work
-    return cudaLaunchKernel(fh, dim3(heavy_grid), dim3(block), args, smem, s);
+    return launch_pass(fh, heavy_grid, block, smem, args, overlap, s);
 }
 
 }  // namespace fm

@@ -119,7 +119,7 @@ struct StaticRun {
             int grid = (int)std::min<uint64_t>(want, (uint64_t)full);
             if (grid < 1) grid = 1;
             FM_CUDA(cudaMemsetAsync(ctl, 0, sizeof(LaunchCtl), s));
-            FM_CUDA(launch_expand(p, mode, roots, dups, grid, full, block, smem, s));
+            FM_CUDA(launch_expand(p, mode, roots, dups, false, grid, full, block, smem, s));
             LaunchCtl c;
             FM_CUDA(cudaMemcpyAsync(&c, ctl, sizeof(LaunchCtl), cudaMemcpyDeviceToHost, s));
             FM_CUDA(cudaStreamSynchronize(s));
@@ -276,6 +276,7 @@ extern "C" fm_status fm_match_static(const fm_graph* graph, const fm_query* quer
     b.tot = tot;
     b.heavy = heavy;
     b.heavy_cap = kStaticHeavyCap;
+    b.max_list = g.max_len;
     // the totals must start at zero: the scratch keeps the previous call's contents
     FM_CUDA(cudaMemsetAsync(tot, 0, sizeof(MatchTotals), s));
     st = run.level_pass(1, g.V, true);

@@ -23,7 +23,8 @@ def ctx():
     c.close()
 
 
-@pytest.mark.parametrize("n", [3, 4, 31, 32, 33, 34, 65])
+# 17 and 18: the longest list (16, 17) without and with a heavy pass
+@pytest.mark.parametrize("n", [3, 4, 17, 18, 31, 32, 33, 34, 65])
 def test_every_candidate_passes(ctx, n):
     V, s, d, l = complete_graph(n)
     g = fm.Graph.from_edges(ctx, V, 2, s, d, l)
