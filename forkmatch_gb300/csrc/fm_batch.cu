@@ -45,6 +45,10 @@ struct BatchParams {
     const uint32_t* nbr;
     const uint32_t* bm;                       // list bitmaps (see DeviceGraph)
     uint32_t bm_words;
+    const uint32_t* efilter;                  // e-line filter and its slices by label (see DeviceGraph)
+    const uint32_t* efilter_off;
+    uint32_t L;                               // label slots
+    uint32_t max_list;                        // the graph's longest list
     uint32_t V;
     // parents: columns 0..d-1, query id in column d (null at depth 1: roots)
     const uint32_t* pin;
@@ -90,9 +94,11 @@ using dev::seg_has;
 using dev::SlotWalk;
 
 constexpr int kBWarps = 8;
-constexpr uint32_t kBStage = 128;
+constexpr uint32_t kBStage = 96;
 constexpr uint32_t kBSlots = 2;            // candidate slots per lane per round
+constexpr uint32_t kBPend = 32 * kBSlots + 32;   // candidates that wait for their exact test
 constexpr uint32_t kHeavyMaxPieces = 65536;
+constexpr uint32_t kBHeavyLeast = 512;     // no chunk above this many candidates: no heavy pass
 
 struct BTune {
     unsigned long long n_parents, n_items;
@@ -114,7 +120,7 @@ __device__ __forceinline__ BTune make_btune(const BatchParams& P) {
     t.credit_block = (uint32_t)(cb < 1024 ? cb : 1024);
     const uint32_t base = t.n_items >= 4 * all_warps ? 2048u : (t.n_items >= all_warps ? 512u : 128u);
     t.heavy_piece = base << P.piece_shift;
-    t.heavy_thresh = 2 * t.heavy_piece;
+    t.heavy_thresh = 32ull * P.max_list <= kBHeavyLeast ? 0xffffffffu : 2 * t.heavy_piece;
     // roots cost about the same per chunk: big batches; deeper chunks vary:
     // small batches keep the warps balanced
     const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x / 32);
@@ -124,25 +130,32 @@ __device__ __forceinline__ BTune make_btune(const BatchParams& P) {
 }
 
 // Per-warp shared memory: rows, records, drivers, per-parent query data, stage.
+// Kept small: what blocks do not take of an SM's 256 KB is its L1.
 struct BMem {
     uint32_t* rows_s;   // [d][32]
-    uint4* segs_s;      // [kmax][32]
+    uint4* segs_s;      // [brecs][32] the driver's record, or all (list stage)
+    uint16_t* ref_s;    // [kmax][32] column and label << 8 of each back edge
     uint2* start_s;     // [32] parents with candidates: first slot, lane (dev::SlotWalk)
-    uint32_t* drv_s;    // [32]
-    uint32_t* k_s;      // [32] requirements of the parent's query at this depth
     uint32_t* qid_s;    // [32]
-    uint32_t* pidx_s;   // [32] parent index in the level (root vertex at depth 1)
-    uint32_t* fin_s;    // [32] 1: the parent's query ends at this depth; 2: it is pre-counted here
+    uint8_t* drv_s;     // [32]
+    uint8_t* k_s;       // [32] requirements of the parent's query at this depth
+    uint8_t* fin_s;     // [32] 1: the parent's query ends at this depth; 2: it is pre-counted here
     uint32_t* stp;      // [kBStage] staged parent index
     uint32_t* stx;      // [kBStage] staged vertex
     uint32_t* stq;      // [kBStage] staged query id
+    uint32_t* px;       // [kBPend] candidates the filter let pass: vertex
+    uint8_t* pj;        // [kBPend] and parent (lane) in the chunk
     uint64_t* mbar;     // completion barrier of the list stage's bulk copies
     uint32_t* stage;    // [stage_words] membership lists copied in by TMA (optional)
 };
 
+// Records kept per parent (see n_recs of the single-query kernel).
+__host__ __device__ constexpr uint32_t brecs(uint32_t kmax, uint32_t stage_words) { return stage_words ? kmax : 1; }
+
 __host__ __device__ constexpr uint32_t bper_warp_bytes(uint32_t d, uint32_t kmax, uint32_t stage_words = 0) {
-    return 128 * d + 512 * kmax + 7 * 128 + 12 * kBStage + 4 * stage_words;
+    return 128 * d + 512 * brecs(kmax, stage_words) + 64 * kmax + 256 + 128 + 96 + 12 * kBStage + 5 * kBPend + 4 * stage_words;
 }
+static_assert((96 + 12 * kBStage + 5 * kBPend) % 16 == 0, "the list stage is 16-byte aligned");
 
 __device__ __forceinline__ BMem bmem(unsigned char* smem, uint32_t warp, uint32_t d, uint32_t kmax,
                                      uint32_t stage_words, uint64_t* mbar_s) {
@@ -150,19 +163,37 @@ __device__ __forceinline__ BMem bmem(unsigned char* smem, uint32_t warp, uint32_
     BMem m;
     m.rows_s = (uint32_t*)w;
     m.segs_s = (uint4*)(w + 128 * d);
-    uint32_t* s = (uint32_t*)(w + 128 * d + 512 * kmax);
-    m.start_s = (uint2*)s;
-    m.drv_s = s + 64;
-    m.k_s = s + 96;
-    m.qid_s = s + 128;
-    m.pidx_s = s + 160;
-    m.fin_s = s + 192;
-    m.stp = s + 224;
+    m.ref_s = (uint16_t*)(m.segs_s + 32 * brecs(kmax, stage_words));
+    m.start_s = (uint2*)(m.ref_s + 32 * kmax);
+    m.qid_s = (uint32_t*)(m.start_s + 32);
+    m.drv_s = (uint8_t*)(m.qid_s + 32);
+    m.k_s = m.drv_s + 32;
+    m.fin_s = m.k_s + 32;
+    m.stp = (uint32_t*)(m.fin_s + 32);
     m.stx = m.stp + kBStage;
     m.stq = m.stx + kBStage;
+    m.px = m.stq + kBStage;
+    m.pj = (uint8_t*)(m.px + kBPend);
     m.mbar = mbar_s + warp;
-    m.stage = (uint32_t*)(w + 128 * d + 512 * kmax + 7 * 128 + 12 * kBStage);
+    m.stage = (uint32_t*)(m.pj + kBPend);
     return m;
+}
+
+// Filter slices of every label, one copy per block (after the warps' memory).
+struct BSlices {
+    const uint2* s;                  // first word, words
+    __device__ __forceinline__ dev::FilterSlice at(const BatchParams& P, uint32_t label) const {
+        return {P.efilter + s[label].x, s[label].y};
+    }
+};
+
+__device__ __forceinline__ BSlices bslices_init(const BatchParams& P, uint2* buf) {
+    for (uint32_t l = threadIdx.x; l < P.L; l += blockDim.x) {
+        const uint32_t a = __ldg(P.efilter_off + l);
+        buf[l] = make_uint2(a, __ldg(P.efilter_off + l + 1) - a);
+    }
+    __syncthreads();
+    return {buf};
 }
 
 constexpr uint32_t kBStageMaxList = 2048;
@@ -228,20 +259,18 @@ __device__ __forceinline__ uint32_t bload_chunk(const BatchParams& P, const BMem
                                                 uint32_t d, unsigned long long n_parents, bool& valid,
                                                 uint32_t& k_out, unsigned long long& words, uint32_t sw,
                                                 uint32_t& phase, bool& stage_ok, unsigned long long& rule_cnt,
-                                                uint32_t& cont_total, uint32_t& excl, uint32_t& n) {
-    uint32_t qid, pidx;
+                                                uint32_t& cont_total, uint32_t& excl, uint32_t& n, const BSlices& S) {
+    uint32_t qid;
     if (ROOTS) {
         qid = chunk / P.chunks_per_query;
         const uint32_t r = (chunk - qid * P.chunks_per_query) * 32 + lane;
         valid = qid < P.nq && r < P.plans[qid].n_roots;
-        pidx = valid ? __ldg(P.heads + P.plans[qid].root_off + r) : 0u;   // the root vertex
-        m.rows_s[lane] = pidx;
+        m.rows_s[lane] = valid ? __ldg(P.heads + P.plans[qid].root_off + r) : 0u;   // the root vertex
     } else {
         const uint64_t p = (uint64_t)chunk * 32 + lane;
         valid = p < n_parents;
-        pidx = (uint32_t)p;
-        qid = valid ? __ldg(P.pin + (uint64_t)d * P.pstride + p) : 0u;
-        for (uint32_t c = 0; c < d; c++) m.rows_s[c * 32 + lane] = valid ? __ldg(P.pin + c * P.pstride + p) : 0u;
+        qid = valid ? __ldcg(P.pin + (uint64_t)d * P.pstride + p) : 0u;
+        for (uint32_t c = 0; c < d; c++) m.rows_s[c * 32 + lane] = valid ? __ldcg(P.pin + c * P.pstride + p) : 0u;
     }
     uint32_t drv = 0, k = 0, fin = 0;
     n = 0;
@@ -254,29 +283,32 @@ __device__ __forceinline__ uint32_t bload_chunk(const BatchParams& P, const BMem
         fin = (pl.q == d + 1) ? 1u : 0u;
         if (pl.q == d + 2 && pl.pre_ok && (!P.table_mode || pl.count_only)) fin = 2u;
         const uint32_t rb = pl.req_begin[d];
-        uint32_t best = 0xffffffffu;
+        uint4 best = make_uint4(0xffffffffu, 0, 0, 0);
         for (uint32_t i = 0; i < k; i++) {
             const uint32_t anc = pl.req_anc[rb + i];
             const uint32_t lab = pl.req_label[rb + i];
             const uint32_t v = m.rows_s[anc * 32 + lane];
             const uint4 sg = ldg4(P.seg + (uint64_t)lab * P.V + v);
-            m.segs_s[i * 32 + lane] = sg;
+            if (sw) m.segs_s[i * 32 + lane] = sg;
+            m.ref_s[i * 32 + lane] = (uint16_t)(anc | lab << 8);
             words += sg.x;
-            if (sg.x < best) {
-                best = sg.x;
+            if (sg.x < best.x) {
+                best = sg;
                 drv = i;
             }
         }
-        n = best;
-        if (k > 2) drv = dev::order_lists(m.segs_s, lane, k, drv);
+        n = best.x;
+        if (!sw) m.segs_s[lane] = best;
         if (fin == 1u && k == 1 && (!P.table_mode || pl.count_only)) {
             // Count rule (the query's count only): every entry of the single
             // list extends the parent except the parent's own vertices, so the
             // extensions are counted, not enumerated.  The caller adds the
             // count once, when the main pass keeps the chunk (a chunk can be
             // loaded again after a deferral or for each heavy piece).
-            const uint4 sg = m.segs_s[lane];
-            rule_cnt = sg.x - dev::count_members(sg, m.rows_s, lane, d, 0u, false, P.nbr, P.bm, P.bm_words);
+            const uint4 sg = best;
+            const uint32_t ref = m.ref_s[lane];
+            rule_cnt = sg.x - dev::count_members_f(sg, S.at(P, ref >> 8), m.rows_s[(ref & 0xffu) * 32 + lane], m.rows_s,
+                                                   lane, d, 0u, false, P.nbr, P.bm, P.bm_words);
             n = 0;
         }
     }
@@ -290,11 +322,10 @@ __device__ __forceinline__ uint32_t bload_chunk(const BatchParams& P, const BMem
         if ((int)lane >= o) incl += t;
     }
     excl = incl - n;
-    m.drv_s[lane] = drv;
-    m.k_s[lane] = k;
+    m.drv_s[lane] = (uint8_t)drv;
+    m.k_s[lane] = (uint8_t)k;
     m.qid_s[lane] = qid;
-    m.pidx_s[lane] = pidx;
-    m.fin_s[lane] = fin;
+    m.fin_s[lane] = (uint8_t)fin;
     // candidate slots of the parents whose query goes on past this depth: the
     // only ones whose survivors can take rows of the next level
     cont_total = __reduce_add_sync(kFull, fin == 0u ? n : 0u);
@@ -314,7 +345,7 @@ __device__ __forceinline__ void bflush(const BatchParams& P, const BMem& m, uint
         uint32_t* col = P.pout + c * P.ocap + pos0;
         for (uint32_t i = lane; i < nst; i += 32) {
             const uint32_t p = m.stp[i];
-            col[i] = ROOTS ? p : ((p >> 5) == cur ? m.rows_s[c * 32 + (p & 31)] : __ldg(P.pin + c * P.pstride + p));
+            col[i] = ROOTS ? p : ((p >> 5) == cur ? m.rows_s[c * 32 + (p & 31)] : __ldcg(P.pin + c * P.pstride + p));
         }
     }
     uint32_t* colx = P.pout + d * P.ocap + pos0;
@@ -351,8 +382,8 @@ __device__ __forceinline__ void bfinal(const BatchParams& P, const BMem& m, bool
 // A survivor counted by pre-count (its query's last depth has one back edge):
 // its extensions are the entries of that list minus the row's vertices (the
 // parent's and x) found in it.  Lanes of the same query share one atomic.
-__device__ __forceinline__ void bprecount(const BatchParams& P, const BMem& m, bool pre, uint32_t j, uint32_t x,
-                                          uint32_t lane, uint32_t d) {
+__device__ __forceinline__ void bprecount(const BatchParams& P, const BMem& m, const BSlices& S, bool pre, uint32_t j,
+                                          uint32_t x, uint32_t lane, uint32_t d) {
     if (!__ballot_sync(kFull, pre)) return;
     uint32_t c = 0, qid = 0xffffffffu;
     if (pre) {
@@ -360,8 +391,10 @@ __device__ __forceinline__ void bprecount(const BatchParams& P, const BMem& m, b
         const BatchPlan& pl = P.plans[qid];
         const uint32_t rb = pl.req_begin[d + 1];
         const uint32_t anc = pl.req_anc[rb];
-        const uint4 sg = ldg4(P.seg + (uint64_t)pl.req_label[rb] * P.V + (anc == d ? x : m.rows_s[anc * 32 + j]));
-        c = sg.x - dev::count_members(sg, m.rows_s, j, d, x, P.self_loops || anc != d, P.nbr, P.bm, P.bm_words);
+        const uint32_t lab = pl.req_label[rb], v = anc == d ? x : m.rows_s[anc * 32 + j];
+        const uint4 sg = ldg4(P.seg + (uint64_t)lab * P.V + v);
+        c = sg.x - dev::count_members_f(sg, S.at(P, lab), v, m.rows_s, j, d, x, P.self_loops || anc != d, P.nbr, P.bm,
+                                        P.bm_words);
     }
     const unsigned grp = __match_any_sync(kFull, qid);
     const unsigned lo = __reduce_add_sync(grp, c & 0xffffu);
@@ -370,58 +403,107 @@ __device__ __forceinline__ void bprecount(const BatchParams& P, const BMem& m, b
         atomicAdd(&P.qpos[qid], ((unsigned long long)hi << 16) + lo);
 }
 
-// Evaluate slots [begin, end) of the loaded chunk, kBSlots per lane per round
-// with every driver load of the round issued before any check (as in the
-// single-query kernel); each slot's survivor is then counted or written
-// (its query ends here), pre-counted, or staged for the next level.
+// What survives a warp round: each survivor is counted or written (its query
+// ends here), pre-counted, or staged for the next level.
 template <bool ROOTS>
-__device__ __forceinline__ void bprocess(const BatchParams& P, const BMem& m, uint32_t chunk, uint32_t excl, uint32_t n,
-                                         uint32_t begin, uint32_t end, uint32_t lane, uint32_t d, uint32_t& nst) {
+__device__ __forceinline__ void bemit(const BatchParams& P, const BMem& m, const BSlices& S, uint32_t chunk, bool ok,
+                                      uint32_t j, uint32_t x, uint32_t lane, uint32_t d, uint32_t& nst) {
+    const uint32_t fs = ok ? m.fin_s[j] : 0u;
+    bfinal(P, m, fs == 1u, j, x, lane, d);
+    bprecount(P, m, S, fs == 2u, j, x, lane, d);
+    const bool stage = ok && fs == 0u;
+    const unsigned b = __ballot_sync(kFull, stage);
+    if (stage) {
+        const uint32_t q0 = nst + __popc(b & ((1u << lane) - 1u));
+        m.stp[q0] = ROOTS ? m.rows_s[j] : chunk * 32 + j;
+        m.stx[q0] = x;
+        m.stq[q0] = m.qid_s[j];
+    }
+    nst += __popc(b);
+    __syncwarp();
+    if (nst > kBStage - 32) {
+        bflush<ROOTS>(P, m, nst, lane, d, chunk);
+        nst = 0;
+        __syncwarp();
+    }
+}
+
+// Evaluate slots [begin, end) of the loaded chunk, kBSlots per lane per round
+// with every driver load of the round issued before any check; the filter
+// rejects, and what it lets pass is tested exactly 32 at a time (as in the
+// single-query kernel).  A chunk none of whose parents has a second back edge
+// goes straight on.
+template <bool ROOTS>
+__device__ __forceinline__ void bprocess(const BatchParams& P, const BMem& m, const BSlices& S, uint32_t chunk,
+                                         uint32_t excl, uint32_t n, uint32_t begin, uint32_t end, uint32_t lane,
+                                         uint32_t d, uint32_t sw, uint32_t& nst) {
     SlotWalk walk(m.start_s, excl, n, begin, lane);
+    const uint32_t kk = __reduce_max_sync(kFull, n ? m.k_s[lane] : 0u);
+    uint32_t pend = 0;
     for (uint32_t base = begin; base < end; base += 32 * kBSlots) {
-        uint32_t j[kBSlots], t[kBSlots], x[kBSlots];
+        uint32_t j[kBSlots], t[kBSlots], x[kBSlots], dj[kBSlots];
         bool ok[kBSlots];
 #pragma unroll
         for (uint32_t u = 0; u < kBSlots; u++) {
             walk.window(m.start_s, base + 32 * u, lane, j[u], t[u]);
-            x[u] = 0;
+            x[u] = dj[u] = 0;
             ok[u] = base + 32 * u + lane < end;
             if (ok[u]) {
-                x[u] = seg_at(m.segs_s[m.drv_s[j[u]] * 32 + j[u]], t[u], P.nbr);
+                dj[u] = m.drv_s[j[u]];
+                x[u] = seg_at(m.segs_s[(sw ? dj[u] * 32 : 0u) + j[u]], t[u], P.nbr);
+            }
+        }
+        if (kk == 1) {
+#pragma unroll
+            for (uint32_t u = 0; u < kBSlots; u++)
+                for (uint32_t c = 0; c < d && ok[u]; c++) ok[u] = m.rows_s[c * 32 + j[u]] != x[u];
+#pragma unroll
+            for (uint32_t u = 0; u < kBSlots; u++) bemit<ROOTS>(P, m, S, chunk, ok[u], j[u], x[u], lane, d, nst);
+            continue;
+        }
+        for (uint32_t i = 0; i < kk; i++) {
+#pragma unroll
+            for (uint32_t u = 0; u < kBSlots; u++) {
+                if (!ok[u] || dj[u] == i || i >= m.k_s[j[u]]) continue;
+                const uint32_t ref = m.ref_s[i * 32 + j[u]];
+                ok[u] = dev::filter_has(S.at(P, ref >> 8), dev::filter_seed(m.rows_s[(ref & 0xffu) * 32 + j[u]]), x[u]);
             }
         }
 #pragma unroll
         for (uint32_t u = 0; u < kBSlots; u++) {
-            if (!ok[u]) continue;
-            const uint32_t jj = j[u], dj = m.drv_s[jj], k = m.k_s[jj];
-            for (uint32_t i = 0; i < k && ok[u]; i++) {
-                if (i == dj) continue;
-                ok[u] = dev::seg_has_st(m.segs_s[i * 32 + jj], x[u], 1, P.nbr, P.bm, P.bm_words, m.stage);
+            const unsigned b = __ballot_sync(kFull, ok[u]);
+            if (ok[u]) {
+                const uint32_t q = pend + __popc(b & ((1u << lane) - 1u));
+                m.px[q] = x[u];
+                m.pj[q] = (uint8_t)j[u];
             }
-            for (uint32_t c = 0; c < d && ok[u]; c++) ok[u] = m.rows_s[c * 32 + jj] != x[u];
+            pend += __popc(b);
         }
-#pragma unroll
-        for (uint32_t u = 0; u < kBSlots; u++) {
-            const uint32_t fs = ok[u] ? m.fin_s[j[u]] : 0u;
-            bfinal(P, m, fs == 1u, j[u], x[u], lane, d);
-            bprecount(P, m, fs == 2u, j[u], x[u], lane, d);
-            const bool stage = ok[u] && fs == 0u;
-            const unsigned b = __ballot_sync(kFull, stage);
-            if (stage) {
-                const uint32_t q0 = nst + __popc(b & ((1u << lane) - 1u));
-                m.stp[q0] = m.pidx_s[j[u]];
-                m.stx[q0] = x[u];
-                m.stq[q0] = m.qid_s[j[u]];
-            }
-            nst += __popc(b);
-        }
-        if (nst > kBStage - 32 * kBSlots) {
+        const bool last = base + 32 * kBSlots >= end;
+        while (pend >= 32 || (last && pend)) {
+            const uint32_t take = min(pend, 32u);
+            pend -= take;
             __syncwarp();
-            bflush<ROOTS>(P, m, nst, lane, d, chunk);
-            nst = 0;
+            bool in = lane < take;
+            uint32_t jj = 0, xx = 0;
+            if (in) {
+                jj = m.pj[pend + lane];
+                xx = m.px[pend + lane];
+                const uint32_t dd = m.drv_s[jj], k = m.k_s[jj];
+                for (uint32_t i = 0; i < k && in; i++) {
+                    if (i == dd) continue;
+                    const uint32_t ref = m.ref_s[i * 32 + jj];
+                    const uint4 r = sw ? m.segs_s[i * 32 + jj]
+                                       : ldg4(P.seg + (uint64_t)(ref >> 8) * P.V + m.rows_s[(ref & 0xffu) * 32 + jj]);
+                    in = dev::seg_has_st(r, xx, 1, P.nbr, P.bm, P.bm_words, m.stage);
+                }
+                for (uint32_t c = 0; c < d && in; c++) in = m.rows_s[c * 32 + jj] != xx;
+            }
+            bemit<ROOTS>(P, m, S, chunk, in, jj, xx, lane, d, nst);
         }
         __syncwarp();
     }
+    __syncwarp();
 }
 
 __device__ __forceinline__ uint32_t bitem_chunk(const BatchParams& P, unsigned long long item) {
@@ -437,8 +519,8 @@ __device__ __forceinline__ void bdefer(const BatchParams& P, uint32_t chunk) {
 }
 
 template <bool ROOTS>
-__device__ __forceinline__ void bexpand_main(const BatchParams& P, unsigned char* smem_raw, uint64_t* mbar_s,
-                                             uint32_t& phase) {
+__device__ __forceinline__ void bexpand_main(const BatchParams& P, unsigned char* smem_raw, const BSlices& S,
+                                             uint64_t* mbar_s, uint32_t& phase) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t d = P.depth;
     const uint32_t sw = P.kmax >= 2 ? P.stage_words : 0;   // only levels with membership tests stage lists
@@ -470,7 +552,7 @@ __device__ __forceinline__ void bexpand_main(const BatchParams& P, unsigned char
             unsigned long long w, rule_cnt;
             uint32_t cont, excl, n;
             const uint32_t total = bload_chunk<ROOTS>(P, m, chunk, lane, d, T.n_parents, valid, k, w, sw, phase,
-                                                      stage_ok, rule_cnt, cont, excl, n);
+                                                      stage_ok, rule_cnt, cont, excl, n, S);
             last_chunk = chunk;
             if (!stage_ok) {
                 done = true;
@@ -533,7 +615,7 @@ __device__ __forceinline__ void bexpand_main(const BatchParams& P, unsigned char
                 pub = __shfl_sync(kFull, pub, 0);
                 if (pub) continue;
             }
-            bprocess<ROOTS>(P, m, chunk, excl, n, 0, total, lane, d, nst);
+            bprocess<ROOTS>(P, m, S, chunk, excl, n, 0, total, lane, d, sw, nst);
             // the stage refers to this chunk's query ids only through stq, and to
             // its parents through pidx: it can outlive the chunk
         }
@@ -553,8 +635,8 @@ __device__ __forceinline__ void bexpand_main(const BatchParams& P, unsigned char
 }
 
 template <bool ROOTS>
-__device__ __forceinline__ void bexpand_heavy(const BatchParams& P, unsigned char* smem_raw, uint64_t* mbar_s,
-                                              uint32_t& phase) {
+__device__ __forceinline__ void bexpand_heavy(const BatchParams& P, unsigned char* smem_raw, const BSlices& S,
+                                              uint64_t* mbar_s, uint32_t& phase) {
     const unsigned long long h = *(volatile unsigned long long*)&P.ctl->heavy;
     const uint32_t nent = (uint32_t)(h >> 32);
     const uint32_t npieces = (uint32_t)h;
@@ -574,10 +656,11 @@ __device__ __forceinline__ void bexpand_heavy(const BatchParams& P, unsigned cha
         uint32_t lo = 0, hi = nent;
         while (hi - lo > 1) {
             const uint32_t mid = (lo + hi) >> 1;
-            if (P.heavy[mid].piece0 <= gp) lo = mid;
+            if (__ldcg(&P.heavy[mid].piece0) <= gp) lo = mid;
             else hi = mid;
         }
-        const HeavyEntry e = P.heavy[lo];
+        const uint4 ev = __ldcg((const uint4*)(P.heavy + lo));
+        const HeavyEntry e = {ev.x, ev.y, ev.z, ev.w};
         const uint32_t begin = ((uint32_t)gp - e.piece0) * T.heavy_piece;
         const uint32_t end = min(begin + T.heavy_piece, e.total);
         bool valid, stage_ok;
@@ -585,10 +668,10 @@ __device__ __forceinline__ void bexpand_heavy(const BatchParams& P, unsigned cha
         unsigned long long w, rule_cnt;   // counted by the main pass
         uint32_t cont, excl, n;
         bload_chunk<ROOTS>(P, m, e.chunk, lane, d, T.n_parents, valid, k, w, sw, phase, stage_ok, rule_cnt, cont, excl,
-                           n);
+                           n, S);
         last_chunk = e.chunk;
         if (!stage_ok) break;
-        bprocess<ROOTS>(P, m, e.chunk, excl, n, begin, end, lane, d, nst);
+        bprocess<ROOTS>(P, m, S, e.chunk, excl, n, begin, end, lane, d, sw, nst);
     }
     if (nst) bflush<ROOTS>(P, m, nst, lane, d, last_chunk);
 }
@@ -597,18 +680,26 @@ template <bool ROOTS>
 __global__ void __launch_bounds__(kBWarps * 32, 6) k_bexpand(const __grid_constant__ BatchParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint64_t mbar_s[kBWarps];
+    __shared__ uint2 slices_s[FM_MAX_LABEL + 1];
+    dev::pass_begin();
+    const BSlices S = bslices_init(P, slices_s);
     dev::stage_barriers_init(mbar_s);
+    dev::pass_wait();
     uint32_t phase = 0;
-    bexpand_main<ROOTS>(P, smem_raw, mbar_s, phase);
+    bexpand_main<ROOTS>(P, smem_raw, S, mbar_s, phase);
 }
 
 template <bool ROOTS>
 __global__ void __launch_bounds__(kBWarps * 32, 6) k_bexpand_heavy(const __grid_constant__ BatchParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint64_t mbar_s[kBWarps];
+    __shared__ uint2 slices_s[FM_MAX_LABEL + 1];
+    dev::pass_begin();
+    const BSlices S = bslices_init(P, slices_s);
     dev::stage_barriers_init(mbar_s);
+    dev::pass_wait();
     uint32_t phase = 0;
-    bexpand_heavy<ROOTS>(P, smem_raw, mbar_s, phase);
+    bexpand_heavy<ROOTS>(P, smem_raw, S, mbar_s, phase);
 }
 
 // Persistent batch engine: one cooperative launch runs every level pass of
@@ -638,6 +729,8 @@ __global__ void __launch_bounds__(kBWarps * 32, 5) k_bpersist(const __grid_const
         uint32_t* dst = (uint32_t*)&P;
         for (uint32_t i = threadIdx.x; i < sizeof(BatchParams) / 4; i += blockDim.x) dst[i] = src[i];
     }
+    __shared__ uint2 slices_s[FM_MAX_LABEL + 1];
+    const BSlices SL = bslices_init(P0, slices_s);
     dev::stage_barriers_init(mbar_s);
     uint32_t phase = 0;       // of this warp's stage barrier, carried across passes
     bool first = true;
@@ -673,12 +766,12 @@ __global__ void __launch_bounds__(kBWarps * 32, 5) k_bpersist(const __grid_const
         __syncthreads();
         const unsigned d = cur_s;
         if (d == 0) break;
-        if (d == 1) bexpand_main<true>(P, smem_raw, mbar_s, phase);
-        else bexpand_main<false>(P, smem_raw, mbar_s, phase);
+        if (d == 1) bexpand_main<true>(P, smem_raw, SL, mbar_s, phase);
+        else bexpand_main<false>(P, smem_raw, SL, mbar_s, phase);
         if (!dev::grid_barrier(S, first && A.hold_first_barrier && blockIdx.x == 0, &flag_s)) break;
         first = false;
-        if (d == 1) bexpand_heavy<true>(P, smem_raw, mbar_s, phase);
-        else bexpand_heavy<false>(P, smem_raw, mbar_s, phase);
+        if (d == 1) bexpand_heavy<true>(P, smem_raw, SL, mbar_s, phase);
+        else bexpand_heavy<false>(P, smem_raw, SL, mbar_s, phase);
         if (!dev::grid_barrier(S, false, &flag_s)) break;
         if (blockIdx.x == 0 && threadIdx.x == 0)
             dev::sched_advance(S, P0.ctl, d, d + 1 < A.maxq, P.n_items, P.ndef_in, P.def_room, false);
@@ -688,13 +781,7 @@ __global__ void __launch_bounds__(kBWarps * 32, 5) k_bpersist(const __grid_const
 
 int bpersist_blocks_per_sm(size_t smem) {
     allow_dynamic_smem((const void*)&k_bpersist);
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, (const void*)&k_bpersist, kBWarps * 32, smem) !=
-        cudaSuccess) {
-        cudaGetLastError();
-        n = 0;
-    }
-    return n;
+    return blocks_per_sm((const void*)&k_bpersist, kBWarps * 32, smem);
 }
 
 cudaError_t launch_bpersist(const BatchParams& p, const BatchPersistArgs& a, int grid, size_t smem,
@@ -716,16 +803,17 @@ cudaError_t launch_bpersist(const BatchParams& p, const BatchPersistArgs& a, int
     return cudaLaunchKernelExC(&cfg, (const void*)&k_bpersist, args);
 }
 
-cudaError_t launch_batch_level(const BatchParams& p, bool roots, int grid, int heavy_grid, size_t smem,
+// `overlap`: the pass may start while the launch before it drains.
+cudaError_t launch_batch_level(const BatchParams& p, bool roots, bool overlap, int grid, int heavy_grid, size_t smem,
                                cudaStream_t s) {
     void* f = roots ? (void*)&k_bexpand<true> : (void*)&k_bexpand<false>;
     void* fh = roots ? (void*)&k_bexpand_heavy<true> : (void*)&k_bexpand_heavy<false>;
     BatchParams q = p;
     q.max_warps = (uint32_t)heavy_grid * kBWarps;
     void* args[] = {(void*)&q};
-    cudaError_t e = cudaLaunchKernel(f, dim3(grid), dim3(kBWarps * 32), args, smem, s);
-    if (e != cudaSuccess) return e;
-    return cudaLaunchKernel(fh, dim3(heavy_grid), dim3(kBWarps * 32), args, smem, s);
+    cudaError_t e = launch_pass(f, grid, kBWarps * 32, smem, args, overlap, s);
+    if (e != cudaSuccess || 32ull * p.max_list <= kBHeavyLeast) return e;
+    return launch_pass(fh, heavy_grid, kBWarps * 32, smem, args, overlap, s);
 }
 
 int batch_blocks_per_sm(bool roots, size_t smem) {
@@ -733,9 +821,7 @@ int batch_blocks_per_sm(bool roots, size_t smem) {
     void* fh = roots ? (void*)&k_bexpand_heavy<true> : (void*)&k_bexpand_heavy<false>;
     allow_dynamic_smem(f);
     allow_dynamic_smem(fh);
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, kBWarps * 32, smem) != cudaSuccess || n < 1) n = 1;
-    return n;
+    return std::max(1, blocks_per_sm(f, kBWarps * 32, smem));
 }
 
 }  // namespace
@@ -1065,6 +1151,7 @@ struct BatchRun {
     // CUDA graph captures.
     fm_status enqueue_all() {
         FM_CUDA(cudaMemsetAsync(b->d_qpos, 0, nq * sizeof(unsigned long long), s));
+        FM_CUDA(cudaMemsetAsync(cv.ctl, 0, b->maxq * sizeof(LaunchCtl), s));
         for (uint32_t d = 1; d < b->maxq; d++) {
             BatchParams p = level_params(d);
             if (d == 1) {
@@ -1075,8 +1162,7 @@ struct BatchRun {
             }
             p.ndef_in = 0;
             p.fresh_base = 0;
-            FM_CUDA(cudaMemsetAsync(cv.ctl + d, 0, sizeof(LaunchCtl), s));
-            FM_CUDA(launch_batch_level(p, d == 1, main_grid(d), full_grid(d), smem(d), s));
+            FM_CUDA(launch_batch_level(p, d == 1, d > 1, main_grid(d), full_grid(d), smem(d), s));
         }
         FM_CUDA(cudaMemcpyAsync(cv.h_ctl, cv.ctl, b->maxq * sizeof(LaunchCtl), cudaMemcpyDeviceToHost, s));
         FM_CUDA(cudaMemcpyAsync(b->h_qpos, b->d_qpos, nq * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
@@ -1099,7 +1185,7 @@ struct BatchRun {
             p.def_out = def_b;
             FM_CUDA(cudaMemsetAsync(cv.ctl + d, 0, sizeof(LaunchCtl), s));
             const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((items + 7) / 8, (uint64_t)full_grid(d)));
-            FM_CUDA(launch_batch_level(p, d == 1, grid, full_grid(d), smem(d), s));
+            FM_CUDA(launch_batch_level(p, d == 1, false, grid, full_grid(d), smem(d), s));
             b->launches++;
             FM_CUDA(cudaMemcpyAsync(cv.h_ctl + d, cv.ctl + d, sizeof(LaunchCtl), cudaMemcpyDeviceToHost, s));
             FM_CUDA(cudaStreamSynchronize(s));
@@ -1354,6 +1440,10 @@ fm_status fm_batch_run(fm_batch* b, uint64_t* counts, fm_batch_stats* stats) {
         run.base.nbr = g.nbr;
         run.base.bm = g.bitmaps;
         run.base.bm_words = g.bm_words;
+        run.base.efilter = g.efilter;
+        run.base.efilter_off = g.efilter_off;
+        run.base.L = g.L;
+        run.base.max_list = g.max_len;
         run.base.V = g.V;
         uint32_t longest = 1;
         for (const BatchPlan& bp : b->h_plans) longest = std::max(longest, bp.n_roots);

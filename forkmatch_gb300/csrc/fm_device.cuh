@@ -181,6 +181,18 @@ __device__ __forceinline__ uint32_t member_mask(const uint4& s, const uint32_t* 
     return mask;
 }
 
+// How many of the row's vertices and, with `extra`, x, are in the list s of
+// vertex v: count_members with the filter in front.
+__device__ __forceinline__ uint32_t count_members_f(const uint4& s, const FilterSlice& f, uint32_t v,
+                                                    const uint32_t* rows_s, uint32_t j, uint32_t n_row, uint32_t x,
+                                                    bool extra, const uint32_t* __restrict__ nbr,
+                                                    const uint32_t* __restrict__ bm, uint32_t bm_words) {
+    if (s.x == 0) return 0;
+    uint32_t n = __popc(member_mask(s, rows_s, j, n_row, 0xffffffffu, f, v, nbr, bm, bm_words));
+    if (extra && filter_has(f, filter_seed(v), x)) n += seg_has(s, x, 1, nbr, bm, bm_words) ? 1u : 0u;
+    return n;
+}
+
 // ------------------------------------------------- staged membership lists
 //
 // A list tested for membership by many candidates of a chunk is copied once

@@ -479,9 +479,8 @@ struct MatchRun {
     uint2* vsum = nullptr;                  // null: the rule needs none
 
     size_t level_smem(uint32_t d) const {
-        const uint32_t k = sums && d == last_depth() ? 2u : nreq_depth[d];
-        return expand_smem_bytes(d, k, block / 32, nreq_depth[d] >= 2 ? base.stage_words : 0,
-                                 mode_of(d) != kModeLastCount);
+        return expand_smem_bytes(d, nreq_depth[d], block / 32, nreq_depth[d] >= 2 ? base.stage_words : 0,
+                                 mode_of(d) != kModeLastCount, dups, sums && d == last_depth());
     }
     cudaError_t vertex_sums(const ExpandParams& p, const unsigned long long* parents) {
         if (!vsum) return cudaSuccess;

@@ -301,8 +301,10 @@ cudaError_t launch_pass(const void* f, int grid, int block, size_t smem, void** 
 // Resident blocks per SM of kernel f (0: does not fit), asked of the driver
 // once per kernel and shared memory size.
 int blocks_per_sm(const void* f, int block, size_t smem);
-// `staged`: the level writes survivors (a middle or a table level).
-size_t expand_smem_bytes(uint32_t depth, uint32_t nreq, int warps, uint32_t stage_words, bool staged);
+// `staged`: the level writes survivors (a middle or a table level); `sums`: it
+// may be pre-counted by sums.
+size_t expand_smem_bytes(uint32_t depth, uint32_t nreq, int warps, uint32_t stage_words, bool staged, bool dups,
+                         bool sums);
 // Vertex sums of pre-count by sums for the lists of `label` (n root-list
 // entries at `heads`); with `parents` set, skipped on the device when the level
 // has too few parents for the rule.

@@ -134,7 +134,7 @@ __device__ __forceinline__ void defer_chunk(const ExpandParams& P, uint32_t chun
 // Per-warp shared memory.
 struct WarpMem {
     uint32_t* rows_s;   // [d][32] parent rows of the current chunk, column-major
-    uint4* segs_s;      // [k][32] segment records
+    uint4* segs_s;      // [n_recs][32] segment records (all k of a parent, or its driver's)
     uint2* start_s;     // [32] parents with candidates: first slot, lane (dev::SlotWalk)
     uint8_t* drv_s;     // [32] driver list of each parent
     uint32_t* stp;      // [stage_rows] staged survivors: parent index in the level
@@ -150,18 +150,27 @@ struct WarpMem {
 // records, lists and filter words (with 6 blocks, 33 KB a block instead of 31
 // leaves 28 KB of L1 instead of 60 and made the counting level of a 5-vertex
 // path 1.5 times slower).
-__host__ __device__ constexpr uint32_t per_warp_bytes(uint32_t d, uint32_t k, uint32_t stage_words, bool staged) {
-    return 128 * d + 512 * k + 256 + 32 + (staged ? 8 * stage_rows(k) : 0u) + (k == 1 ? 0u : 5 * kPend) + 4 * stage_words;
+__host__ __device__ constexpr uint32_t per_warp_bytes(uint32_t d, uint32_t k, uint32_t recs, uint32_t stage_words,
+                                                      bool staged) {
+    return 128 * d + 512 * recs + 256 + 32 + (staged ? 8 * stage_rows(k) : 0u) + (k == 1 ? 0u : 5 * kPend) + 4 * stage_words;
 }
 static_assert(5 * kPend % 16 == 0 && 8 * kStage % 16 == 0, "the list stage is 16-byte aligned");
 
-__device__ __forceinline__ WarpMem warp_mem(unsigned char* smem_raw, uint32_t warp, uint32_t d, uint32_t k,
+// Records kept per parent: only the driver's.  The other lists are asked through
+// the filter, and the few exact tests load their record again.  Graphs with
+// duplicates test every candidate exactly and the list stage rewrites records,
+// so those keep all.
+__host__ __device__ constexpr uint32_t n_recs(uint32_t k, bool dups, uint32_t stage_words) {
+    return dups || stage_words ? k : 1;
+}
+
+__device__ __forceinline__ WarpMem warp_mem(unsigned char* smem_raw, uint32_t warp, uint32_t d, uint32_t k, uint32_t recs,
                                             uint32_t stage_words, bool staged, uint64_t* mbar_s) {
-    unsigned char* ws = smem_raw + warp * per_warp_bytes(d, k, stage_words, staged);
+    unsigned char* ws = smem_raw + warp * per_warp_bytes(d, k, recs, stage_words, staged);
     WarpMem m;
     m.rows_s = (uint32_t*)ws;
     m.segs_s = (uint4*)(ws + 128 * d);
-    m.start_s = (uint2*)(ws + 128 * d + 512 * k);
+    m.start_s = (uint2*)(ws + 128 * d + 512 * recs);
     m.drv_s = (uint8_t*)(m.start_s + 32);
     m.stp = (uint32_t*)(m.drv_s + 32);
     m.stx = m.stp + stage_rows(k);
@@ -321,20 +330,22 @@ __device__ __forceinline__ uint32_t load_chunk(const ExpandParams& P, const Warp
     n = 0;
     words = 0;
     if (valid) {
-        uint32_t best = 0xffffffffu;
+        const bool all = DUPS || P.stage_words;
+        uint4 best = make_uint4(0xffffffffu, 0, 0, 0);
         for (uint32_t i = 0; i < k; i++) {
             const uint32_t anc = P.plan.req_anc[rb + i];
             const uint32_t lab = P.plan.req_label[rb + i];
             const uint32_t v = m.rows_s[anc * 32 + lane];
             const uint4 sg = ldg4(P.seg + (uint64_t)lab * P.V + v);
-            m.segs_s[i * 32 + lane] = sg;
+            if (all) m.segs_s[i * 32 + lane] = sg;
             words += sg.x;
-            if (sg.x < best) {
-                best = sg.x;
+            if (sg.x < best.x) {
+                best = sg;
                 drv = i;
             }
         }
-        n = best;
+        n = best.x;
+        if (!all) m.segs_s[lane] = best;
         // shortest list first where every candidate is tested exactly
         if (DUPS && k > 2) drv = dev::order_lists(m.segs_s, lane, k, drv);
     }
@@ -379,6 +390,7 @@ __device__ __forceinline__ void flush_pre(const ExpandParams& P, PreAcc& pre, ui
 // parent (in shared memory, one copy per block).
 struct LevelLists {
     uint2 slice[kMaxQ];              // first word, words
+    const uint4* records[kMaxQ];     // of the back edge's label
     uint8_t anc[kMaxQ];
     __device__ __forceinline__ dev::FilterSlice at(const ExpandParams& P, uint32_t i) const {
         return {P.efilter + slice[i].x, slice[i].y};
@@ -390,6 +402,7 @@ __device__ __forceinline__ void level_lists_init(const ExpandParams& P, LevelLis
     if (threadIdx.x < k) {
         const uint32_t l = P.plan.req_label[rb + threadIdx.x];
         L.anc[threadIdx.x] = P.plan.req_anc[rb + threadIdx.x];
+        L.records[threadIdx.x] = P.seg + (uint64_t)l * P.V;
         if (P.efilter) {
             const uint32_t a = __ldg(P.efilter_off + l);
             L.slice[threadIdx.x] = make_uint2(a, __ldg(P.efilter_off + l + 1) - a);
@@ -420,8 +433,11 @@ __device__ __forceinline__ void emit(const ExpandParams& P, const WarpMem& m, ui
         const uint32_t rb = P.plan.req_begin[d + 1];
         const uint32_t anc = P.plan.req_anc[rb];
         const uint4* segl = P.seg + (uint64_t)P.plan.req_label[rb] * P.V;
-        const uint4 sg = ldg4(segl + (anc == d ? x : m.rows_s[anc * 32 + j]));
-        e.lane_count += sg.x - dev::count_members(sg, m.rows_s, j, d, x, P.self_loops || anc != d, P.nbr, P.bm, P.bm_words);
+        const uint32_t v = anc == d ? x : m.rows_s[anc * 32 + j];
+        const uint4 sg = ldg4(segl + v);
+        const dev::FilterSlice f = dev::filter_slice(P.efilter, P.efilter_off, P.plan.req_label[rb]);
+        e.lane_count += sg.x - dev::count_members_f(sg, f, v, m.rows_s, j, d, x, P.self_loops || anc != d, P.nbr, P.bm,
+                                                    P.bm_words);
         pre.parents += 1;
         pre.words += sg.x;
         return;
@@ -462,6 +478,7 @@ __device__ __forceinline__ void process_slots(const ExpandParams& P, const WarpM
     Emit e{nst, stage_rows(k), n_count};
     SlotWalk walk(m.start_s, excl, n, begin, lane);
     uint32_t pend = 0;
+    const bool all = DUPS || (P.stage_words && k >= 2);      // every record is in segs_s
     for (uint32_t base = begin; base < end; base += 32 * kSlots) {
         uint32_t j[kSlots], t[kSlots], x[kSlots], dj[kSlots];
         bool ok[kSlots];
@@ -473,7 +490,7 @@ __device__ __forceinline__ void process_slots(const ExpandParams& P, const WarpM
             ok[u] = base + 32 * u + lane < end;
             if (ok[u]) {
                 dj[u] = m.drv_s[j[u]];
-                x[u] = seg_at(m.segs_s[dj[u] * 32 + j[u]], t[u], P.nbr);
+                x[u] = seg_at(m.segs_s[(all ? dj[u] * 32 : 0u) + j[u]], t[u], P.nbr);
             }
         }
         if (DUPS || k == 1) {
@@ -526,9 +543,12 @@ __device__ __forceinline__ void process_slots(const ExpandParams& P, const WarpM
                     jj = m.pj[pend + lane];
                     xx = m.px[pend + lane];
                     const uint32_t dd = m.drv_s[jj];
-                    for (uint32_t i = 0; i < k && in; i++)
-                        if (i != dd)
-                            in = dev::seg_has_st(m.segs_s[i * 32 + jj], xx, 1, P.nbr, P.bm, P.bm_words, m.stage);
+                    for (uint32_t i = 0; i < k && in; i++) {
+                        if (i == dd) continue;
+                        const uint4 r = all ? m.segs_s[i * 32 + jj]
+                                            : ldg4(L.records[i] + m.rows_s[L.anc[i] * 32 + jj]);
+                        in = dev::seg_has_st(r, xx, 1, P.nbr, P.bm, P.bm_words, m.stage);
+                    }
                     for (uint32_t c = 0; c < d && in; c++) in = m.rows_s[c * 32 + jj] != xx;
                 }
                 emit<MODE, ROOTS, DUPS>(P, m, chunk, in, jj, xx, lane, d, col_depth_s, e, pre);
@@ -581,7 +601,7 @@ __device__ __forceinline__ void expand_main(const ExpandParams& P, unsigned char
     const uint32_t k = P.plan.nreq[d];
     const uint32_t rb = P.plan.req_begin[d];
     const uint32_t sw = k >= 2 ? P.stage_words : 0;   // only levels with membership tests stage lists
-    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, k, sw, MODE != kModeLastCount, mbar_s);
+    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, k, n_recs(k, DUPS, sw), sw, MODE != kModeLastCount, mbar_s);
     const Tune T = make_tune(P, true);
 
     unsigned long long n_count = 0, n_lookups = 0, n_words = 0, n_parents = 0;
@@ -731,7 +751,7 @@ __device__ __forceinline__ void expand_heavy(const ExpandParams& P, unsigned cha
     const uint32_t k = P.plan.nreq[d];
     const uint32_t rb = P.plan.req_begin[d];
     const uint32_t sw = k >= 2 ? P.stage_words : 0;
-    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, k, sw, MODE != kModeLastCount, mbar_s);
+    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, k, n_recs(k, DUPS, sw), sw, MODE != kModeLastCount, mbar_s);
     const Tune T = make_tune(P, false);
     unsigned long long n_count = 0, n_flushed = 0;
     PreAcc pre;
@@ -909,7 +929,7 @@ __device__ __forceinline__ bool sum_needs(const SumPlan& sp, uint32_t d, uint32_
 __device__ __forceinline__ void expand_sum_main(const ExpandParams& P, unsigned char* smem_raw, uint64_t* mbar_s) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t d = P.depth;
-    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, 2, 0, false, mbar_s);
+    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, 2, 2, 0, false, mbar_s);
     const Tune T = make_tune(P, true);
     const SumPlan sp = sum_plan(P);
     const bool chain = sp.last_anc == d;
@@ -1012,7 +1032,7 @@ __device__ __forceinline__ void expand_sum_heavy(const ExpandParams& P, unsigned
     if (nent == 0) return;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t d = P.depth;
-    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, 2, 0, false, mbar_s);
+    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, 2, 2, 0, false, mbar_s);
     const Tune T = make_tune(P, false);
     const SumPlan sp = sum_plan(P);
     unsigned long long hits = 0;
@@ -1309,7 +1329,8 @@ cudaError_t launch_sched_init(SchedState* S, unsigned q, unsigned long long n_ro
 size_t persist_smem_bytes(const DevPlan& plan, const uint32_t* nreq_depth, uint32_t stage_words) {
     size_t best = 0;
     for (uint32_t d = 1; d < plan.q; d++)
-        best = std::max<size_t>(best, per_warp_bytes(d, nreq_depth[d], nreq_depth[d] >= 2 ? stage_words : 0, true));
+        best = std::max<size_t>(best, per_warp_bytes(d, nreq_depth[d], nreq_depth[d],
+                                                     nreq_depth[d] >= 2 ? stage_words : 0, true));
     return best * kWarps;
 }
 
@@ -1362,8 +1383,10 @@ cudaError_t launch_vertex_sums(const ExpandParams& p, const uint32_t* heads, uin
                        parents != nullptr, s);
 }
 
-size_t expand_smem_bytes(uint32_t depth, uint32_t nreq, int warps, uint32_t stage_words, bool staged) {
-    return (size_t)warps * per_warp_bytes(depth, nreq, stage_words, staged);
+size_t expand_smem_bytes(uint32_t depth, uint32_t nreq, int warps, uint32_t stage_words, bool staged, bool dups,
+                         bool sums) {
+    return (size_t)warps * per_warp_bytes(depth, sums ? 2 : nreq, sums ? 2 : n_recs(nreq, dups, stage_words), stage_words,
+                                          staged);
 }
 
 void allow_dynamic_smem(const void* f) {
