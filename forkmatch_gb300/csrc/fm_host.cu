@@ -478,9 +478,15 @@ struct MatchRun {
     uint32_t sum_label = 0, sum_last = 0;
     uint2* vsum = nullptr;                  // null: the rule needs none
 
+    // The two oldest back edges of depth d leave the newest column alone:
+    // parents of a run share their intersection (lists staged by TMA exclude it).
+    bool shares(uint32_t d) const {
+        const uint32_t k = nreq_depth[d];
+        return !dups && !base.stage_words && k >= 2 && base.plan.req_anc[base.plan.req_begin[d] + k - 2] + 1u < d;
+    }
     size_t level_smem(uint32_t d) const {
         return expand_smem_bytes(d, nreq_depth[d], block / 32, nreq_depth[d] >= 2 ? base.stage_words : 0,
-                                 mode_of(d) != kModeLastCount, dups, sums && d == last_depth());
+                                 mode_of(d) != kModeLastCount, dups, sums && d == last_depth(), shares(d));
     }
     cudaError_t vertex_sums(const ExpandParams& p, const unsigned long long* parents) {
         if (!vsum) return cudaSuccess;
@@ -562,7 +568,8 @@ struct MatchRun {
             const int mode = mode_of(d);
             const bool roots = d == 1;
             const size_t smem = level_smem(d);
-            const int per_sm = expand_blocks_per_sm(mode, roots, dups, smem, block);
+            const bool share = shares(d);
+            const int per_sm = expand_blocks_per_sm(mode, roots, dups, share, smem, block);
             const int full = ctx->sms * per_sm;
             ExpandParams p = base;
             p.pin = roots ? nullptr : level[d];
@@ -589,7 +596,7 @@ struct MatchRun {
                 p.sum_rule = 1;
                 FM_CUDA(vertex_sums(p, p.n_parents_dev));
             }
-            FM_CUDA(launch_expand(p, mode, roots, dups, !roots, grid, full, block, smem, s));
+            FM_CUDA(launch_expand(p, mode, roots, dups, share, !roots, grid, full, block, smem, s));
             if (profile) FM_CUDA(cudaEventRecord(ev[d][1], s));
         }
         FM_TRY(read_back());
@@ -702,7 +709,8 @@ struct MatchRun {
         const int mode = mode_of(d);
         const uint64_t n_chunks = (n_parents + 31) / 32;
         const size_t smem = level_smem(d);
-        const int per_sm = expand_blocks_per_sm(mode, roots, dups, smem, block);
+        const bool share = shares(d);
+        const int per_sm = expand_blocks_per_sm(mode, roots, dups, share, smem, block);
         (void)q;
         while (true) {
             const uint64_t items = ndef_in + (n_chunks - fresh);
@@ -735,7 +743,7 @@ struct MatchRun {
                 }
                 p.sum_rule = sums_ready ? 2 : 0;
             }
-            FM_CUDA(launch_expand(p, mode, roots, dups, false, grid, ctx->sms * per_sm, block, smem, s));
+            FM_CUDA(launch_expand(p, mode, roots, dups, share, false, grid, ctx->sms * per_sm, block, smem, s));
             if (profile) FM_CUDA(cudaEventRecord(e1, s));
             FM_CUDA(cudaMemcpyAsync(ctx->h_ctl + d, ctx->ctl + d, sizeof(LaunchCtl), cudaMemcpyDeviceToHost, s));
             FM_CUDA(cudaStreamSynchronize(s));

@@ -227,6 +227,7 @@ struct ExpandParams {
     const uint2* vsum;              // per vertex v with a list of the level's label: the sum of its
                                     // neighbours' last-label list lengths, and the neighbours that are
                                     // also in v's own last-label list
+    uint32_t share_words;           // words of each warp's buffer for shared intersections; 0: none
 };
 constexpr unsigned int kLimitFlag = 2u;
 
@@ -295,16 +296,16 @@ cudaError_t launch_sched_init(SchedState* S, unsigned q, unsigned long long n_ro
 // Launch one level expansion: the main pass, then the heavy-chunk pass
 // (fm_match.cu).
 // `overlap`: the pass may start while the launch before it drains.
-cudaError_t launch_expand(const ExpandParams& p, int mode, bool roots, bool dups, bool overlap, int grid,
+cudaError_t launch_expand(const ExpandParams& p, int mode, bool roots, bool dups, bool share, bool overlap, int grid,
                           int heavy_grid, int block, size_t smem, cudaStream_t s);
 cudaError_t launch_pass(const void* f, int grid, int block, size_t smem, void** args, bool overlap, cudaStream_t s);
 // Resident blocks per SM of kernel f (0: does not fit), asked of the driver
 // once per kernel and shared memory size.
 int blocks_per_sm(const void* f, int block, size_t smem);
 // `staged`: the level writes survivors (a middle or a table level); `sums`: it
-// may be pre-counted by sums.
+// may be pre-counted by sums; `share`: it shares intersections.
 size_t expand_smem_bytes(uint32_t depth, uint32_t nreq, int warps, uint32_t stage_words, bool staged, bool dups,
-                         bool sums);
+                         bool sums, bool share);
 // Vertex sums of pre-count by sums for the lists of `label` (n root-list
 // entries at `heads`); with `parents` set, skipped on the device when the level
 // has too few parents for the rule.
@@ -313,7 +314,7 @@ cudaError_t launch_vertex_sums(const ExpandParams& p, const uint32_t* heads, uin
 // Let kernel f launch with up to the device's opt-in shared memory (once per
 // device; safe from several host threads).
 void allow_dynamic_smem(const void* f);
-int expand_blocks_per_sm(int mode, bool roots, bool dups, size_t smem, int block);
+int expand_blocks_per_sm(int mode, bool roots, bool dups, bool share, size_t smem, int block);
 
 // The parts of a context other translation units use (fm_host.cu owns it).
 struct ContextView {

@@ -110,6 +110,9 @@ __device__ __forceinline__ Tune make_tune(const ExpandParams& P, bool main_pass)
     t.credit_block = (uint32_t)(cb < 1024 ? cb : 1024);
     t.heavy_thresh = t.n_items >= 4 * all_warps ? 4096u : (t.n_items >= all_warps ? 1024u : 256u);
     if (32ull * P.max_list <= kHeavyLeast) t.heavy_thresh = 0xffffffffu;   // there is no heavy pass
+    // a piece of a chunk with shared intersections computes them again, so its
+    // pieces are long (2048 to 16384 slots: 32.3 to 27.2 ms on the level below)
+    if (P.share_words && t.n_items >= 4 * all_warps) t.heavy_thresh = 32768u;
     t.heavy_piece = t.heavy_thresh / 2;
     return t;
 }
@@ -143,6 +146,7 @@ struct WarpMem {
     uint8_t* pj;        // [kPend] and parent (lane) in the chunk
     uint64_t* mbar;     // completion barrier of the list stage's bulk copies
     uint32_t* stage;    // [stage_words] membership lists copied in by TMA (optional)
+    uint32_t* shared;   // [share_words] intersections that parents of the chunk share (optional)
 };
 
 // Counting levels store no survivors and have no stage.  The bytes matter: what
@@ -151,8 +155,9 @@ struct WarpMem {
 // leaves 28 KB of L1 instead of 60 and made the counting level of a 5-vertex
 // path 1.5 times slower).
 __host__ __device__ constexpr uint32_t per_warp_bytes(uint32_t d, uint32_t k, uint32_t recs, uint32_t stage_words,
-                                                      bool staged) {
-    return 128 * d + 512 * recs + 256 + 32 + (staged ? 8 * stage_rows(k) : 0u) + (k == 1 ? 0u : 5 * kPend) + 4 * stage_words;
+                                                      bool staged, uint32_t share_words) {
+    return 128 * d + 512 * recs + 256 + 32 + (staged ? 8 * stage_rows(k) : 0u) + (k == 1 ? 0u : 5 * kPend) +
+           4 * stage_words + 4 * share_words;
 }
 static_assert(5 * kPend % 16 == 0 && 8 * kStage % 16 == 0, "the list stage is 16-byte aligned");
 
@@ -165,8 +170,9 @@ __host__ __device__ constexpr uint32_t n_recs(uint32_t k, bool dups, uint32_t st
 }
 
 __device__ __forceinline__ WarpMem warp_mem(unsigned char* smem_raw, uint32_t warp, uint32_t d, uint32_t k, uint32_t recs,
-                                            uint32_t stage_words, bool staged, uint64_t* mbar_s) {
-    unsigned char* ws = smem_raw + warp * per_warp_bytes(d, k, recs, stage_words, staged);
+                                            uint32_t stage_words, bool staged, uint32_t share_words,
+                                            uint64_t* mbar_s) {
+    unsigned char* ws = smem_raw + warp * per_warp_bytes(d, k, recs, stage_words, staged, share_words);
     WarpMem m;
     m.rows_s = (uint32_t*)ws;
     m.segs_s = (uint4*)(ws + 128 * d);
@@ -178,6 +184,7 @@ __device__ __forceinline__ WarpMem warp_mem(unsigned char* smem_raw, uint32_t wa
     m.pj = (uint8_t*)(m.px + kPend);
     m.mbar = mbar_s + warp;
     m.stage = (uint32_t*)(m.pj + kPend);
+    m.shared = m.stage + stage_words;
     return m;
 }
 
@@ -311,14 +318,133 @@ __device__ __forceinline__ void flush_stage(const ExpandParams& P, const WarpMem
     }
 }
 
+// The back edges' filter slices and columns of a level, the same for every
+// parent (in shared memory, one copy per block).
+struct LevelLists {
+    uint2 slice[kMaxQ];              // first word, words
+    const uint4* records[kMaxQ];     // of the back edge's label
+    uint8_t anc[kMaxQ];
+    __device__ __forceinline__ dev::FilterSlice at(const ExpandParams& P, uint32_t i) const {
+        return {P.efilter + slice[i].x, slice[i].y};
+    }
+};
+
+__device__ __forceinline__ void level_lists_init(const ExpandParams& P, LevelLists& L, uint32_t d) {
+    const uint32_t k = P.plan.nreq[d], rb = P.plan.req_begin[d];
+    if (threadIdx.x < k) {
+        const uint32_t l = P.plan.req_label[rb + threadIdx.x];
+        L.anc[threadIdx.x] = P.plan.req_anc[rb + threadIdx.x];
+        L.records[threadIdx.x] = P.seg + (uint64_t)l * P.V;
+        if (P.efilter) {
+            const uint32_t a = __ldg(P.efilter_off + l);
+            L.slice[threadIdx.x] = make_uint2(a, __ldg(P.efilter_off + l + 1) - a);
+        }
+    }
+    __syncthreads();
+}
+
+// -------------------------------------------------- shared intersections
+//
+// The rows of a level come in runs: parents that extend the same earlier match
+// differ only in their newest column.  Where the two oldest back edges of a
+// level leave the newest column alone, the intersection T of their lists is
+// the same for the whole run; it is computed once by the warp, kept in shared
+// memory for the next chunks of the run, and drives where it is shorter than
+// every list of the parent: far fewer candidates, and two tests less for each.
+// A run needs 4 parents in the chunk and as many candidates, over them, as
+// building T reads; T must fit the buffer.  Levels with less than four chunks a
+// warp are left alone: there the time is one chunk's latency, which building T
+// adds to.
+//
+// Closing level of 4-cliques on a 2^18-vertex power-law graph of 2 labels (3.8e7
+// parents with 280 candidates each between hub lists, 70 with T): 27.2 ms, 66.4
+// without.  1024 words a warp: 40.4 ms with the pieces of 512's 32.3, for the
+// blocks and the L1 they cost.
+constexpr uint32_t kShareWords = 512;
+constexpr uint32_t kDrvShared = 0xff;         // drv_s: T drives
+static_assert(kDrvShared >= kMaxQ, "no list index");
+
+struct ShareState {
+    unsigned long long key = ~0ull, bad = ~0ull;   // run whose T is at the buffer's start; run whose T did not fit
+    uint32_t n = 0;                                // entries of that T
+};
+
+// T for runs of lanes with equal `key` (the vertices of back edges q0 and
+// q0 + 1): returns its length and offset in m.shared for this lane, or
+// 0xffffffff.  `work`: the lane's candidates without it (0: no parent).
+// Whether a run is shared depends on the chunk alone, never on what the warp
+// did before: the heavy pass has to find the same slots.
+__device__ __forceinline__ uint32_t share_lists(const ExpandParams& P, const WarpMem& m, const LevelLists& L,
+                                                uint32_t lane, uint32_t q0, unsigned long long key, uint32_t work,
+                                                ShareState& st, uint32_t& off_out) {
+    const unsigned same = __match_any_sync(kFull, key);
+    unsigned todo = __ballot_sync(kFull, work > 0 && __popc(same) >= 4);
+    uint32_t used = 0, mine = 0xffffffffu;
+    while (todo) {
+        const int leader = __ffs(todo) - 1;
+        const unsigned grp = __shfl_sync(kFull, same, leader);
+        todo &= ~grp;
+        const unsigned long long gkey = __shfl_sync(kFull, key, leader);
+        const bool in = (grp >> lane) & 1u;
+        const uint32_t va = (uint32_t)(gkey >> 32), vb = (uint32_t)gkey;
+        const uint4 ra = ldg4(L.records[q0] + va), rb = ldg4(L.records[q0 + 1] + vb);
+        const bool first = ra.x <= rb.x;
+        const uint4 base = first ? ra : rb, other = first ? rb : ra;
+        const uint32_t all = __reduce_add_sync(kFull, in ? min(work, 1u << 24) : 0u);
+        if (gkey == st.bad || all < base.x) continue;
+        uint32_t n = 0;
+        const uint32_t off = used;
+        if (used == 0 && gkey == st.key) {
+            n = st.n;                              // still there from the chunk before
+        } else {
+            if (used == 0) st.key = ~0ull;
+            const dev::FilterSlice f = L.at(P, first ? q0 + 1 : q0);
+            const uint32_t seed = dev::filter_seed(first ? vb : va);
+            __syncwarp();
+            for (uint32_t t0 = 0; t0 < base.x; t0 += 32) {
+                const uint32_t t = t0 + lane;
+                uint32_t x = 0;
+                bool ok = t < base.x;
+                if (ok) {
+                    x = seg_at(base, t, P.nbr);
+                    ok = dev::filter_has(f, seed, x) && seg_has(other, x, 1, P.nbr, P.bm, P.bm_words);
+                }
+                const unsigned b = __ballot_sync(kFull, ok);
+                if (off + n + __popc(b) > P.share_words) {
+                    n = 0xffffffffu;
+                    break;
+                }
+                if (ok) m.shared[off + n + __popc(b & ((1u << lane) - 1u))] = x;
+                n += __popc(b);
+            }
+            __syncwarp();
+            if (n == 0xffffffffu) {
+                if (off == 0) st.bad = gkey;       // alone it never fits
+                continue;
+            }
+            if (off == 0) {
+                st.key = gkey;
+                st.n = n;
+            }
+        }
+        if (in) {
+            mine = n;
+            off_out = off;
+        }
+        used = off + n;
+    }
+    return mine;
+}
+
 // Load the 32 parents of `chunk`, look up their k lists (independent 16-byte
 // loads), pick each parent's shortest list as its driver and prefix-sum the
 // driver lengths.  Returns the chunk's candidate slots (warp-uniform).
-template <bool ROOTS, bool DUPS>
+template <bool ROOTS, bool DUPS, bool SHARE>
 __device__ __forceinline__ uint32_t load_chunk(const ExpandParams& P, const WarpMem& m, uint32_t chunk, uint32_t lane,
                                                uint32_t d, uint32_t k, uint32_t rb, unsigned long long n_parents,
                                                bool& valid, unsigned long long& words, uint32_t& phase,
-                                               bool& stage_ok, uint32_t& excl, uint32_t& n) {
+                                               bool& stage_ok, uint32_t& excl, uint32_t& n, const LevelLists& L,
+                                               bool share_on, ShareState& share) {
     const uint64_t p = (uint64_t)chunk * 32 + lane;
     valid = p < n_parents;
     if (ROOTS) {
@@ -348,6 +474,19 @@ __device__ __forceinline__ uint32_t load_chunk(const ExpandParams& P, const Warp
         if (!all) m.segs_s[lane] = best;
         // shortest list first where every candidate is tested exactly
         if (DUPS && k > 2) drv = dev::order_lists(m.segs_s, lane, k, drv);
+    }
+    if (SHARE && share_on) {
+        // back edges are ordered by climb: the two oldest come last
+        const uint32_t q0 = k - 2;
+        const unsigned long long key =
+            (unsigned long long)m.rows_s[L.anc[q0] * 32 + lane] << 32 | m.rows_s[L.anc[q0 + 1] * 32 + lane];
+        uint32_t off = 0;
+        const uint32_t nt = share_lists(P, m, L, lane, q0, key, valid ? n : 0u, share, off);
+        if (nt < n) {
+            n = nt;
+            drv = kDrvShared;
+            m.segs_s[lane] = make_uint4(nt, dev::kStagedMark | off, 0, 0);
+        }
     }
     stage_ok = true;
     if (P.stage_words && k >= 2) stage_ok = stage_lists(P, m, lane, k, drv, n, valid, phase);
@@ -384,31 +523,6 @@ __device__ __forceinline__ void flush_pre(const ExpandParams& P, PreAcc& pre, ui
         atomicAdd(&next->lookups, pre.parents);
         atomicAdd(&next->list_words, pre.words);
     }
-}
-
-// The back edges' filter slices and columns of a level, the same for every
-// parent (in shared memory, one copy per block).
-struct LevelLists {
-    uint2 slice[kMaxQ];              // first word, words
-    const uint4* records[kMaxQ];     // of the back edge's label
-    uint8_t anc[kMaxQ];
-    __device__ __forceinline__ dev::FilterSlice at(const ExpandParams& P, uint32_t i) const {
-        return {P.efilter + slice[i].x, slice[i].y};
-    }
-};
-
-__device__ __forceinline__ void level_lists_init(const ExpandParams& P, LevelLists& L, uint32_t d) {
-    const uint32_t k = P.plan.nreq[d], rb = P.plan.req_begin[d];
-    if (threadIdx.x < k) {
-        const uint32_t l = P.plan.req_label[rb + threadIdx.x];
-        L.anc[threadIdx.x] = P.plan.req_anc[rb + threadIdx.x];
-        L.records[threadIdx.x] = P.seg + (uint64_t)l * P.V;
-        if (P.efilter) {
-            const uint32_t a = __ldg(P.efilter_off + l);
-            L.slice[threadIdx.x] = make_uint2(a, __ldg(P.efilter_off + l + 1) - a);
-        }
-    }
-    __syncthreads();
 }
 
 // What survives a warp round at its level: lane's candidate x of parent j,
@@ -469,7 +583,7 @@ __device__ __forceinline__ void emit(const ExpandParams& P, const WarpMem& m, ui
 // slots and by the L1's rate for scattered words.  Closing level of a 4-cycle on
 // a 2^20-vertex R-MAT graph with 64 labels (1.7e7 parents): 740 us, 1100 us with
 // an exact test per candidate and a binary search per slot for its parent.
-template <int MODE, bool ROOTS, bool DUPS>
+template <int MODE, bool ROOTS, bool DUPS, bool SHARE>
 __device__ __forceinline__ void process_slots(const ExpandParams& P, const WarpMem& m, uint32_t chunk,
                                               uint32_t excl, uint32_t n, uint32_t begin, uint32_t end, uint32_t lane,
                                               uint32_t d, uint32_t k, const LevelLists& L,
@@ -490,7 +604,9 @@ __device__ __forceinline__ void process_slots(const ExpandParams& P, const WarpM
             ok[u] = base + 32 * u + lane < end;
             if (ok[u]) {
                 dj[u] = m.drv_s[j[u]];
-                x[u] = seg_at(m.segs_s[(all ? dj[u] * 32 : 0u) + j[u]], t[u], P.nbr);
+                const uint4 r = m.segs_s[(all ? dj[u] * 32 : 0u) + j[u]];
+                if (SHARE && dj[u] == kDrvShared) x[u] = m.shared[(r.y & ~dev::kStagedMark) + t[u]];
+                else x[u] = seg_at(r, t[u], P.nbr);
             }
         }
         if (DUPS || k == 1) {
@@ -520,7 +636,8 @@ __device__ __forceinline__ void process_slots(const ExpandParams& P, const WarpM
                 const uint32_t* col = m.rows_s + L.anc[i] * 32;
 #pragma unroll
                 for (uint32_t u = 0; u < kSlots; u++)
-                    if (ok[u] && dj[u] != i) ok[u] = dev::filter_has(f, dev::filter_seed(col[j[u]]), x[u]);
+                    if (ok[u] && dj[u] != i && !(SHARE && dj[u] == kDrvShared && i + 2 >= k))
+                        ok[u] = dev::filter_has(f, dev::filter_seed(col[j[u]]), x[u]);
             }
 #pragma unroll
             for (uint32_t u = 0; u < kSlots; u++) {
@@ -544,7 +661,7 @@ __device__ __forceinline__ void process_slots(const ExpandParams& P, const WarpM
                     xx = m.px[pend + lane];
                     const uint32_t dd = m.drv_s[jj];
                     for (uint32_t i = 0; i < k && in; i++) {
-                        if (i == dd) continue;
+                        if (i == dd || (SHARE && dd == kDrvShared && i + 2 >= k)) continue;
                         const uint4 r = all ? m.segs_s[i * 32 + jj]
                                             : ldg4(L.records[i] + m.rows_s[L.anc[i] * 32 + jj]);
                         in = dev::seg_has_st(r, xx, 1, P.nbr, P.bm, P.bm_words, m.stage);
@@ -593,7 +710,7 @@ __device__ __forceinline__ bool over_limit(const ExpandParams& P, uint32_t lane,
 
 // Main pass: warps claim batches of chunks; long candidate ranges are
 // published to the heavy list instead of being walked by one warp.
-template <int MODE, bool ROOTS, bool DUPS>
+template <int MODE, bool ROOTS, bool DUPS, bool SHARE>
 __device__ __forceinline__ void expand_main(const ExpandParams& P, unsigned char* smem_raw, const LevelLists& L,
                                             const uint8_t* col_depth_s, uint64_t* mbar_s, uint32_t& phase) {
     const uint32_t lane = threadIdx.x & 31;
@@ -601,8 +718,11 @@ __device__ __forceinline__ void expand_main(const ExpandParams& P, unsigned char
     const uint32_t k = P.plan.nreq[d];
     const uint32_t rb = P.plan.req_begin[d];
     const uint32_t sw = k >= 2 ? P.stage_words : 0;   // only levels with membership tests stage lists
-    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, k, n_recs(k, DUPS, sw), sw, MODE != kModeLastCount, mbar_s);
+    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, k, n_recs(k, DUPS, sw), sw, MODE != kModeLastCount,
+                               SHARE ? P.share_words : 0, mbar_s);
     const Tune T = make_tune(P, true);
+    const bool share_on = SHARE && T.n_items >= 4ull * P.max_warps;
+    ShareState share;
 
     unsigned long long n_count = 0, n_lookups = 0, n_words = 0, n_parents = 0;
     unsigned long long n_flushed = 0;  // part of n_count already added to tot->count (lane 0)
@@ -639,8 +759,8 @@ __device__ __forceinline__ void expand_main(const ExpandParams& P, unsigned char
             bool valid, stage_ok;
             unsigned long long w;
             uint32_t excl, n;
-            const uint32_t total = load_chunk<ROOTS, DUPS>(P, m, chunk, lane, d, k, rb, T.n_parents, valid, w, phase,
-                                                     stage_ok, excl, n);
+            const uint32_t total = load_chunk<ROOTS, DUPS, SHARE>(P, m, chunk, lane, d, k, rb, T.n_parents, valid, w, phase,
+                                                     stage_ok, excl, n, L, share_on, share);
             last_chunk = chunk;
             if (!stage_ok) {
                 done = true;
@@ -713,7 +833,7 @@ __device__ __forceinline__ void expand_main(const ExpandParams& P, unsigned char
                 pub = __shfl_sync(kFull, pub, 0);
                 if (pub) continue;
             }
-            process_slots<MODE, ROOTS, DUPS>(P, m, chunk, excl, n, 0, total, lane, d, k, L, col_depth_s, nst, n_count,
+            process_slots<MODE, ROOTS, DUPS, SHARE>(P, m, chunk, excl, n, 0, total, lane, d, k, L, col_depth_s, nst, n_count,
                                              pre);
         }
     }
@@ -739,7 +859,7 @@ __device__ __forceinline__ void expand_main(const ExpandParams& P, unsigned char
 // chunks, reloads that chunk and walks its piece of the slots -- the warps
 // that finished their own chunks take over the work of the hub chunks.  The
 // main pass already holds the chunk's output budget and counted its work.
-template <int MODE, bool ROOTS, bool DUPS>
+template <int MODE, bool ROOTS, bool DUPS, bool SHARE>
 __device__ __forceinline__ void expand_heavy(const ExpandParams& P, unsigned char* smem_raw, const LevelLists& L,
                                              const uint8_t* col_depth_s, uint64_t* mbar_s, uint32_t& phase) {
     const unsigned long long h = *(volatile unsigned long long*)&P.ctl->heavy;
@@ -751,8 +871,11 @@ __device__ __forceinline__ void expand_heavy(const ExpandParams& P, unsigned cha
     const uint32_t k = P.plan.nreq[d];
     const uint32_t rb = P.plan.req_begin[d];
     const uint32_t sw = k >= 2 ? P.stage_words : 0;
-    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, k, n_recs(k, DUPS, sw), sw, MODE != kModeLastCount, mbar_s);
+    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, k, n_recs(k, DUPS, sw), sw, MODE != kModeLastCount,
+                               SHARE ? P.share_words : 0, mbar_s);
     const Tune T = make_tune(P, false);
+    const bool share_on = SHARE && T.n_items >= 4ull * P.max_warps;
+    ShareState share;
     unsigned long long n_count = 0, n_flushed = 0;
     PreAcc pre;
     uint32_t last_chunk = 0xffffffffu;   // chunk whose rows are in m.rows_s
@@ -775,10 +898,10 @@ __device__ __forceinline__ void expand_heavy(const ExpandParams& P, unsigned cha
         bool valid, stage_ok;
         unsigned long long w;
         uint32_t excl, n;
-        load_chunk<ROOTS, DUPS>(P, m, e.chunk, lane, d, k, rb, T.n_parents, valid, w, phase, stage_ok, excl, n);
+        load_chunk<ROOTS, DUPS, SHARE>(P, m, e.chunk, lane, d, k, rb, T.n_parents, valid, w, phase, stage_ok, excl, n, L, share_on, share);
         last_chunk = e.chunk;
         if (!stage_ok) break;
-        process_slots<MODE, ROOTS, DUPS>(P, m, e.chunk, excl, n, begin, end, lane, d, k, L, col_depth_s, nst, n_count,
+        process_slots<MODE, ROOTS, DUPS, SHARE>(P, m, e.chunk, excl, n, begin, end, lane, d, k, L, col_depth_s, nst, n_count,
                                              pre);
     }
     if (MODE != kModeLastCount && nst) flush_stage<MODE, ROOTS>(P, m, nst, lane, d, col_depth_s, last_chunk);
@@ -929,7 +1052,7 @@ __device__ __forceinline__ bool sum_needs(const SumPlan& sp, uint32_t d, uint32_
 __device__ __forceinline__ void expand_sum_main(const ExpandParams& P, unsigned char* smem_raw, uint64_t* mbar_s) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t d = P.depth;
-    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, 2, 2, 0, false, mbar_s);
+    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, 2, 2, 0, false, 0, mbar_s);
     const Tune T = make_tune(P, true);
     const SumPlan sp = sum_plan(P);
     const bool chain = sp.last_anc == d;
@@ -1032,7 +1155,7 @@ __device__ __forceinline__ void expand_sum_heavy(const ExpandParams& P, unsigned
     if (nent == 0) return;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t d = P.depth;
-    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, 2, 2, 0, false, mbar_s);
+    const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, 2, 2, 0, false, 0, mbar_s);
     const Tune T = make_tune(P, false);
     const SumPlan sp = sum_plan(P);
     unsigned long long hits = 0;
@@ -1140,7 +1263,7 @@ __global__ void __launch_bounds__(kWarps * 32) k_vertex_sums(const __grid_consta
     }
 }
 
-template <int MODE, bool ROOTS, bool DUPS>
+template <int MODE, bool ROOTS, bool DUPS, bool SHARE>
 __global__ void __launch_bounds__(kWarps * 32, 6) k_expand(const __grid_constant__ ExpandParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint8_t col_depth_s[kMaxQ];
@@ -1151,15 +1274,15 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_expand(const __grid_constant
     if (threadIdx.x < (unsigned)kMaxQ) col_depth_s[threadIdx.x] = P.plan.col_depth[threadIdx.x];
     dev::stage_barriers_init(mbar_s);
     dev::pass_wait();
-    if (MODE == kModeLastCount && !ROOTS && !DUPS && P.sum_rule && sum_rule_on(P, make_tune(P, true).n_parents)) {
+    if (MODE == kModeLastCount && !ROOTS && !DUPS && !SHARE && P.sum_rule && sum_rule_on(P, make_tune(P, true).n_parents)) {
         expand_sum_main(P, smem_raw, mbar_s);
         return;
     }
     uint32_t phase = 0;
-    expand_main<MODE, ROOTS, DUPS>(P, smem_raw, L, col_depth_s, mbar_s, phase);
+    expand_main<MODE, ROOTS, DUPS, SHARE>(P, smem_raw, L, col_depth_s, mbar_s, phase);
 }
 
-template <int MODE, bool ROOTS, bool DUPS>
+template <int MODE, bool ROOTS, bool DUPS, bool SHARE>
 __global__ void __launch_bounds__(kWarps * 32, 6) k_expand_heavy(const __grid_constant__ ExpandParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint8_t col_depth_s[kMaxQ];
@@ -1170,12 +1293,12 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_expand_heavy(const __grid_co
     if (threadIdx.x < (unsigned)kMaxQ) col_depth_s[threadIdx.x] = P.plan.col_depth[threadIdx.x];
     dev::stage_barriers_init(mbar_s);
     dev::pass_wait();
-    if (MODE == kModeLastCount && !ROOTS && !DUPS && P.sum_rule && sum_rule_on(P, make_tune(P, false).n_parents)) {
+    if (MODE == kModeLastCount && !ROOTS && !DUPS && !SHARE && P.sum_rule && sum_rule_on(P, make_tune(P, false).n_parents)) {
         expand_sum_heavy(P, smem_raw, mbar_s);
         return;
     }
     uint32_t phase = 0;
-    expand_heavy<MODE, ROOTS, DUPS>(P, smem_raw, L, col_depth_s, mbar_s, phase);
+    expand_heavy<MODE, ROOTS, DUPS, SHARE>(P, smem_raw, L, col_depth_s, mbar_s, phase);
 }
 
 // ------------------------------------------------------- persistent engine
@@ -1193,11 +1316,11 @@ template <int LAST, bool DUPS>
 __device__ __forceinline__ void persist_main(const ExpandParams& P, unsigned char* smem, const uint8_t* cd,
                                              bool roots, bool last, const LevelLists& L, uint64_t* mb, uint32_t& ph) {
     if (last) {
-        if (roots) expand_main<LAST, true, DUPS>(P, smem, L, cd, mb, ph);
-        else expand_main<LAST, false, DUPS>(P, smem, L, cd, mb, ph);
+        if (roots) expand_main<LAST, true, DUPS, false>(P, smem, L, cd, mb, ph);
+        else expand_main<LAST, false, DUPS, false>(P, smem, L, cd, mb, ph);
     } else {
-        if (roots) expand_main<kModeMid, true, DUPS>(P, smem, L, cd, mb, ph);
-        else expand_main<kModeMid, false, DUPS>(P, smem, L, cd, mb, ph);
+        if (roots) expand_main<kModeMid, true, DUPS, false>(P, smem, L, cd, mb, ph);
+        else expand_main<kModeMid, false, DUPS, false>(P, smem, L, cd, mb, ph);
     }
 }
 
@@ -1205,11 +1328,11 @@ template <int LAST, bool DUPS>
 __device__ __forceinline__ void persist_heavy(const ExpandParams& P, unsigned char* smem, const uint8_t* cd,
                                               bool roots, bool last, const LevelLists& L, uint64_t* mb, uint32_t& ph) {
     if (last) {
-        if (roots) expand_heavy<LAST, true, DUPS>(P, smem, L, cd, mb, ph);
-        else expand_heavy<LAST, false, DUPS>(P, smem, L, cd, mb, ph);
+        if (roots) expand_heavy<LAST, true, DUPS, false>(P, smem, L, cd, mb, ph);
+        else expand_heavy<LAST, false, DUPS, false>(P, smem, L, cd, mb, ph);
     } else {
-        if (roots) expand_heavy<kModeMid, true, DUPS>(P, smem, L, cd, mb, ph);
-        else expand_heavy<kModeMid, false, DUPS>(P, smem, L, cd, mb, ph);
+        if (roots) expand_heavy<kModeMid, true, DUPS, false>(P, smem, L, cd, mb, ph);
+        else expand_heavy<kModeMid, false, DUPS, false>(P, smem, L, cd, mb, ph);
     }
 }
 
@@ -1277,14 +1400,16 @@ __global__ void __launch_bounds__(kWarps * 32, 5) k_persist(const __grid_constan
     }
 }
 
-template <int MODE, bool ROOTS, bool DUPS>
+template <int MODE, bool ROOTS, bool DUPS, bool SHARE = false>
 void* kernel_ptr(bool heavy) {
-    return heavy ? (void*)&k_expand_heavy<MODE, ROOTS, DUPS> : (void*)&k_expand<MODE, ROOTS, DUPS>;
+    return heavy ? (void*)&k_expand_heavy<MODE, ROOTS, DUPS, SHARE> : (void*)&k_expand<MODE, ROOTS, DUPS, SHARE>;
 }
 
-void* pick(int mode, bool roots, bool dups, bool heavy) {
+// `share`: the level has a buffer for shared intersections.
+void* pick(int mode, bool roots, bool dups, bool share, bool heavy) {
 #define FM_PICK(M)                                                                                     \
     if (mode == M) {                                                                                   \
+        if (share) return kernel_ptr<M, false, false, true>(heavy);                                    \
         if (roots) return dups ? kernel_ptr<M, true, true>(heavy) : kernel_ptr<M, true, false>(heavy); \
         return dups ? kernel_ptr<M, false, true>(heavy) : kernel_ptr<M, false, false>(heavy);          \
     }
@@ -1330,7 +1455,7 @@ size_t persist_smem_bytes(const DevPlan& plan, const uint32_t* nreq_depth, uint3
     size_t best = 0;
     for (uint32_t d = 1; d < plan.q; d++)
         best = std::max<size_t>(best, per_warp_bytes(d, nreq_depth[d], nreq_depth[d],
-                                                     nreq_depth[d] >= 2 ? stage_words : 0, true));
+                                                     nreq_depth[d] >= 2 ? stage_words : 0, true, 0));
     return best * kWarps;
 }
 
@@ -1384,9 +1509,9 @@ cudaError_t launch_vertex_sums(const ExpandParams& p, const uint32_t* heads, uin
 }
 
 size_t expand_smem_bytes(uint32_t depth, uint32_t nreq, int warps, uint32_t stage_words, bool staged, bool dups,
-                         bool sums) {
+                         bool sums, bool share) {
     return (size_t)warps * per_warp_bytes(depth, sums ? 2 : nreq, sums ? 2 : n_recs(nreq, dups, stage_words), stage_words,
-                                          staged);
+                                          staged, share ? kShareWords : 0);
 }
 
 void allow_dynamic_smem(const void* f) {
@@ -1428,22 +1553,23 @@ int blocks_per_sm(const void* f, int block, size_t smem) {
     return n;
 }
 
-int expand_blocks_per_sm(int mode, bool roots, bool dups, size_t smem, int block) {
-    void* f = pick(mode, roots, dups, false);
+int expand_blocks_per_sm(int mode, bool roots, bool dups, bool share, size_t smem, int block) {
+    void* f = pick(mode, roots, dups, share, false);
     allow_dynamic_smem(f);
-    allow_dynamic_smem(pick(mode, roots, dups, true));
+    allow_dynamic_smem(pick(mode, roots, dups, share, true));
     return std::max(1, blocks_per_sm(f, block, smem));
 }
 
-cudaError_t launch_expand(const ExpandParams& p, int mode, bool roots, bool dups, bool overlap, int grid,
+cudaError_t launch_expand(const ExpandParams& p, int mode, bool roots, bool dups, bool share, bool overlap, int grid,
                           int heavy_grid, int block, size_t smem, cudaStream_t s) {
-    void* f = pick(mode, roots, dups, false);
-    void* fh = pick(mode, roots, dups, true);
+    void* f = pick(mode, roots, dups, share, false);
+    void* fh = pick(mode, roots, dups, share, true);
     if (!f || !fh) return cudaErrorInvalidValue;
     ExpandParams q = p;
     // both passes tune themselves on the device (make_tune) from the level size
     // and from max_warps, the warps of the heavy pass
     q.max_warps = (uint32_t)heavy_grid * (uint32_t)(block / 32);
+    q.share_words = share ? kShareWords : 0;
     void* args[] = {(void*)&q};
     cudaError_t e = launch_pass(f, grid, block, smem, args, overlap, s);
     if (e != cudaSuccess || 32ull * p.max_list <= kHeavyLeast) return e;

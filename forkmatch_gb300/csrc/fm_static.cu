@@ -91,8 +91,8 @@ struct StaticRun {
         uint32_t* def_b = def_a + kStaticDefCap;
         uint32_t ndef_in = 0;
         uint64_t fresh = 0;
-        const size_t smem = expand_smem_bytes(d, nreq[d], block / 32, 0, mode != kModeLastCount, dups, false);
-        const int per_sm = expand_blocks_per_sm(mode, roots, dups, smem, block);
+        const size_t smem = expand_smem_bytes(d, nreq[d], block / 32, 0, mode != kModeLastCount, dups, false, false);
+        const int per_sm = expand_blocks_per_sm(mode, roots, dups, false, smem, block);
         // A launch defers at most 8 chunks per warp (the largest claim batch),
         // so a grid of at most kStaticDefCap / (8 * warps per block) blocks
         // keeps one launch's deferred chunks within a list whatever the SM
@@ -119,7 +119,7 @@ struct StaticRun {
             int grid = (int)std::min<uint64_t>(want, (uint64_t)full);
             if (grid < 1) grid = 1;
             FM_CUDA(cudaMemsetAsync(ctl, 0, sizeof(LaunchCtl), s));
-            FM_CUDA(launch_expand(p, mode, roots, dups, false, grid, full, block, smem, s));
+            FM_CUDA(launch_expand(p, mode, roots, dups, false, false, grid, full, block, smem, s));
             LaunchCtl c;
             FM_CUDA(cudaMemcpyAsync(&c, ctl, sizeof(LaunchCtl), cudaMemcpyDeviceToHost, s));
             FM_CUDA(cudaStreamSynchronize(s));

@@ -49,3 +49,30 @@ def test_one_edge_per_label(ctx, labels):
     q = fm.Query.from_text(S.query_cycle(3, [1, min(2, labels), min(3, labels)]).to_g_text())
     assert fm.match(ctx, g, q, mode=fm.MODE_COUNT).count == (6 if labels == 1 else 1)
     g.close()
+
+
+def test_shared_intersections(ctx):
+    """Levels with enough chunks to share the intersection of their two oldest lists: it fits the buffer (complete
+    graph), it does not for pairs of hubs and does for a hub and a leaf (hubs joined to everything), and it is the
+    whole candidate list (a vertex on two old ones, the newest column free)."""
+    V, s, d, l = complete_graph(104)
+    g = fm.Graph.from_edges(ctx, V, 2, s, d, l)
+    k4 = fm.Query.from_text(S.query_clique(4, [1]).to_g_text())
+    assert fm.match(ctx, g, k4, mode=fm.MODE_COUNT).count == math.perm(104, 4)
+    g.close()
+    hubs, leaves = 40, 1100
+    e = np.array([(a, b) for a in range(hubs) for b in range(a)] +
+                 [(a, hubs + b) for a in range(hubs) for b in range(leaves)], dtype=np.uint32)
+    src, dst = np.concatenate([e[:, 0], e[:, 1]]), np.concatenate([e[:, 1], e[:, 0]])
+    g = fm.Graph.from_edges(ctx, hubs + leaves, 2, src, dst, np.ones(len(src), dtype=np.uint32))
+    for order in (fm.ORDER_AUTO, fm.ORDER_REFERENCE):
+        r = fm.match(ctx, g, k4, mode=fm.MODE_COUNT, order=order)
+        assert r.count == math.perm(hubs, 4) + 4 * math.perm(hubs, 3) * leaves
+    g.close()
+    V, s, d, l = complete_graph(40)
+    g = fm.Graph.from_edges(ctx, V, 2, s, d, l)
+    q = S.Query(5, [(0, 1, 1), (0, 2, 1), (1, 2, 1), (2, 3, 1), (0, 4, 1), (1, 4, 1)])
+    query = fm.Query.from_text(q.to_g_text())
+    for order in (fm.ORDER_AUTO, fm.ORDER_REFERENCE):
+        assert fm.match(ctx, g, query, mode=fm.MODE_COUNT, order=order).count == math.perm(40, 5)
+    g.close()
