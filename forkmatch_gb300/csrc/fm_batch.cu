@@ -529,7 +529,7 @@ __device__ __forceinline__ void bexpand_main(const BatchParams& P, unsigned char
     unsigned long long n_lookups = 0, n_words = 0, n_parents = 0, credit = 0;
     uint32_t nst = 0;
     uint32_t last_chunk = 0xffffffffu;   // chunk whose rows are in m.rows_s
-    bool done = false;
+    bool done = !dev::warp_needed(T.n_items);
     while (!done) {
         unsigned long long first = 0;
         if (lane == 0) first = atomicAdd(&P.ctl->claim, (unsigned long long)T.claim_batch);
@@ -640,7 +640,7 @@ __device__ __forceinline__ void bexpand_heavy(const BatchParams& P, unsigned cha
     const unsigned long long h = *(volatile unsigned long long*)&P.ctl->heavy;
     const uint32_t nent = (uint32_t)(h >> 32);
     const uint32_t npieces = (uint32_t)h;
-    if (nent == 0) return;
+    if (nent == 0 || !dev::warp_needed(npieces)) return;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t d = P.depth;
     const uint32_t sw = P.kmax >= 2 ? P.stage_words : 0;

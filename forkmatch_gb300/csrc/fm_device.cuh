@@ -320,6 +320,15 @@ __device__ __forceinline__ uint32_t order_lists(uint4* recs, uint32_t lane, uint
     return 0;
 }
 
+// Warps are numbered across the blocks first, so that the warps that a small
+// pass needs are spread over the SMs.  A warp whose number is not below the
+// pass's work items claims nothing: the others take every item, and thousands
+// of claims on one counter (about 1 ns each) were most of a small pass's time
+// (twelve levels, eight of them nearly empty, of 912 blocks: 315 to 299 us).
+__device__ __forceinline__ bool warp_needed(unsigned long long items) {
+    return (unsigned long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x < items;
+}
+
 // Which parent a candidate slot of a chunk belongs to.  The parents with
 // candidates are listed in order (`start`: first slot and lane of each); a
 // window of 32 consecutive slots starts in the middle of some parent's range,

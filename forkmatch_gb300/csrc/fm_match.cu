@@ -730,7 +730,7 @@ __device__ __forceinline__ void expand_main(const ExpandParams& P, unsigned char
     uint32_t last_chunk = 0xffffffffu;   // chunk whose rows are in m.rows_s
     unsigned long long credit = 0;   // level budget held by this warp (lane 0)
     uint32_t nst = 0;
-    bool done = false;
+    bool done = !dev::warp_needed(T.n_items);
     while (!done) {
         unsigned long long first = 0;
         if (lane == 0) first = atomicAdd(&P.ctl->claim, (unsigned long long)T.claim_batch);
@@ -865,7 +865,7 @@ __device__ __forceinline__ void expand_heavy(const ExpandParams& P, unsigned cha
     const unsigned long long h = *(volatile unsigned long long*)&P.ctl->heavy;
     const uint32_t nent = (uint32_t)(h >> 32);
     const uint32_t npieces = (uint32_t)h;
-    if (nent == 0) return;
+    if (nent == 0 || !dev::warp_needed(npieces)) return;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t d = P.depth;
     const uint32_t k = P.plan.nreq[d];
@@ -1058,7 +1058,7 @@ __device__ __forceinline__ void expand_sum_main(const ExpandParams& P, unsigned 
     const bool chain = sp.last_anc == d;
     unsigned long long n_count = 0, n_parents = 0, n_words = 0;   // lane-private
     PreAcc pre;
-    for (;;) {
+    while (dev::warp_needed(T.n_items)) {
         unsigned long long first = 0;
         if (lane == 0) first = atomicAdd(&P.ctl->claim, (unsigned long long)T.claim_batch);
         first = __shfl_sync(kFull, first, 0);
@@ -1152,7 +1152,7 @@ __device__ __forceinline__ void expand_sum_heavy(const ExpandParams& P, unsigned
     const unsigned long long h = *(volatile unsigned long long*)&P.ctl->heavy;
     const uint32_t nent = (uint32_t)(h >> 32);
     const uint32_t npieces = (uint32_t)h;
-    if (nent == 0) return;
+    if (nent == 0 || !dev::warp_needed(npieces)) return;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t d = P.depth;
     const WarpMem m = warp_mem(smem_raw, threadIdx.x >> 5, d, 2, 2, 0, false, 0, mbar_s);
