@@ -564,6 +564,9 @@ struct MatchRun {
         const uint32_t q = plan->q;
         const uint32_t last = last_depth();
         cudaEvent_t ev[kMaxQ][2] = {};
+        // What a level can hold at most: the roots times the longest list per
+        // depth.  On a small graph that needs few blocks.
+        uint64_t most = n_roots;
         for (uint32_t d = 1; d <= last; d++) {
             const int mode = mode_of(d);
             const bool roots = d == 1;
@@ -590,6 +593,8 @@ struct MatchRun {
                 grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((p.n_items + 7) / 8, (uint64_t)full));
             } else {
                 p.n_parents_dev = &ctx->ctl[d - 1].produced;
+                most = std::min<uint64_t>(level_cap, most * std::max(1u, g->max_len));
+                grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((most + 255) / 256, (uint64_t)full));
             }
             if (profile) FM_TRY(begin_timing(ev[d][0], ev[d][1]));
             if (sums && d == last) {
@@ -799,6 +804,14 @@ __global__ void k_iota_rows(uint32_t* out, uint64_t n, uint32_t first, uint64_t 
 
 namespace {
 
+// Whether a match may count its last two depths by sums, its plan permitting:
+// counting, no vertex in its own list, no duplicates, no work limit (which
+// counts candidate by candidate), the level-launch engine.
+bool sums_allowed(const DeviceGraph& g, const fm_match_opts& opts) {
+    return opts.mode != FM_MODE_TABLE && !g.has_dups && !g.has_self_loops && !opts.work_limit && pre_count_knob() &&
+           (opts.engine != FM_ENGINE_PERSISTENT || opts.profile);
+}
+
 // fm_match with the table written into `region` (device memory, `region_rows`
 // rows) instead of the start of OUTPUT_PREALLOC when `region` is set.
 fm_status match_impl(fm_context* ctx, const fm_graph* graph, const fm_query* query, const fm_match_opts& opts,
@@ -849,6 +862,19 @@ fm_status match_impl(fm_context* ctx, const fm_graph* graph, const fm_query* que
     if (!use_ref) {
         choose_order(pl, g, order);
         if (!order_requirements(pl, order, nreq, climb, rlab)) use_ref = true;
+    }
+    // Counting by sums intersects, for a chain at the end of the order, one list
+    // per row vertex, and for a fork (both last vertices hang on earlier ones)
+    // only one: an order with the same prefix cost that ends in a fork is
+    // better.  5-vertex path on 2^22 vertices: 6.5 ms for the counting level,
+    // 14.4 with the chain's order.
+    if (!use_ref && sums_allowed(g, opts) && q >= 5 && nreq[q - 1] == 1 && nreq[q - 2] == 1 && climb[q - 1][0] == 1 &&
+        g.symmetric) {
+        uint32_t fork[kMaxQ];
+        if (choose_fork_order(pl, g, order, fork)) {
+            std::memcpy(order, fork, sizeof(order));
+            if (!order_requirements(pl, order, nreq, climb, rlab)) use_ref = true;
+        }
     }
     if (use_ref) {
         for (uint32_t d = 0; d < q; d++) {
@@ -925,8 +951,7 @@ fm_status match_impl(fm_context* ctx, const fm_graph* graph, const fm_query* que
         // bytes a vertex of the level memory, at most an eighth of it, and a
         // launch of their own: below 4096 lists that launch (3 us) is more
         // than the level saves (300 vertices: 86 us a match with, 83 without).
-        if (run.pre && q >= 4 && nreq[q - 2] == 1 && !g.has_self_loops && !opts.work_limit &&
-            (opts.engine != FM_ENGINE_PERSISTENT || opts.profile)) {
+        if (run.pre && q >= 4 && nreq[q - 2] == 1 && sums_allowed(g, opts)) {
             const uint32_t a = dp.req_anc[dp.req_begin[q - 2]], l = dp.req_label[dp.req_begin[q - 2]];
             const uint32_t b = dp.req_anc[dp.req_begin[q - 1]], ll = dp.req_label[dp.req_begin[q - 1]];
             const bool chain = b == q - 2;

@@ -455,68 +455,146 @@ bool order_requirements(const Plan& P, const uint32_t* order, uint32_t nreq[kMax
 // possible), ties broken by more back e-lines, larger degree, lower local
 // index; the start with the smallest summed partial-match estimate wins, and
 // ties keep the reference's start (local index 0 comes first).
-void choose_order(const Plan& P, const DeviceGraph& g, uint32_t order[kMaxQ]) {
-    const uint32_t q = P.q;
-    for (uint32_t d = 0; d < q; d++) order[d] = P.order_local[d];
-    if (q <= 2 || g.V == 0) return;
-    const double V = (double)g.V;
-    auto avg = [&](uint32_t l) {
-        uint64_t c = l < g.label_count.size() ? g.label_count[l] : 0;
-        return (double)c / V;
-    };
-    const RowIndex row(P);
-    std::vector<double> line_avg(P.rows.size());
-    for (size_t r = 0; r < P.rows.size(); r++) line_avg[r] = avg(P.rows[r].l);
-    auto deg = [&](uint32_t v) { return row.begin[v + 1] - row.begin[v]; };
-    double best = -1;
-    uint32_t cand[kMaxQ];
-    for (uint32_t start = 0; start < q; start++) {
+namespace {
+
+struct OrderModel {
+    const Plan& P;
+    RowIndex row;
+    double V;
+    std::vector<double> line_avg;
+
+    OrderModel(const Plan& plan, const DeviceGraph& g) : P(plan), row(plan), V((double)g.V), line_avg(plan.rows.size()) {
+        for (size_t r = 0; r < P.rows.size(); r++) {
+            const uint32_t l = P.rows[r].l;
+            line_avg[r] = (double)(l < g.label_count.size() ? g.label_count[l] : 0) / V;
+        }
+    }
+    uint32_t deg(uint32_t v) const { return row.begin[v + 1] - row.begin[v]; }
+
+    // Back e-lines of v to matched vertices and its estimated factor.
+    uint32_t factor(uint32_t v, const bool* matched, double& f) const {
+        double mn = 1e300, prod = 1.0;
+        uint32_t back = 0;
+        for (uint32_t r = row.begin[v]; r < row.begin[v + 1]; r++) {
+            if (!matched[P.rows[r].b]) continue;
+            const double a = line_avg[r];
+            back++;
+            if (a < mn) {
+                if (mn < 1e299) prod *= mn / V;
+                mn = a;
+            } else {
+                prod *= a / V;
+            }
+        }
+        f = mn * prod;
+        return back;
+    }
+
+    // Greedy order of the n vertices not `left` from `start`; its summed
+    // partial-match estimate, or -1 if they are not connected.
+    double greedy(uint32_t start, const bool* left, uint32_t n, uint32_t* cand) const {
         bool matched[kMaxQ] = {};
         matched[start] = true;
         cand[0] = start;
         double card = V, cost = V;
-        bool ok = true;
-        for (uint32_t d = 1; d < q && ok; d++) {
+        for (uint32_t d = 1; d < n; d++) {
             int pick = -1;
             double pf = 0;
             uint32_t pback = 0;
-            for (uint32_t v = 0; v < q; v++) {
-                if (matched[v]) continue;
-                double mn = 1e300, prod = 1.0;
-                uint32_t back = 0;
-                for (uint32_t r = row.begin[v]; r < row.begin[v + 1]; r++) {
-                    if (!matched[P.rows[r].b]) continue;
-                    const double a = line_avg[r];
-                    back++;
-                    if (a < mn) {
-                        if (mn < 1e299) prod *= mn / V;
-                        mn = a;
-                    } else {
-                        prod *= a / V;
-                    }
-                }
+            for (uint32_t v = 0; v < P.q; v++) {
+                if (matched[v] || left[v]) continue;
+                double f;
+                const uint32_t back = factor(v, matched, f);
                 if (!back) continue;
-                double f = mn * prod;
-                bool better = pick < 0 || f < pf * (1 - 1e-12) ||
-                              (f <= pf * (1 + 1e-12) && (back > pback || (back == pback && deg(v) > deg(pick))));
+                const bool better = pick < 0 || f < pf * (1 - 1e-12) ||
+                                    (f <= pf * (1 + 1e-12) && (back > pback || (back == pback && deg(v) > deg(pick))));
                 if (better) {
                     pick = (int)v;
                     pf = f;
                     pback = back;
                 }
             }
-            if (pick < 0) { ok = false; break; }
+            if (pick < 0) return -1;
             matched[pick] = true;
             cand[d] = (uint32_t)pick;
             card *= pf;
             cost += card;
         }
-        if (!ok) continue;
-        if (best < 0 || cost < best * (1 - 1e-9)) {
-            best = cost;
-            for (uint32_t d = 0; d < q; d++) order[d] = cand[d];
+        return cost;
+    }
+
+    // The cheapest greedy order over every start; -1 if none.
+    double best(const bool* left, uint32_t n, uint32_t* order) const {
+        double best = -1;
+        uint32_t cand[kMaxQ];
+        for (uint32_t start = 0; start < P.q; start++) {
+            if (left[start]) continue;
+            const double cost = greedy(start, left, n, cand);
+            if (cost < 0) continue;
+            if (best < 0 || cost < best * (1 - 1e-9)) {
+                best = cost;
+                for (uint32_t d = 0; d < n; d++) order[d] = cand[d];
+            }
+        }
+        return best;
+    }
+};
+
+}  // namespace
+
+void choose_order(const Plan& P, const DeviceGraph& g, uint32_t order[kMaxQ]) {
+    const uint32_t q = P.q;
+    for (uint32_t d = 0; d < q; d++) order[d] = P.order_local[d];
+    if (q <= 2 || g.V == 0) return;
+    const bool none[kMaxQ] = {};
+    OrderModel(P, g).best(none, q, order);
+}
+
+bool choose_fork_order(const Plan& P, const DeviceGraph& g, const uint32_t* order, uint32_t fork[kMaxQ]) {
+    const uint32_t q = P.q;
+    if (q < 4 || g.V == 0) return false;
+    const OrderModel M(P, g);
+    // a query e-line is a requirement of the end matched later, so only a query
+    // that lists every e-line from both ends may be matched in any order
+    for (const auto& e : P.rows) {
+        bool back = false;
+        for (uint32_t r = M.row.begin[e.b]; r < M.row.begin[e.b + 1]; r++)
+            back |= P.rows[r].b == e.a && P.rows[r].l == e.l;
+        if (!back) return false;
+    }
+    // what the given order's first q - 2 vertices cost
+    double limit = M.V;
+    {
+        bool matched[kMaxQ] = {};
+        matched[order[0]] = true;
+        double card = M.V;
+        for (uint32_t d = 1; d + 2 < q; d++) {
+            double f;
+            if (!M.factor(order[d], matched, f)) return false;
+            card *= f;
+            limit += card;
+            matched[order[d]] = true;
         }
     }
+    double best = -1;
+    uint32_t tried = 0;
+    for (uint32_t a = 0; a < q; a++) {
+        if (M.deg(a) != 1) continue;
+        for (uint32_t b = a + 1; b < q && tried < 16; b++) {       // bounded planning work on stars
+            if (M.deg(b) != 1 || P.rows[M.row.begin[a]].b == b) continue;
+            tried++;
+            bool left[kMaxQ] = {};
+            left[a] = left[b] = true;
+            uint32_t cand[kMaxQ];
+            const double cost = M.best(left, q - 2, cand);
+            if (cost < 0 || cost > 1.25 * limit || (best >= 0 && cost >= best * (1 - 1e-9))) continue;
+            best = cost;
+            for (uint32_t d = 0; d + 2 < q; d++) fork[d] = cand[d];
+            fork[q - 2] = a;
+            fork[q - 1] = b;
+        }
+    }
+    return best >= 0;
 }
 
 void estimate_level_rows(const Plan& P, const DeviceGraph& g, double est[kMaxQ]) {
