@@ -76,3 +76,21 @@ def test_shared_intersections(ctx):
     for order in (fm.ORDER_AUTO, fm.ORDER_REFERENCE):
         assert fm.match(ctx, g, query, mode=fm.MODE_COUNT, order=order).count == math.perm(40, 5)
     g.close()
+
+
+@pytest.mark.parametrize("n", [2, 45, 46, 64])
+def test_tables_around_the_first_read_back(ctx, n):
+    """Tables just below, at and above the 16 KiB that are read back with the totals, and host buffers smaller than
+    the table: 2-vertex rows of a complete graph (45 * 44 * 8 bytes is 15840, 46 * 45 * 8 is 16560)."""
+    V, s, d, l = complete_graph(n)
+    g = fm.Graph.from_edges(ctx, V, 2, s, d, l)
+    q = fm.Query.from_text(S.query_path(2, [1]).to_g_text())
+    want = sorted((int(a), int(b)) for a in range(n) for b in range(n) if a != b)
+    for cap in {1, len(want) - 1, len(want), len(want) + 7}:
+        buf = np.full((cap + 1) * 2, 7, dtype=np.uint32)
+        r = fm.match(ctx, g, q, host_rows=buf[:cap * 2])
+        assert r.count == len(want) and r.rows_copied == min(cap, len(want))
+        rows = list(map(tuple, buf[:2 * r.rows_copied].reshape(-1, 2).tolist()))
+        assert len(set(rows)) == len(rows) and set(rows) <= set(want)
+        assert (buf[2 * r.rows_copied:] == 7).all()
+    g.close()
