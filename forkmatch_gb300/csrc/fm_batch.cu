@@ -36,7 +36,15 @@ struct BatchPlan {                    // per query, in device memory
     uint32_t count_only;              // no table for this query (count rule allowed)
     uint32_t pre_ok;                  // last depth has one back edge: when counting, depth q-2 counts
                                       // each survivor's extensions and depth q-1 is never reached
+    uint32_t sum_kind;                // pre-counted by sums (see SumKind), 0: candidate by candidate
+    const uint2* vsum;                // its vertex sums (chains, forks of one vertex by two labels)
 };
+
+// Pre-count by sums in a batch (see expand_sum_main in fm_match.cu): the lane adds
+// its parent's closed part, and at most one list intersection is walked in its
+// place, each of whose members takes one off.  So chains are taken at depth 2
+// only (one row vertex besides r_a), forks at any depth.
+enum SumKind : uint32_t { kSumNone = 0, kSumChain = 1, kSumFork = 2, kSumForkOne = 3, kSumForkSame = 4 };
 
 struct BatchParams {
     const BatchPlan* plans;
@@ -139,7 +147,8 @@ struct BMem {
     uint32_t* qid_s;    // [32]
     uint8_t* drv_s;     // [32]
     uint8_t* k_s;       // [32] requirements of the parent's query at this depth
-    uint8_t* fin_s;     // [32] 1: the parent's query ends at this depth; 2: it is pre-counted here
+    uint8_t* fin_s;     // [32] 1: the parent's query ends at this depth; 2: it is pre-counted here;
+                        //      3: it is pre-counted by sums here (survivors are taken off)
     uint32_t* stp;      // [kBStage] staged parent index
     uint32_t* stx;      // [kBStage] staged vertex
     uint32_t* stq;      // [kBStage] staged query id
@@ -254,6 +263,47 @@ __device__ __forceinline__ bool bstage_lists(const BatchParams& P, const BMem& m
     return ok;
 }
 
+// A parent counted by sums: its closed part; the shorter of the two lists whose
+// members are to be taken off goes to `drv_rec` (index `drv`, length `n`).
+__device__ __forceinline__ unsigned long long bsum_parent(const BatchParams& P, const BMem& m, const BSlices& S,
+                                                          const BatchPlan& pl, const uint4 a, uint32_t anc, uint32_t lab,
+                                                          uint32_t lane, uint32_t d, uint4& drv_rec, uint32_t& drv,
+                                                          uint32_t& n) {
+    const uint32_t rl = pl.req_begin[d + 1], last_anc = pl.req_anc[rl], ll = pl.req_label[rl];
+    const uint4* last = P.seg + (uint64_t)ll * P.V;
+    const uint32_t va = m.rows_s[anc * 32 + lane];
+    uint32_t in_a = dev::member_mask(a, m.rows_s, lane, d, anc, S.at(P, lab), va, P.nbr, P.bm, P.bm_words);
+    const unsigned long long free_a = a.x - __popc(in_a);
+    unsigned long long c;
+    uint32_t u = last_anc;
+    if (pl.sum_kind == kSumChain) {
+        const uint2 w = __ldcg(pl.vsum + va);
+        c = (unsigned long long)w.x - w.y;
+        if (in_a) {
+            const uint4 own = ldg4(last + va);
+            for (; in_a; in_a &= in_a - 1) {
+                const uint32_t v = m.rows_s[(__ffs(in_a) - 1) * 32 + lane];
+                c -= __ldg(&last[v].x);
+                c += seg_has(own, v, 1, P.nbr, P.bm, P.bm_words) ? 1u : 0u;
+            }
+        }
+        u = 1 - anc;                     // depth 2: the other row vertex
+    } else {
+        const uint32_t vb = m.rows_s[last_anc * 32 + lane];
+        const uint4 b = ldg4(last + vb);
+        const uint32_t in_b = dev::member_mask(b, m.rows_s, lane, d, last_anc, S.at(P, ll), vb, P.nbr, P.bm, P.bm_words);
+        c = free_a * (b.x - __popc(in_b));
+        if (pl.sum_kind == kSumForkSame) return c - free_a;
+        if (pl.sum_kind == kSumForkOne) return c - (__ldcg(&pl.vsum[va].y) - __popc(in_a & in_b));
+    }
+    const uint4 b = ldg4(last + m.rows_s[u * 32 + lane]);
+    m.ref_s[32 + lane] = (uint16_t)(u | ll << 8);
+    drv = b.x < a.x ? 1u : 0u;
+    drv_rec = drv ? b : a;
+    n = drv_rec.x;
+    return c;
+}
+
 template <bool ROOTS>
 __device__ __forceinline__ uint32_t bload_chunk(const BatchParams& P, const BMem& m, uint32_t chunk, uint32_t lane,
                                                 uint32_t d, unsigned long long n_parents, bool& valid,
@@ -281,7 +331,7 @@ __device__ __forceinline__ uint32_t bload_chunk(const BatchParams& P, const BMem
         k = pl.nreq[d];
         // bit 0: the query ends at this depth; bit 1: it is counted here (pre-count)
         fin = (pl.q == d + 1) ? 1u : 0u;
-        if (pl.q == d + 2 && pl.pre_ok && (!P.table_mode || pl.count_only)) fin = 2u;
+        if (pl.q == d + 2 && pl.pre_ok && (!P.table_mode || pl.count_only)) fin = pl.sum_kind ? 3u : 2u;
         const uint32_t rb = pl.req_begin[d];
         uint4 best = make_uint4(0xffffffffu, 0, 0, 0);
         for (uint32_t i = 0; i < k; i++) {
@@ -298,6 +348,12 @@ __device__ __forceinline__ uint32_t bload_chunk(const BatchParams& P, const BMem
             }
         }
         n = best.x;
+        if (fin == 3u) {
+            const uint32_t ref = m.ref_s[lane];
+            n = 0;
+            if (best.x) rule_cnt = bsum_parent(P, m, S, pl, best, ref & 0xffu, ref >> 8, lane, d, best, drv, n);
+            if (n) k = 2;
+        }
         if (!sw) m.segs_s[lane] = best;
         if (fin == 1u && k == 1 && (!P.table_mode || pl.count_only)) {
             // Count rule (the query's count only): every entry of the single
@@ -411,6 +467,11 @@ __device__ __forceinline__ void bemit(const BatchParams& P, const BMem& m, const
     const uint32_t fs = ok ? m.fin_s[j] : 0u;
     bfinal(P, m, fs == 1u, j, x, lane, d);
     bprecount(P, m, S, fs == 2u, j, x, lane, d);
+    if (__ballot_sync(kFull, fs == 3u)) {
+        const uint32_t key = fs == 3u ? m.qid_s[j] : 0xffffffffu;
+        const unsigned grp = __match_any_sync(kFull, key);
+        if (fs == 3u && (int)lane == __ffs(grp) - 1) atomicAdd(&P.qpos[key], 0ull - (unsigned long long)__popc(grp));
+    }
     const bool stage = ok && fs == 0u;
     const unsigned b = __ballot_sync(kFull, stage);
     if (stage) {
@@ -588,13 +649,16 @@ __device__ __forceinline__ void bexpand_main(const BatchParams& P, unsigned char
                 n_parents += 1;
             }
             {
-                // count-rule counts: one atomic per query present in the chunk
-                // (each lane's count is below 2^27, a warp's sum below 2^32)
+                // count-rule and sum counts: one atomic per query present in the
+                // chunk, summed in three parts of at most 26 bits
                 const uint32_t key = rule_cnt ? m.qid_s[lane] : 0xffffffffu;
                 const unsigned grp = __match_any_sync(kFull, key);
-                const unsigned sum = __reduce_add_sync(grp, (unsigned)rule_cnt);
+                const unsigned lo = __reduce_add_sync(grp, (unsigned)(rule_cnt & 0x3ffffffu));
+                const unsigned mid = __reduce_add_sync(grp, (unsigned)(rule_cnt >> 26) & 0x3ffffffu);
+                const unsigned hi = __reduce_add_sync(grp, (unsigned)(rule_cnt >> 52));
                 if (key != 0xffffffffu && (int)lane == __ffs(grp) - 1)
-                    atomicAdd(&P.qpos[key], (unsigned long long)sum);
+                    atomicAdd(&P.qpos[key],
+                              lo + ((unsigned long long)mid << 26) + ((unsigned long long)hi << 52));
             }
             if (total > T.heavy_thresh) {
                 int pub = 0;
@@ -939,6 +1003,14 @@ struct fm_batch {
     // buffers, crowds out the others; it runs on the single-query engine
     // with the whole level memory, after the shared run, its table written
     // into its own region.  Indices are positions in `batched`.
+    // Vertex sums of the queries counted by sums: one table per (label, last
+    // label), at the end of the level region; recomputed by every run.
+    struct SumTable {
+        uint32_t label, last;
+        uint2* at;
+    };
+    std::vector<SumTable> sum_tables;
+
     std::vector<uint8_t> solo;
     std::vector<uint32_t> roots_all;      // n_roots of every batched plan (solo plans get 0 in h_plans)
     uint32_t n_solo = 0;
@@ -1055,12 +1127,38 @@ struct BatchRun {
         return m * kBWarps;
     }
 
+    // The tables of vertex sums that a counting query of this run reads.
+    fm_status enqueue_sums() {
+        for (const fm_batch::SumTable& t : b->sum_tables) {
+            bool used = false;
+            for (size_t i = 0; i < b->h_plans.size(); i++) {
+                const BatchPlan& bp = b->h_plans[i];
+                used |= bp.vsum == t.at && bp.n_roots && (!base.table_mode || bp.count_only);
+            }
+            if (!used) continue;
+            ExpandParams p;
+            std::memset(&p, 0, sizeof(p));
+            p.seg = g->seg;
+            p.nbr = g->nbr;
+            p.bm = g->bitmaps;
+            p.bm_words = g->bm_words;
+            p.efilter = g->efilter;
+            p.efilter_off = g->efilter_off;
+            p.V = g->V;
+            const uint64_t h = g->head_off[t.label];
+            FM_CUDA(launch_vertex_sums(p, g->heads + h, (uint32_t)(g->head_off[t.label + 1] - h), t.label, t.last, t.at,
+                                       nullptr, s));
+        }
+        return FM_OK;
+    }
+
     // The persistent run as stream work (what the CUDA graph captures): clear
     // the per-query results and control blocks, write the initial schedule,
     // one cooperative launch, read back the schedule and the per-query results.
     fm_status enqueue_persist() {
         FM_CUDA(cudaMemsetAsync(b->d_qpos, 0, nq * sizeof(unsigned long long), s));
         FM_CUDA(cudaMemsetAsync(cv.ctl, 0, b->maxq * sizeof(LaunchCtl), s));
+        FM_TRY(enqueue_sums());
         FM_CUDA(launch_sched_init(cv.sched, b->maxq, (unsigned long long)nq * base.chunks_per_query * 32, 0,
                                   60000ull * 1000000ull, s));
         BatchParams p = base;
@@ -1152,6 +1250,7 @@ struct BatchRun {
     fm_status enqueue_all() {
         FM_CUDA(cudaMemsetAsync(b->d_qpos, 0, nq * sizeof(unsigned long long), s));
         FM_CUDA(cudaMemsetAsync(cv.ctl, 0, b->maxq * sizeof(LaunchCtl), s));
+        FM_TRY(enqueue_sums());
         for (uint32_t d = 1; d < b->maxq; d++) {
             BatchParams p = level_params(d);
             if (d == 1) {
@@ -1342,15 +1441,47 @@ fm_status batch_create_impl(fm_context* ctx, const fm_graph* graph, const fm_que
     }
     const uint32_t nq = (uint32_t)plans.size();
     if (nq) {
-        for (uint32_t d = 1; d < b->maxq; d++) {
-            uint32_t km = 1;
-            for (auto& bp : plans)
-                if (d < bp.q) km = std::max(km, bp.nreq[d]);
-            b->kmax[d] = km;
-        }
         uint64_t sum_cols = 0;   // level d+1 rows hold d+1 vertices and a query id
         for (uint32_t d = 2; d < b->maxq; d++) sum_cols += d + 1;
-        uint64_t cap = sum_cols ? cv.soln_bytes / (4ull * sum_cols) : 0;
+        // queries counted by sums: as in fm_match, with at most an eighth of the
+        // level memory for their tables
+        uint64_t soln = cv.soln_bytes;
+        if (!stage_words_knob() && !g.has_self_loops) {
+            const uint64_t vbytes = ((uint64_t)g.V * sizeof(uint2) + 255) & ~255ull;
+            for (auto& bp : plans) {
+                const uint32_t q = bp.q;
+                if (!bp.pre_ok || q < 4 || bp.nreq[q - 2] != 1) continue;
+                const uint32_t a = bp.req_anc[bp.req_begin[q - 2]], l = bp.req_label[bp.req_begin[q - 2]];
+                const uint32_t c = bp.req_anc[bp.req_begin[q - 1]], ll = bp.req_label[bp.req_begin[q - 1]];
+                const bool chain = c == q - 2;
+                if (g.head_off[l + 1] - g.head_off[l] < 4096 || (chain && (q != 4 || !g.symmetric))) continue;
+                const uint32_t kind = chain ? kSumChain : a != c ? kSumFork : l != ll ? kSumForkOne : kSumForkSame;
+                if (kind == kSumChain || kind == kSumForkOne) {
+                    uint2* at = nullptr;
+                    for (auto& t : b->sum_tables)
+                        if (t.label == l && t.last == ll) at = t.at;
+                    if (!at) {
+                        if (soln < vbytes + 256 || cv.soln_bytes - soln + vbytes > cv.soln_bytes / 8 ||
+                            (soln - vbytes - 256) / (4ull * sum_cols) < (uint64_t)g.max_len * 32 + 32)
+                            continue;
+                        soln = (soln - vbytes) & ~255ull;
+                        at = (uint2*)(cv.soln + soln);
+                        b->sum_tables.push_back({l, ll, at});
+                    }
+                    bp.vsum = at;
+                }
+                bp.sum_kind = kind;
+            }
+        }
+        for (uint32_t d = 1; d < b->maxq; d++) {
+            uint32_t km = 1;
+            for (auto& bp : plans) {
+                if (d < bp.q) km = std::max(km, bp.nreq[d]);
+                if (bp.sum_kind && d + 2 == bp.q) km = std::max(km, 2u);   // the list it is met with
+            }
+            b->kmax[d] = km;
+        }
+        uint64_t cap = sum_cols ? soln / (4ull * sum_cols) : 0;
         cap = std::min<uint64_t>(cap, 0xffffffffull - 64);
         if (sum_cols && cap < (uint64_t)g.max_len * 32 + 32) {
             set_error("SOLN_PREALLOC cannot hold one 32-parent chunk per level for this graph");

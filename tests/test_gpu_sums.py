@@ -70,7 +70,7 @@ def test_sums_equal_enumeration(ctx, monkeypatch, kind, bitmaps):
     V, (src, dst, lab) = _edges(kind)
     g = fm.Graph.from_edges(ctx, V, 4, src, dst, lab)
     og = O.Graph.from_edges(V, 4, src, dst, lab)
-    small = fm.Context(prealloc_bytes=256 << 20, soln_prealloc_bytes=8 * 4 * 5 * (32 * g.info().max_list + 64) + 8 * V,
+    small = fm.Context(prealloc_bytes=256 << 20, soln_prealloc_bytes=8 * 4 * 7 * (32 * g.info().max_list + 64) + 128 * V,
                        output_prealloc_bytes=1 << 20, bank_rows=1)
     for text in _queries():
         p = O.plan(text, enumerate_aut=0)
@@ -89,5 +89,17 @@ def test_sums_equal_enumeration(ctx, monkeypatch, kind, bitmaps):
             assert r.level[d].parents == st.partials[d - 1], ("parents", d)
         for d in range(1, p.q - 1):
             assert r.level[d].produced == st.partials[d], ("produced", d)
+    # the same queries in shared launches, counting and as count-only ones of a table batch
+    queries = [fm.Query.from_text(t) for t in _queries()]
+    want = [fm.match(ctx, g, q, mode=fm.MODE_COUNT).count for q in queries]
+    for mode, engine in ((fm.MODE_COUNT, fm.ENGINE_LEVELS), (fm.MODE_COUNT, fm.ENGINE_PERSISTENT),
+                         (fm.MODE_TABLE, fm.ENGINE_LEVELS)):
+        for c in (ctx, small):
+            b = fm.Batch(c, g, queries, mode=mode)
+            b.set_engine(engine)
+            for i in range(len(queries)):
+                b.set_query_mode(i, fm.MODE_COUNT)
+            assert b.run()[0] == want and b.run()[0] == want
+            b.close()
     small.close()
     g.close()
