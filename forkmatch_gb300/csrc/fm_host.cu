@@ -874,10 +874,11 @@ fm_status match_impl(fm_context* ctx, const fm_graph* graph, const fm_query* que
     }
     // Counting by sums intersects, for a chain at the end of the order, one list
     // per row vertex, and for a fork (both last vertices hang on earlier ones)
-    // only one: an order with the same prefix cost that ends in a fork is
-    // better.  5-vertex path on 2^22 vertices: 6.5 ms for the counting level,
+    // only one: an order with about the same prefix cost that ends in a fork is
+    // better.  Over the full root range only: the count of a part of it belongs
+    // to the order's first vertex.  5-vertex path on 2^22 vertices: 6.5 ms for the counting level,
     // 14.4 with the chain's order.
-    if (!use_ref && sums_allowed(g, opts) && q >= 5 && nreq[q - 1] == 1 && nreq[q - 2] == 1 && climb[q - 1][0] == 1 &&
+    if (!use_ref && rb == 0 && re == g.V && sums_allowed(g, opts) && q >= 5 && nreq[q - 1] == 1 && nreq[q - 2] == 1 && climb[q - 1][0] == 1 &&
         g.symmetric) {
         uint32_t fork[kMaxQ];
         if (choose_fork_order(pl, g, order, fork)) {

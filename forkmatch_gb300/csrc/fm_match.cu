@@ -16,15 +16,18 @@
 //      turns the 32 parents' candidate lists into one range of slots;
 //   3. lanes take 64 consecutive slots per round, two per lane with both driver
 //      loads in flight (load-balanced across parents, so a hub parent keeps all
-//      32 lanes busy), reject values already in the row, test membership in
-//      the other k-1 lists (inline compare or binary search), and stage
-//      survivors as (parent index, value) in shared memory;
-//   4. the stage outlives the chunk: it is flushed with one atomic per 448+
-//      survivors and fully coalesced stores, column by column into the next
-//      level or as contiguous row-major rows into the table.
+//      32 lanes busy); one word of the e-line filter per other list rejects
+//      almost every candidate that is not in it, and what passes is queued
+//      and tested exactly 32 at a time (inline compare, bitmap or binary
+//      search, then against the row), and survivors are staged as (parent
+//      index, value) in shared memory;
+//   4. the stage outlives the chunk: it is flushed with one atomic per 96+
+//      survivors (224+ where every candidate survives) and fully coalesced
+//      stores, column by column into the next level or as contiguous
+//      row-major rows into the table.
 // A chunk whose candidate range is long (a hub) is not walked by one warp: it
 // is published to a heavy list and cut into pieces that every warp of a second
-// launch shares.  Lists of length <= 3 are inline in the segment record, so
+// launch shares; launches of one match overlap (dev::pass_wait).  Lists of length <= 3 are inline in the segment record, so
 // the common case needs no second memory access.  With duplicate e-lines the
 // value at rank r of its run in the driver list survives only if every other
 // list holds at least r + 1 copies (min-multiplicity semantics of the

@@ -103,7 +103,8 @@ typedef struct fm_graph_info {
     uint64_t nbr_words;         /* u32 words of out-of-line storage (16 B aligned) */
     uint32_t max_list;          /* longest (label, vertex) list */
     int32_t has_duplicates;     /* some (label, src, dst) e-line occurs twice */
-    uint64_t device_bytes;      /* graph bytes resident on the device */
+    uint64_t device_bytes;      /* records, lists, root lists and bitmaps on the device (the e-line
+                                   filter adds 2 bytes per e-line) */
     double build_ms;            /* device build time */
     uint32_t bitmaps;           /* lists that also have a membership bitmap over all vertices */
     uint32_t bitmap_min_len;    /* shortest list given a bitmap (0: none) */
