@@ -740,8 +740,13 @@ __device__ __forceinline__ void bexpand_heavy(const BatchParams& P, unsigned cha
     if (nst) bflush<ROOTS>(P, m, nst, lane, d, last_chunk);
 }
 
+// 4 blocks per SM (64 registers): a batch's passes are mostly small and the
+// per-lane plans spill at 40 registers.  48 mixed queries 13.7 ms at 6 blocks,
+// 13.4 at 5, 12.9 at 4, 13.7 at 3; 32 served walk counts 1.49, 1.40, 1.29, 1.27.
+constexpr int kBBlocks = 4;
+
 template <bool ROOTS>
-__global__ void __launch_bounds__(kBWarps * 32, 6) k_bexpand(const __grid_constant__ BatchParams P) {
+__global__ void __launch_bounds__(kBWarps * 32, kBBlocks) k_bexpand(const __grid_constant__ BatchParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint64_t mbar_s[kBWarps];
     __shared__ uint2 slices_s[FM_MAX_LABEL + 1];
@@ -754,7 +759,7 @@ __global__ void __launch_bounds__(kBWarps * 32, 6) k_bexpand(const __grid_consta
 }
 
 template <bool ROOTS>
-__global__ void __launch_bounds__(kBWarps * 32, 6) k_bexpand_heavy(const __grid_constant__ BatchParams P) {
+__global__ void __launch_bounds__(kBWarps * 32, kBBlocks) k_bexpand_heavy(const __grid_constant__ BatchParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint64_t mbar_s[kBWarps];
     __shared__ uint2 slices_s[FM_MAX_LABEL + 1];

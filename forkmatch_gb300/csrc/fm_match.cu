@@ -1266,8 +1266,17 @@ __global__ void __launch_bounds__(kWarps * 32) k_vertex_sums(const __grid_consta
     }
 }
 
+// Blocks per SM a pass is compiled for.  Closing and counting levels, which hold
+// most of a large match's work, want every warp they can get (6 blocks, 40
+// registers; 4 blocks: closing a 4-cycle 12 % slower).  Middle levels of walk
+// queries are mostly small, and there fewer, unspilled warps and fewer blocks to
+// start win: 4 blocks (64 registers) took a 13-vertex walk's match from 312 to
+// 267 us and left the large ones where they were (4-cycle 1069 and 1057 us, 3
+// blocks: 8-vertex walks and 4-cliques slower again).
+constexpr int min_blocks(int mode) { return mode == kModeMid ? 4 : 6; }
+
 template <int MODE, bool ROOTS, bool DUPS, bool SHARE>
-__global__ void __launch_bounds__(kWarps * 32, 6) k_expand(const __grid_constant__ ExpandParams P) {
+__global__ void __launch_bounds__(kWarps * 32, min_blocks(MODE)) k_expand(const __grid_constant__ ExpandParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint8_t col_depth_s[kMaxQ];
     __shared__ uint64_t mbar_s[kWarps];
@@ -1286,7 +1295,7 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_expand(const __grid_constant
 }
 
 template <int MODE, bool ROOTS, bool DUPS, bool SHARE>
-__global__ void __launch_bounds__(kWarps * 32, 6) k_expand_heavy(const __grid_constant__ ExpandParams P) {
+__global__ void __launch_bounds__(kWarps * 32, min_blocks(MODE)) k_expand_heavy(const __grid_constant__ ExpandParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint8_t col_depth_s[kMaxQ];
     __shared__ uint64_t mbar_s[kWarps];
