@@ -821,6 +821,58 @@ bool sums_allowed(const DeviceGraph& g, const fm_match_opts& opts) {
            (opts.engine != FM_ENGINE_PERSISTENT || opts.profile);
 }
 
+// What counting the last two depths by sums needs (see expand_sum_main).
+struct SumsPlan {
+    uint32_t label = 0, last = 0;    // of the last two depths' back edges
+    uint32_t lists = 0;              // lists of `label`
+    bool vertex = false;             // reads vertex sums, at `voff` of the level memory
+    uint64_t voff = 0;
+    uint64_t cap = 0;                // rows per level buffer beside them
+};
+
+// Lists of the counting level's label below which the rule is off.
+constexpr uint64_t kSumsMinLists = 4096;
+
+// Rows of every level buffer, depths 2 .. stored - 1, in `bytes` of level memory.
+uint64_t level_rows(uint64_t bytes, uint32_t stored, uint64_t bank) {
+    uint64_t sum_cols = 0;
+    for (uint32_t d = 2; d < stored; d++) sum_cols += d;
+    uint64_t cap = sum_cols ? bytes / (4ull * sum_cols) : 0;
+    cap = std::min<uint64_t>(cap, 0xffffffffull - 64);   // parent indices are 32-bit
+    return cap / bank * bank;
+}
+
+// One 32-parent chunk fits a level buffer of `cap` rows.
+bool rows_enough(const DeviceGraph& g, uint32_t stored, uint64_t cap) {
+    return stored <= 2 || (cap >= (uint64_t)g.max_len * 32 + 32 && cap > 0);
+}
+
+// Whether an order's last two depths can be counted by sums: one back edge
+// each, and a chain's lists can be read from either end.  Depth 1 is left to
+// enumeration: its parents are the label's lists, each of which the vertex sums
+// would walk once as well.  The sums take 8 bytes a vertex of the level memory,
+// at most an eighth of it, and a launch of their own: below 4096 lists that
+// launch (3 us) is more than the level saves (300 vertices: 86 us a match with,
+// 83 without).
+bool sums_plan(const fm_context* ctx, const DeviceGraph& g, uint32_t q, const uint32_t* nreq,
+               const uint32_t (*climb)[kMaxQ], const uint32_t (*rlab)[kMaxQ], SumsPlan& out) {
+    if (q < 4 || nreq[q - 2] != 1 || nreq[q - 1] != 1) return false;
+    out.label = rlab[q - 2][0];
+    out.last = rlab[q - 1][0];
+    if (out.label >= g.L || out.last >= g.L) return false;
+    const bool chain = climb[q - 1][0] == 1;
+    const bool same_vertex = climb[q - 1][0] == climb[q - 2][0] + 1;
+    out.vertex = chain || (same_vertex && out.label != out.last);
+    const uint64_t lists = g.head_off[out.label + 1] - g.head_off[out.label];
+    out.lists = (uint32_t)lists;
+    if ((chain && !g.symmetric) || lists < kSumsMinLists) return false;
+    const uint64_t vbytes = out.vertex ? (uint64_t)g.V * sizeof(uint2) : 0;
+    if (8 * vbytes > ctx->soln_bytes) return false;
+    out.voff = (ctx->soln_bytes - vbytes) & ~255ull;
+    out.cap = level_rows(out.voff, q - 1, ctx->knobs.bank_rows);
+    return rows_enough(g, q - 1, out.cap);
+}
+
 // fm_match with the table written into `region` (device memory, `region_rows`
 // rows) instead of the start of OUTPUT_PREALLOC when `region` is set.
 fm_status match_impl(fm_context* ctx, const fm_graph* graph, const fm_query* query, const fm_match_opts& opts,
@@ -875,15 +927,20 @@ fm_status match_impl(fm_context* ctx, const fm_graph* graph, const fm_query* que
     // Counting by sums intersects, for a chain at the end of the order, one list
     // per row vertex, and for a fork (both last vertices hang on earlier ones)
     // only one: an order with about the same prefix cost that ends in a fork is
-    // better.  Over the full root range only: the count of a part of it belongs
-    // to the order's first vertex.  5-vertex path on 2^22 vertices: 6.5 ms for the counting level,
-    // 14.4 with the chain's order.
-    if (!use_ref && rb == 0 && re == g.V && sums_allowed(g, opts) && q >= 5 && nreq[q - 1] == 1 && nreq[q - 2] == 1 && climb[q - 1][0] == 1 &&
-        g.symmetric) {
-        uint32_t fork[kMaxQ];
-        if (choose_fork_order(pl, g, order, fork)) {
+    // better, where its last two depths will be counted by sums (their candidates
+    // were never costed).  Over the full root range only: the count of a part of
+    // it belongs to the order's first vertex.  5-vertex path on 2^22 vertices:
+    // 6.5 ms for the counting level, 14.4 with the chain's order.
+    if (!use_ref && rb == 0 && re == g.V && sums_allowed(g, opts) && q >= 5 && nreq[q - 1] == 1 &&
+        nreq[q - 2] == 1 && climb[q - 1][0] == 1 && g.symmetric) {
+        uint32_t fork[kMaxQ], fnreq[kMaxQ], fclimb[kMaxQ][kMaxQ], flab[kMaxQ][kMaxQ];
+        SumsPlan sp;
+        if (choose_fork_order(pl, g, order, kSumsMinLists, fork) &&
+            order_requirements(pl, fork, fnreq, fclimb, flab) && sums_plan(ctx, g, q, fnreq, fclimb, flab, sp)) {
             std::memcpy(order, fork, sizeof(order));
-            if (!order_requirements(pl, order, nreq, climb, rlab)) use_ref = true;
+            std::memcpy(nreq, fnreq, sizeof(nreq));
+            std::memcpy(climb, fclimb, sizeof(climb));
+            std::memcpy(rlab, flab, sizeof(rlab));
         }
     }
     if (use_ref) {
@@ -939,46 +996,21 @@ fm_status match_impl(fm_context* ctx, const fm_graph* graph, const fm_query* que
         // level buffer (graphs with duplicate e-lines enumerate it)
         run.pre = !table && !g.has_dups && q >= 3 && nreq[q - 1] == 1 && pre_count_knob();
         const uint32_t stored = q - (run.pre ? 1u : 0u);   // depths with a level buffer: 2 .. stored-1
-        uint64_t sum_cols = 0;
-        for (uint32_t d = 2; d < stored; d++) sum_cols += d;
-        const uint64_t bank = ctx->knobs.bank_rows;
-        auto rows_in = [&](uint64_t bytes) {
-            uint64_t cap = sum_cols ? bytes / (4ull * sum_cols) : 0;
-            cap = std::min<uint64_t>(cap, 0xffffffffull - 64);   // parent indices are 32-bit
-            return cap / bank * bank;
-        };
-        auto enough = [&](uint64_t cap) { return !sum_cols || (cap >= (uint64_t)g.max_len * 32 + 32 && cap > 0); };
-        uint64_t cap = rows_in(ctx->soln_bytes);
-        if (!enough(cap)) {
+        uint64_t cap = level_rows(ctx->soln_bytes, stored, ctx->knobs.bank_rows);
+        if (!rows_enough(g, stored, cap)) {
             set_error("SOLN_PREALLOC cannot hold one 32-parent chunk per level for this graph");
             return FM_ERR_POOL;
         }
-        // Pre-count by sums: the counting level has one back edge too, no
-        // vertex is in its own list, and a chain's lists can be read from
-        // either end.  A work limit counts candidate by candidate.  Depth 1
-        // is left to enumeration: its parents are the label's lists, each of
-        // which the vertex sums would walk once as well.  The sums take 8
-        // bytes a vertex of the level memory, at most an eighth of it, and a
-        // launch of their own: below 4096 lists that launch (3 us) is more
-        // than the level saves (300 vertices: 86 us a match with, 83 without).
-        if (run.pre && q >= 4 && nreq[q - 2] == 1 && sums_allowed(g, opts)) {
-            const uint32_t a = dp.req_anc[dp.req_begin[q - 2]], l = dp.req_label[dp.req_begin[q - 2]];
-            const uint32_t b = dp.req_anc[dp.req_begin[q - 1]], ll = dp.req_label[dp.req_begin[q - 1]];
-            const bool chain = b == q - 2;
-            const bool vertex = chain || (a == b && l != ll);
-            const uint64_t vbytes = vertex ? (uint64_t)g.V * sizeof(uint2) : 0;
-            const uint64_t voff = 8 * vbytes <= ctx->soln_bytes ? (ctx->soln_bytes - vbytes) & ~255ull : 0;
-            const uint64_t lists = l < g.L ? g.head_off[l + 1] - g.head_off[l] : 0;
-            if ((!chain || g.symmetric) && lists >= 4096 && enough(rows_in(voff))) {
-                run.sums = true;
-                run.sum_label = l;
-                run.sum_last = ll;
-                cap = rows_in(voff);
-                if (vertex) {
-                    run.vsum = (uint2*)(ctx->soln + voff);
-                    run.base.vsum = run.vsum;
-                    run.base.sum_heads = (uint32_t)lists;
-                }
+        SumsPlan sp;
+        if (run.pre && sums_allowed(g, opts) && sums_plan(ctx, g, q, nreq, climb, rlab, sp)) {
+            run.sums = true;
+            run.sum_label = sp.label;
+            run.sum_last = sp.last;
+            cap = sp.cap;
+            if (sp.vertex) {
+                run.vsum = (uint2*)(ctx->soln + sp.voff);
+                run.base.vsum = run.vsum;
+                run.base.sum_heads = sp.lists;
             }
         }
         run.ctx = ctx;

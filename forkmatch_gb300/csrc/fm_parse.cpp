@@ -550,10 +550,30 @@ void choose_order(const Plan& P, const DeviceGraph& g, uint32_t order[kMaxQ]) {
     OrderModel(P, g).best(none, q, order);
 }
 
-bool choose_fork_order(const Plan& P, const DeviceGraph& g, const uint32_t* order, uint32_t fork[kMaxQ]) {
+bool choose_fork_order(const Plan& P, const DeviceGraph& g, const uint32_t* order, uint64_t min_lists,
+                       uint32_t fork[kMaxQ]) {
     const uint32_t q = P.q;
     if (q < 4 || g.V == 0) return false;
     const OrderModel M(P, g);
+    // The leaves over the most frequent labels: leaving two of those to the end
+    // leaves the cheapest prefix, so the pairs of the first three are planned and
+    // no others (each is a plan of its own, as dear as choose_order's: 150 us for a
+    // 32-vertex tree, which has up to 190 pairs).
+    uint32_t leaf[kMaxQ], leaves = 0;
+    bool any = false;
+    auto line = [&](uint32_t v) { return M.row.begin[v]; };
+    auto enough = [&](uint32_t v) {
+        const uint32_t l = P.rows[line(v)].l;
+        return l < g.L && g.head_off[l + 1] - g.head_off[l] >= min_lists;
+    };
+    for (uint32_t v = 0; v < q; v++) {
+        if (M.deg(v) != 1) continue;
+        leaf[leaves++] = v;
+        any |= enough(v);
+    }
+    if (leaves < 2 || !any) return false;
+    std::stable_sort(leaf, leaf + leaves,
+                     [&](uint32_t x, uint32_t y) { return M.line_avg[line(x)] > M.line_avg[line(y)]; });
     // a query e-line is a requirement of the end matched later, so only a query
     // that lists every e-line from both ends may be matched in any order
     for (const auto& e : P.rows) {
@@ -577,12 +597,13 @@ bool choose_fork_order(const Plan& P, const DeviceGraph& g, const uint32_t* orde
         }
     }
     double best = -1;
-    uint32_t tried = 0;
-    for (uint32_t a = 0; a < q; a++) {
-        if (M.deg(a) != 1) continue;
-        for (uint32_t b = a + 1; b < q && tried < 16; b++) {       // bounded planning work on stars
-            if (M.deg(b) != 1 || P.rows[M.row.begin[a]].b == b) continue;
-            tried++;
+    const uint32_t first = std::min(leaves, 3u);
+    for (uint32_t i = 0; i < first; i++) {
+        for (uint32_t j = i + 1; j < first; j++) {
+            uint32_t a = std::min(leaf[i], leaf[j]), b = std::max(leaf[i], leaf[j]);
+            if (P.rows[line(a)].b == b) continue;
+            if (!enough(a)) std::swap(a, b);
+            if (!enough(a)) continue;
             bool left[kMaxQ] = {};
             left[a] = left[b] = true;
             uint32_t cand[kMaxQ];

@@ -103,3 +103,28 @@ def test_sums_equal_enumeration(ctx, monkeypatch, kind, bitmaps):
             b.close()
     small.close()
     g.close()
+
+
+def _uneven(n, m):
+    """n vertices, about m edges; one edge in 50 carries label 1, the others 2 to 4 (fewer than 4096 lists of each)."""
+    rng = np.random.default_rng(3)
+    a, b = rng.integers(0, n, m), rng.integers(0, n, m)
+    lab = np.where(rng.random(m) < 0.02, 1, rng.integers(2, 5, m))
+    keep = a != b
+    e = np.unique(np.stack([np.minimum(a, b)[keep], np.maximum(a, b)[keep]], 1), axis=0, return_index=True)[1]
+    a, b, lab = a[keep][e], b[keep][e], lab[keep][e]
+    return [np.concatenate(x).astype(np.uint32) for x in ((a, b), (b, a), (lab, lab))]
+
+
+@pytest.mark.parametrize("edges,labels", [(20000, [2, 3, 4, 2]), (60000, [2, 3, 4, 2]), (60000, [1, 2, 1, 3]),
+                                          (400000, [3, 1, 2, 1])])
+def test_order_of_a_count_that_sums_cannot_serve(ctx, edges, labels):
+    """Too few lists for counting by sums: the count walks the table's matching order, not one chosen for the sums."""
+    g = fm.Graph.from_edges(ctx, 3000, 5, *_uneven(3000, edges))
+    q = fm.Query.from_text(S.query_path(5, labels).to_g_text())
+    t = fm.match(ctx, g, q, mode=fm.MODE_TABLE, allow_truncation=True)
+    c = fm.match(ctx, g, q, mode=fm.MODE_COUNT)
+    assert c.count == t.count
+    for d in range(1, 5):
+        assert (c.level[d].parents, c.level[d].list_words) == (t.level[d].parents, t.level[d].list_words), d
+    g.close()
