@@ -258,7 +258,7 @@ __device__ __forceinline__ bool stage_lists(const ExpandParams& P, const WarpMem
 template <bool ROOTS>
 __device__ __forceinline__ uint32_t parent_col(const ExpandParams& P, uint32_t c, uint32_t p) {
     if (ROOTS) return P.root_list ? __ldg(P.root_list + p) : P.root_begin + p;
-    return __ldcg(P.pin + c * P.pstride + p);
+    return P.pin[c * P.pstride + p];
 }
 
 // Column c of staged parent p: from the warp's copy of chunk `cur` in shared
@@ -453,7 +453,7 @@ __device__ __forceinline__ uint32_t load_chunk(const ExpandParams& P, const Warp
     if (ROOTS) {
         m.rows_s[lane] = !P.root_list ? P.root_begin + (uint32_t)p : valid ? __ldg(P.root_list + p) : 0u;
     } else {
-        for (uint32_t c = 0; c < d; c++) m.rows_s[c * 32 + lane] = valid ? __ldcg(P.pin + c * P.pstride + p) : 0u;
+        for (uint32_t c = 0; c < d; c++) m.rows_s[c * 32 + lane] = valid ? P.pin[c * P.pstride + p] : 0u;
     }
     uint32_t drv = 0;
     n = 0;
@@ -530,18 +530,19 @@ __device__ __forceinline__ void flush_pre(const ExpandParams& P, PreAcc& pre, ui
 
 // What survives a warp round at its level: lane's candidate x of parent j,
 // `ok` if it survived.  Counted, pre-counted, or staged for the next level or
-// the table; the stage is flushed when it cannot take another round.
+// the table; the stage is flushed when it cannot take another round, unless
+// `more` follows at once.
 struct Emit {
-    uint32_t& nst;                        // staged survivors (warp-uniform), of cap
-    uint32_t cap;
+    uint32_t& nst;                        // staged survivors (warp-uniform)
+    uint32_t flush_at;                    // flushed above this many
     unsigned long long& n_count;          // counted (warp-uniform)
     unsigned long long lane_count = 0;    // pre-counted by this lane
 };
 
 template <int MODE, bool ROOTS, bool DUPS>
 __device__ __forceinline__ void emit(const ExpandParams& P, const WarpMem& m, uint32_t chunk, bool ok, uint32_t j,
-                                     uint32_t x, uint32_t lane, uint32_t d, const uint8_t* col_depth_s, Emit& e,
-                                     PreAcc& pre) {
+                                     uint32_t x, uint32_t lane, uint32_t d, const uint8_t* col_depth_s, bool more,
+                                     Emit& e, PreAcc& pre) {
     if (MODE == kModeLastCount && !DUPS && P.pre_count) {
         // Pre-count: each survivor's extensions at the last depth (one back
         // edge: ancestor anc, label lab) are the entries of that list minus
@@ -570,8 +571,9 @@ __device__ __forceinline__ void emit(const ExpandParams& P, const WarpMem& m, ui
         m.stx[q] = x;
     }
     e.nst += __popc(b);
+    if (more) return;
     __syncwarp();
-    if (e.nst > e.cap - 32) {
+    if (e.nst > e.flush_at) {
         flush_stage<MODE, ROOTS>(P, m, e.nst, lane, d, col_depth_s, chunk);
         e.nst = 0;
         __syncwarp();
@@ -592,7 +594,8 @@ __device__ __forceinline__ void process_slots(const ExpandParams& P, const WarpM
                                               uint32_t d, uint32_t k, const LevelLists& L,
                                               const uint8_t* col_depth_s, uint32_t& nst,
                                               unsigned long long& n_count, PreAcc& pre) {
-    Emit e{nst, stage_rows(k), n_count};
+    // with one back edge both slots of a round are staged before one look at the stage
+    Emit e{nst, stage_rows(k) - (k == 1 ? 32 * kSlots : 32), n_count};
     SlotWalk walk(m.start_s, excl, n, begin, lane);
     uint32_t pend = 0;
     const bool all = DUPS || (P.stage_words && k >= 2);      // every record is in segs_s
@@ -618,7 +621,8 @@ __device__ __forceinline__ void process_slots(const ExpandParams& P, const WarpM
 #pragma unroll
             for (uint32_t u = 0; u < kSlots; u++) {
                 if (ok[u]) {
-                    if (DUPS) {
+                    // (with one list every copy survives: no rank is asked)
+                    if (DUPS && k > 1) {
                         const uint32_t need = seg_rank(m.segs_s[dj[u] * 32 + j[u]], t[u], x[u], P.nbr) + 1;
                         for (uint32_t i = 0; i < k && ok[u]; i++)
                             if (i != dj[u])
@@ -630,7 +634,8 @@ __device__ __forceinline__ void process_slots(const ExpandParams& P, const WarpM
             }
 #pragma unroll
             for (uint32_t u = 0; u < kSlots; u++)
-                emit<MODE, ROOTS, DUPS>(P, m, chunk, ok[u], j[u], x[u], lane, d, col_depth_s, e, pre);
+                emit<MODE, ROOTS, DUPS>(P, m, chunk, ok[u], j[u], x[u], lane, d, col_depth_s,
+                                        u + 1 < kSlots && (!DUPS || k == 1), e, pre);
             continue;
         }
         if constexpr (!DUPS) {
@@ -671,7 +676,7 @@ __device__ __forceinline__ void process_slots(const ExpandParams& P, const WarpM
                     }
                     for (uint32_t c = 0; c < d && in; c++) in = m.rows_s[c * 32 + jj] != xx;
                 }
-                emit<MODE, ROOTS, DUPS>(P, m, chunk, in, jj, xx, lane, d, col_depth_s, e, pre);
+                emit<MODE, ROOTS, DUPS>(P, m, chunk, in, jj, xx, lane, d, col_depth_s, false, e, pre);
             }
             __syncwarp();
         }
