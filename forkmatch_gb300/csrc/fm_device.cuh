@@ -15,8 +15,8 @@ __device__ __forceinline__ uint4 ldg4(const uint4* p) { return __ldg(p); }
 // Every block lets the next pass start (`pass_begin`, first thing) and waits
 // for the pass before it (`pass_wait`) ahead of reading anything that pass
 // wrote: the control blocks, the level's rows, heavy entries and vertex sums.
-// Those are read past the L1 (`ldcg`), never through the read-only path, whose
-// contract ends at a grid's launch.  Without the launch attribute both are
+// Those are read with ordinary, volatile or `ldcg` loads after the wait, never
+// through the read-only path, whose contract ends at a grid's launch.  Without the launch attribute both are
 // no-ops.  With one clear and one read-back a match instead of one a level, and
 // no heavy pass where no chunk can need one, a 4-vertex count on 300 vertices
 // takes 46 us instead of 83, twelve nearly empty levels 296 us instead of 375.

@@ -22,16 +22,18 @@
 //      search, then against the row), and survivors are staged as (parent
 //      index, value) in shared memory;
 //   4. the stage outlives the chunk: it is flushed with one atomic per 96+
-//      survivors (224+ where every candidate survives) and fully coalesced
+//      survivors (192+ where every candidate survives) and fully coalesced
 //      stores, column by column into the next level or as contiguous
 //      row-major rows into the table.
 // A chunk whose candidate range is long (a hub) is not walked by one warp: it
 // is published to a heavy list and cut into pieces that every warp of a second
-// launch shares; launches of one match overlap (dev::pass_wait).  Lists of length <= 3 are inline in the segment record, so
-// the common case needs no second memory access.  With duplicate e-lines the
-// value at rank r of its run in the driver list survives only if every other
-// list holds at least r + 1 copies (min-multiplicity semantics of the
-// reference's merge).
+// launch shares; launches of one match overlap (dev::pass_wait).  Lists of length <= 3
+// are inline in the segment record, so the common case needs no second memory
+// access.  With duplicate e-lines the value at rank r of its run in the driver
+// list survives only if every other list holds at least r + 1 copies
+// (min-multiplicity semantics of the reference's merge); with no other list
+// every copy survives and no rank is asked (4-vertex path with its table, 2.2e8
+// rows: 1.85 ms, 2.79 with the ranks).
 //
 // Bounded memory: before expanding a chunk a warp holds output budget for its
 // candidate upper bound (reserved from the level in blocks); when a
@@ -254,7 +256,9 @@ __device__ __forceinline__ bool stage_lists(const ExpandParams& P, const WarpMem
     return ok;
 }
 
-// Column c of parent p of the level being expanded.
+// Column c of parent p of the level being expanded.  An ordinary load: the rows
+// of a run repeat their older columns and a flush reads them once a survivor, so
+// the L1 serves most of it.
 template <bool ROOTS>
 __device__ __forceinline__ uint32_t parent_col(const ExpandParams& P, uint32_t c, uint32_t p) {
     if (ROOTS) return P.root_list ? __ldg(P.root_list + p) : P.root_begin + p;
@@ -594,7 +598,10 @@ __device__ __forceinline__ void process_slots(const ExpandParams& P, const WarpM
                                               uint32_t d, uint32_t k, const LevelLists& L,
                                               const uint8_t* col_depth_s, uint32_t& nst,
                                               unsigned long long& n_count, PreAcc& pre) {
-    // with one back edge both slots of a round are staged before one look at the stage
+    // With one back edge both slots of a round are staged before one look at the
+    // stage: a look after each, with its copy of the flush, made large tables
+    // slower (4-vertex star on a 2^20-vertex R-MAT graph with 64 labels, 3.8e9
+    // embeddings: 17.8 ms, 16.0 now; 4-vertex path, 3.1e8 rows: 2.88 and 2.61).
     Emit e{nst, stage_rows(k) - (k == 1 ? 32 * kSlots : 32), n_count};
     SlotWalk walk(m.start_s, excl, n, begin, lane);
     uint32_t pend = 0;
