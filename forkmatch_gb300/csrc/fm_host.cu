@@ -1033,6 +1033,7 @@ fm_status match_impl(fm_context* ctx, const fm_graph* graph, const fm_query* que
         b.nbr = g.nbr;
         b.bm = g.bitmaps;
         b.bm_words = g.bm_words;
+        b.bm_near = g.bitmaps_near();
         b.efilter = g.efilter;
         b.efilter_off = g.efilter_off;
         b.V = g.V;

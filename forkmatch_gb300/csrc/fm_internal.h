@@ -60,6 +60,8 @@ struct DeviceGraph {
     uint32_t* efilter = nullptr;
     uint32_t* efilter_off = nullptr;
     uint32_t n_bitmaps = 0;
+    // All bitmaps take at most half of the L2 (64 of 129 MB).
+    bool bitmaps_near() const { return (uint64_t)n_bitmaps * bm_words * 4 <= (64ull << 20); }
     uint32_t bm_min_len = 0;
     uint64_t nbr_words = 0;
     uint64_t segments = 0, long_segments = 0;
@@ -167,6 +169,7 @@ struct ExpandParams {
     const uint32_t* nbr;
     const uint32_t* bm;             // list bitmaps (see DeviceGraph)
     uint32_t bm_words;
+    uint32_t bm_near;               // they stay in the L2 (see dev::count_members_f)
     const uint32_t* efilter;        // e-line filter and its slices by label (see DeviceGraph)
     const uint32_t* efilter_off;
     uint32_t V;

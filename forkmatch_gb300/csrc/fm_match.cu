@@ -559,7 +559,7 @@ __device__ __forceinline__ void emit(const ExpandParams& P, const WarpMem& m, ui
         const uint4 sg = ldg4(segl + v);
         const dev::FilterSlice f = dev::filter_slice(P.efilter, P.efilter_off, P.plan.req_label[rb]);
         e.lane_count += sg.x - dev::count_members_f(sg, f, v, m.rows_s, j, d, x, P.self_loops || anc != d, P.nbr, P.bm,
-                                                    P.bm_words);
+                                                    P.bm_words, P.bm_near);
         pre.parents += 1;
         pre.words += sg.x;
         return;

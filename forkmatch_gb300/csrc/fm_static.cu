@@ -265,6 +265,7 @@ extern "C" fm_status fm_match_static(const fm_graph* graph, const fm_query* quer
     b.nbr = g.nbr;
     b.bm = g.bitmaps;
     b.bm_words = g.bm_words;
+    b.bm_near = g.bitmaps_near();
     b.efilter = g.efilter;
     b.efilter_off = g.efilter_off;
     b.V = g.V;
