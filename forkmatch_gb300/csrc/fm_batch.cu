@@ -103,7 +103,12 @@ using dev::seg_has;
 using dev::SlotWalk;
 
 constexpr int kBWarps = 8;
-constexpr uint32_t kBStage = 96;
+// Staged survivors per warp: levels where no query has a second back edge flush
+// every candidate and have no filter queue.  With 96 rows there too, eight counts
+// of 5-vertex paths on a random graph of 2^20 vertices (7.7e7 rows at one level)
+// took 11.1 ms instead of 9.8.
+constexpr uint32_t kBStage = 96, kBStageOne = 256;
+__host__ __device__ constexpr uint32_t bstage_rows(uint32_t kmax) { return kmax == 1 ? kBStageOne : kBStage; }
 constexpr uint32_t kBSlots = 2;            // candidate slots per lane per round
 constexpr uint32_t kBPend = 32 * kBSlots + 32;   // candidates that wait for their exact test
 constexpr uint32_t kHeavyMaxPieces = 65536;
@@ -150,9 +155,9 @@ struct BMem {
     uint8_t* k_s;       // [32] requirements of the parent's query at this depth
     uint8_t* fin_s;     // [32] 1: the parent's query ends at this depth; 2: it is pre-counted here;
                         //      3: it is pre-counted by sums here (survivors are taken off)
-    uint32_t* stp;      // [kBStage] staged parent index
-    uint32_t* stx;      // [kBStage] staged vertex
-    uint32_t* stq;      // [kBStage] staged query id
+    uint32_t* stp;      // [bstage_rows] staged parent index
+    uint32_t* stx;      // [bstage_rows] staged vertex
+    uint32_t* stq;      // [bstage_rows] staged query id
     uint32_t* px;       // [kBPend] candidates the filter let pass: vertex
     uint8_t* pj;        // [kBPend] and parent (lane) in the chunk
     uint64_t* mbar;     // completion barrier of the list stage's bulk copies
@@ -163,9 +168,11 @@ struct BMem {
 __host__ __device__ constexpr uint32_t brecs(uint32_t kmax, uint32_t stage_words) { return stage_words ? kmax : 1; }
 
 __host__ __device__ constexpr uint32_t bper_warp_bytes(uint32_t d, uint32_t kmax, uint32_t stage_words = 0) {
-    return 128 * d + 512 * brecs(kmax, stage_words) + 64 * kmax + 256 + 128 + 96 + 12 * kBStage + 5 * kBPend + 4 * stage_words;
+    return 128 * d + 512 * brecs(kmax, stage_words) + 64 * kmax + 256 + 128 + 96 + 12 * bstage_rows(kmax) +
+           (kmax == 1 ? 0u : 5 * kBPend) + 4 * stage_words;
 }
 static_assert((96 + 12 * kBStage + 5 * kBPend) % 16 == 0, "the list stage is 16-byte aligned");
+static_assert((96 + 12 * kBStageOne) % 16 == 0, "the next warp's memory is 16-byte aligned");
 
 __device__ __forceinline__ BMem bmem(unsigned char* smem, uint32_t warp, uint32_t d, uint32_t kmax,
                                      uint32_t stage_words, uint64_t* mbar_s) {
@@ -180,9 +187,9 @@ __device__ __forceinline__ BMem bmem(unsigned char* smem, uint32_t warp, uint32_
     m.k_s = m.drv_s + 32;
     m.fin_s = m.k_s + 32;
     m.stp = (uint32_t*)(m.fin_s + 32);
-    m.stx = m.stp + kBStage;
-    m.stq = m.stx + kBStage;
-    m.px = m.stq + kBStage;
+    m.stx = m.stp + bstage_rows(kmax);
+    m.stq = m.stx + bstage_rows(kmax);
+    m.px = m.stq + bstage_rows(kmax);
     m.pj = (uint8_t*)(m.px + kBPend);
     m.mbar = mbar_s + warp;
     m.stage = (uint32_t*)(m.pj + kBPend);
@@ -483,7 +490,7 @@ __device__ __forceinline__ void bemit(const BatchParams& P, const BMem& m, const
     }
     nst += __popc(b);
     __syncwarp();
-    if (nst > kBStage - 32) {
+    if (nst > bstage_rows(P.kmax) - 32) {
         bflush<ROOTS>(P, m, nst, lane, d, chunk);
         nst = 0;
         __syncwarp();
@@ -515,52 +522,70 @@ __device__ __forceinline__ void bprocess(const BatchParams& P, const BMem& m, co
                 x[u] = seg_at(m.segs_s[(sw ? dj[u] * 32 : 0u) + j[u]], t[u], P.nbr);
             }
         }
-        if (kk == 1) {
+        const bool direct = kk == 1, last = base + 32 * kBSlots >= end;
+        if (!direct) {
+            for (uint32_t i = 0; i < kk; i++) {
 #pragma unroll
-            for (uint32_t u = 0; u < kBSlots; u++)
-                for (uint32_t c = 0; c < d && ok[u]; c++) ok[u] = m.rows_s[c * 32 + j[u]] != x[u];
-#pragma unroll
-            for (uint32_t u = 0; u < kBSlots; u++) bemit<ROOTS>(P, m, S, chunk, ok[u], j[u], x[u], lane, d, nst);
-            continue;
-        }
-        for (uint32_t i = 0; i < kk; i++) {
+                for (uint32_t u = 0; u < kBSlots; u++) {
+                    if (!ok[u] || dj[u] == i || i >= m.k_s[j[u]]) continue;
+                    const uint32_t ref = m.ref_s[i * 32 + j[u]];
+                    ok[u] =
+                        dev::filter_has(S.at(P, ref >> 8), dev::filter_seed(m.rows_s[(ref & 0xffu) * 32 + j[u]]), x[u]);
+                }
+            }
 #pragma unroll
             for (uint32_t u = 0; u < kBSlots; u++) {
-                if (!ok[u] || dj[u] == i || i >= m.k_s[j[u]]) continue;
-                const uint32_t ref = m.ref_s[i * 32 + j[u]];
-                ok[u] = dev::filter_has(S.at(P, ref >> 8), dev::filter_seed(m.rows_s[(ref & 0xffu) * 32 + j[u]]), x[u]);
-            }
-        }
-#pragma unroll
-        for (uint32_t u = 0; u < kBSlots; u++) {
-            const unsigned b = __ballot_sync(kFull, ok[u]);
-            if (ok[u]) {
-                const uint32_t q = pend + __popc(b & ((1u << lane) - 1u));
-                m.px[q] = x[u];
-                m.pj[q] = (uint8_t)j[u];
-            }
-            pend += __popc(b);
-        }
-        const bool last = base + 32 * kBSlots >= end;
-        while (pend >= 32 || (last && pend)) {
-            const uint32_t take = min(pend, 32u);
-            pend -= take;
-            __syncwarp();
-            bool in = lane < take;
-            uint32_t jj = 0, xx = 0;
-            if (in) {
-                jj = m.pj[pend + lane];
-                xx = m.px[pend + lane];
-                const uint32_t dd = m.drv_s[jj], k = m.k_s[jj];
-                for (uint32_t i = 0; i < k && in; i++) {
-                    if (i == dd) continue;
-                    const uint32_t ref = m.ref_s[i * 32 + jj];
-                    const uint4 r = sw ? m.segs_s[i * 32 + jj]
-                                       : ldg4(P.seg + (uint64_t)(ref >> 8) * P.V + m.rows_s[(ref & 0xffu) * 32 + jj]);
-                    in = dev::seg_has_st(r, xx, 1, P.nbr, P.bm, P.bm_words, m.stage);
+                const unsigned b = __ballot_sync(kFull, ok[u]);
+                if (ok[u]) {
+                    const uint32_t q = pend + __popc(b & ((1u << lane) - 1u));
+                    m.px[q] = x[u];
+                    m.pj[q] = (uint8_t)j[u];
                 }
-                for (uint32_t c = 0; c < d && in; c++) in = m.rows_s[c * 32 + jj] != xx;
+                pend += __popc(b);
             }
+        }
+        // One loop, and one copy of bemit, for the slots that go straight on and for
+        // the queue.  With a copy for each slot and the queue the code missed the
+        // instruction cache (8.4 of a warp's 20 cycles between two instructions):
+        // eight counts of 5-vertex paths took 8.0 ms on a random graph of 2^16
+        // vertices with 4 labels (5.6 now) and 52.1 ms on a 2^20-vertex R-MAT graph
+        // (37.7).
+        uint32_t slot = 0;
+#pragma unroll 1
+        while (direct ? slot < kBSlots : pend >= 32 || (last && pend)) {
+            bool in;
+            uint32_t jj = 0, xx = 0;
+            if (direct) {
+                in = ok[0];
+                jj = j[0];
+                xx = x[0];
+#pragma unroll
+                for (uint32_t u = 1; u < kBSlots; u++) {
+                    if (slot != u) continue;
+                    in = ok[u];
+                    jj = j[u];
+                    xx = x[u];
+                }
+                slot++;
+            } else {
+                const uint32_t take = min(pend, 32u);
+                pend -= take;
+                __syncwarp();
+                in = lane < take;
+                if (in) {
+                    jj = m.pj[pend + lane];
+                    xx = m.px[pend + lane];
+                    const uint32_t dd = m.drv_s[jj], k = m.k_s[jj];
+                    for (uint32_t i = 0; i < k && in; i++) {
+                        if (i == dd) continue;
+                        const uint32_t ref = m.ref_s[i * 32 + jj];
+                        const uint4 r = sw ? m.segs_s[i * 32 + jj]
+                                           : ldg4(P.seg + (uint64_t)(ref >> 8) * P.V + m.rows_s[(ref & 0xffu) * 32 + jj]);
+                        in = dev::seg_has_st(r, xx, 1, P.nbr, P.bm, P.bm_words, m.stage);
+                    }
+                }
+            }
+            for (uint32_t c = 0; c < d && in; c++) in = m.rows_s[c * 32 + jj] != xx;
             bemit<ROOTS>(P, m, S, chunk, in, jj, xx, lane, d, nst);
         }
         __syncwarp();
@@ -787,7 +812,7 @@ struct BatchPersistArgs {
     int hold_first_barrier;
 };
 
-__global__ void __launch_bounds__(kBWarps * 32, 5) k_bpersist(const __grid_constant__ BatchParams P0,
+__global__ void __launch_bounds__(kBWarps * 32, kBBlocks) k_bpersist(const __grid_constant__ BatchParams P0,
                                                               const __grid_constant__ BatchPersistArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ __align__(16) BatchParams P;

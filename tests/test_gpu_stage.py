@@ -52,3 +52,26 @@ def test_every_candidate_is_staged(ctx, leaves, dup):
                 assert table_sha(b.rows(i, n)) == table_sha(rows)
     b.close()
     g.close()
+
+
+@pytest.mark.parametrize("n", [7, 33, 48])
+def test_a_batch_mixes_levels_with_one_and_two_back_edges(ctx, n):
+    """Shared levels that take both ways at once: chunks whose parents have one back edge go straight on, chunks of a
+    triangle's last depth through the filter, into one stage."""
+    src, dst = np.nonzero(~np.eye(n, dtype=bool))
+    lab = 1 + (src + dst) % 2
+    g = fm.Graph.from_edges(ctx, n, 3, *[x.astype(np.uint32) for x in (src, dst, lab)])
+    og = O.Graph.from_edges(n, 3, *[x.astype(np.uint32) for x in (src, dst, lab)])
+    texts = [q.to_g_text() for q in (S.query_path(4, [1, 2, 1]), S.query_cycle(3, [1, 1, 2]), S.query_path(3, [1, 1]),
+                                     S.Query(4, [(0, 1, 1), (1, 2, 2), (0, 2, 1), (2, 3, 1)]))]
+    want = [O.match(og, O.plan(t, enumerate_aut=0), table=True) for t in texts]
+    for mode in (fm.MODE_TABLE, fm.MODE_COUNT):
+        b = fm.Batch(ctx, g, [fm.Query.from_text(t) for t in texts], mode=mode)
+        for engine in (fm.ENGINE_LEVELS, fm.ENGINE_PERSISTENT):
+            b.set_engine(engine)
+            assert b.run()[0] == [c for c, _, _ in want] and b.run()[0] == [c for c, _, _ in want]
+            if mode == fm.MODE_TABLE:
+                for i, (c, rows, _) in enumerate(want):
+                    assert table_sha(b.rows(i, c)) == table_sha(rows)
+        b.close()
+    g.close()
