@@ -24,6 +24,7 @@ MODE_TABLE, MODE_COUNT = 0, 1
 COLUMNS_REFERENCE, COLUMNS_QUERY_ID = 0, 1
 ORDER_AUTO, ORDER_REFERENCE = 0, 1
 ENGINE_LEVELS, ENGINE_PERSISTENT = 0, 1
+ROUTE_SUMS, ROUTE_SHARED, ROUTE_SHARED_PIECES, ROUTE_FORK = 1, 2, 4, 8      # bits of Result.routes
 
 STATUS_NAMES = {
     0: "FM_OK", 1: "FM_ERR_ARG", 2: "FM_ERR_IO", 3: "FM_ERR_DATA_HEADER0", 4: "FM_ERR_DATA_TRAILER",
@@ -90,7 +91,7 @@ class Result(ctypes.Structure):
                 ("device_ms", ctypes.c_double), ("launches", ctypes.c_uint64), ("h2d_bytes", ctypes.c_uint64),
                 ("d2h_bytes", ctypes.c_uint64), ("level", LevelStats * MAXQ), ("engine", ctypes.c_int32),
                 ("passes", ctypes.c_uint32), ("max_wait_ns", ctypes.c_uint64), ("pre_counted", ctypes.c_int32),
-                ("reserved", ctypes.c_uint32)]
+                ("routes", ctypes.c_uint32)]
 
 
 class BatchStats(ctypes.Structure):

@@ -898,6 +898,8 @@ cudaError_t launch_bpersist(const BatchParams& p, const BatchPersistArgs& a, int
     return cudaLaunchKernelExC(&cfg, (const void*)&k_bpersist, args);
 }
 
+uint32_t batch_level_launches(uint32_t max_list) { return 32ull * max_list <= kBHeavyLeast ? 1 : 2; }
+
 // `overlap`: the pass may start while the launch before it drains.
 cudaError_t launch_batch_level(const BatchParams& p, bool roots, bool overlap, int grid, int heavy_grid, size_t smem,
                                cudaStream_t s) {
@@ -907,7 +909,7 @@ cudaError_t launch_batch_level(const BatchParams& p, bool roots, bool overlap, i
     q.max_warps = (uint32_t)heavy_grid * kBWarps;
     void* args[] = {(void*)&q};
     cudaError_t e = launch_pass(f, grid, kBWarps * 32, smem, args, overlap, s);
-    if (e != cudaSuccess || 32ull * p.max_list <= kBHeavyLeast) return e;
+    if (e != cudaSuccess || batch_level_launches(p.max_list) == 1) return e;
     return launch_pass(fh, heavy_grid, kBWarps * 32, smem, args, overlap, s);
 }
 
@@ -1041,6 +1043,7 @@ struct fm_batch {
         uint2* at;
     };
     std::vector<SumTable> sum_tables;
+    uint32_t sum_launches[2] = {0, 0};    // of one run, counting and table mode
 
     std::vector<uint8_t> solo;
     std::vector<uint32_t> roots_all;      // n_roots of every batched plan (solo plans get 0 in h_plans)
@@ -1160,6 +1163,8 @@ struct BatchRun {
 
     // The tables of vertex sums that a counting query of this run reads.
     fm_status enqueue_sums() {
+        uint32_t& launched = b->sum_launches[base.table_mode ? 1 : 0];
+        launched = 0;
         for (const fm_batch::SumTable& t : b->sum_tables) {
             bool used = false;
             for (size_t i = 0; i < b->h_plans.size(); i++) {
@@ -1177,6 +1182,7 @@ struct BatchRun {
             p.efilter_off = g->efilter_off;
             p.V = g->V;
             const uint64_t h = g->head_off[t.label];
+            launched++;
             FM_CUDA(launch_vertex_sums(p, g->heads + h, (uint32_t)(g->head_off[t.label + 1] - h), t.label, t.last, t.at,
                                        nullptr, s));
         }
@@ -1236,7 +1242,8 @@ struct BatchRun {
         }
         if (!ran) FM_TRY(enqueue_persist());
         FM_CUDA(cudaStreamSynchronize(s));
-        b->launches += 2;   // the schedule initialisation and the persistent kernel
+        // the schedule initialisation, the persistent kernel and the vertex sums
+        b->launches += 2 + b->sum_launches[base.table_mode ? 1 : 0];
         const SchedState& h = *cv.h_sched;
         for (uint32_t d = 0; d < (uint32_t)kMaxQ; d++) b->vol[d] = 0;
         for (uint32_t d = 1; d + 1 < b->maxq; d++) b->vol[d + 1] = h.lv[d].produced;
@@ -1316,7 +1323,7 @@ struct BatchRun {
             FM_CUDA(cudaMemsetAsync(cv.ctl + d, 0, sizeof(LaunchCtl), s));
             const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((items + 7) / 8, (uint64_t)full_grid(d)));
             FM_CUDA(launch_batch_level(p, d == 1, false, grid, full_grid(d), smem(d), s));
-            b->launches++;
+            b->launches += batch_level_launches(g->max_len);
             FM_CUDA(cudaMemcpyAsync(cv.h_ctl + d, cv.ctl + d, sizeof(LaunchCtl), cudaMemcpyDeviceToHost, s));
             FM_CUDA(cudaStreamSynchronize(s));
             const LaunchCtl c = cv.h_ctl[d];
@@ -1375,7 +1382,8 @@ struct BatchRun {
             FM_TRY(enqueue_all());
         }
         FM_CUDA(cudaStreamSynchronize(s));
-        b->launches += 2 * (b->maxq - 1);
+        b->launches += (uint64_t)batch_level_launches(g->max_len) * (b->maxq - 1) +
+                       b->sum_launches[base.table_mode ? 1 : 0];
         LaunchCtl snap[kMaxQ];
         std::memcpy(snap, cv.h_ctl, b->maxq * sizeof(LaunchCtl));
         uint64_t n_parents[kMaxQ] = {};

@@ -601,6 +601,7 @@ fm_status build_from_keys(DeviceGraph& g, uint32_t V, uint32_t L, uint64_t E, Bu
         char* f = (char*)g.heads + head_bytes + bm_bytes;
         g.efilter = (uint32_t*)f;
         g.efilter_off = (uint32_t*)(f + filter_bytes);
+        g.filter_bytes = foff[L] * 4ull + (L + 1) * 4ull;
         FM_CUDA(cudaMemsetAsync(g.efilter, 0, filter_bytes, s));
         FM_CUDA(cudaMemcpyAsync(g.efilter_off, foff.data(), (L + 1) * 4, cudaMemcpyHostToDevice, s));
         k_filter<<<grid_for(E, sms), 256, 0, s>>>(sorted, E, vbits, g.efilter_off, g.efilter);

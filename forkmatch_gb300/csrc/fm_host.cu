@@ -399,7 +399,8 @@ fm_status fm_graph_get_info(const fm_graph* g, fm_graph_info* info) {
     info->bitmaps = d.n_bitmaps;
     info->bitmap_min_len = d.bm_min_len;
     info->bitmap_bytes = (uint64_t)d.n_bitmaps * d.bm_words * 4;
-    info->device_bytes = (uint64_t)d.L * d.V * 16 + d.nbr_words * 4 + d.segments * 4 + info->bitmap_bytes;
+    info->device_bytes =
+        (uint64_t)d.L * d.V * 16 + d.nbr_words * 4 + d.segments * 4 + info->bitmap_bytes + d.filter_bytes;
     info->build_ms = d.build_ms;
     return FM_OK;
 }
@@ -496,6 +497,7 @@ struct MatchRun {
     }
     cudaError_t vertex_sums(const ExpandParams& p, const unsigned long long* parents) {
         if (!vsum) return cudaSuccess;
+        res->launches++;
         const uint64_t h = g->head_off[sum_label];
         return launch_vertex_sums(p, g->heads + h, (uint32_t)(g->head_off[sum_label + 1] - h), sum_label, sum_last, vsum,
                                   parents, s);
@@ -521,6 +523,7 @@ struct MatchRun {
     fm_status read_back() {
         FM_CUDA(cudaEventRecord(ctx->ev1, s));
         FM_CUDA(cudaMemcpyAsync(ctx->h_ctl, ctx->ctl, sizeof(MatchCtl), cudaMemcpyDeviceToHost, s));
+        res->d2h_bytes += sizeof(MatchCtl) + first_rows;
         if (first_rows) FM_CUDA(cudaMemcpyAsync(ctx->h_rows, base.table, first_rows, cudaMemcpyDeviceToHost, s));
         FM_CUDA(cudaStreamSynchronize(s));
         return FM_OK;
@@ -556,12 +559,21 @@ struct MatchRun {
     void add_stats(uint32_t d, const LaunchCtl& c) {
         fm_level_stats& ls = res->level[d];
         ls.launches++;
-        res->launches++;
+        res->launches += expand_launches(base.max_list);
         res->passes++;
         ls.parents += c.parents;
         ls.lookups += c.lookups;
         ls.list_words += c.list_words;
         if (mode_of(d) == kModeMid) ls.produced += c.produced;
+    }
+
+    // Which ways a pass of depth d took: of `parents` rows in `items` chunks, on
+    // `warps` warps (the rules of the kernels, which decide on the device).
+    void add_routes(uint32_t d, uint64_t parents, uint64_t items, uint64_t warps, bool by_sums, const LaunchCtl& c) {
+        if (by_sums && parents) res->routes |= FM_ROUTE_SUMS;
+        if (!shares(d) || items < 4 * warps) return;
+        res->routes |= FM_ROUTE_SHARED;
+        if (c.heavy) res->routes |= FM_ROUTE_SHARED_PIECES;
     }
 
     // Optimistic pass: every level launched back to back, level d reading its
@@ -573,6 +585,7 @@ struct MatchRun {
         const uint32_t q = plan->q;
         const uint32_t last = last_depth();
         cudaEvent_t ev[kMaxQ][2] = {};
+        uint64_t warps[kMaxQ] = {};
         // What a level can hold at most: the roots times the longest list per
         // depth.  On a small graph that needs few blocks.
         uint64_t most = n_roots;
@@ -583,6 +596,7 @@ struct MatchRun {
             const bool share = shares(d);
             const int per_sm = expand_blocks_per_sm(mode, roots, dups, share, smem, block);
             const int full = ctx->sms * per_sm;
+            warps[d] = (uint64_t)full * (block / 32);
             ExpandParams p = base;
             p.pin = roots ? nullptr : level[d];
             p.pstride = level_cap;
@@ -619,6 +633,8 @@ struct MatchRun {
             const LaunchCtl& c = ctx->h_ctl[d];
             n_parents[d] = d == 1 ? n_roots : ctx->h_ctl[d - 1].produced;
             add_stats(d, c);
+            add_routes(d, n_parents[d], (n_parents[d] + 31) / 32, warps[d],
+                       sums && d == last && 4 * n_parents[d] >= base.sum_heads, c);
             if (profile) {
                 float ms = 0;
                 cudaEventElapsedTime(&ms, ev[d][0], ev[d][1]);
@@ -680,6 +696,7 @@ struct MatchRun {
         p.ctl = ctx->ctl;
         FM_CUDA(launch_persist(p, a, last_mode, dups, grid, smem, s));
         FM_CUDA(cudaMemcpyAsync(&h, ctx->sched, sizeof(h), cudaMemcpyDeviceToHost, s));
+        res->d2h_bytes += sizeof(h);
         FM_TRY(read_back());
         for (uint32_t d = 1; d < q; d++) {
             fm_level_stats& ls = res->level[d];
@@ -760,6 +777,7 @@ struct MatchRun {
             FM_CUDA(launch_expand(p, mode, roots, dups, share, false, grid, ctx->sms * per_sm, block, smem, s));
             if (profile) FM_CUDA(cudaEventRecord(e1, s));
             FM_CUDA(cudaMemcpyAsync(ctx->h_ctl + d, ctx->ctl + d, sizeof(LaunchCtl), cudaMemcpyDeviceToHost, s));
+            res->d2h_bytes += sizeof(LaunchCtl);
             FM_CUDA(cudaStreamSynchronize(s));
             const LaunchCtl c = ctx->h_ctl[d];
             if (profile) {
@@ -768,6 +786,7 @@ struct MatchRun {
                 res->level[d].kernel_ms += ms;
             }
             add_stats(d, c);
+            add_routes(d, n_parents, items, (uint64_t)ctx->sms * per_sm * (block / 32), p.sum_rule == 2, c);
             if (c.error) {
                 set_error((c.error & 2u) ? "a list stage's bounded wait ran out" : "deferred-chunk list overflow");
                 return FM_ERR_DEVICE;
@@ -941,6 +960,7 @@ fm_status match_impl(fm_context* ctx, const fm_graph* graph, const fm_query* que
             std::memcpy(nreq, fnreq, sizeof(nreq));
             std::memcpy(climb, fclimb, sizeof(climb));
             std::memcpy(rlab, flab, sizeof(rlab));
+            out->routes |= FM_ROUTE_FORK;
         }
     }
     if (use_ref) {
@@ -1104,18 +1124,19 @@ fm_status match_impl(fm_context* ctx, const fm_graph* graph, const fm_query* que
     if (q > 1) out->level[q - 1].produced = out->count;
     if (direct) {
         out->rows_copied = out->rows;   // already in host memory
+        out->d2h_bytes += out->rows * q * 4;
     } else if (table && opts.host_rows && out->rows) {
         uint64_t n = std::min<uint64_t>(out->rows, opts.host_rows_cap);
         if (launched && n * q * 4 <= run.first_rows) {
             std::memcpy(opts.host_rows, ctx->h_rows, n * q * 4);
         } else {
+            out->d2h_bytes += n * q * 4;
             FM_CUDA(cudaMemcpyAsync(opts.host_rows, table_ptr, n * q * 4, cudaMemcpyDeviceToHost, s));
             FM_CUDA(cudaStreamSynchronize(s));
         }
         out->rows_copied = n;
     }
     out->h2d_bytes = out->launches * sizeof(ExpandParams);
-    out->d2h_bytes = out->launches * sizeof(LaunchCtl) + sizeof(MatchTotals) + out->rows_copied * q * 4;
     if (limited || (ctx->h_tot->error & kLimitFlag)) {
         set_error("work limit reached; count and rows are a lower bound");
         return FM_ERR_LIMIT;

@@ -59,6 +59,7 @@ struct DeviceGraph {
     // efilter_off[l + 1])).  Null for graphs with duplicate e-lines.
     uint32_t* efilter = nullptr;
     uint32_t* efilter_off = nullptr;
+    uint64_t filter_bytes = 0;           // of both
     uint32_t n_bitmaps = 0;
     // All bitmaps take at most half of the L2 (64 of 129 MB).
     bool bitmaps_near() const { return (uint64_t)n_bitmaps * bm_words * 4 <= (64ull << 20); }
@@ -307,6 +308,8 @@ cudaError_t launch_sched_init(SchedState* S, unsigned q, unsigned long long n_ro
 // `overlap`: the pass may start while the launch before it drains.
 cudaError_t launch_expand(const ExpandParams& p, int mode, bool roots, bool dups, bool share, bool overlap, int grid,
                           int heavy_grid, int block, size_t smem, cudaStream_t s);
+// Kernel launches of one level pass on a graph whose longest list is `max_list`.
+uint32_t expand_launches(uint32_t max_list);
 cudaError_t launch_pass(const void* f, int grid, int block, size_t smem, void** args, bool overlap, cudaStream_t s);
 // Resident blocks per SM of kernel f (0: does not fit), asked of the driver
 // once per kernel and shared memory size.

@@ -1584,6 +1584,8 @@ int expand_blocks_per_sm(int mode, bool roots, bool dups, bool share, size_t sme
     return std::max(1, blocks_per_sm(f, block, smem));
 }
 
+uint32_t expand_launches(uint32_t max_list) { return 32ull * max_list <= kHeavyLeast ? 1 : 2; }
+
 cudaError_t launch_expand(const ExpandParams& p, int mode, bool roots, bool dups, bool share, bool overlap, int grid,
                           int heavy_grid, int block, size_t smem, cudaStream_t s) {
     void* f = pick(mode, roots, dups, share, false);
@@ -1596,7 +1598,7 @@ cudaError_t launch_expand(const ExpandParams& p, int mode, bool roots, bool dups
     q.share_words = share ? kShareWords : 0;
     void* args[] = {(void*)&q};
     cudaError_t e = launch_pass(f, grid, block, smem, args, overlap, s);
-    if (e != cudaSuccess || 32ull * p.max_list <= kHeavyLeast) return e;
+    if (e != cudaSuccess || expand_launches(p.max_list) == 1) return e;
     // the heavy pass always gets a full grid: a few heavy chunks can hold most of the work
     return launch_pass(fh, heavy_grid, block, smem, args, overlap, s);
 }

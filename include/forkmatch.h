@@ -103,8 +103,7 @@ typedef struct fm_graph_info {
     uint64_t nbr_words;         /* u32 words of out-of-line storage (16 B aligned) */
     uint32_t max_list;          /* longest (label, vertex) list */
     int32_t has_duplicates;     /* some (label, src, dst) e-line occurs twice */
-    uint64_t device_bytes;      /* records, lists, root lists and bitmaps on the device (the e-line
-                                   filter adds 2 bytes per e-line) */
+    uint64_t device_bytes;      /* graph bytes resident on the device */
     double build_ms;            /* device build time */
     uint32_t bitmaps;           /* lists that also have a membership bitmap over all vertices */
     uint32_t bitmap_min_len;    /* shortest list given a bitmap (0: none) */
@@ -235,9 +234,10 @@ typedef struct fm_result {
     int32_t truncated;          /* table capacity exceeded */
     uint32_t q;                 /* row width */
     double device_ms;           /* matching window on the device (CUDA events) */
-    uint64_t launches;          /* expansion kernel launches */
+    uint64_t launches;          /* kernel launches: the level passes' (main, heavy) and vertex sums */
     uint64_t h2d_bytes;         /* host->device bytes this match moved (kernel parameter blocks) */
-    uint64_t d2h_bytes;         /* device->host bytes (control blocks, totals, copied rows) */
+    uint64_t d2h_bytes;         /* device->host bytes (control blocks, totals, the first rows read
+                                   back with them, copied rows) */
     fm_level_stats level[FM_MAX_QUERY_VERTICES];
     int32_t engine;             /* fm_engine that ran */
     uint32_t passes;            /* level passes over all depths */
@@ -245,8 +245,18 @@ typedef struct fm_result {
     int32_t pre_counted;        /* count mode, last depth with one back edge: its extensions were
                                    counted from depth q-2 (its survivors are not stored), so the
                                    last depth was not launched; level[q-1] still reports its work */
-    uint32_t reserved;
+    uint32_t routes;            /* fm_route bits: what some level pass of this match did */
 } fm_result;
+
+/* Ways a level pass may take; results and work counters do not depend on them. */
+typedef enum fm_route {
+    FM_ROUTE_SUMS = 1,          /* the last two depths were counted by sums of list lengths and list
+                                   intersections, no candidate of them was looked at */
+    FM_ROUTE_SHARED = 2,        /* parents of one run shared the intersection of their oldest lists */
+    FM_ROUTE_SHARED_PIECES = 4, /* and a chunk of such a level was cut into pieces */
+    FM_ROUTE_FORK = 8           /* an order was chosen for the sums: both last vertices are leaves on
+                                   earlier ones */
+} fm_route;
 
 fm_status fm_match(fm_context* ctx, const fm_graph* g, const fm_query* q,
                    const fm_match_opts* opts, fm_result* out);
