@@ -15,7 +15,9 @@
 #include <algorithm>
 #include <chrono>
 #include <cstring>
+#include <map>
 #include <memory>
+#include <utility>
 #include <vector>
 
 #include "fm_device.cuh"
@@ -1129,6 +1131,47 @@ void build_plan(const Plan& pl, const DeviceGraph& g, BatchPlan& bp, bool& impos
     }
 }
 
+// How a query's last two depths may be counted by sums: kSumNone if they may not.
+uint32_t sum_kind_of(const BatchPlan& bp, const DeviceGraph& g) {
+    const uint32_t q = bp.q;
+    if (!bp.pre_ok || q < 4 || bp.nreq[q - 2] != 1 || g.has_self_loops || stage_words_knob()) return kSumNone;
+    const uint32_t a = bp.req_anc[bp.req_begin[q - 2]], l = bp.req_label[bp.req_begin[q - 2]];
+    const uint32_t c = bp.req_anc[bp.req_begin[q - 1]], ll = bp.req_label[bp.req_begin[q - 1]];
+    const bool chain = c == q - 2;
+    if (g.head_off[l + 1] - g.head_off[l] < 4096 || (chain && (q != 4 || !g.symmetric))) return kSumNone;
+    return chain ? kSumChain : a != c ? kSumFork : l != ll ? kSumForkOne : kSumForkSame;
+}
+
+// Estimated candidates of a query's counting level: rows reached through an
+// e-line of label l meet lists of label_pairs / label_count more.
+double sum_candidates(const BatchPlan& bp, const DeviceGraph& g) {
+    const double V = (double)g.V;
+    auto avg = [&](uint32_t l) { return (double)g.label_count[l] / V; };
+    auto seen = [&](uint32_t l) {
+        return g.label_count[l] ? std::max(avg(l), (double)g.label_pairs[l] / (double)g.label_count[l]) : 0.0;
+    };
+    double rows = V;
+    for (uint32_t d = 1; d + 1 < bp.q; d++) {
+        const uint8_t* l = bp.req_label + bp.req_begin[d];
+        double shortest = d == 1 || bp.nreq[d] > 1 ? avg(l[0]) : seen(l[0]), rest = 1.0;
+        for (uint32_t i = 1; i < bp.nreq[d]; i++) {
+            rest *= std::max(shortest, avg(l[i])) / V;
+            shortest = std::min(shortest, avg(l[i]));
+        }
+        rows *= shortest * rest;
+    }
+    return rows;
+}
+
+// A table of vertex sums pays if it spares its queries this many candidates per
+// e-line of its label, each of which it reads.  Unlike fm_match, which decides on
+// the device from the parents it counted, a batch computes its tables before its
+// first level.  32 paths of 4 vertices on a 2^20-vertex random graph with 40
+// labels (0.8 candidates per e-line): 2151 us with tables, 1477 without; with 10
+// labels (3.1) the two are even, with 4 labels (7.6) tables take 1050 of 1595 us
+// a path.  Paths that start at a rare label (0.0001): 552 us with, 82 without.
+constexpr double kSumsSpare = 3.0;
+
 struct BatchRun {
     fm_batch* b;
     ContextView cv;
@@ -1485,32 +1528,35 @@ fm_status batch_create_impl(fm_context* ctx, const fm_graph* graph, const fm_que
         // queries counted by sums: as in fm_match, with at most an eighth of the
         // level memory for their tables
         uint64_t soln = cv.soln_bytes;
-        if (!stage_words_knob() && !g.has_self_loops) {
-            const uint64_t vbytes = ((uint64_t)g.V * sizeof(uint2) + 255) & ~255ull;
-            for (auto& bp : plans) {
-                const uint32_t q = bp.q;
-                if (!bp.pre_ok || q < 4 || bp.nreq[q - 2] != 1) continue;
-                const uint32_t a = bp.req_anc[bp.req_begin[q - 2]], l = bp.req_label[bp.req_begin[q - 2]];
-                const uint32_t c = bp.req_anc[bp.req_begin[q - 1]], ll = bp.req_label[bp.req_begin[q - 1]];
-                const bool chain = c == q - 2;
-                if (g.head_off[l + 1] - g.head_off[l] < 4096 || (chain && (q != 4 || !g.symmetric))) continue;
-                const uint32_t kind = chain ? kSumChain : a != c ? kSumFork : l != ll ? kSumForkOne : kSumForkSame;
-                if (kind == kSumChain || kind == kSumForkOne) {
-                    uint2* at = nullptr;
-                    for (auto& t : b->sum_tables)
-                        if (t.label == l && t.last == ll) at = t.at;
-                    if (!at) {
-                        if (soln < vbytes + 256 || cv.soln_bytes - soln + vbytes > cv.soln_bytes / 8 ||
-                            (soln - vbytes - 256) / (4ull * sum_cols) < (uint64_t)g.max_len * 32 + 32)
-                            continue;
-                        soln = (soln - vbytes) & ~255ull;
-                        at = (uint2*)(cv.soln + soln);
-                        b->sum_tables.push_back({l, ll, at});
-                    }
-                    bp.vsum = at;
+        const uint64_t vbytes = ((uint64_t)g.V * sizeof(uint2) + 255) & ~255ull;
+        auto pair_of = [](const BatchPlan& bp) {
+            return std::make_pair<uint32_t, uint32_t>(bp.req_label[bp.req_begin[bp.q - 2]],
+                                                      bp.req_label[bp.req_begin[bp.q - 1]]);
+        };
+        std::map<std::pair<uint32_t, uint32_t>, double> spared;   // per table: candidates of its queries
+        for (const auto& bp : plans) {
+            const uint32_t kind = sum_kind_of(bp, g);
+            if (kind == kSumChain || kind == kSumForkOne) spared[pair_of(bp)] += sum_candidates(bp, g);
+        }
+        for (auto& bp : plans) {
+            const uint32_t kind = sum_kind_of(bp, g);
+            if (kind == kSumChain || kind == kSumForkOne) {
+                const auto pr = pair_of(bp);
+                if (spared[pr] < kSumsSpare * (double)g.label_count[pr.first]) continue;
+                uint2* at = nullptr;
+                for (auto& t : b->sum_tables)
+                    if (t.label == pr.first && t.last == pr.second) at = t.at;
+                if (!at) {
+                    if (soln < vbytes + 256 || cv.soln_bytes - soln + vbytes > cv.soln_bytes / 8 ||
+                        (soln - vbytes - 256) / (4ull * sum_cols) < (uint64_t)g.max_len * 32 + 32)
+                        continue;
+                    soln = (soln - vbytes) & ~255ull;
+                    at = (uint2*)(cv.soln + soln);
+                    b->sum_tables.push_back({pr.first, pr.second, at});
                 }
-                bp.sum_kind = kind;
+                bp.vsum = at;
             }
+            bp.sum_kind = kind;
         }
         for (uint32_t d = 1; d < b->maxq; d++) {
             uint32_t km = 1;

@@ -133,14 +133,16 @@ __global__ void k_seg_starts(const uint64_t* __restrict__ keys, uint64_t E, uint
 __device__ __forceinline__ uint32_t len16_of(uint32_t n) { return n > 3 ? (n + 3) / 4 : 0; }
 
 // Segment lengths: the 16-byte units each tile of segments stores out of line,
-// the longest list, the long lists, the list lengths by floor(log2), and the
-// first segment of every label.  The totals are gathered per block and added
+// the longest list, the long lists, the list lengths by floor(log2), the pairs
+// in a list summed per label, and the first segment of every label.  The totals are gathered per block and added
 // once (one atomic per segment on shared counters was the slowest kernel of
 // the build: 250 us for 7.1 M segments, now 30).
 __global__ void k_seg_lens(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ seg_start,
                            uint32_t vbits, uint32_t* __restrict__ tile16, BuildStats* __restrict__ st) {
     __shared__ uint32_t hist_s[32], red_s[kBlock / 32], max_s;
+    __shared__ unsigned long long pairs_s[FM_MAX_LABEL + 1];
     if (threadIdx.x < 32) hist_s[threadIdx.x] = 0;
+    for (uint32_t i = threadIdx.x; i <= FM_MAX_LABEL; i += blockDim.x) pairs_s[i] = 0;
     if (threadIdx.x == 0) max_s = 0;
     __syncthreads();
     const uint32_t nseg = st->nseg;
@@ -151,19 +153,31 @@ __global__ void k_seg_lens(const uint64_t* __restrict__ keys, const uint32_t* __
 #pragma unroll
         for (uint32_t j = 0; j < kTileSegs / kBlock; j++) {
             const uint64_t s = t * kTileSegs + j * kBlock + threadIdx.x;
-            uint32_t n = 0;
+            uint32_t n = 0, l = 0;
             if (s < nseg) {
                 const uint32_t b = seg_start[s];
                 n = seg_start[s + 1] - b;
                 sum += len16_of(n);
                 mx = max(mx, n);
                 if (n > 3) atomicAdd(&hist_s[31 - __clz((int)n)], 1u);
-                const uint32_t l = (uint32_t)(keys[b] >> (2 * vbits));
+                l = (uint32_t)(keys[b] >> (2 * vbits));
                 if (s == 0 || (uint32_t)(keys[b - 1] >> (2 * vbits)) != l) st->first[l] = s;
             }
             // most lists are this short: counted by ballot, not by colliding atomics
             one += __popc(__ballot_sync(0xffffffffu, n == 1));
             two += __popc(__ballot_sync(0xffffffffu, n == 2 || n == 3));
+            // segments come label by label: nearly always one label a warp
+            const unsigned many = __ballot_sync(0xffffffffu, n > 1);
+            if (!many) continue;
+            unsigned long long pr = n > 1 ? (unsigned long long)n * (n - 1) : 0ull;
+            const uint32_t l0 = __shfl_sync(0xffffffffu, l, __ffs(many) - 1);
+            if (__all_sync(0xffffffffu, n <= 1 || l == l0)) {
+#pragma unroll
+                for (int o = 16; o; o >>= 1) pr += __shfl_xor_sync(0xffffffffu, pr, o);
+                if (lane == 0) atomicAdd(&pairs_s[l0], pr);
+            } else if (pr) {
+                atomicAdd(&pairs_s[l], pr);
+            }
         }
         sum = __reduce_add_sync(0xffffffffu, sum);
         mx = __reduce_max_sync(0xffffffffu, mx);
@@ -184,6 +198,8 @@ __global__ void k_seg_lens(const uint64_t* __restrict__ keys, const uint32_t* __
     __syncthreads();
     if (threadIdx.x < 32 && hist_s[threadIdx.x]) atomicAdd(&st->hist[threadIdx.x], hist_s[threadIdx.x]);
     if (threadIdx.x == 0 && max_s) atomicMax(&st->max_len, max_s);
+    for (uint32_t i = threadIdx.x; i <= FM_MAX_LABEL; i += blockDim.x)
+        if (pairs_s[i]) atomicAdd(&st->pairs[i], pairs_s[i]);
 }
 
 // Out-of-line offset of every segment, in 16-byte units.  A thread takes four
@@ -548,6 +564,7 @@ fm_status build_from_keys(DeviceGraph& g, uint32_t V, uint32_t L, uint64_t E, Bu
     g.has_self_loops = h.loops ? 1 : 0;
     g.long_segments = nseg - h.hist[0] - h.hist[1];   // lists of 4 entries and more
     g.label_count.assign(h.label_count, h.label_count + L);
+    g.label_pairs.assign(h.pairs, h.pairs + L);
     // a label without segments starts where the next label with one does
     g.head_off.assign(L + 1, nseg);
     if (E)

@@ -73,6 +73,9 @@ struct DeviceGraph {
     int device = 0;
     double build_ms = 0;
     std::vector<uint64_t> label_count;   // e-lines per label slot
+    // per label slot, the pairs of distinct e-lines out of one vertex: over
+    // label_count, how many more e-lines of the label the source of one has on average
+    std::vector<uint64_t> label_pairs;
 };
 
 // ----------------------------------------------------------------- query plan
@@ -392,6 +395,7 @@ struct BuildStats {
     unsigned long long lines;         // text: lines
     unsigned long long label_count[FM_MAX_LABEL + 1];
     unsigned long long first[FM_MAX_LABEL + 1];   // first segment of a label; all ones: none
+    unsigned long long pairs[FM_MAX_LABEL + 1];   // n (n - 1) summed over a label's lists
 };
 
 // Every temporary of one build, in one device allocation sized for `cap` keys

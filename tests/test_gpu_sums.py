@@ -128,3 +128,31 @@ def test_order_of_a_count_that_sums_cannot_serve(ctx, edges, labels):
     for d in range(1, 5):
         assert (c.level[d].parents, c.level[d].list_words) == (t.level[d].parents, t.level[d].list_words), d
     g.close()
+
+
+def test_batches_compute_vertex_sums_only_where_they_pay(ctx):
+    """A table of vertex sums reads every e-line of its label.  Paths whose first label is rare meet few of them: no
+    table; paths over frequent labels of a graph with long lists: one a pair of labels, shared by its queries."""
+    rng = np.random.default_rng(4)
+    n = 5000
+    e = np.unique(np.sort(rng.integers(0, n, (100000, 2)), axis=1), axis=0)
+    e = e[e[:, 0] != e[:, 1]]
+    lab = rng.integers(2, 4, len(e))
+    lab[:40] = 1
+    src, dst, lab = [np.concatenate(x).astype(np.uint32) for x in ((e[:, 0], e[:, 1]), (e[:, 1], e[:, 0]), (lab, lab))]
+    g = fm.Graph.from_edges(ctx, n, 4, src, dst, lab)
+    per = 2 if g.info().max_list > 16 else 1
+    for labels, shared in (([[1, 2, 3], [1, 3, 2], [1, 2, 2]], None), ([[2, 3, 2], [2, 3, 2]], 1),
+                           ([[2, 3, 2], [2, 2, 2], [3, 3, 3]], 0)):
+        qs = [fm.Query.from_text(S.query_path(4, l).to_g_text()) for l in labels]
+        b = fm.Batch(ctx, g, qs, mode=fm.MODE_COUNT)
+        want = [fm.match(ctx, g, q, mode=fm.MODE_COUNT, order=fm.ORDER_REFERENCE).count for q in qs]
+        # a count of its own launches the vertex sums if its order needs them
+        alone = [fm.match(ctx, g, q, mode=fm.MODE_COUNT) for q in qs]
+        tables = 0 if shared is None else sum(r.launches - per * r.passes for r in alone) - shared
+        assert shared is None or tables >= 1
+        for _ in range(2):
+            counts, st = b.run()
+            assert counts == want and st.launches == 3 * per + tables
+        b.close()
+    g.close()
