@@ -967,6 +967,7 @@ struct fm_batch {
     uint64_t cap_floor = 0;               // smallest level buffer one chunk per level needs
     uint32_t bank_shift = 0;              // tuned: level buffers of cap_full >> bank_shift rows
     char* soln = nullptr;
+    uint64_t soln_bytes = 0;              // the level region
 
     uint64_t lcap[kMaxQ] = {};            // rows of the level buffer of depth d (d >= 2)
     uint64_t vol[kMaxQ] = {};             // rows that passed through level d in the last run
@@ -1027,6 +1028,17 @@ struct fm_batch {
         }
         return true;
     }
+    // Vertex sums of the queries counted by sums: one table per (label, last
+    // label), at the end of the level region; recomputed by every run.
+    struct SumTable {
+        uint32_t label, last;
+        uint2* at;
+    };
+    std::vector<SumTable> sum_tables;
+    uint32_t sum_launches[2] = {0, 0};    // of one run, counting and table mode
+    bool sums_counting = true;            // reserved for a run that counts every query (see reserve_sums)
+    bool sums_stale = false;              // the queries in the shared launches changed since
+
     std::vector<uint64_t> counts;
     std::vector<uint64_t> single_counts;
     uint64_t launches = 0;
@@ -1038,15 +1050,6 @@ struct fm_batch {
     // buffers, crowds out the others; it runs on the single-query engine
     // with the whole level memory, after the shared run, its table written
     // into its own region.  Indices are positions in `batched`.
-    // Vertex sums of the queries counted by sums: one table per (label, last
-    // label), at the end of the level region; recomputed by every run.
-    struct SumTable {
-        uint32_t label, last;
-        uint2* at;
-    };
-    std::vector<SumTable> sum_tables;
-    uint32_t sum_launches[2] = {0, 0};    // of one run, counting and table mode
-
     std::vector<uint8_t> solo;
     std::vector<uint32_t> roots_all;      // n_roots of every batched plan (solo plans get 0 in h_plans)
     uint32_t n_solo = 0;
@@ -1059,6 +1062,7 @@ struct fm_batch {
             n_solo += s[i] ? 1u : 0u;
         }
         plans_dirty = true;
+        sums_stale = true;
         drop_graphs();                    // the captured launches bake in the longest root list
     }
 
@@ -1171,6 +1175,72 @@ double sum_candidates(const BatchPlan& bp, const DeviceGraph& g) {
 // labels (3.1) the two are even, with 4 labels (7.6) tables take 1050 of 1595 us
 // a path.  Paths that start at a rare label (0.0001): 552 us with, 82 without.
 constexpr double kSumsSpare = 3.0;
+
+// Which queries of the coming runs are counted by sums, the tables of vertex sums
+// that they read (at most an eighth of the level region, at its end) and the
+// level buffers before those.  `counting`: the run counts every query (a count
+// batch, or the first run of a table batch, which sizes the tables); otherwise
+// only the queries set to count only are counted, and the level region has no
+// tables of the others.
+void reserve_sums(fm_batch& b, bool counting) {
+    const DeviceGraph& g = b.graph->g;
+    uint64_t sum_cols = 0;
+    for (uint32_t d = 2; d < b.maxq; d++) sum_cols += d + 1;
+    uint64_t soln = b.soln_bytes;
+    const uint64_t vbytes = ((uint64_t)g.V * sizeof(uint2) + 255) & ~255ull;
+    auto pair_of = [](const BatchPlan& bp) {
+        return std::make_pair<uint32_t, uint32_t>(bp.req_label[bp.req_begin[bp.q - 2]],
+                                                  bp.req_label[bp.req_begin[bp.q - 1]]);
+    };
+    auto kind_of = [&](size_t i) {
+        const BatchPlan& bp = b.h_plans[i];
+        return (counting || bp.count_only) && !b.solo[i] ? sum_kind_of(bp, g) : (uint32_t)kSumNone;
+    };
+    b.sum_tables.clear();
+    std::map<std::pair<uint32_t, uint32_t>, double> spared;   // per table: candidates of its queries
+    for (size_t i = 0; i < b.h_plans.size(); i++) {
+        const uint32_t kind = kind_of(i);
+        if (kind == kSumChain || kind == kSumForkOne) spared[pair_of(b.h_plans[i])] += sum_candidates(b.h_plans[i], g);
+    }
+    for (size_t i = 0; i < b.h_plans.size(); i++) {
+        BatchPlan& bp = b.h_plans[i];
+        bp.sum_kind = kSumNone;
+        bp.vsum = nullptr;
+        const uint32_t kind = kind_of(i);
+        if (kind == kSumChain || kind == kSumForkOne) {
+            const auto pr = pair_of(bp);
+            if (spared[pr] < kSumsSpare * (double)g.label_count[pr.first]) continue;
+            uint2* at = nullptr;
+            for (auto& t : b.sum_tables)
+                if (t.label == pr.first && t.last == pr.second) at = t.at;
+            if (!at) {
+                if (soln < vbytes + 256 || b.soln_bytes - soln + vbytes > b.soln_bytes / 8 ||
+                    (soln - vbytes - 256) / (4ull * sum_cols) < b.cap_floor)
+                    continue;
+                soln = (soln - vbytes) & ~255ull;
+                at = (uint2*)(b.soln + soln);
+                b.sum_tables.push_back({pr.first, pr.second, at});
+            }
+            bp.vsum = at;
+        }
+        bp.sum_kind = kind;
+    }
+    for (uint32_t d = 1; d < b.maxq; d++) {
+        uint32_t km = 1;
+        for (const auto& bp : b.h_plans) {
+            if (d < bp.q) km = std::max(km, bp.nreq[d]);
+            if (bp.sum_kind && d + 2 == bp.q) km = std::max(km, 2u);   // the list it is met with
+        }
+        b.kmax[d] = km;
+    }
+    b.cap_full = std::min<uint64_t>(sum_cols ? soln / (4ull * sum_cols) : 0, 0xffffffffull - 64);
+    if (!b.weighted || !b.layout_weighted())
+        b.layout_levels(sum_cols ? std::max(b.cap_full >> b.bank_shift, b.cap_floor) : 0);
+    b.sums_counting = counting;
+    b.sums_stale = false;
+    b.plans_dirty = true;
+    b.drop_graphs();                      // they hold the level buffers and tables
+}
 
 struct BatchRun {
     fm_batch* b;
@@ -1525,60 +1595,18 @@ fm_status batch_create_impl(fm_context* ctx, const fm_graph* graph, const fm_que
     if (nq) {
         uint64_t sum_cols = 0;   // level d+1 rows hold d+1 vertices and a query id
         for (uint32_t d = 2; d < b->maxq; d++) sum_cols += d + 1;
-        // queries counted by sums: as in fm_match, with at most an eighth of the
-        // level memory for their tables
-        uint64_t soln = cv.soln_bytes;
-        const uint64_t vbytes = ((uint64_t)g.V * sizeof(uint2) + 255) & ~255ull;
-        auto pair_of = [](const BatchPlan& bp) {
-            return std::make_pair<uint32_t, uint32_t>(bp.req_label[bp.req_begin[bp.q - 2]],
-                                                      bp.req_label[bp.req_begin[bp.q - 1]]);
-        };
-        std::map<std::pair<uint32_t, uint32_t>, double> spared;   // per table: candidates of its queries
-        for (const auto& bp : plans) {
-            const uint32_t kind = sum_kind_of(bp, g);
-            if (kind == kSumChain || kind == kSumForkOne) spared[pair_of(bp)] += sum_candidates(bp, g);
-        }
-        for (auto& bp : plans) {
-            const uint32_t kind = sum_kind_of(bp, g);
-            if (kind == kSumChain || kind == kSumForkOne) {
-                const auto pr = pair_of(bp);
-                if (spared[pr] < kSumsSpare * (double)g.label_count[pr.first]) continue;
-                uint2* at = nullptr;
-                for (auto& t : b->sum_tables)
-                    if (t.label == pr.first && t.last == pr.second) at = t.at;
-                if (!at) {
-                    if (soln < vbytes + 256 || cv.soln_bytes - soln + vbytes > cv.soln_bytes / 8 ||
-                        (soln - vbytes - 256) / (4ull * sum_cols) < (uint64_t)g.max_len * 32 + 32)
-                        continue;
-                    soln = (soln - vbytes) & ~255ull;
-                    at = (uint2*)(cv.soln + soln);
-                    b->sum_tables.push_back({pr.first, pr.second, at});
-                }
-                bp.vsum = at;
-            }
-            bp.sum_kind = kind;
-        }
-        for (uint32_t d = 1; d < b->maxq; d++) {
-            uint32_t km = 1;
-            for (auto& bp : plans) {
-                if (d < bp.q) km = std::max(km, bp.nreq[d]);
-                if (bp.sum_kind && d + 2 == bp.q) km = std::max(km, 2u);   // the list it is met with
-            }
-            b->kmax[d] = km;
-        }
-        uint64_t cap = sum_cols ? soln / (4ull * sum_cols) : 0;
-        cap = std::min<uint64_t>(cap, 0xffffffffull - 64);
-        if (sum_cols && cap < (uint64_t)g.max_len * 32 + 32) {
+        if (sum_cols && cv.soln_bytes / (4ull * sum_cols) < (uint64_t)g.max_len * 32 + 32) {
             set_error("SOLN_PREALLOC cannot hold one 32-parent chunk per level for this graph");
             return FM_ERR_POOL;
         }
         b->soln = cv.soln;
-        b->cap_full = cap;
+        b->soln_bytes = cv.soln_bytes;
         b->cap_floor = (uint64_t)g.max_len * 32 + 32;
-        b->layout_levels(cap);
         b->h_plans = plans;
         b->solo.assign(nq, 0);
         for (auto& bp : plans) b->roots_all.push_back(bp.n_roots);
+        reserve_sums(*b, true);
+        b->plans_dirty = false;              // uploaded here
         if (scr) {
             // caller-owned scratch: no allocation (a server must not call
             // cudaMalloc/cudaFree while other slots run)
@@ -1594,7 +1622,7 @@ fm_status batch_create_impl(fm_context* ctx, const fm_graph* graph, const fm_que
                                     cv.stream));
         } else {
             FM_CUDA(cudaMalloc(&b->d_plans, nq * sizeof(BatchPlan)));
-            FM_CUDA(cudaMemcpy(b->d_plans, plans.data(), nq * sizeof(BatchPlan), cudaMemcpyHostToDevice));
+            FM_CUDA(cudaMemcpy(b->d_plans, b->h_plans.data(), nq * sizeof(BatchPlan), cudaMemcpyHostToDevice));
             FM_CUDA(cudaMalloc(&b->d_qpos, nq * sizeof(unsigned long long)));
             FM_CUDA(cudaHostAlloc(&b->h_qpos, nq * sizeof(unsigned long long), cudaHostAllocDefault));
         }
@@ -1643,6 +1671,8 @@ fm_status fm_batch_run(fm_batch* b, uint64_t* counts, fm_batch_stats* stats) {
     const uint32_t nq = (uint32_t)b->batched.size();
     int truncated = 0;
     if (nq) {
+        const bool counting = !b->table || !b->regions_exact;
+        if (b->sums_stale || b->sums_counting != counting) reserve_sums(*b, counting);
         BatchRun run;
         run.b = b;
         run.cv = cv;
@@ -1734,6 +1764,7 @@ fm_status fm_batch_run(fm_batch* b, uint64_t* counts, fm_batch_stats* stats) {
                 done[i] = (b->h_plans[i].count_only || b->solo[i]) ? 1 : 0;
                 if (b->h_plans[i].count_only) b->h_plans[i].n_roots = 0;
             }
+            reserve_sums(*b, false);
             FM_CUDA(cudaMemcpyAsync(b->d_plans, b->h_plans.data(), nq * sizeof(BatchPlan), cudaMemcpyHostToDevice,
                                     cv.stream));
             b->regions_exact = true;

@@ -130,9 +130,8 @@ def test_order_of_a_count_that_sums_cannot_serve(ctx, edges, labels):
     g.close()
 
 
-def test_batches_compute_vertex_sums_only_where_they_pay(ctx):
-    """A table of vertex sums reads every e-line of its label.  Paths whose first label is rare meet few of them: no
-    table; paths over frequent labels of a graph with long lists: one a pair of labels, shared by its queries."""
+def _long_lists(ctx):
+    """5000 vertices, 100000 edges of labels 2 and 3 and 40 of label 1."""
     rng = np.random.default_rng(4)
     n = 5000
     e = np.unique(np.sort(rng.integers(0, n, (100000, 2)), axis=1), axis=0)
@@ -140,7 +139,13 @@ def test_batches_compute_vertex_sums_only_where_they_pay(ctx):
     lab = rng.integers(2, 4, len(e))
     lab[:40] = 1
     src, dst, lab = [np.concatenate(x).astype(np.uint32) for x in ((e[:, 0], e[:, 1]), (e[:, 1], e[:, 0]), (lab, lab))]
-    g = fm.Graph.from_edges(ctx, n, 4, src, dst, lab)
+    return fm.Graph.from_edges(ctx, n, 4, src, dst, lab)
+
+
+def test_batches_compute_vertex_sums_only_where_they_pay(ctx):
+    """A table of vertex sums reads every e-line of its label.  Paths whose first label is rare meet few of them: no
+    table; paths over frequent labels of a graph with long lists: one a pair of labels, shared by its queries."""
+    g = _long_lists(ctx)
     per = 2 if g.info().max_list > 16 else 1
     for labels, shared in (([[1, 2, 3], [1, 3, 2], [1, 2, 2]], None), ([[2, 3, 2], [2, 3, 2]], 1),
                            ([[2, 3, 2], [2, 2, 2], [3, 3, 3]], 0)):
@@ -155,4 +160,40 @@ def test_batches_compute_vertex_sums_only_where_they_pay(ctx):
             counts, st = b.run()
             assert counts == want and st.launches == 3 * per + tables
         b.close()
+    g.close()
+
+
+def test_table_batches_keep_their_level_memory(ctx):
+    """A table batch counts every query once, to size the tables; after that the level region has no tables of vertex
+    sums but those of its count-only queries, and its level buffers take the rest."""
+    g = _long_lists(ctx)
+    qs = [fm.Query.from_text(S.query_path(4, l).to_g_text()) for l in ([2, 3, 2], [2, 2, 2])] + \
+        [fm.Query.from_text(S.query_cycle(3, [1, 2, 3]).to_g_text())]
+    want = [fm.match(ctx, g, q, mode=fm.MODE_COUNT, order=fm.ORDER_REFERENCE).count for q in qs]
+    full = (512 << 20) // (4 * (3 + 4))              # rows of 3 and 4 words at depths 2 and 3
+    c = fm.Batch(ctx, g, qs, mode=fm.MODE_COUNT)
+    counted, st = c.run()
+    assert counted == want and st.level_rows < full
+    c.close()
+    b = fm.Batch(ctx, g, qs, mode=fm.MODE_TABLE)
+    for engine in (fm.ENGINE_LEVELS, fm.ENGINE_PERSISTENT):
+        b.set_engine(engine)
+        for _ in range(3):                           # sizing, captured and replayed
+            counted, st = b.run(allow_truncation=True)
+            assert counted == want and st.level_rows == full
+    b.set_query_mode(0, fm.MODE_COUNT)               # sized again, then one query counted by sums
+    for _ in range(3):
+        counted, st = b.run(allow_truncation=True)
+        assert counted == want and st.level_rows < full
+    b.set_solo(0, True)                              # matched alone: its table goes
+    for _ in range(2):
+        counted, st = b.run(allow_truncation=True)
+        assert counted == want and st.level_rows == full
+    b.set_solo(0, False)
+    b.set_query_mode(0, fm.MODE_TABLE)
+    for _ in range(2):
+        counted, st = b.run(allow_truncation=True)
+        assert counted == want and st.level_rows == full
+    assert len(b.rows(2, want[2])) == want[2]
+    b.close()
     g.close()
