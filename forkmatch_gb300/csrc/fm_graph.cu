@@ -398,14 +398,6 @@ uint32_t bits_for(uint64_t x) {   // bits needed to store values 0..x
     return b;
 }
 
-uint64_t env_bytes(const char* name, uint64_t dflt) {
-    const char* v = std::getenv(name);
-    if (!v || !*v) return dflt;
-    char* end = nullptr;
-    const unsigned long long x = std::strtoull(v, &end, 10);
-    return (end && *end == 0) ? (uint64_t)x : dflt;
-}
-
 uint64_t up256(uint64_t x) { return (x + 255) & ~255ull; }
 
 int grid_for(uint64_t n, int sms) {
@@ -425,6 +417,14 @@ struct Events {                      // destroyed on every return path
 };
 
 }  // namespace
+
+uint64_t env_bytes(const char* name, uint64_t dflt) {
+    const char* v = std::getenv(name);
+    if (!v || !*v) return dflt;
+    char* end = nullptr;
+    const unsigned long long x = std::strtoull(v, &end, 10);
+    return (end && *end == 0) ? (uint64_t)x : dflt;
+}
 
 cudaError_t scan_tiles_u64(unsigned long long* v, uint64_t n, unsigned long long* total, cudaStream_t s) {
     k_scan_tiles<unsigned long long><<<1, 1024, 0, s>>>(v, n, total);

@@ -249,8 +249,9 @@ fm_status parse_data_text_device(const char* text, uint64_t len, cudaStream_t s,
     // lines (a text with more lines has its first bad line among those).
     // Texts up to 64 MiB use that bound for the build's arrays (33 bytes per
     // possible line) and put body and arrays in one allocation; larger ones,
-    // where the bound would cost gigabytes, count the lines first.
-    const bool bound = blen <= (64ull << 20);
+    // where the bound would cost gigabytes, count the lines first
+    // (FM_INGEST_BOUND_BYTES sets the limit).
+    const bool bound = blen <= env_bytes("FM_INGEST_BOUND_BYTES", 64ull << 20);
     BuildArena arena;
     DBuf d_text;
     uint64_t cap = blen / 6 + 1;

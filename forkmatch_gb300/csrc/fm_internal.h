@@ -379,6 +379,9 @@ fm_status batch_create_scratch(fm_context* ctx, const fm_graph* graph, const fm_
 // (independent e-lines, label frequencies): the server's footprint model.
 void estimate_level_rows(const Plan& P, const DeviceGraph& g, double est[kMaxQ]);
 
+// An environment variable's byte count; `dflt` if it is unset or not a number.
+uint64_t env_bytes(const char* name, uint64_t dflt);
+
 // Device graph build (fm_graph.cu).
 // What the build finds out on the device, read back once.
 struct BuildStats {

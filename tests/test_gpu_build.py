@@ -62,3 +62,30 @@ def test_build_totals_and_lists(ctx, form, E, V, L, hub, dup):
         want = list(zip(src[m].tolist(), dst[m].tolist()))
         assert got == sorted(want) or got == sorted((b, a) for a, b in want)
     g.close()
+
+
+@pytest.mark.parametrize("E,V,L,hub,dup", [(0, 5, 2, 0, 0), (1, 1, 2, 0, 0), (513, 3000, 2, 513, 0), (4095, 65, 4, 60, 0),
+                                           (4097, 9000, 3, 4000, 3), (70001, 30011, 5, 9001, 1)])
+def test_texts_whose_lines_are_counted_first(ctx, monkeypatch, E, V, L, hub, dup):
+    """The way of texts above the size limit, where the lines are counted before the build's arrays are sized."""
+    monkeypatch.setenv("FM_INGEST_BOUND_BYTES", "0")
+    test_build_totals_and_lists(ctx, "text", E, V, L, hub, dup)
+
+
+@pytest.mark.parametrize("body,status", [
+    ("", 0), ("\n" * 5000, 6), ("v 0 1\n" * 3 + "\n" * 900, 6), ("e 0 1 1\ne 1 0 1\n", 0), ("e 0 1 1\n" * 4, 6),
+    ("v 0 1\ne 0 1 1\ne 0 4 1\ne 1 0 1\n", 6), ("e 0 1 1\nx 1 0 1\n", 6), ("e 0 1 1\ne 1 0 4294967296\n", 6),
+    ("e 0 1 1\ne 1 0 1", 6), ("v 4 1\n" * 700, 6), ("v 3 1\n" * 700 + "v 3\n" + "v 4 1\n" * 700, 6)])
+def test_both_ways_of_texts_refuse_the_same_lines(ctx, monkeypatch, body, status):
+    """4 vertices, a header of 2 e-lines; FM_ERR_DATA_LINE is 6."""
+    text = "t # 0\n4 2 1 2\n" + body + "t # -1"
+    got = []
+    for limit in (str(1 << 30), "0"):
+        monkeypatch.setenv("FM_INGEST_BOUND_BYTES", limit)
+        try:
+            g = fm.Graph.from_text(ctx, text)
+            got.append((0, g.info().edges, ""))
+            g.close()
+        except fm.FMError as e:
+            got.append((e.status, 0, str(e)))
+    assert got[0] == got[1] and got[0][0] == status
