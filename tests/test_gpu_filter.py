@@ -8,7 +8,8 @@ import pytest
 
 import forkmatch_gb300 as fm
 from forkmatch_gb300 import synth as S
-from tests.helpers import complete_graph
+from oracle import oracle as O
+from tests.helpers import complete_graph, table_sha
 
 pytestmark = pytest.mark.gpu
 
@@ -93,4 +94,46 @@ def test_tables_around_the_first_read_back(ctx, n):
         rows = list(map(tuple, buf[:2 * r.rows_copied].reshape(-1, 2).tolist()))
         assert len(set(rows)) == len(rows) and set(rows) <= set(want)
         assert (buf[2 * r.rows_copied:] == 7).all()
+    g.close()
+
+
+def test_shared_intersections_of_tables_and_middle_levels(ctx):
+    """A dense random graph with 1.1e6 ordered triangles: the table level of 4-cliques and the middle level of 5-cliques
+    share; the rows are the oracle's."""
+    rng = np.random.default_rng(11)
+    n = 420
+    a, b = np.nonzero(np.triu(rng.random((n, n)) < 0.25, 1))
+    src, dst = [np.concatenate(x).astype(np.uint32) for x in ((a, b), (b, a))]
+    lab = np.ones(len(src), dtype=np.uint32)
+    g = fm.Graph.from_edges(ctx, n, 2, src, dst, lab)
+    og = O.Graph.from_edges(n, 2, src, dst, lab)
+    t4, t5 = [S.query_clique(k, [1]).to_g_text() for k in (4, 5)]
+    want, rows, _ = O.match(og, O.plan(t4, enumerate_aut=0), table=True, table_cap=1 << 23)
+    assert want == len(rows) > 1 << 22
+    buf = np.zeros(want * 4, dtype=np.uint32)
+    r = fm.match(ctx, g, fm.Query.from_text(t4), host_rows=buf)
+    assert r.count == want == r.rows_copied and r.routes == fm.ROUTE_SHARED
+    assert table_sha(buf.reshape(-1, 4)) == table_sha(rows)
+    r = fm.match(ctx, g, fm.Query.from_text(t5), mode=fm.MODE_COUNT)
+    assert r.count == O.match(og, O.plan(t5, enumerate_aut=0), count_rule=True)[0] and r.routes & fm.ROUTE_SHARED
+    g.close()
+
+
+def test_shared_intersections_in_pieces(ctx):
+    """Two groups of 20 hubs, all hubs joined, each group joined to 1400 leaves of its own.  Two hubs of one group have
+    1438 common neighbours, which do not fit the buffer, and the rows of such a pair with a third hub have about 1439
+    candidates each; hubs of different groups have 38, which fit.  Rows of both kinds meet in chunks of more than
+    32768 candidates, which the heavy pass loads again, piece by piece."""
+    hubs, leaves = 40, 1400
+    a, b = np.triu_indices(hubs, 1)
+    h, x = [v.ravel() for v in np.meshgrid(np.arange(hubs), np.arange(leaves))]
+    a, b = np.concatenate([a, h]), np.concatenate([b, hubs + (h % 2) * leaves + x])
+    src, dst = [np.concatenate(v).astype(np.uint32) for v in ((a, b), (b, a))]
+    g = fm.Graph.from_edges(ctx, hubs + 2 * leaves, 2, src, dst, np.ones(len(src), dtype=np.uint32))
+    want = math.perm(hubs, 4) + 2 * 4 * math.perm(hubs // 2, 3) * leaves
+    k4 = fm.Query.from_text(S.query_clique(4, [1]).to_g_text())
+    for mode in (fm.MODE_COUNT, fm.MODE_TABLE):
+        for order in (fm.ORDER_AUTO, fm.ORDER_REFERENCE):
+            r = fm.match(ctx, g, k4, mode=mode, order=order, allow_truncation=True)
+            assert r.count == want and r.routes == fm.ROUTE_SHARED | fm.ROUTE_SHARED_PIECES
     g.close()
