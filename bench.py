@@ -91,11 +91,18 @@ def match_alg_bytes(r, qi, count_only):
     table rows, or only counted).  A count-only last depth with one back edge
     is charged its lookups only (the count rule: one record per parent, the
     parent's vertices tested against it), and the depth before it stores
-    nothing when the match counted from there (pre-count)."""
+    nothing when the match counted from there (pre-count).  Last two depths
+    counted by sums are charged a parent's row and its two records alone: no
+    candidate is looked at, and the words of the list that is intersected are
+    not reported, so their figure is a lower bound."""
     q = qi.q
     b = 0
+    sums = getattr(r, "routes", 0) & 1           # forkmatch_gb300.ROUTE_SUMS
     for d in range(1, q):
         lv = r.level[d]
+        if sums and d >= q - 2:
+            b += (4 * d + 32) * lv.parents if d == q - 2 else 0
+            continue
         rule = count_only and d == q - 1 and qi.nreq[d] == 1
         stored = d < q - 1 and not (r.pre_counted and d == q - 2)
         b += 16 * lv.lookups + (0 if rule else 4 * lv.list_words) + (8 * lv.produced if stored else 0)
@@ -669,8 +676,9 @@ def run_batched(args, rank, world, local):
         cnt, rows, _ = fm.match_table(ctx, g, queries[i], max_rows=max(1, rec[i]))
         plain_rows[i] = rows[np.lexsort(rows.T[::-1])] if len(rows) else rows
 
-    # roofline numerator: the algorithmic bytes of every query (same matching
-    # order in both forms), from the plain form's per-level counters
+    # roofline numerator: the algorithmic bytes of every query, from the plain
+    # form's per-level counters (a batch matches some count-only paths in
+    # another order, and not all of them by sums)
     prof = []
     plain_step(collect=prof, profile=True)
     alg_each = [match_alg_bytes(r, qi, c_only) for r, qi, c_only in zip(prof, qinfo, counted)]
@@ -809,14 +817,17 @@ def run_batched(args, rank, world, local):
                          "traffic": batched_traffic(alg_bytes / max(1, world) - alg_alone, alg_alone),
                          "kernel": "one batch run: k_bexpand + k_bexpand_heavy for the shared launches (k_bpersist "
                                    "when the tuner picks the persistent engine), k_expand + k_expand_heavy for the "
-                                   "queries matched alone (the dominant one: the pre-count level of the 5-vertex "
-                                   "count-only paths)",
+                                   "queries matched alone (the dominant one: the counting level of the 5-vertex "
+                                   "count-only paths, by sums)",
                          "peak_kind": peak_kind, "algorithmic_bytes_per_step": alg_bytes,
                          "traffic_source": "profiles/k_bexpand_batched.md (DRAM bytes per algorithmic byte of "
                                            "the batch kernels and of the single-query kernels, captured on every "
                                            "32nd query at 2^20 vertices, applied to this run's shared and alone "
                                            "queries)",
-                         "note": "achieved = algorithmic bytes of all queries / device time of one batch run"},
+                         "note": "achieved = algorithmic bytes of all queries / device time of one batch run; they "
+                                 "hold every looked-up list at its full length, of which the kernels read one list "
+                                 "and one filter word a candidate, and a lower bound for depths counted by sums: "
+                                 "traffic is what DRAM moves"},
             "cpu_baseline": cpu,
             "e2e_paths": e2e_paths, "e2e": e2e,
             "gpu_launches": b_launch, "clocks": clocks,

@@ -62,3 +62,15 @@ def test_batched_traffic_uses_both_kernel_families():
     got = bench.batched_traffic(1_000_000_000, 3_000_000_000)
     want = 1e9 * ratios["traffic_bytes_per_algorithmic_byte"] + 3e9 * ratios["traffic_bytes_per_algorithmic_byte_single"]
     assert got == pytest.approx(want, rel=1e-9)
+
+
+def test_depths_counted_by_sums_charge_rows_and_records():
+    # q = 4, the last two depths by sums: 80 parents of depth 2 read a row of 2 and two records each
+    r = _result([(0, 0, 0), (10, 40, 30), (80, 5000, 0), (900, 70000, 123456)], count=123456, pre_counted=1)
+    r.level[2].parents = 80
+    r.routes = 1
+    want = (16 * 10 + 4 * 40 + 8 * 30) + 80 * (4 * 2 + 2 * 16)
+    assert bench.match_alg_bytes(r, _info(4, [0, 1, 1, 1]), True) == want
+    r.routes = 2                                     # shared intersections alone change nothing
+    assert bench.match_alg_bytes(r, _info(4, [0, 1, 1, 1]), True) == \
+        (16 * 10 + 4 * 40 + 8 * 30) + (16 * 80 + 4 * 5000) + 16 * 900
