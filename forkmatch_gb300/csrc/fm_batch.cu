@@ -276,8 +276,8 @@ __device__ __forceinline__ bool bstage_lists(const BatchParams& P, const BMem& m
 // A parent counted by sums: its closed part; the shorter of the two lists whose
 // members are to be taken off goes to `drv_rec` (index `drv`, length `n`).
 __device__ __forceinline__ unsigned long long bsum_parent(const BatchParams& P, const BMem& m, const BSlices& S,
-                                                          const BatchPlan& pl, const uint4 a, uint32_t anc, uint32_t lab,
-                                                          uint32_t lane, uint32_t d, uint4& drv_rec, uint32_t& drv,
+                                                          const BatchPlan& pl, const uint4 a, uint32_t anc,
+                                                          uint32_t lab, uint32_t lane, uint32_t d, uint4& drv_rec, uint32_t& drv,
                                                           uint32_t& n) {
     const uint32_t rl = pl.req_begin[d + 1], last_anc = pl.req_anc[rl], ll = pl.req_label[rl];
     const uint4* last = P.seg + (uint64_t)ll * P.V;
@@ -301,7 +301,8 @@ __device__ __forceinline__ unsigned long long bsum_parent(const BatchParams& P, 
     } else {
         const uint32_t vb = m.rows_s[last_anc * 32 + lane];
         const uint4 b = ldg4(last + vb);
-        const uint32_t in_b = dev::member_mask(b, m.rows_s, lane, d, last_anc, S.at(P, ll), vb, P.nbr, P.bm, P.bm_words);
+        const uint32_t in_b =
+            dev::member_mask(b, m.rows_s, lane, d, last_anc, S.at(P, ll), vb, P.nbr, P.bm, P.bm_words);
         c = free_a * (b.x - __popc(in_b));
         if (pl.sum_kind == kSumForkSame) return c - free_a;
         if (pl.sum_kind == kSumForkOne) return c - (__ldcg(&pl.vsum[va].y) - __popc(in_a & in_b));
@@ -581,8 +582,8 @@ __device__ __forceinline__ void bprocess(const BatchParams& P, const BMem& m, co
                     for (uint32_t i = 0; i < k && in; i++) {
                         if (i == dd) continue;
                         const uint32_t ref = m.ref_s[i * 32 + jj];
-                        const uint4 r = sw ? m.segs_s[i * 32 + jj]
-                                           : ldg4(P.seg + (uint64_t)(ref >> 8) * P.V + m.rows_s[(ref & 0xffu) * 32 + jj]);
+                        const uint32_t v = m.rows_s[(ref & 0xffu) * 32 + jj];
+                        const uint4 r = sw ? m.segs_s[i * 32 + jj] : ldg4(P.seg + (uint64_t)(ref >> 8) * P.V + v);
                         in = dev::seg_has_st(r, xx, 1, P.nbr, P.bm, P.bm_words, m.stage);
                     }
                 }
@@ -708,8 +709,8 @@ __device__ __forceinline__ void bexpand_main(const BatchParams& P, unsigned char
                 if (pub) continue;
             }
             bprocess<ROOTS>(P, m, S, chunk, excl, n, 0, total, lane, d, sw, nst);
-            // the stage refers to this chunk's query ids only through stq, and to
-            // its parents through pidx: it can outlive the chunk
+            // the stage holds the survivors' query ids (stq) and parents' indices
+            // in the level (stp): it can outlive the chunk
         }
     }
     if (nst) bflush<ROOTS>(P, m, nst, lane, d, last_chunk);

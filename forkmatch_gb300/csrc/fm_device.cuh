@@ -16,10 +16,11 @@ __device__ __forceinline__ uint4 ldg4(const uint4* p) { return __ldg(p); }
 // for the pass before it (`pass_wait`) ahead of reading anything that pass
 // wrote: the control blocks, the level's rows, heavy entries and vertex sums.
 // Those are read with ordinary, volatile or `ldcg` loads after the wait, never
-// through the read-only path, whose contract ends at a grid's launch.  Without the launch attribute both are
-// no-ops.  With one clear and one read-back a match instead of one a level, and
-// no heavy pass where no chunk can need one, a 4-vertex count on 300 vertices
-// takes 46 us instead of 83, twelve nearly empty levels 296 us instead of 375.
+// through the read-only path, whose contract ends at a grid's launch.  Without
+// the launch attribute both are no-ops.  With one clear and one read-back a match
+// instead of one a level, and no heavy pass where no chunk can need one, a
+// 4-vertex count on 300 vertices takes 46 us instead of 83, twelve nearly empty
+// levels 296 us instead of 375.
 __device__ __forceinline__ void pass_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pass_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -499,8 +499,8 @@ struct MatchRun {
         if (!vsum) return cudaSuccess;
         res->launches++;
         const uint64_t h = g->head_off[sum_label];
-        return launch_vertex_sums(p, g->heads + h, (uint32_t)(g->head_off[sum_label + 1] - h), sum_label, sum_last, vsum,
-                                  parents, s);
+        return launch_vertex_sums(p, g->heads + h, (uint32_t)(g->head_off[sum_label + 1] - h), sum_label, sum_last,
+                                  vsum, parents, s);
     }
 
     uint32_t last_depth() const { return plan->q - 1 - (pre ? 1u : 0u); }
@@ -872,7 +872,10 @@ bool rows_enough(const DeviceGraph& g, uint32_t stored, uint64_t cap) {
 // would walk once as well.  The sums take 8 bytes a vertex of the level memory,
 // at most an eighth of it, and a launch of their own: below 4096 lists that
 // launch (3 us) is more than the level saves (300 vertices: 86 us a match with,
-// 83 without).
+// 83 without).  Forks that need no vertex sums are held to the same minimum, for
+// the plan of the order that they cost: without it sparse graphs of 3000 vertices
+// lose 3 us of 75, dense ones would gain (5-vertex path, 200 neighbours a vertex:
+// 1.6 ms by sums, 4.0 candidate by candidate).
 bool sums_plan(const fm_context* ctx, const DeviceGraph& g, uint32_t q, const uint32_t* nreq,
                const uint32_t (*climb)[kMaxQ], const uint32_t (*rlab)[kMaxQ], SumsPlan& out) {
     if (q < 4 || nreq[q - 2] != 1 || nreq[q - 1] != 1) return false;
@@ -1081,7 +1084,8 @@ fm_status match_impl(fm_context* ctx, const fm_graph* graph, const fm_query* que
         if (table && opts.host_rows && !direct && cudaPointerGetAttributes(&at, opts.host_rows) != cudaSuccess)
             cudaGetLastError();
         if (table && opts.host_rows && !direct && at.type != cudaMemoryTypeDevice)
-            run.first_rows = std::min<uint64_t>(kFirstRowBytes, std::min<uint64_t>(table_cap, opts.host_rows_cap) * q * 4);
+            run.first_rows =
+                std::min<uint64_t>(kFirstRowBytes, std::min<uint64_t>(table_cap, opts.host_rows_cap) * q * 4);
         b.table_vec4 = (q % 4 == 0 && ((uintptr_t)table_ptr % 16) == 0) ? 1u : 0u;
         b.ctl = ctx->ctl;
         b.tot = ctx->tot;

@@ -174,8 +174,8 @@ __host__ __device__ constexpr uint32_t n_recs(uint32_t k, bool dups, uint32_t st
     return dups || stage_words ? k : 1;
 }
 
-__device__ __forceinline__ WarpMem warp_mem(unsigned char* smem_raw, uint32_t warp, uint32_t d, uint32_t k, uint32_t recs,
-                                            uint32_t stage_words, bool staged, uint32_t share_words,
+__device__ __forceinline__ WarpMem warp_mem(unsigned char* smem_raw, uint32_t warp, uint32_t d, uint32_t k,
+                                            uint32_t recs, uint32_t stage_words, bool staged, uint32_t share_words,
                                             uint64_t* mbar_s) {
     unsigned char* ws = smem_raw + warp * per_warp_bytes(d, k, recs, stage_words, staged, share_words);
     WarpMem m;
@@ -774,8 +774,8 @@ __device__ __forceinline__ void expand_main(const ExpandParams& P, unsigned char
             bool valid, stage_ok;
             unsigned long long w;
             uint32_t excl, n;
-            const uint32_t total = load_chunk<ROOTS, DUPS, SHARE>(P, m, chunk, lane, d, k, rb, T.n_parents, valid, w, phase,
-                                                     stage_ok, excl, n, L, share_on, share);
+            const uint32_t total = load_chunk<ROOTS, DUPS, SHARE>(P, m, chunk, lane, d, k, rb, T.n_parents, valid, w,
+                                                                  phase, stage_ok, excl, n, L, share_on, share);
             last_chunk = chunk;
             if (!stage_ok) {
                 done = true;
@@ -848,8 +848,8 @@ __device__ __forceinline__ void expand_main(const ExpandParams& P, unsigned char
                 pub = __shfl_sync(kFull, pub, 0);
                 if (pub) continue;
             }
-            process_slots<MODE, ROOTS, DUPS, SHARE>(P, m, chunk, excl, n, 0, total, lane, d, k, L, col_depth_s, nst, n_count,
-                                             pre);
+            process_slots<MODE, ROOTS, DUPS, SHARE>(P, m, chunk, excl, n, 0, total, lane, d, k, L, col_depth_s, nst,
+                                                    n_count, pre);
         }
     }
     if (MODE != kModeLastCount && nst) flush_stage<MODE, ROOTS>(P, m, nst, lane, d, col_depth_s, last_chunk);
@@ -913,11 +913,12 @@ __device__ __forceinline__ void expand_heavy(const ExpandParams& P, unsigned cha
         bool valid, stage_ok;
         unsigned long long w;
         uint32_t excl, n;
-        load_chunk<ROOTS, DUPS, SHARE>(P, m, e.chunk, lane, d, k, rb, T.n_parents, valid, w, phase, stage_ok, excl, n, L, share_on, share);
+        load_chunk<ROOTS, DUPS, SHARE>(P, m, e.chunk, lane, d, k, rb, T.n_parents, valid, w, phase, stage_ok, excl, n,
+                                       L, share_on, share);
         last_chunk = e.chunk;
         if (!stage_ok) break;
-        process_slots<MODE, ROOTS, DUPS, SHARE>(P, m, e.chunk, excl, n, begin, end, lane, d, k, L, col_depth_s, nst, n_count,
-                                             pre);
+        process_slots<MODE, ROOTS, DUPS, SHARE>(P, m, e.chunk, excl, n, begin, end, lane, d, k, L, col_depth_s, nst,
+                                                n_count, pre);
     }
     if (MODE != kModeLastCount && nst) flush_stage<MODE, ROOTS>(P, m, nst, lane, d, col_depth_s, last_chunk);
     if (MODE == kModeLastCount && lane == 0 && n_count > n_flushed) atomicAdd(&P.tot->count, n_count - n_flushed);
@@ -1280,9 +1281,11 @@ __global__ void __launch_bounds__(kWarps * 32) k_vertex_sums(const __grid_consta
 
 // Blocks per SM a pass is compiled for.  Closing and counting levels, which hold
 // most of a large match's work, want every warp they can get (6 blocks, 40
-// registers; 4 blocks: closing a 4-cycle 12 % slower).  Middle levels of walk
-// queries are mostly small, and there fewer, unspilled warps and fewer blocks to
-// start win: 4 blocks (64 registers) took a 13-vertex walk's match from 312 to
+// registers, spilling 100 to 400 bytes; 4 blocks: closing a 4-cycle 12 % slower;
+// 5 for table levels: 4-vertex stars 2 % faster, closing a 4-cycle 4 % slower).
+// Middle levels of walk queries are mostly small, and there fewer warps, which
+// spill nothing (with shared intersections 84 bytes), and fewer blocks to start
+// win: 4 blocks (64 registers) took a 13-vertex walk's match from 312 to
 // 267 us and left the large ones where they were (4-cycle 1069 and 1057 us, 3
 // blocks: 8-vertex walks and 4-cliques slower again).
 constexpr int min_blocks(int mode) { return mode == kModeMid ? 4 : 6; }
@@ -1298,7 +1301,8 @@ __global__ void __launch_bounds__(kWarps * 32, min_blocks(MODE)) k_expand(const 
     if (threadIdx.x < (unsigned)kMaxQ) col_depth_s[threadIdx.x] = P.plan.col_depth[threadIdx.x];
     dev::stage_barriers_init(mbar_s);
     dev::pass_wait();
-    if (MODE == kModeLastCount && !ROOTS && !DUPS && !SHARE && P.sum_rule && sum_rule_on(P, make_tune(P, true).n_parents)) {
+    if (MODE == kModeLastCount && !ROOTS && !DUPS && !SHARE && P.sum_rule &&
+        sum_rule_on(P, make_tune(P, true).n_parents)) {
         expand_sum_main(P, smem_raw, mbar_s);
         return;
     }
@@ -1307,7 +1311,8 @@ __global__ void __launch_bounds__(kWarps * 32, min_blocks(MODE)) k_expand(const 
 }
 
 template <int MODE, bool ROOTS, bool DUPS, bool SHARE>
-__global__ void __launch_bounds__(kWarps * 32, min_blocks(MODE)) k_expand_heavy(const __grid_constant__ ExpandParams P) {
+__global__ void __launch_bounds__(kWarps * 32, min_blocks(MODE))
+    k_expand_heavy(const __grid_constant__ ExpandParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint8_t col_depth_s[kMaxQ];
     __shared__ uint64_t mbar_s[kWarps];
@@ -1317,7 +1322,8 @@ __global__ void __launch_bounds__(kWarps * 32, min_blocks(MODE)) k_expand_heavy(
     if (threadIdx.x < (unsigned)kMaxQ) col_depth_s[threadIdx.x] = P.plan.col_depth[threadIdx.x];
     dev::stage_barriers_init(mbar_s);
     dev::pass_wait();
-    if (MODE == kModeLastCount && !ROOTS && !DUPS && !SHARE && P.sum_rule && sum_rule_on(P, make_tune(P, false).n_parents)) {
+    if (MODE == kModeLastCount && !ROOTS && !DUPS && !SHARE && P.sum_rule &&
+        sum_rule_on(P, make_tune(P, false).n_parents)) {
         expand_sum_heavy(P, smem_raw, mbar_s);
         return;
     }

@@ -463,7 +463,8 @@ struct OrderModel {
     double V;
     std::vector<double> line_avg;
 
-    OrderModel(const Plan& plan, const DeviceGraph& g) : P(plan), row(plan), V((double)g.V), line_avg(plan.rows.size()) {
+    OrderModel(const Plan& plan, const DeviceGraph& g)
+        : P(plan), row(plan), V((double)g.V), line_avg(plan.rows.size()) {
         for (size_t r = 0; r < P.rows.size(); r++) {
             const uint32_t l = P.rows[r].l;
             line_avg[r] = (double)(l < g.label_count.size() ? g.label_count[l] : 0) / V;
