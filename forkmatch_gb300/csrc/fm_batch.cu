@@ -55,7 +55,7 @@ struct BatchParams {
     const uint32_t* nbr;
     const uint32_t* bm;                       // list bitmaps (see DeviceGraph)
     uint32_t bm_words;
-    uint32_t bm_near;
+    uint32_t bm_common;                       // DeviceGraph::bitmaps_common
     const uint32_t* efilter;                  // e-line filter and its slices by label (see DeviceGraph)
     const uint32_t* efilter_off;
     uint32_t L;                               // label slots
@@ -375,7 +375,7 @@ __device__ __forceinline__ uint32_t bload_chunk(const BatchParams& P, const BMem
             const uint4 sg = best;
             const uint32_t ref = m.ref_s[lane];
             rule_cnt = sg.x - dev::count_members_f(sg, S.at(P, ref >> 8), m.rows_s[(ref & 0xffu) * 32 + lane], m.rows_s,
-                                                   lane, d, 0u, false, P.nbr, P.bm, P.bm_words, P.bm_near);
+                                                   lane, d, 0u, false, P.nbr, P.bm, P.bm_words, P.bm_common);
             n = 0;
         }
     }
@@ -461,7 +461,7 @@ __device__ __forceinline__ void bprecount(const BatchParams& P, const BMem& m, c
         const uint32_t lab = pl.req_label[rb], v = anc == d ? x : m.rows_s[anc * 32 + j];
         const uint4 sg = ldg4(P.seg + (uint64_t)lab * P.V + v);
         c = sg.x - dev::count_members_f(sg, S.at(P, lab), v, m.rows_s, j, d, x, P.self_loops || anc != d, P.nbr, P.bm,
-                                        P.bm_words, P.bm_near);
+                                        P.bm_words, P.bm_common);
     }
     const unsigned grp = __match_any_sync(kFull, qid);
     const unsigned lo = __reduce_add_sync(grp, c & 0xffffu);
@@ -1687,7 +1687,7 @@ fm_status fm_batch_run(fm_batch* b, uint64_t* counts, fm_batch_stats* stats) {
         run.base.nbr = g.nbr;
         run.base.bm = g.bitmaps;
         run.base.bm_words = g.bm_words;
-        run.base.bm_near = g.bitmaps_near();
+        run.base.bm_common = g.bitmaps_common();
         run.base.efilter = g.efilter;
         run.base.efilter_off = g.efilter_off;
         run.base.L = g.L;

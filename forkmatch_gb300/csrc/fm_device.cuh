@@ -183,21 +183,24 @@ __device__ __forceinline__ uint32_t member_mask(const uint4& s, const uint32_t* 
 }
 
 // How many of the row's vertices and, with `extra`, x, are in the list s of
-// vertex v: count_members with the filter in front.  `bm_near`: a list's bitmap
-// is asked instead, which is one load a value and none of the filter's 20
-// instructions: better while the bitmaps stay in the L2 (5-vertex path on 3000
-// vertices and 400000 edges, 3 MB of bitmaps: 12.0 ms, 17.4 with the filter; 13.4
-// before there was one), worse when they do not (2^20-vertex R-MAT graph, 2 GB:
-// 34.9 and 33.2 ms).
+// vertex v: count_members with the filter in front.  `bm_common`: a list's bitmap
+// is asked instead, which is one load a value, none of the filter's 20
+// instructions and no exact test.  Better where enough of the lists have one that
+// lanes mostly agree, whatever the bitmaps take (5-vertex paths, share of lists
+// with a bitmap, time against the filter's: random graphs 0.03 1.06, 0.17 0.96,
+// 0.24 0.93, 0.64 0.80, 1.0 0.69 to 1.02, with 511 MB of them 0.91; R-MAT and
+// power-law graphs, whose hubs' lists are few, 0.001 to 0.09: 1.00 to 1.10): from
+// an eighth of the lists on.
 __device__ __forceinline__ uint32_t count_members_f(const uint4& s, const FilterSlice& f, uint32_t v,
                                                     const uint32_t* rows_s, uint32_t j, uint32_t n_row, uint32_t x,
                                                     bool extra, const uint32_t* __restrict__ nbr,
                                                     const uint32_t* __restrict__ bm, uint32_t bm_words,
-                                                    uint32_t bm_near) {
+                                                    uint32_t bm_common) {
     if (s.x == 0) return 0;
-    if (bm_near && s.x > 3 && (s.z & kBitmapMark)) {
+    if (bm_common && s.x > 3 && (s.z & kBitmapMark)) {
         const uint32_t* b = bm + (uint64_t)(s.z & ~kBitmapMark) * bm_words;
         uint32_t n = extra ? (__ldg(b + (x >> 5)) >> (x & 31)) & 1u : 0u;
+#pragma unroll 1
         for (uint32_t i = 0; i < n_row; i++) {
             const uint32_t w = rows_s[i * 32 + j];
             n += (__ldg(b + (w >> 5)) >> (w & 31)) & 1u;

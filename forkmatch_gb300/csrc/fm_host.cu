@@ -594,7 +594,7 @@ struct MatchRun {
             const bool roots = d == 1;
             const size_t smem = level_smem(d);
             const bool share = shares(d);
-            const int per_sm = expand_blocks_per_sm(mode, roots, dups, share, smem, block);
+            const int per_sm = expand_blocks_per_sm(mode, roots, dups, share, base.bm_common != 0, smem, block);
             const int full = ctx->sms * per_sm;
             warps[d] = (uint64_t)full * (block / 32);
             ExpandParams p = base;
@@ -741,7 +741,7 @@ struct MatchRun {
         const uint64_t n_chunks = (n_parents + 31) / 32;
         const size_t smem = level_smem(d);
         const bool share = shares(d);
-        const int per_sm = expand_blocks_per_sm(mode, roots, dups, share, smem, block);
+        const int per_sm = expand_blocks_per_sm(mode, roots, dups, share, base.bm_common != 0, smem, block);
         (void)q;
         while (true) {
             const uint64_t items = ndef_in + (n_chunks - fresh);
@@ -1056,7 +1056,7 @@ fm_status match_impl(fm_context* ctx, const fm_graph* graph, const fm_query* que
         b.nbr = g.nbr;
         b.bm = g.bitmaps;
         b.bm_words = g.bm_words;
-        b.bm_near = g.bitmaps_near();
+        b.bm_common = g.bitmaps_common();
         b.efilter = g.efilter;
         b.efilter_off = g.efilter_off;
         b.V = g.V;

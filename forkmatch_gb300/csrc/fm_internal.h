@@ -61,8 +61,8 @@ struct DeviceGraph {
     uint32_t* efilter_off = nullptr;
     uint64_t filter_bytes = 0;           // of both
     uint32_t n_bitmaps = 0;
-    // All bitmaps take at most half of the L2 (64 of 129 MB).
-    bool bitmaps_near() const { return (uint64_t)n_bitmaps * bm_words * 4 <= (64ull << 20); }
+    // At least an eighth of all lists have a bitmap (see dev::count_members_f).
+    bool bitmaps_common() const { return n_bitmaps && 8ull * n_bitmaps >= segments; }
     uint32_t bm_min_len = 0;
     uint64_t nbr_words = 0;
     uint64_t segments = 0, long_segments = 0;
@@ -173,7 +173,7 @@ struct ExpandParams {
     const uint32_t* nbr;
     const uint32_t* bm;             // list bitmaps (see DeviceGraph)
     uint32_t bm_words;
-    uint32_t bm_near;               // they stay in the L2 (see dev::count_members_f)
+    uint32_t bm_common;             // DeviceGraph::bitmaps_common
     const uint32_t* efilter;        // e-line filter and its slices by label (see DeviceGraph)
     const uint32_t* efilter_off;
     uint32_t V;
@@ -329,7 +329,7 @@ cudaError_t launch_vertex_sums(const ExpandParams& p, const uint32_t* heads, uin
 // Let kernel f launch with up to the device's opt-in shared memory (once per
 // device; safe from several host threads).
 void allow_dynamic_smem(const void* f);
-int expand_blocks_per_sm(int mode, bool roots, bool dups, bool share, size_t smem, int block);
+int expand_blocks_per_sm(int mode, bool roots, bool dups, bool share, bool common, size_t smem, int block);
 
 // The parts of a context other translation units use (fm_host.cu owns it).
 struct ContextView {

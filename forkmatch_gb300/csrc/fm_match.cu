@@ -543,7 +543,7 @@ struct Emit {
     unsigned long long lane_count = 0;    // pre-counted by this lane
 };
 
-template <int MODE, bool ROOTS, bool DUPS>
+template <int MODE, bool ROOTS, bool DUPS, bool COMMON>
 __device__ __forceinline__ void emit(const ExpandParams& P, const WarpMem& m, uint32_t chunk, bool ok, uint32_t j,
                                      uint32_t x, uint32_t lane, uint32_t d, const uint8_t* col_depth_s, bool more,
                                      Emit& e, PreAcc& pre) {
@@ -559,7 +559,7 @@ __device__ __forceinline__ void emit(const ExpandParams& P, const WarpMem& m, ui
         const uint4 sg = ldg4(segl + v);
         const dev::FilterSlice f = dev::filter_slice(P.efilter, P.efilter_off, P.plan.req_label[rb]);
         e.lane_count += sg.x - dev::count_members_f(sg, f, v, m.rows_s, j, d, x, P.self_loops || anc != d, P.nbr, P.bm,
-                                                    P.bm_words, P.bm_near);
+                                                    P.bm_words, COMMON ? P.bm_common : 0u);
         pre.parents += 1;
         pre.words += sg.x;
         return;
@@ -592,7 +592,7 @@ __device__ __forceinline__ void emit(const ExpandParams& P, const WarpMem& m, ui
 // slots and by the L1's rate for scattered words.  Closing level of a 4-cycle on
 // a 2^20-vertex R-MAT graph with 64 labels (1.7e7 parents): 740 us, 1100 us with
 // an exact test per candidate and a binary search per slot for its parent.
-template <int MODE, bool ROOTS, bool DUPS, bool SHARE>
+template <int MODE, bool ROOTS, bool DUPS, bool SHARE, bool COMMON>
 __device__ __forceinline__ void process_slots(const ExpandParams& P, const WarpMem& m, uint32_t chunk,
                                               uint32_t excl, uint32_t n, uint32_t begin, uint32_t end, uint32_t lane,
                                               uint32_t d, uint32_t k, const LevelLists& L,
@@ -641,7 +641,7 @@ __device__ __forceinline__ void process_slots(const ExpandParams& P, const WarpM
             }
 #pragma unroll
             for (uint32_t u = 0; u < kSlots; u++)
-                emit<MODE, ROOTS, DUPS>(P, m, chunk, ok[u], j[u], x[u], lane, d, col_depth_s,
+                emit<MODE, ROOTS, DUPS, COMMON>(P, m, chunk, ok[u], j[u], x[u], lane, d, col_depth_s,
                                         u + 1 < kSlots && (!DUPS || k == 1), e, pre);
             continue;
         }
@@ -683,7 +683,7 @@ __device__ __forceinline__ void process_slots(const ExpandParams& P, const WarpM
                     }
                     for (uint32_t c = 0; c < d && in; c++) in = m.rows_s[c * 32 + jj] != xx;
                 }
-                emit<MODE, ROOTS, DUPS>(P, m, chunk, in, jj, xx, lane, d, col_depth_s, false, e, pre);
+                emit<MODE, ROOTS, DUPS, COMMON>(P, m, chunk, in, jj, xx, lane, d, col_depth_s, false, e, pre);
             }
             __syncwarp();
         }
@@ -725,7 +725,7 @@ __device__ __forceinline__ bool over_limit(const ExpandParams& P, uint32_t lane,
 
 // Main pass: warps claim batches of chunks; long candidate ranges are
 // published to the heavy list instead of being walked by one warp.
-template <int MODE, bool ROOTS, bool DUPS, bool SHARE>
+template <int MODE, bool ROOTS, bool DUPS, bool SHARE, bool COMMON>
 __device__ __forceinline__ void expand_main(const ExpandParams& P, unsigned char* smem_raw, const LevelLists& L,
                                             const uint8_t* col_depth_s, uint64_t* mbar_s, uint32_t& phase) {
     const uint32_t lane = threadIdx.x & 31;
@@ -848,7 +848,7 @@ __device__ __forceinline__ void expand_main(const ExpandParams& P, unsigned char
                 pub = __shfl_sync(kFull, pub, 0);
                 if (pub) continue;
             }
-            process_slots<MODE, ROOTS, DUPS, SHARE>(P, m, chunk, excl, n, 0, total, lane, d, k, L, col_depth_s, nst,
+            process_slots<MODE, ROOTS, DUPS, SHARE, COMMON>(P, m, chunk, excl, n, 0, total, lane, d, k, L, col_depth_s, nst,
                                                     n_count, pre);
         }
     }
@@ -874,7 +874,7 @@ __device__ __forceinline__ void expand_main(const ExpandParams& P, unsigned char
 // chunks, reloads that chunk and walks its piece of the slots -- the warps
 // that finished their own chunks take over the work of the hub chunks.  The
 // main pass already holds the chunk's output budget and counted its work.
-template <int MODE, bool ROOTS, bool DUPS, bool SHARE>
+template <int MODE, bool ROOTS, bool DUPS, bool SHARE, bool COMMON>
 __device__ __forceinline__ void expand_heavy(const ExpandParams& P, unsigned char* smem_raw, const LevelLists& L,
                                              const uint8_t* col_depth_s, uint64_t* mbar_s, uint32_t& phase) {
     const unsigned long long h = *(volatile unsigned long long*)&P.ctl->heavy;
@@ -917,7 +917,7 @@ __device__ __forceinline__ void expand_heavy(const ExpandParams& P, unsigned cha
                                        L, share_on, share);
         last_chunk = e.chunk;
         if (!stage_ok) break;
-        process_slots<MODE, ROOTS, DUPS, SHARE>(P, m, e.chunk, excl, n, begin, end, lane, d, k, L, col_depth_s, nst,
+        process_slots<MODE, ROOTS, DUPS, SHARE, COMMON>(P, m, e.chunk, excl, n, begin, end, lane, d, k, L, col_depth_s, nst,
                                                 n_count, pre);
     }
     if (MODE != kModeLastCount && nst) flush_stage<MODE, ROOTS>(P, m, nst, lane, d, col_depth_s, last_chunk);
@@ -1290,7 +1290,7 @@ __global__ void __launch_bounds__(kWarps * 32) k_vertex_sums(const __grid_consta
 // blocks: 8-vertex walks and 4-cliques slower again).
 constexpr int min_blocks(int mode) { return mode == kModeMid ? 4 : 6; }
 
-template <int MODE, bool ROOTS, bool DUPS, bool SHARE>
+template <int MODE, bool ROOTS, bool DUPS, bool SHARE, bool COMMON>
 __global__ void __launch_bounds__(kWarps * 32, min_blocks(MODE)) k_expand(const __grid_constant__ ExpandParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint8_t col_depth_s[kMaxQ];
@@ -1307,10 +1307,10 @@ __global__ void __launch_bounds__(kWarps * 32, min_blocks(MODE)) k_expand(const 
         return;
     }
     uint32_t phase = 0;
-    expand_main<MODE, ROOTS, DUPS, SHARE>(P, smem_raw, L, col_depth_s, mbar_s, phase);
+    expand_main<MODE, ROOTS, DUPS, SHARE, COMMON>(P, smem_raw, L, col_depth_s, mbar_s, phase);
 }
 
-template <int MODE, bool ROOTS, bool DUPS, bool SHARE>
+template <int MODE, bool ROOTS, bool DUPS, bool SHARE, bool COMMON>
 __global__ void __launch_bounds__(kWarps * 32, min_blocks(MODE))
     k_expand_heavy(const __grid_constant__ ExpandParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1328,7 +1328,7 @@ __global__ void __launch_bounds__(kWarps * 32, min_blocks(MODE))
         return;
     }
     uint32_t phase = 0;
-    expand_heavy<MODE, ROOTS, DUPS, SHARE>(P, smem_raw, L, col_depth_s, mbar_s, phase);
+    expand_heavy<MODE, ROOTS, DUPS, SHARE, COMMON>(P, smem_raw, L, col_depth_s, mbar_s, phase);
 }
 
 // ------------------------------------------------------- persistent engine
@@ -1346,11 +1346,11 @@ template <int LAST, bool DUPS>
 __device__ __forceinline__ void persist_main(const ExpandParams& P, unsigned char* smem, const uint8_t* cd,
                                              bool roots, bool last, const LevelLists& L, uint64_t* mb, uint32_t& ph) {
     if (last) {
-        if (roots) expand_main<LAST, true, DUPS, false>(P, smem, L, cd, mb, ph);
-        else expand_main<LAST, false, DUPS, false>(P, smem, L, cd, mb, ph);
+        if (roots) expand_main<LAST, true, DUPS, false, true>(P, smem, L, cd, mb, ph);
+        else expand_main<LAST, false, DUPS, false, true>(P, smem, L, cd, mb, ph);
     } else {
-        if (roots) expand_main<kModeMid, true, DUPS, false>(P, smem, L, cd, mb, ph);
-        else expand_main<kModeMid, false, DUPS, false>(P, smem, L, cd, mb, ph);
+        if (roots) expand_main<kModeMid, true, DUPS, false, true>(P, smem, L, cd, mb, ph);
+        else expand_main<kModeMid, false, DUPS, false, true>(P, smem, L, cd, mb, ph);
     }
 }
 
@@ -1358,11 +1358,11 @@ template <int LAST, bool DUPS>
 __device__ __forceinline__ void persist_heavy(const ExpandParams& P, unsigned char* smem, const uint8_t* cd,
                                               bool roots, bool last, const LevelLists& L, uint64_t* mb, uint32_t& ph) {
     if (last) {
-        if (roots) expand_heavy<LAST, true, DUPS, false>(P, smem, L, cd, mb, ph);
-        else expand_heavy<LAST, false, DUPS, false>(P, smem, L, cd, mb, ph);
+        if (roots) expand_heavy<LAST, true, DUPS, false, true>(P, smem, L, cd, mb, ph);
+        else expand_heavy<LAST, false, DUPS, false, true>(P, smem, L, cd, mb, ph);
     } else {
-        if (roots) expand_heavy<kModeMid, true, DUPS, false>(P, smem, L, cd, mb, ph);
-        else expand_heavy<kModeMid, false, DUPS, false>(P, smem, L, cd, mb, ph);
+        if (roots) expand_heavy<kModeMid, true, DUPS, false, true>(P, smem, L, cd, mb, ph);
+        else expand_heavy<kModeMid, false, DUPS, false, true>(P, smem, L, cd, mb, ph);
     }
 }
 
@@ -1430,13 +1430,19 @@ __global__ void __launch_bounds__(kWarps * 32, 5) k_persist(const __grid_constan
     }
 }
 
-template <int MODE, bool ROOTS, bool DUPS, bool SHARE = false>
+template <int MODE, bool ROOTS, bool DUPS, bool SHARE = false, bool COMMON = false>
 void* kernel_ptr(bool heavy) {
-    return heavy ? (void*)&k_expand_heavy<MODE, ROOTS, DUPS, SHARE> : (void*)&k_expand<MODE, ROOTS, DUPS, SHARE>;
+    return heavy ? (void*)&k_expand_heavy<MODE, ROOTS, DUPS, SHARE, COMMON>
+                 : (void*)&k_expand<MODE, ROOTS, DUPS, SHARE, COMMON>;
 }
 
-// `share`: the level has a buffer for shared intersections.
-void* pick(int mode, bool roots, bool dups, bool share, bool heavy) {
+// `share`: the level has a buffer for shared intersections; `common`: bitmaps are
+// common (DeviceGraph::bitmaps_common).  A counting level on a graph without them
+// has a kernel of its own: the code that asks them cost it 2 to 4 % (5-vertex path
+// counted candidate by candidate, 2^16 vertices with lists of 8: 0.514 and 0.501 ms).
+void* pick(int mode, bool roots, bool dups, bool share, bool common, bool heavy) {
+    if (common && mode == kModeLastCount && !roots && !dups && !share)
+        return kernel_ptr<kModeLastCount, false, false, false, true>(heavy);
 #define FM_PICK(M)                                                                                     \
     if (mode == M) {                                                                                   \
         if (share) return kernel_ptr<M, false, false, true>(heavy);                                    \
@@ -1583,10 +1589,10 @@ int blocks_per_sm(const void* f, int block, size_t smem) {
     return n;
 }
 
-int expand_blocks_per_sm(int mode, bool roots, bool dups, bool share, size_t smem, int block) {
-    void* f = pick(mode, roots, dups, share, false);
+int expand_blocks_per_sm(int mode, bool roots, bool dups, bool share, bool common, size_t smem, int block) {
+    void* f = pick(mode, roots, dups, share, common, false);
     allow_dynamic_smem(f);
-    allow_dynamic_smem(pick(mode, roots, dups, share, true));
+    allow_dynamic_smem(pick(mode, roots, dups, share, common, true));
     return std::max(1, blocks_per_sm(f, block, smem));
 }
 
@@ -1594,8 +1600,8 @@ uint32_t expand_launches(uint32_t max_list) { return 32ull * max_list <= kHeavyL
 
 cudaError_t launch_expand(const ExpandParams& p, int mode, bool roots, bool dups, bool share, bool overlap, int grid,
                           int heavy_grid, int block, size_t smem, cudaStream_t s) {
-    void* f = pick(mode, roots, dups, share, false);
-    void* fh = pick(mode, roots, dups, share, true);
+    void* f = pick(mode, roots, dups, share, p.bm_common != 0, false);
+    void* fh = pick(mode, roots, dups, share, p.bm_common != 0, true);
     if (!f || !fh) return cudaErrorInvalidValue;
     ExpandParams q = p;
     // both passes tune themselves on the device (make_tune) from the level size

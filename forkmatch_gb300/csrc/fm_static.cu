@@ -92,7 +92,7 @@ struct StaticRun {
         uint32_t ndef_in = 0;
         uint64_t fresh = 0;
         const size_t smem = expand_smem_bytes(d, nreq[d], block / 32, 0, mode != kModeLastCount, dups, false, false);
-        const int per_sm = expand_blocks_per_sm(mode, roots, dups, false, smem, block);
+        const int per_sm = expand_blocks_per_sm(mode, roots, dups, false, base.bm_common != 0, smem, block);
         // A launch defers at most 8 chunks per warp (the largest claim batch),
         // so a grid of at most kStaticDefCap / (8 * warps per block) blocks
         // keeps one launch's deferred chunks within a list whatever the SM
@@ -265,7 +265,7 @@ extern "C" fm_status fm_match_static(const fm_graph* graph, const fm_query* quer
     b.nbr = g.nbr;
     b.bm = g.bitmaps;
     b.bm_words = g.bm_words;
-    b.bm_near = g.bitmaps_near();
+    b.bm_common = g.bitmaps_common();
     b.efilter = g.efilter;
     b.efilter_off = g.efilter_off;
     b.V = g.V;

@@ -190,21 +190,21 @@ def test_pre_count_equals_the_launched_last_depth(ctx):
     g.close()
 
 
-@pytest.mark.parametrize("stride", [1, 100])
-def test_pre_count_asks_bitmaps_or_filter(ctx, monkeypatch, stride):
-    """The same lists with bitmaps that fit half of the L2 (asked) and with ones that do not (the filter is asked):
-    ids spread over 100 times as many vertices make every bitmap 100 times as long."""
-    monkeypatch.setenv("FM_BITMAP_MIN_LEN", "4")
+@pytest.mark.parametrize("edges,common", [(11000, False), (14000, True), (30000, True)])
+def test_pre_count_asks_bitmaps_or_filter(ctx, monkeypatch, edges, common):
+    """Lists of which less than an eighth have a bitmap (the filter is asked) and of which more do (they are asked)."""
+    monkeypatch.setenv("FM_BITMAP_MIN_LEN", "8")
     n = 2500                                             # fewer than 4096 lists: candidate by candidate
     rng = np.random.default_rng(5)
-    e = np.unique(np.sort(rng.integers(0, n, (30000, 2)), axis=1), axis=0)
+    e = np.unique(np.sort(rng.integers(0, n, (edges, 2)), axis=1), axis=0)
     e = e[e[:, 0] != e[:, 1]]
     lab = rng.integers(1, 3, len(e))
     src, dst, lab = [np.concatenate(x).astype(np.uint32) for x in
-                     ((e[:, 0] * stride, e[:, 1] * stride), (e[:, 1] * stride, e[:, 0] * stride), (lab, lab))]
-    g = fm.Graph.from_edges(ctx, n * stride, 3, src, dst, lab)
-    assert g.info().bitmaps > 4000 and (g.info().bitmap_bytes <= 64 << 20) == (stride == 1)
-    og = O.Graph.from_edges(n * stride, 3, src, dst, lab)
+                     ((e[:, 0], e[:, 1]), (e[:, 1], e[:, 0]), (lab, lab))]
+    g = fm.Graph.from_edges(ctx, n, 3, src, dst, lab)
+    i = g.info()
+    assert i.bitmaps > 100 and (8 * i.bitmaps >= i.segments) == common
+    og = O.Graph.from_edges(n, 3, src, dst, lab)
     for q in (S.query_path(3, [1, 2]), S.query_path(4, [1, 2, 1]), S.query_star(4, [1, 1, 2]),
               S.Query(4, [(0, 1, 1), (1, 2, 1), (0, 2, 2), (2, 3, 1)])):
         want = O.match(og, O.plan(q.to_g_text(), enumerate_aut=0), count_rule=True)[0]
