@@ -134,20 +134,26 @@ __device__ __forceinline__ uint32_t len16_of(uint32_t n) { return n > 3 ? (n + 3
 
 // Segment lengths: the 16-byte units each tile of segments stores out of line,
 // the longest list, the long lists, the list lengths by floor(log2), the pairs
-// in a list summed per label, and the first segment of every label.  The totals are gathered per block and added
-// once (one atomic per segment on shared counters was the slowest kernel of
-// the build: 250 us for 7.1 M segments, now 30).
+// in a list summed per label, and the first segment of every label.  The totals
+// are gathered per block, the pairs per warp, and added once (one atomic per
+// segment on shared counters was the slowest kernel of the build: 250 us for
+// 7.1 M segments, now 30).
 __global__ void k_seg_lens(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ seg_start,
                            uint32_t vbits, uint32_t* __restrict__ tile16, BuildStats* __restrict__ st) {
     __shared__ uint32_t hist_s[32], red_s[kBlock / 32], max_s;
-    __shared__ unsigned long long pairs_s[FM_MAX_LABEL + 1];
     if (threadIdx.x < 32) hist_s[threadIdx.x] = 0;
-    for (uint32_t i = threadIdx.x; i <= FM_MAX_LABEL; i += blockDim.x) pairs_s[i] = 0;
     if (threadIdx.x == 0) max_s = 0;
     __syncthreads();
     const uint32_t nseg = st->nseg;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t one = 0, two = 0;
+    uint32_t one = 0, two = 0, pairs_of = 0;      // label of the pairs summed so far
+    unsigned long long pairs = 0;                 // (lane's part)
+    auto add_pairs = [&]() {
+#pragma unroll
+        for (int o = 16; o; o >>= 1) pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
+        if (lane == 0 && pairs) atomicAdd(&st->pairs[pairs_of], pairs);
+        pairs = 0;
+    };
     for (uint64_t t = blockIdx.x; t * kTileSegs < nseg; t += gridDim.x) {
         uint32_t sum = 0, mx = 0;
 #pragma unroll
@@ -169,15 +175,14 @@ __global__ void k_seg_lens(const uint64_t* __restrict__ keys, const uint32_t* __
             // segments come label by label: nearly always one label a warp
             const unsigned many = __ballot_sync(0xffffffffu, n > 1);
             if (!many) continue;
-            unsigned long long pr = n > 1 ? (unsigned long long)n * (n - 1) : 0ull;
             const uint32_t l0 = __shfl_sync(0xffffffffu, l, __ffs(many) - 1);
-            if (__all_sync(0xffffffffu, n <= 1 || l == l0)) {
-#pragma unroll
-                for (int o = 16; o; o >>= 1) pr += __shfl_xor_sync(0xffffffffu, pr, o);
-                if (lane == 0) atomicAdd(&pairs_s[l0], pr);
-            } else if (pr) {
-                atomicAdd(&pairs_s[l], pr);
+            if (l0 != pairs_of) {
+                add_pairs();
+                pairs_of = l0;
             }
+            const unsigned long long pr = n > 1 ? (unsigned long long)n * (n - 1) : 0ull;
+            if (l == l0) pairs += pr;
+            else if (pr) atomicAdd(&st->pairs[l], pr);
         }
         sum = __reduce_add_sync(0xffffffffu, sum);
         mx = __reduce_max_sync(0xffffffffu, mx);
@@ -198,8 +203,7 @@ __global__ void k_seg_lens(const uint64_t* __restrict__ keys, const uint32_t* __
     __syncthreads();
     if (threadIdx.x < 32 && hist_s[threadIdx.x]) atomicAdd(&st->hist[threadIdx.x], hist_s[threadIdx.x]);
     if (threadIdx.x == 0 && max_s) atomicMax(&st->max_len, max_s);
-    for (uint32_t i = threadIdx.x; i <= FM_MAX_LABEL; i += blockDim.x)
-        if (pairs_s[i]) atomicAdd(&st->pairs[i], pairs_s[i]);
+    add_pairs();
 }
 
 // Out-of-line offset of every segment, in 16-byte units.  A thread takes four
