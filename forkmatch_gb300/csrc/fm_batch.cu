@@ -109,9 +109,11 @@ constexpr int kBWarps = 8;
 // every candidate and have no filter queue.  With 96 rows there too, eight counts
 // of 5-vertex paths on a random graph of 2^20 vertices (7.7e7 rows at one level)
 // took 11.1 ms instead of 9.8.
-constexpr uint32_t kBStage = 96, kBStageOne = 256;
+constexpr uint32_t kBStage = 128, kBStageOne = 256;
 __host__ __device__ constexpr uint32_t bstage_rows(uint32_t kmax) { return kmax == 1 ? kBStageOne : kBStage; }
 constexpr uint32_t kBSlots = 2;            // candidate slots per lane per round
+// The stage is flushed above this many rows: whatever follows, a round fits.
+__host__ __device__ constexpr uint32_t bflush_at(uint32_t kmax) { return bstage_rows(kmax) - 32 * kBSlots; }
 constexpr uint32_t kBPend = 32 * kBSlots + 32;   // candidates that wait for their exact test
 constexpr uint32_t kHeavyMaxPieces = 65536;
 constexpr uint32_t kBHeavyLeast = 512;     // no chunk above this many candidates: no heavy pass
@@ -493,7 +495,7 @@ __device__ __forceinline__ void bemit(const BatchParams& P, const BMem& m, const
     }
     nst += __popc(b);
     __syncwarp();
-    if (nst > bstage_rows(P.kmax) - 32) {
+    if (nst > bflush_at(P.kmax)) {
         bflush<ROOTS>(P, m, nst, lane, d, chunk);
         nst = 0;
         __syncwarp();
@@ -540,6 +542,44 @@ __device__ __forceinline__ void bcount_slots(const BatchParams& P, const BMem& m
     __syncwarp();
 }
 
+// Slots [begin, end) of a chunk whose parents' queries all go on past this depth
+// over one back edge: what is not in its row is staged, with one look at the stage
+// a round.
+template <bool ROOTS>
+__device__ __forceinline__ void bstage_slots(const BatchParams& P, const BMem& m, SlotWalk& walk, uint32_t chunk,
+                                             uint32_t begin, uint32_t end, uint32_t lane, uint32_t d, uint32_t& nst) {
+    for (uint32_t base = begin; base < end; base += 32 * kBSlots) {
+        uint32_t j[kBSlots], t[kBSlots], x[kBSlots];
+        bool ok[kBSlots];
+#pragma unroll
+        for (uint32_t u = 0; u < kBSlots; u++) {
+            walk.window(m.start_s, base + 32 * u, lane, j[u], t[u]);
+            x[u] = 0;
+            ok[u] = base + 32 * u + lane < end;
+            if (ok[u]) x[u] = seg_at(m.segs_s[j[u]], t[u], P.nbr);   // its first record is its only one
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < kBSlots; u++) {
+            for (uint32_t c = 0; c < d && ok[u]; c++) ok[u] = m.rows_s[c * 32 + j[u]] != x[u];
+            const unsigned b = __ballot_sync(kFull, ok[u]);
+            if (ok[u]) {
+                const uint32_t q = nst + __popc(b & ((1u << lane) - 1u));
+                m.stp[q] = ROOTS ? m.rows_s[j[u]] : chunk * 32 + j[u];
+                m.stx[q] = x[u];
+                m.stq[q] = m.qid_s[j[u]];
+            }
+            nst += __popc(b);
+        }
+        __syncwarp();
+        if (nst > bflush_at(P.kmax)) {
+            bflush<ROOTS>(P, m, nst, lane, d, chunk);
+            nst = 0;
+            __syncwarp();
+        }
+    }
+    __syncwarp();
+}
+
 // Evaluate slots [begin, end) of the loaded chunk, kBSlots per lane per round
 // with every driver load of the round issued before any check; the filter
 // rejects, and what it lets pass is tested exactly 32 at a time (as in the
@@ -555,6 +595,10 @@ __device__ __forceinline__ void bprocess(const BatchParams& P, const BMem& m, co
     const uint32_t q0 = m.qid_s[has ? __ffs(has) - 1 : 0];
     if (kk == 1 && __all_sync(kFull, n == 0 || (m.fin_s[lane] == 2u && m.qid_s[lane] == q0))) {
         bcount_slots(P, m, S, walk, q0, begin, end, lane, d);
+        return;
+    }
+    if (kk == 1 && __all_sync(kFull, n == 0 || m.fin_s[lane] == 0u)) {
+        bstage_slots<ROOTS>(P, m, walk, chunk, begin, end, lane, d, nst);
         return;
     }
     uint32_t pend = 0;
