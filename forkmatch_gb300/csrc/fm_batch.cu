@@ -1233,8 +1233,9 @@ uint32_t sum_kind_of(const BatchPlan& bp, const DeviceGraph& g) {
     const uint32_t a = bp.req_anc[bp.req_begin[q - 2]], l = bp.req_label[bp.req_begin[q - 2]];
     const uint32_t c = bp.req_anc[bp.req_begin[q - 1]], ll = bp.req_label[bp.req_begin[q - 1]];
     const bool chain = c == q - 2;
-    if (g.head_off[l + 1] - g.head_off[l] < 4096 || (chain && (q != 4 || !g.symmetric))) return kSumNone;
-    return chain ? kSumChain : a != c ? kSumFork : l != ll ? kSumForkOne : kSumForkSame;
+    const uint32_t kind = chain ? kSumChain : a != c ? kSumFork : l != ll ? kSumForkOne : kSumForkSame;
+    if (chain && (q != 4 || !g.symmetric)) return kSumNone;
+    return sums_lists_enough(g, l, kind == kSumChain || kind == kSumForkOne) ? kind : (uint32_t)kSumNone;
 }
 
 // Estimated candidates of a query's counting level: rows reached through an

@@ -849,9 +849,6 @@ struct SumsPlan {
     uint64_t cap = 0;                // rows per level buffer beside them
 };
 
-// Lists of the counting level's label below which the rule is off.
-constexpr uint64_t kSumsMinLists = 4096;
-
 // Rows of every level buffer, depths 2 .. stored - 1, in `bytes` of level memory.
 uint64_t level_rows(uint64_t bytes, uint32_t stored, uint64_t bank) {
     uint64_t sum_cols = 0;
@@ -870,12 +867,7 @@ bool rows_enough(const DeviceGraph& g, uint32_t stored, uint64_t cap) {
 // each, and a chain's lists can be read from either end.  Depth 1 is left to
 // enumeration: its parents are the label's lists, each of which the vertex sums
 // would walk once as well.  The sums take 8 bytes a vertex of the level memory,
-// at most an eighth of it, and a launch of their own: below 4096 lists that
-// launch (3 us) is more than the level saves (300 vertices: 86 us a match with,
-// 83 without).  Forks that need no vertex sums are held to the same minimum, for
-// the plan of the order that they cost: without it sparse graphs of 3000 vertices
-// lose 3 us of 75, dense ones would gain (5-vertex path, 200 neighbours a vertex:
-// 1.6 ms by sums, 4.0 candidate by candidate).
+// at most an eighth of it.
 bool sums_plan(const fm_context* ctx, const DeviceGraph& g, uint32_t q, const uint32_t* nreq,
                const uint32_t (*climb)[kMaxQ], const uint32_t (*rlab)[kMaxQ], SumsPlan& out) {
     if (q < 4 || nreq[q - 2] != 1 || nreq[q - 1] != 1) return false;
@@ -887,7 +879,7 @@ bool sums_plan(const fm_context* ctx, const DeviceGraph& g, uint32_t q, const ui
     out.vertex = chain || (same_vertex && out.label != out.last);
     const uint64_t lists = g.head_off[out.label + 1] - g.head_off[out.label];
     out.lists = (uint32_t)lists;
-    if ((chain && !g.symmetric) || lists < kSumsMinLists) return false;
+    if ((chain && !g.symmetric) || !sums_lists_enough(g, out.label, out.vertex)) return false;
     const uint64_t vbytes = out.vertex ? (uint64_t)g.V * sizeof(uint2) : 0;
     if (8 * vbytes > ctx->soln_bytes) return false;
     out.voff = (ctx->soln_bytes - vbytes) & ~255ull;
@@ -957,7 +949,7 @@ fm_status match_impl(fm_context* ctx, const fm_graph* graph, const fm_query* que
         nreq[q - 2] == 1 && climb[q - 1][0] == 1 && g.symmetric) {
         uint32_t fork[kMaxQ], fnreq[kMaxQ], fclimb[kMaxQ][kMaxQ], flab[kMaxQ][kMaxQ];
         SumsPlan sp;
-        if (choose_fork_order(pl, g, order, kSumsMinLists, fork) &&
+        if (choose_fork_order(pl, g, order, fork) &&
             order_requirements(pl, fork, fnreq, fclimb, flab) && sums_plan(ctx, g, q, fnreq, fclimb, flab, sp)) {
             std::memcpy(order, fork, sizeof(order));
             std::memcpy(nreq, fnreq, sizeof(nreq));

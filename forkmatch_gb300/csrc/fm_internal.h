@@ -117,12 +117,14 @@ bool order_requirements(const Plan& P, const uint32_t* order, uint32_t nreq[kMax
                         uint32_t climb[kMaxQ][kMaxQ], uint32_t label[kMaxQ][kMaxQ]);
 // Cost-based matching order for a data graph (fm_parse.cpp).
 void choose_order(const Plan& P, const DeviceGraph& g, uint32_t order[kMaxQ]);
+// Whether counting by sums pays over the lists of `label`, the label of the
+// counting level; `vertex`: it reads vertex sums.
+bool sums_lists_enough(const DeviceGraph& g, uint32_t label, bool vertex);
 // An order that ends with two leaves on earlier vertices (a fork), the first of
-// them over a label of at least `min_lists` lists, and whose other vertices cost
+// them over a label for which sums_lists_enough holds, and whose other vertices cost
 // at most a quarter more, by the same model, than those of `order` (each list
 // intersection less saves more than that).  Returns false if there is none.
-bool choose_fork_order(const Plan& P, const DeviceGraph& g, const uint32_t* order, uint64_t min_lists,
-                       uint32_t fork[kMaxQ]);
+bool choose_fork_order(const Plan& P, const DeviceGraph& g, const uint32_t* order, uint32_t fork[kMaxQ]);
 
 // Per-launch control block in device memory.
 struct LaunchCtl {

@@ -551,8 +551,16 @@ void choose_order(const Plan& P, const DeviceGraph& g, uint32_t order[kMaxQ]) {
     OrderModel(P, g).best(none, q, order);
 }
 
-bool choose_fork_order(const Plan& P, const DeviceGraph& g, const uint32_t* order, uint64_t min_lists,
-                       uint32_t fork[kMaxQ]) {
+// The vertex sums take a launch of their own, 3 us, which below 4096 lists is more
+// than the level saves (300 vertices: 86 us a match with, 83 without).  A fork
+// without them saves at every size: 5-vertex path on random graphs of 300 and 3000
+// vertices with 2 neighbours a vertex 48 -> 45 and 58 -> 53 us, with 16 135 -> 103
+// and 301 -> 185; 4-vertex star with one label, 4 neighbours, 44 -> 33 us.
+bool sums_lists_enough(const DeviceGraph& g, uint32_t label, bool vertex) {
+    return label < g.L && (!vertex || g.head_off[label + 1] - g.head_off[label] >= 4096);
+}
+
+bool choose_fork_order(const Plan& P, const DeviceGraph& g, const uint32_t* order, uint32_t fork[kMaxQ]) {
     const uint32_t q = P.q;
     if (q < 4 || g.V == 0) return false;
     const OrderModel M(P, g);
@@ -563,14 +571,15 @@ bool choose_fork_order(const Plan& P, const DeviceGraph& g, const uint32_t* orde
     uint32_t leaf[kMaxQ], leaves = 0;
     bool any = false;
     auto line = [&](uint32_t v) { return M.row.begin[v]; };
-    auto enough = [&](uint32_t v) {
-        const uint32_t l = P.rows[line(v)].l;
-        return l < g.L && g.head_off[l + 1] - g.head_off[l] >= min_lists;
+    // leaf a at the counting level, leaf b last
+    auto enough = [&](uint32_t a, uint32_t b) {
+        const LocalELine &x = P.rows[line(a)], &y = P.rows[line(b)];
+        return sums_lists_enough(g, x.l, x.b == y.b && x.l != y.l);
     };
     for (uint32_t v = 0; v < q; v++) {
         if (M.deg(v) != 1) continue;
         leaf[leaves++] = v;
-        any |= enough(v);
+        any |= sums_lists_enough(g, P.rows[line(v)].l, false);
     }
     if (leaves < 2 || !any) return false;
     std::stable_sort(leaf, leaf + leaves,
@@ -603,8 +612,8 @@ bool choose_fork_order(const Plan& P, const DeviceGraph& g, const uint32_t* orde
         for (uint32_t j = i + 1; j < first; j++) {
             uint32_t a = std::min(leaf[i], leaf[j]), b = std::max(leaf[i], leaf[j]);
             if (P.rows[line(a)].b == b) continue;
-            if (!enough(a)) std::swap(a, b);
-            if (!enough(a)) continue;
+            if (!enough(a, b)) std::swap(a, b);
+            if (!enough(a, b)) continue;
             bool left[kMaxQ] = {};
             left[a] = left[b] = true;
             uint32_t cand[kMaxQ];
