@@ -279,8 +279,8 @@ __device__ __forceinline__ bool bstage_lists(const BatchParams& P, const BMem& m
 // members are to be taken off goes to `drv_rec` (index `drv`, length `n`).
 __device__ __forceinline__ unsigned long long bsum_parent(const BatchParams& P, const BMem& m, const BSlices& S,
                                                           const BatchPlan& pl, const uint4 a, uint32_t anc,
-                                                          uint32_t lab, uint32_t lane, uint32_t d, uint4& drv_rec, uint32_t& drv,
-                                                          uint32_t& n) {
+                                                          uint32_t lab, uint32_t lane, uint32_t d, uint4& drv_rec,
+                                                          uint32_t& drv, uint32_t& n) {
     const uint32_t rl = pl.req_begin[d + 1], last_anc = pl.req_anc[rl], ll = pl.req_label[rl];
     const uint4* last = P.seg + (uint64_t)ll * P.V;
     const uint32_t va = m.rows_s[anc * 32 + lane];
@@ -639,10 +639,8 @@ __device__ __forceinline__ void bprocess(const BatchParams& P, const BMem& m, co
         }
         // One loop, and one copy of bemit, for the slots that go straight on and for
         // the queue.  With a copy for each slot and the queue the code missed the
-        // instruction cache (8.4 of a warp's 20 cycles between two instructions):
-        // eight counts of 5-vertex paths took 8.0 ms on a random graph of 2^16
-        // vertices with 4 labels (5.6 now) and 52.1 ms on a 2^20-vertex R-MAT graph
-        // (37.7).
+        // instruction cache (8.4 of a warp's 20 cycles between two instructions) and
+        // counts of 5-vertex paths took 1.4 times as long.
         uint32_t slot = 0;
 #pragma unroll 1
         while (direct ? slot < kBSlots : pend >= 32 || (last && pend)) {
@@ -860,8 +858,10 @@ __device__ __forceinline__ void bexpand_heavy(const BatchParams& P, unsigned cha
 }
 
 // 4 blocks per SM (64 registers): a batch's passes are mostly small and the
-// per-lane plans spill at 40 registers.  48 mixed queries 13.7 ms at 6 blocks,
-// 13.4 at 5, 12.9 at 4, 13.7 at 3; 32 served walk counts 1.49, 1.40, 1.29, 1.27.
+// per-lane plans spill at fewer registers.  48 mixed queries 12.4 ms, 13.1 with 5
+// blocks; 4-vertex counts on a 2^20-vertex random graph with 40 labels 2.13 and
+// 2.28.  Batches of large levels alone would take 5: cycles, triangles and cliques
+// on a 2^18-vertex random graph with 2 labels 219 and 205 ms.
 constexpr int kBBlocks = 4;
 
 template <bool ROOTS>

@@ -848,8 +848,8 @@ __device__ __forceinline__ void expand_main(const ExpandParams& P, unsigned char
                 pub = __shfl_sync(kFull, pub, 0);
                 if (pub) continue;
             }
-            process_slots<MODE, ROOTS, DUPS, SHARE, COMMON>(P, m, chunk, excl, n, 0, total, lane, d, k, L, col_depth_s, nst,
-                                                    n_count, pre);
+            process_slots<MODE, ROOTS, DUPS, SHARE, COMMON>(P, m, chunk, excl, n, 0, total, lane, d, k, L,
+                                                            col_depth_s, nst, n_count, pre);
         }
     }
     if (MODE != kModeLastCount && nst) flush_stage<MODE, ROOTS>(P, m, nst, lane, d, col_depth_s, last_chunk);
@@ -917,8 +917,8 @@ __device__ __forceinline__ void expand_heavy(const ExpandParams& P, unsigned cha
                                        L, share_on, share);
         last_chunk = e.chunk;
         if (!stage_ok) break;
-        process_slots<MODE, ROOTS, DUPS, SHARE, COMMON>(P, m, e.chunk, excl, n, begin, end, lane, d, k, L, col_depth_s, nst,
-                                                n_count, pre);
+        process_slots<MODE, ROOTS, DUPS, SHARE, COMMON>(P, m, e.chunk, excl, n, begin, end, lane, d, k, L,
+                                                        col_depth_s, nst, n_count, pre);
     }
     if (MODE != kModeLastCount && nst) flush_stage<MODE, ROOTS>(P, m, nst, lane, d, col_depth_s, last_chunk);
     if (MODE == kModeLastCount && lane == 0 && n_count > n_flushed) atomicAdd(&P.tot->count, n_count - n_flushed);
