@@ -133,6 +133,16 @@ def test_fork_orders_come_with_sums(ctx, edges, labels):
     g.close()
 
 
+def test_no_fork_order_is_planned_for_few_candidates(ctx):
+    """A 24-vertex path on a graph with half a neighbour a label: nothing to spare, no plan."""
+    g = fm.Graph.from_edges(ctx, 3000, 5, *_uneven(3000, 3000))
+    q = fm.Query.from_text(S.query_path(24, [2 + i % 3 for i in range(23)]).to_g_text())
+    t = fm.match(ctx, g, q, mode=fm.MODE_TABLE, allow_truncation=True)
+    c = fm.match(ctx, g, q, mode=fm.MODE_COUNT)
+    assert c.count == t.count and not c.routes & fm.ROUTE_FORK
+    g.close()
+
+
 def _long_lists(ctx):
     """5000 vertices, 100000 edges of labels 2 and 3 and 40 of label 1."""
     rng = np.random.default_rng(4)
